@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <algorithm>
 #include <cstring>
+#include <future>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -73,6 +74,29 @@ int upload_v(fv_solver* s, const std::vector<T>& v, const T** out) {
     if (!v.empty()) CK(cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
     *out = d;
     return FV_OK;
+}
+// the fused kernel's arrays over two-ring tiles (build_fused)
+template <class S>
+int upload_fused(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2,
+                 bool exact, double K) {
+    FusedArrays<S> a;
+    build_fused<S>(m, fa, ta, t2, exact, K, a);
+    FusedParams& F = s->FPm;
+    F.nf = a.nf;
+    const int32_t* info; const uint32_t* hd; const S *rec, *rec2, *sl, *eg;
+    int rc;
+    if ((rc = upload_v(s, a.info, &info)) || (rc = upload_v(s, a.hd, &hd)) || (rc = upload_v(s, a.rec, &rec)) || (rc = upload_v(s, a.rec2, &rec2)) || (rc = upload_v(s, a.sl, &sl)) ||
+        (rc = upload_v(s, a.eg, &eg)) || (rc = upload_v(s, a.ria, &F.ria)))
+        return rc;
+    F.info = reinterpret_cast<const int4*>(info);
+    F.hd = reinterpret_cast<const uint4*>(hd);
+    F.rec = rec; F.rec2 = rec2; F.sl = sl; F.eg = eg;
+    return FV_OK;
+}
+// lanes per cell of the fused kernel's gradient and update phases
+int fused_lanes(const fv_solver* s) {
+    (void)s;
+    return 1;
 }
 }  // namespace
 
@@ -365,6 +389,16 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     const int tile_cells = (opt && opt->tile_cells) ? opt->tile_cells : 128;
     if (tile_cells != 64 && tile_cells != 128 && tile_cells != 256)
         return fail(FV_ERR_ARG, "tile_cells must be 64, 128 or 256");
+    // one fused kernel per stage for the second-order Roe kinds; the fast
+    // modes' split layout runs over the two-ring tiles as well, which are
+    // built beside the one-ring tiles
+    const int sk = opt ? opt->stage_kernels : FV_STAGE_AUTO;
+    const bool can_fuse = ph->V == 4 && ph->order2 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST) &&
+                          !ph->diffusive && !ph->smooth_residuals;
+    const bool two_ring = can_fuse && (sk != FV_STAGE_SPLIT || precision != FV_PREC_FP64_EXACT);
+    Tile2Arrays t2;
+    std::future<void> t2_built;
+    if (two_ring) t2_built = std::async(std::launch::async, [&] { build_tiles2(m, fa, tile_cells, t2); });
     build_tiles(m, fa, tile_cells, ta);
     if (ta.max_halo + tile_cells > 65535 || ta.max_edges > kFaceEdgeMask)
         return fail(FV_ERR_MESH, "tile halo too large for 16-bit local indices");
@@ -420,49 +454,30 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     s->new2ref = const_cast<int32_t*>(n2r);
     CK(tile::prepare(precision, TP));
     {
-        // one fused kernel per stage for the second-order Roe kinds
-        const int sk = opt ? opt->stage_kernels : FV_STAGE_AUTO;
         if (sk < FV_STAGE_AUTO || sk > FV_STAGE_HYBRID) return fail(FV_ERR_ARG, "unknown stage_kernels");
-        const bool can_fuse = ph->V == 4 && ph->order2 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST) &&
-                              !ph->diffusive && !ph->smooth_residuals;
         if ((sk == FV_STAGE_FUSED || sk == FV_STAGE_HYBRID) && !can_fuse)
             return fail(FV_ERR_UNSUPPORTED, "the fused stage kernel needs a second-order Roe kind without "
                                             "diffusive terms or residual smoothing");
-        if (can_fuse && sk != FV_STAGE_SPLIT) {
-            Tile2Arrays t2;
-            build_tiles2(m, fa, tile_cells, t2);
+        if (two_ring) {
+            t2_built.get();
             FusedParams& F = s->FPm;
             F.T = tile_cells;
-            F.max_slots = t2.max_slots; F.max_grad = t2.max_grad;
-            F.max_edges = t2.max_edges; F.max_flux = t2.max_flux;
-            const bool fits = t2.max_slots <= 65535 && t2.max_edges <= kFaceEdgeMask &&
-                              tile::smem_fused(precision, F) <= (size_t)227 * 1024;
+            F.max_slots = t2.max_slots; F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;
+            const bool fits = t2.max_slots < 65535 && t2.max_edges <= kFaceEdgeMask &&
+                              2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= (size_t)227 * 1024;
             if (!fits && (sk == FV_STAGE_FUSED || sk == FV_STAGE_HYBRID))
                 return fail(FV_ERR_MESH, "two-ring tiles too large for the fused stage kernel at this tile size");
             if (fits) {
-                const int32_t* i2; const int32_t* h2; const uint32_t* e2; const uint16_t* f2;
-                if ((rc = upload_v(s.get(), t2.info, &i2))) return rc;
-                F.info = reinterpret_cast<const int4*>(i2);
+                if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, ph->K);
+                else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, ph->K);
+                if (rc) return rc;
+                const int32_t* h2;
                 if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;
                 F.halo = h2;
-                if ((rc = upload_v(s.get(), t2.edge_ij, &e2))) return rc;
-                F.edge_ij = e2;
-                if ((rc = upload_v(s.get(), t2.face, &f2))) return rc;
-                F.face = reinterpret_cast<const uint2*>(f2);
-                if ((rc = upload_s(s.get(), t2.enx, &F.enx))) return rc;
-                if ((rc = upload_s(s.get(), t2.eny, &F.eny))) return rc;
-                if ((rc = upload_s(s.get(), t2.ele, &F.ele))) return rc;
-                if ((rc = upload_s(s.get(), t2.exf, &F.exf))) return rc;
-                if ((rc = upload_s(s.get(), t2.eyf, &F.eyf))) return rc;
-                if ((rc = upload_s(s.get(), t2.eg, &F.eg))) return rc;
-                std::vector<double> cca(4 * (size_t)m.n_total, 0.0);
-                for (size_t n = 0; n < (size_t)m.n_total; ++n) {
-                    cca[4 * n] = ta.ccx[n]; cca[4 * n + 1] = ta.ccy[n]; cca[4 * n + 2] = fa.area[n];
-                }
-                if ((rc = upload_s(s.get(), cca, &F.cca))) return rc;
-                F.threads = tile_cells;
+                F.area = TP.area;
+                s->two_ring = true;
                 CK(tile::prepare_fused(precision, F));
-                s->fused = true;
+                s->fused = sk != FV_STAGE_SPLIT;
                 CK(s->alloc(&s->work, kWorkSlots));
                 CK(cudaMemset(s->work, 0, kWorkSlots * sizeof(int)));
                 s->work_grid = tile::work_grid_fused(precision, F, ta.n_tiles);
@@ -473,6 +488,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
                 if (sk == FV_STAGE_HYBRID && sched == FV_SCHED_WORKLIST)
                     return fail(FV_ERR_ARG, "the work-list schedule needs the dt kernel of the fused layout");
                 s->sched = sched;
+                F.lanes = fused_lanes(s.get());
                 // automatic choice: in FP32 the split first stage (its gradient
                 // kernel computes dt) saves more than it costs; in FP64 the
                 // fused first stage and the separate dt kernel are faster
@@ -590,6 +606,7 @@ int fv_solver_create_tuned(const fv_mesh* fm, const fv_physics* ph, int32_t prec
         };
         for (int variant = can_fuse ? 4 : 0; variant >= 0; --variant) {
             if (variant == 3 && t > kTileMax / 2) continue;
+            if (variant == 4 && precision != FV_PREC_FP64_EXACT) continue;  // the launches of variant 1
             clear_graphs(s);
             set_variant(variant);
             // one untimed step (graph capture), then n_steps timed on the device
@@ -767,6 +784,13 @@ namespace fvgpu {
 
 int set_error(int code, const std::string& msg) { return fail(code, msg); }
 
+// lanes and threads of a fused launch: one lane per cell in a decomposition's
+// parts and in the schedules with their own thread counts
+static void fused_schedule(const fv_solver* s, FusedParams& F, bool part) {
+    if (part || s->sched != FV_SCHED_TILE) F.lanes = 1;
+    F.threads = s->sched == FV_SCHED_TILE2 ? 2 * F.T : F.lanes * F.T;
+}
+
 int step_open(fv_solver* s, const std::vector<double>& alpha, int b, bool first, StepCursor& c, EventLog* log,
               bool with_dt) {
     const TileParams& TP = s->TP;
@@ -783,13 +807,20 @@ int step_open(fv_solver* s, const std::vector<double>& alpha, int b, bool first,
     // the fused stage kernel computes its gradients itself: the step's dt
     // comes from the dt kernel, as in first order
     c.grads = (TP.P.order2 || TP.P.diffusive) && !s->fused;
-    // the split first stage's gradient kernel computes dt
-    c.split_first = s->fused && s->split_first;
+    // the fast modes' split kernels over the two-ring tiles
+    c.fast2 = s->two_ring && s->precision != FV_PREC_FP64_EXACT;
+    // their time step: the CFL and constant kinds (the viscous ones keep k_tile_dt)
+    c.dt2 = c.fast2 && TP.P.dt_kind < 3;
+    // FP64_EXACT's hybrid layout: the split first stage's gradient kernel
+    // computes dt.  In the fast modes the dt kernel over the fused kernel's
+    // tiles and a fused first stage cost less (998k cells, FP32: 80 us against
+    // 104 us for the split first stage), so hybrid launches what fused does.
+    c.split_first = s->fused && s->split_first && s->precision == FV_PREC_FP64_EXACT;
     // the work-list schedule: one tile counter per stage, zeroed by the dt kernel
     c.worklist = s->fused && s->sched == FV_SCHED_WORKLIST && alpha.size() <= (size_t)kWorkSlots;
     c.FPl = s->FPm;
     c.FPl.P = TP.P;
-    c.FPl.threads = (s->sched == FV_SCHED_TILE2) ? 2 * c.FPl.T : c.FPl.T;
+    fused_schedule(s, c.FPl, c.part);
     c.in = s->sbase[b];
     c.out = nullptr;
     if (with_dt) n += step_dt(s, c, log);
@@ -799,10 +830,11 @@ int step_open(fv_solver* s, const std::vector<double>& alpha, int b, bool first,
 int step_dt(fv_solver* s, StepCursor& c, EventLog* log) {
     // every kernel after step_begin is a programmatic dependent of the one
     // before it (its constant tile data is staged during that one's tail)
-    if (c.grads || c.split_first) return 0;
+    if ((c.grads && !c.fast2) || c.split_first) return 0;
     TileIO dio = c.io;
     dio.work_reset = c.worklist ? s->work : nullptr;
-    tile::launch_dt(s->precision, s->TP, dio, s->stream, true);
+    if (c.dt2) tile::launch_fused_split(s->precision, c.FPl, dio, s->stream, true, s->n_tiles, 3);
+    else tile::launch_dt(s->precision, s->TP, dio, s->stream, true);
     if (log) log->mark(KK_DT);
     return 1;
 }
@@ -843,6 +875,13 @@ int step_stage(fv_solver* s, const std::vector<double>& alpha, int k, StepCursor
         }
         c.out = out_s;
         if (r->last) c.in = out_s;
+        return n;
+    }
+    if (c.fast2 && c.grads) {
+        tile::launch_fused_split(s->precision, c.FPl, so, st, pdl, s->n_tiles, 1); ++n; mark(KK_GRADLIM);
+        tile::launch_fused_split(s->precision, c.FPl, so, st, pdl, s->n_tiles, 2); ++n; mark(KK_STAGE);
+        c.in = out_s;
+        c.out = out_s;
         return n;
     }
     if (c.grads) { tile::launch_gradlim(s->precision, TP, so, st, k == 0, pdl); ++n; mark(KK_GRADLIM); }
@@ -1454,7 +1493,7 @@ int adj_forward_step(fv_adjoint* a, const double* q, double* q_next, double* dt_
         // gradient + stage kernels, without writing the gradients out)
         FusedParams FPl = s->FPm;
         FPl.P = TP.P;
-        FPl.threads = (s->sched == FV_SCHED_TILE2) ? 2 * FPl.T : FPl.T;
+        fused_schedule(s, FPl, false);
         for (int k = 0; k < a->S; ++k) {
             double* out = (k == a->S - 1) ? q_next : a->tmp[k % 2];
             TileIO so{};

@@ -5,71 +5,165 @@
 // update_cells + update_bounds of explicit.cpp:112-417 for one stage).
 //
 // A tile stages the states of its cells, of their face neighbours (ring 1)
-// and of the ring-1 cells' other neighbours (ring 2), computes the gradients
-// and limiters of its cells and of ring 1 into shared memory, and then the
-// fluxes of its edges from them.  The limited gradients never leave the
-// chip: per stage the kernel reads the stage state, the base state and the
-// constant geometry once and writes the new state, with one staging round
-// and one kernel boundary instead of two.  Ring-1 gradients are computed by
-// every tile that borders the cell (the same arithmetic in each, so the
-// results are identical and, in the exact policy, bit-identical to the
-// reference's).
+// and of the ring-1 cells' other neighbours (ring 2).  The gradient phase
+// gives one thread (or 2 or 4 lanes, each with its share of the variables,
+// which do not mix there) a cell of the tile or of ring 1: it computes the
+// limited gradients in registers and leaves, for every flux edge of the cell,
+// the cell's face state in shared memory.  The flux phase then reads the two
+// face states of an edge from consecutive addresses, and nothing else of the
+// cells.  The limited gradients never leave the registers: per stage the
+// kernel reads the stage state, the base state and the constant geometry once
+// and writes the new state.  Ring-1 gradients are computed by every tile that
+// borders the cell (the same arithmetic in each, so the results are identical
+// and, in the exact policy, bit-identical to the reference's).
 //
-// Shared-memory records are planes of 16-byte units (one float4, or two
-// double2 planes, per 4-vector), so that reads of random slots are free of
-// bank conflicts.  The time step of the step comes from k_tile_dt, launched
-// before the first stage.
+// The geometry of the gradient phase is stored per (gradient cell, face), in
+// the order the threads read it: the fast policies hold the cell's
+// Green-Gauss coefficient (the gradient is the sum of a_f (q_nb - q), since a
+// closed cell's face normals sum to zero) and the vector to the face centre.
+// It goes from global memory straight into registers, with coalesced 16- or
+// 32-byte loads issued before the dependency wait.
+//
+// What bounds it and why this form: the former kernel kept gradients,
+// centroids and edge arrays in shared memory and gathered them again per edge.
+// Its shared-memory wavefronts (about 345 per 32 cells) and its instructions
+// (46 warp instructions per cell in FP32) each took 37-40 us of a 998k-cell
+// stage by themselves.
 #pragma once
 #include "fv_tile.cuh"
 
 namespace fvgpu {
 
+// Shared-memory layout of one fused tile, in bytes from the start.
+//  - state planes [max_slots] of the staged states;
+//  - face-state planes of the flux edges' first and second cells
+//    [2 * max_flux]; the flux leaving the first cell and entering the second
+//    replaces them, and after the per-cell sums the store holds the residual
+//    warp sums;
+//  - the base state of the owned cells (FP64, [T][4]);
+//  - the limited gradients (and, exact, the limiters) of owned cells with a
+//    boundary ghost, for the ghost fill.
+constexpr int kFusedThreads = 512;  // threads per CTA at most
+struct FusedSmem {
+    int q, fs, qb, gx, gy, lm, total, total_grad;
+    int ls, lf, lt;  // plane strides (units)
+};
+template <class M>
+inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int T) {
+    constexpr int NU = (int)(4 * sizeof(typename M::S) / 16);
+    FusedSmem L{};
+    L.ls = max_slots;
+    L.lf = 2 * max_flux;
+    L.lt = T;
+    int o = 0;
+    L.q = o; o += 16 * NU * max_slots;
+    const int f = 32 * NU * max_flux, red = (kFusedThreads / 32) * 4 * (int)sizeof(double);
+    L.fs = o; o += f > red ? f : red;
+    L.qb = o; o += 32 * T;
+    L.gx = o; o += 16 * NU * T;
+    L.gy = o; o += 16 * NU * T;
+    L.lm = o; if (M::exact) o += 16 * NU * T;
+    L.total = o;
+    // the gradient kernel of the split layout and the dt kernel: the states
+    // and, in the flux store's place, {u, v, c} of the gradient slots
+    L.total_grad = L.fs + 16 * NU * max_grad;
+    return L;
+}
+
 struct FusedParams {
     Params P;
     int T;
-    int threads;               // threads per CTA: T, or 2T (at most kTileMax)
-    int max_slots, max_grad, max_edges, max_flux;  // max_edges rounded up to a multiple of 4
-    const int4* info;          // [n_tiles][2]: {edge_off, n_edges, n_flux, halo_off}, {n1, n2, face_off, 0}
+    int threads;               // threads per CTA: T, 2T (FV_SCHED_TILE2) or lanes * T
+    int lanes;                 // lanes per cell of the gradient and update phases: 1, 2 or 4
+    int nf;                    // faces per gradient slot: 3 (triangles only) or 4
+    int max_slots, max_grad, max_flux;
+    const int4* info;          // [n_tiles][2]: {slot_off, halo_off, flux_off, n_flux}, {n1, n2, owned cells, 0}
     const int32_t* halo;       // device cell of each ring-1, then ring-2 slot
-    const uint32_t* edge_ij;   // local i | local j << 16; each tile's run starts on a multiple of 4
-    const void* enx;           // S [local edges]
-    const void* eny;
-    const void* ele;
-    const void* exf;
-    const void* eyf;
-    const void* eg;
-    const uint2* face;         // four face words per gradient slot
-    const void* cca;           // S [n_total][4]: centroid x, y, area, 0
+    // per gradient slot (T owned, then n1 ring-1 slots of every tile) four
+    // face words: neighbour slot (0xFFFF = no face) | face-state unit << 16
+    // (flux edge + max_flux on the edge's second side) | kWordGhost (the
+    // neighbour is a boundary ghost) | kWordNoFlux (not a flux edge).  FP32
+    // with nf = 3: the fourth word holds `sl`.
+    const uint4* hd;
+    // per gradient slot and face, at nf * slot_off + f * (T + n1) + slot:
+    // fast S[4] {a_x, a_y, d_x, d_y}; exact S[4] {n_x, n_y, length (negative
+    // on the edge's second side), weight} and S[2] {d_x, d_y} in rec2 (d: face
+    // centre - centroid)
+    const void* rec;
+    const void* rec2;
+    const void* sl;            // per gradient slot: fast S 1 / (K sqrt(A))^3; exact double2 {1 / A, (K sqrt(A))^3}
+    const void* eg;            // S[4] per flux edge: n_x, n_y, length, 0
+    const double* ria;         // [n_own] 1 / area
+    const void* area;          // S [n_total]
+    FusedSmem L;               // shared-memory layout (fused_smem)
 };
 
-// 4-vectors in shared-memory planes of 16-byte units: FP32 one float4 plane,
-// FP64 two double2 planes `stride` units apart.
-template <class S>
+constexpr uint32_t kWordGhost = 0x40000000u, kWordNoFlux = 0x80000000u;
+constexpr int kMaxFluxUnits = 0x3FFF;  // 2 * max_flux at most
+__device__ __forceinline__ int word_nbr(uint32_t w) { return (int)(w & 0xFFFFu); }
+__device__ __forceinline__ int word_unit(uint32_t w) { return (int)((w >> 16) & 0x3FFFu); }
+
+// One 4-vector of S at a 16- or 32-byte aligned global address.
+__device__ __forceinline__ void ldg4(const float* p, float* v) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+__device__ __forceinline__ void ldg4(const double* p, double* v) {  // one 256-bit load
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+
+// NV consecutive variables (from v0) of 4-vectors kept in shared-memory
+// planes of 16-byte units (FP32 one float4 plane, FP64 two double2 planes
+// `stride` units apart), so that reads of random slots are free of bank
+// conflicts.
+template <class S, int NV>
 struct Planes;
-template <>
-struct Planes<float> {
-    static constexpr int NU = 1;
-    __device__ static __forceinline__ void get(const uint4* p, int, int r, float* v) {
-        const float4 x = reinterpret_cast<const float4*>(p)[r];
-        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+template <int NV>
+struct Planes<float, NV> {
+    __device__ static __forceinline__ void get(const uint4* p, int, int r, int v0, float* v) {
+        const float* a = reinterpret_cast<const float*>(p + r) + v0;
+        if (NV == 4) {
+            const float4 x = *reinterpret_cast<const float4*>(a);
+            v[0] = x.x; v[1 % NV] = x.y; v[2 % NV] = x.z; v[3 % NV] = x.w;
+        } else if (NV == 2) {
+            const float2 x = *reinterpret_cast<const float2*>(a);
+            v[0] = x.x; v[1 % NV] = x.y;
+        } else {
+            v[0] = a[0];
+        }
     }
-    __device__ static __forceinline__ void put(uint4* p, int, int r, const float* v) {
-        reinterpret_cast<float4*>(p)[r] = make_float4(v[0], v[1], v[2], v[3]);
+    __device__ static __forceinline__ void put(uint4* p, int, int r, int v0, const float* v) {
+        float* a = reinterpret_cast<float*>(p + r) + v0;
+        if (NV == 4) *reinterpret_cast<float4*>(a) = make_float4(v[0], v[1 % NV], v[2 % NV], v[3 % NV]);
+        else if (NV == 2) *reinterpret_cast<float2*>(a) = make_float2(v[0], v[1 % NV]);
+        else a[0] = v[0];
     }
-    // asynchronous copy of the 4-vector at global g into slot r
+    // asynchronous copy of the whole 4-vector at global g into slot r
     __device__ static __forceinline__ void stage(uint4* p, int, int r, const float* g) { cpa16(p + r, g); }
 };
-template <>
-struct Planes<double> {
-    static constexpr int NU = 2;
-    __device__ static __forceinline__ void get(const uint4* p, int stride, int r, double* v) {
-        const double2 x = reinterpret_cast<const double2*>(p)[r];
-        const double2 y = reinterpret_cast<const double2*>(p + stride)[r];
-        v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+template <int NV>
+struct Planes<double, NV> {
+    __device__ static __forceinline__ void get(const uint4* p, int stride, int r, int v0, double* v) {
+        if (NV == 4) {
+            const double2 x = reinterpret_cast<const double2*>(p)[r];
+            const double2 y = reinterpret_cast<const double2*>(p + stride)[r];
+            v[0] = x.x; v[1 % NV] = x.y; v[2 % NV] = y.x; v[3 % NV] = y.y;
+        } else if (NV == 2) {
+            const double2 x = reinterpret_cast<const double2*>(p + (v0 >> 1) * stride)[r];
+            v[0] = x.x; v[1 % NV] = x.y;
+        } else {
+            v[0] = reinterpret_cast<const double*>(p + (v0 >> 1) * stride + r)[v0 & 1];
+        }
     }
-    __device__ static __forceinline__ void put(uint4* p, int stride, int r, const double* v) {
-        reinterpret_cast<double2*>(p)[r] = make_double2(v[0], v[1]);
-        reinterpret_cast<double2*>(p + stride)[r] = make_double2(v[2], v[3]);
+    __device__ static __forceinline__ void put(uint4* p, int stride, int r, int v0, const double* v) {
+        if (NV == 4) {
+            reinterpret_cast<double2*>(p)[r] = make_double2(v[0], v[1 % NV]);
+            reinterpret_cast<double2*>(p + stride)[r] = make_double2(v[2 % NV], v[3 % NV]);
+        } else if (NV == 2) {
+            reinterpret_cast<double2*>(p + (v0 >> 1) * stride)[r] = make_double2(v[0], v[1 % NV]);
+        } else {
+            reinterpret_cast<double*>(p + (v0 >> 1) * stride + r)[v0 & 1] = v[0];
+        }
     }
     __device__ static __forceinline__ void stage(uint4* p, int stride, int r, const double* g) {
         cpa16(p + r, g);
@@ -77,129 +171,205 @@ struct Planes<double> {
     }
 };
 
-// Shared-memory layout of one fused tile, in bytes from the start.
-//  - state planes [max_slots];
-//  - centroids [max_grad]: FP32 one float4 plane (x, y, area, 0); FP64 one
-//    double2 plane (x, y) and the ring-1 areas [max_grad - T] (an owned
-//    cell's area is held by its thread);
-//  - gradient planes [max_grad] (and the limiter in the exact policy);
-//  - edge indices and normal, length, face centre [max_edges];
-//  - the flux store, which before the flux phase holds the Green-Gauss
-//    weights [max_edges] (gradient phase) and the halo indices (staging), and
-//    after the per-cell sums the residual warp sums.
-struct FusedSmem {
-    size_t q, c, ar, gx, gy, lm, ij, geo, flux, halo, total;
-    int ls, lg, em;  // plane strides (units) and edge-array length
-};
-template <class M>
-__host__ __device__ inline FusedSmem fused_smem(int max_slots, int max_grad, int max_edges, int max_flux, int T) {
-    using S = typename M::S;
-    using FT = typename std::conditional<M::exact, double, S>::type;
-    constexpr int NU = (int)(4 * sizeof(S) / 16);
-    FusedSmem L{};
-    L.ls = max_slots;
-    L.lg = max_grad;
-    L.em = max_edges;
-    size_t o = 0;
-    L.q = o; o += (size_t)16 * NU * max_slots;
-    L.c = o; o += (size_t)16 * max_grad;
-    L.ar = o; if (sizeof(S) == 8) o += ((size_t)8 * (max_grad - T) + 15) / 16 * 16;
-    L.gx = o; o += (size_t)16 * NU * max_grad;
-    L.gy = o; o += (size_t)16 * NU * max_grad;
-    L.lm = o; if (M::exact) o += (size_t)16 * NU * max_grad;
-    L.ij = o; o += (size_t)4 * max_edges;
-    L.geo = o; o += (size_t)5 * sizeof(S) * max_edges;
-    o = (o + 15) / 16 * 16;
-    L.flux = o;
-    L.halo = L.flux + ((size_t)sizeof(S) * max_edges + 15) / 16 * 16;
-    size_t fb = (size_t)max_flux * 4 * sizeof(FT);
-    const size_t before = (L.halo - L.flux) + (size_t)max_slots * 4;
-    fb = fb > before ? fb : before;
-    fb = fb > (size_t)(kTileMax / 32) * 4 * sizeof(double) ? fb : (size_t)(kTileMax / 32) * 4 * sizeof(double);
-    o += (fb + 15) / 16 * 16;
-    L.total = o;
-    return L;
+// NV consecutive values of a 4-vector in global memory
+template <class S, int NV>
+__device__ __forceinline__ void ldv(const S* a, S* v) {
+    if (NV == 4 && sizeof(S) == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a);
+        v[0] = (S)x.x; v[1 % NV] = (S)x.y; v[2 % NV] = (S)x.z; v[3 % NV] = (S)x.w;
+    } else if (NV >= 2 && sizeof(S) == 8) {
+#pragma unroll
+        for (int i = 0; i < NV / 2; ++i) {
+            const double2 x = reinterpret_cast<const double2*>(a)[i];
+            v[2 * i] = (S)x.x; v[(2 * i + 1) % NV] = (S)x.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = a[i];
+    }
+}
+template <class S, int NV>
+__device__ __forceinline__ void stv(S* a, const S* v) {
+    if (NV == 4 && sizeof(S) == 4) {
+        *reinterpret_cast<float4*>(a) = make_float4((float)v[0], (float)v[1 % NV], (float)v[2 % NV], (float)v[3 % NV]);
+    } else if (NV >= 2 && sizeof(S) == 8) {
+#pragma unroll
+        for (int i = 0; i < NV / 2; ++i)
+            reinterpret_cast<double2*>(a)[i] = make_double2((double)v[2 * i], (double)v[(2 * i + 1) % NV]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) a[i] = v[i];
+    }
 }
 
-// centroid (x, y) of slot r
-template <class S>
-__device__ __forceinline__ void cent(const uint4* C, int r, S& x, S& y) {
-    if constexpr (sizeof(S) == 4) {
-        const float4 v = reinterpret_cast<const float4*>(C)[r];
-        x = v.x; y = v.y;
+// The NV-variable shares of the 4 / NV lanes of one cell (consecutive lanes
+// of a warp, all in the same branch), as one 4-vector in every lane.
+template <class S, int NV>
+__device__ __forceinline__ void share(const S* v, S* all) {
+    if (NV == 4) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) all[k] = v[k % NV];
     } else {
-        const double2 v = reinterpret_cast<const double2*>(C)[r];
-        x = v.x; y = v.y;
+        constexpr int LP = 4 / NV;
+        const int lane = threadIdx.x & 31, first = lane & ~(LP - 1);
+        const unsigned m = ((1u << LP) - 1u) << first;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) all[k] = __shfl_sync(m, v[k % NV], first + k / NV);
     }
+}
+// this lane's share of a 4-vector
+template <class S, int NV>
+__device__ __forceinline__ void own_share(const S* all, int v0, S* v) {
+    if (NV == 4) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k % NV] = all[k];
+    } else if (NV == 2) {
+        v[0] = v0 ? all[2] : all[0];
+        v[1 % NV] = v0 ? all[3] : all[1];
+    } else {
+        v[0] = v0 == 0 ? all[0] : v0 == 1 ? all[1] : v0 == 2 ? all[2] : all[3];
+    }
+}
+
+// guard_face (fv_tile.cuh) of a face state held in shares
+template <class S, int NV, bool EXACT>
+__device__ __forceinline__ void guard_share(const Params& P, S* qf, const S* qc) {
+    if (!P.positivity_guard) return;
+    S a[4];
+    share<S, NV>(qf, a);
+    if (face_state_bad<S, EXACT>(P, a)) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) qf[i] = qc[i];
+    }
+}
+
+// One gradient slot's geometry: face words and records.
+template <class M, int NF>
+struct SlotGeo {
+    using S = typename M::S;
+    uint32_t w[NF];
+    S sl[M::exact ? 2 : 1];
+    S a[NF][4];
+    S d[M::exact ? NF : 1][2];
+    __device__ __forceinline__ bool face(int f) const { return f < 3 || word_nbr(w[f]) != 0xFFFF; }
+    __device__ __forceinline__ S dx(int f) const { if constexpr (M::exact) return d[f][0]; else return a[f][2]; }
+    __device__ __forceinline__ S dy(int f) const { if constexpr (M::exact) return d[f][1]; else return a[f][3]; }
+    __device__ __forceinline__ void load(const FusedParams& FP, uint32_t slot_off, uint32_t G, uint32_t r) {
+        const uint4 h = __ldg(FP.hd + (slot_off + r));
+        w[0] = h.x; w[1] = h.y; w[2] = h.z;
+        if constexpr (NF == 4) w[NF - 1] = h.w;
+        if constexpr (M::exact) {
+            const double2 x = __ldg(reinterpret_cast<const double2*>(FP.sl) + (slot_off + r));
+            sl[0] = x.x; sl[1] = x.y;
+        } else if constexpr (NF == 3 && sizeof(S) == 4) {
+            sl[0] = __uint_as_float(h.w);
+        } else {
+            sl[0] = __ldg((const S*)FP.sl + (slot_off + r));
+        }
+        const uint32_t b = NF * slot_off + r;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            ldg4((const S*)FP.rec + 4 * (size_t)(b + f * G), a[f]);
+            if constexpr (M::exact) {
+                const double2 x = __ldg(reinterpret_cast<const double2*>(FP.rec2) + (b + f * G));
+                d[f][0] = x.x; d[f][1] = x.y;
+            }
+        }
+    }
+};
+
+// CFL or constant time step of owned cell c (slot l) and of its boundary
+// ghosts from {u, v, c} of the tile's slots (calc_dt of
+// examples/forwardStep/main.cpp:140-185 and examples/naca/main.cpp:142-183;
+// fast policies); returns the ordered-key minimum of the values written.
+template <class S, int NF>
+__device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& FP, const TileIO& io, const uint32_t* fw,
+                                                            const uint4* W, int l, int c, int halo_off, int flux_off) {
+    const Params& P = FP.P;
+    const S cfl = (S)P.cfl, A = __ldg((const S*)FP.area + c);
+    const bool sum = P.dt_kind == 1, constant = P.dt_kind == 0;
+    unsigned long long kmin = ~0ull;
+    S ws[4];
+    Planes<S, 4>::get(W, FP.max_grad, l, 0, ws);
+    S acc = sum ? S(0) : S(1);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const uint32_t w = fw[f];
+        const int o = word_nbr(w);
+        if (f == 3 && o == 0xFFFF) continue;
+        const bool ghost = (w & kWordGhost) != 0;
+        S e[4], wn[4];
+        const int u = word_unit(w);
+        ldg4((const S*)FP.eg + 4 * (size_t)(flux_off + (u < FP.max_flux ? u : u - FP.max_flux)), e);
+        Planes<S, 4>::get(W, FP.max_grad, o, 0, wn);
+        double dg = P.dt_const;
+        if (sum) {
+            const S center = fast::tmax(ws[2] + fabs(fast::fma_(ws[0], e[0], ws[1] * e[1])),
+                                        wn[2] + fabs(fast::fma_(wn[0], e[0], wn[1] * e[1])));
+            acc = fast::fma_(center, e[2], acc);
+            if (ghost) dg = (double)(cfl * __ldg((const S*)FP.area + FP.halo[halo_off + o - FP.T]) * fast::rcp(center * e[2]));
+        } else if (!constant) {
+            const S es = fast::fma_(ws[2] + fabs(ws[0]), e[0], (ws[2] + fabs(ws[1])) * e[1]);
+            acc = fast::tmin(acc, cfl * A * fast::rcp(e[2] * fabs(es)));
+            if (ghost) {
+                const S en = fast::fma_(wn[2] + fabs(wn[0]), e[0], (wn[2] + fabs(wn[1])) * e[1]);
+                const S An = __ldg((const S*)FP.area + FP.halo[halo_off + o - FP.T]);
+                dg = (double)fast::tmin(S(1), cfl * An * fast::rcp(e[2] * fabs(en)));
+            }
+        }
+        if (ghost) {
+            io.dt[FP.halo[halo_off + o - FP.T]] = dg;
+            kmin = kmin_(kmin, tkey(dg));
+        }
+    }
+    const double di = constant ? P.dt_const : (double)(sum ? cfl * A * fast::rcp(acc) : acc);
+    io.dt[c] = di;
+    return kmin_(kmin, tkey(di));
 }
 
 // One tile t.  Returns false when the step is inactive (nothing written).
+// NV: variables per lane of the gradient and update phases (4 / NV lanes per cell).
+// PH 0: the whole stage.  PH 1: the limited gradients of the owned cells only,
+// written to io.gx, io.gy; PH 2: the stage with the gradients read from there
+// (the split layout; fast policies).  PH 3: the step's time step only.
 // PART: a decomposition part's tile, whose owned cells come from the tile
 // info (a part owns fewer real cells than its local mesh holds).
-template <class M, int FLUX, bool REMOTE = false, bool PART = false>
+template <class M, int FLUX, int NV, int NF, int PH, bool REMOTE, bool PART>
 __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& io, const int t, const PartIO& pio) {
     using S = typename M::S;
-    using FT = typename std::conditional<M::exact, double, S>::type;  // flux storage
-    using PL = Planes<S>;
-    constexpr int V = 4;
+    using PL = Planes<S, NV>;
+    using P4 = Planes<S, 4>;
+    constexpr int V = 4, LP = V / NV;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ unsigned long long s_dtkey;
+    __shared__ double s_dt;
     const Params& P = FP.P;
     const int N = P.n_real, T = FP.T;
     const int4 ia = FP.info[2 * t], ib = FP.info[2 * t + 1];
-    const int edge_off = ia.x, n_edges = ia.y, n_flux = ia.z, halo_off = ia.w;
-    const int n1 = ib.x, n2 = ib.y, face_off = ib.z;
-    const int c0 = t * T, nown = PART ? ib.w : min(T, N - c0);
-    const FusedSmem L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_edges, FP.max_flux, FP.T);
+    const int slot_off = ia.x, halo_off = ia.y, flux_off = ia.z, n_flux = ia.w;
+    const int n1 = ib.x, nh = ib.x + ib.y;
+    const int c0 = t * T, nown = PART ? ib.z : min(T, N - c0);
+    const int G = T + n1;
+    const FusedSmem& L = FP.L;
     uint4* Q = reinterpret_cast<uint4*>(smem_raw + L.q);
-    uint4* C = reinterpret_cast<uint4*>(smem_raw + L.c);
-    S* AR = reinterpret_cast<S*>(smem_raw + L.ar);  // FP64: ring-1 areas
+    uint4* FS = reinterpret_cast<uint4*>(smem_raw + L.fs);
+    double* QB = reinterpret_cast<double*>(smem_raw + L.qb);
     uint4* GX = reinterpret_cast<uint4*>(smem_raw + L.gx);
     uint4* GY = reinterpret_cast<uint4*>(smem_raw + L.gy);
     uint4* LM = reinterpret_cast<uint4*>(smem_raw + L.lm);
-    uint32_t* sij = reinterpret_cast<uint32_t*>(smem_raw + L.ij);
-    S* snx = reinterpret_cast<S*>(smem_raw + L.geo);
-    S* sny = snx + L.em; S* sle = sny + L.em; S* sxf = sle + L.em; S* syf = sxf + L.em;
-    FT* sF = reinterpret_cast<FT*>(smem_raw + L.flux);
-    // the Green-Gauss weights (gradient phase) and the halo indices (staging)
-    // are dead before the first flux is stored: they share the flux store
-    S* sg = reinterpret_cast<S*>(smem_raw + L.flux);
-    int* shalo = reinterpret_cast<int*>(smem_raw + L.halo);
     const bool global_dt = io.ctrl != nullptr && P.global_dt;
     const int l = threadIdx.x;
-    const int c = c0 + l;
+    const int r0 = l / LP, rstep = blockDim.x / LP;  // gradient slots of this lane
+    const int v0 = (l % LP) * NV;                    // its first variable
     // ---- constant tile data first (may overlap the previous kernel's tail):
-    // edges in 16-byte chunks, halo indices, centroid/area records of the
-    // owned cells, face words of this thread's gradient slots
-    {
-        const int nch = (n_edges + 3) >> 2;  // 4 edges per chunk of the u32 array
-        for (int k = l; k < nch; k += blockDim.x) cpa16(sij + 4 * k, FP.edge_ij + edge_off + 4 * k);
-        constexpr int EPC = 16 / (int)sizeof(S);  // edges per 16-byte chunk of a geometry array
-        const int ncg = (n_edges + EPC - 1) / EPC;
-        for (int k = l; k < ncg; k += blockDim.x) {
-            const int d = EPC * k, g = edge_off + EPC * k;
-            cpa16(snx + d, (const S*)FP.enx + g);
-            cpa16(sny + d, (const S*)FP.eny + g);
-            cpa16(sle + d, (const S*)FP.ele + g);
-            cpa16(sxf + d, (const S*)FP.exf + g);
-            cpa16(syf + d, (const S*)FP.eyf + g);
-            cpa16(sg + d, (const S*)FP.eg + g);
-        }
-        for (int h = l; h < n1 + n2; h += blockDim.x) cpa4(shalo + h, FP.halo + halo_off + h);
-        for (int r = l; r < nown; r += blockDim.x) cpa16(C + r, (const S*)FP.cca + 4 * (size_t)(c0 + r));
-        cpa_commit();
-    }
-    // the owned cell's area (this thread's gradient slot and update)
-    const S A_own = l < nown ? ((const S*)FP.cca)[4 * (size_t)c + 2] : S(1);
-    // face words of this thread's gradient slots: slot l (pass 0) and slot
-    // l + blockDim.x (pass 1); slots [0, nown) are owned, [T, T + n1) ring 1
-    const uint2 kNoWords = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
-    auto slot_words = [&](int r) {
-        const bool has = r < T ? r < nown : r - T < n1;
-        return has ? FP.face[face_off + r] : kNoWords;
-    };
-    const uint2 fw0 = slot_words(l);
-    const uint2 fw1 = slot_words(l + blockDim.x);
+    // the first gradient slot's geometry and the halo indices, into registers
+    SlotGeo<M, NF> geo;
+    geo.load(FP, slot_off, G, min(r0, G - 1));
+    const int h0 = l < nh ? __ldg(FP.halo + halo_off + l) : 0;
+    // the owned cell of the update phase (r0 < nown there) and its faces
+    const int uc = r0;
+    uint32_t own[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) own[f] = geo.w[f];
     // the tile's case (batches); -1: the tile spans two cases
     const int tc = (global_dt && P.n_cases > 1) ? P.tile_case[t] : 0;
     // reference cell 0 of the tile's case, whose dt carries the NaN rule of min_dt
@@ -207,16 +377,6 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
     pdl_wait();
     // every load of data written by earlier kernels is issued here together
     const bool inactive = t_inactive(io.ctrl);
-    double d0 = 0., dtc = 0.;
-    double qb[V];
-    if (global_dt && tc >= 0) d0 = io.dt[cell0];
-    if (l < nown) {
-        ld<double, V>(io.q_base, c, qb);
-        if (!global_dt) dtc = io.dt[c];
-    }
-    for (int r = l; r < nown; r += blockDim.x) PL::stage(Q, L.ls, r, (const S*)io.q_stage + 4 * (size_t)(c0 + r));
-    cpa_commit();
-    cpa_wait_prior();  // the constant group: edges, halo indices
     if constexpr (REMOTE) {
         // a band tile reads halo cells: wait for the senders' epoch of this
         // stage's input (bounded; a tile that gives up is skipped)
@@ -241,97 +401,103 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
             }
         }
         __syncthreads();
-        if (s_gave_up) {
-            cpa_wait();  // this tile's copies in flight land before it leaves
-            return false;
-        }
+        if (s_gave_up) return false;
     }
-    __syncthreads();
-    for (int h = l; h < n1 + n2; h += blockDim.x) {
-        const int g = shalo[h];
-        PL::stage(Q, L.ls, T + h, (const S*)io.q_stage + 4 * (size_t)g);
-        if (h < n1) {
-            cpa16(C + T + h, (const S*)FP.cca + 4 * (size_t)g);
-            if constexpr (sizeof(S) == 8) cpa8(AR + h, (const S*)FP.cca + 4 * (size_t)g + 2);
-        }
+    double dtc = 0.;
+    if ((PH == 0 || PH == 2) && !global_dt && uc < nown) dtc = io.dt[c0 + uc];
+    // the owned states and, behind them, the base states, in 16-byte chunks of
+    // consecutive threads (a CTA has at least T threads)
+    constexpr int NU = (int)sizeof(S) / 4;
+    const uint4* gq = reinterpret_cast<const uint4*>((const S*)io.q_stage + 4 * (size_t)c0) + l;
+    const uint4* gb = reinterpret_cast<const uint4*>(io.q_base + 4 * (size_t)c0) + l;
+    if (l < NU * nown) cpa16(NU == 1 ? Q + l : Q + (l & 1) * L.ls + (l >> 1), gq);
+    if (NU == 2 && l + T < 2 * nown) cpa16(Q + (l & 1) * L.ls + ((l + T) >> 1), gq + T);
+    for (int h = l; h < nh; h += blockDim.x) {
+        const int g = h == l ? h0 : __ldg(FP.halo + halo_off + h);
+        P4::stage(Q, L.ls, T + h, (const S*)io.q_stage + 4 * (size_t)g);
     }
-    if (global_dt && tc >= 0 && threadIdx.x < 32) {
+    cpa_commit();
+    if (PH == 0 || PH == 2) {
+        if (l < 2 * nown) cpa16(QB + 2 * l, gb);
+        if (l + T < 2 * nown) cpa16(QB + 2 * (l + T), gb + T);
+    }
+    cpa_commit();
+    if ((PH == 0 || PH == 2) && global_dt && tc >= 0 && threadIdx.x < 32) {
+        // min_dt (explicit.cpp:555-564) of the tile's case; a NaN in its dt[0] wins
         const unsigned long long* keys = io.dtkeys + (size_t)tc * kDtSlots;
+        const double d0 = io.dt[cell0];
         unsigned long long k = kmin_(keys[threadIdx.x], keys[threadIdx.x + 32]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) k = kmin_(k, __shfl_xor_sync(0xffffffffu, k, o));
-        if (threadIdx.x == 0) s_dtkey = k;
+        if (threadIdx.x == 0) s_dt = (d0 != d0) ? d0 : tkey_inv(k);
     }
-    cpa_wait();
-    if (inactive) return false;
+    cpa_wait_prior();  // the states; the base state is awaited before the update
+    if (inactive) {
+        cpa_wait();
+        return false;
+    }
     __syncthreads();
 
-    // ---- gradients and limiters of the owned cells and ring 1
-    // (calc_gradients + calc_limiters, explicit.cpp:112-258)
-    for (int r = l, pass = 0; r < T + n1; r += blockDim.x, ++pass) {
-        if (r < T && r >= nown) continue;
-        const uint2 fwv = pass == 0 ? fw0 : (pass == 1 ? fw1 : FP.face[face_off + r]);
-        uint16_t w[kMaxFaces];
-        w[0] = (uint16_t)(fwv.x & 0xFFFF); w[1] = (uint16_t)(fwv.x >> 16);
-        w[2] = (uint16_t)(fwv.y & 0xFFFF); w[3] = (uint16_t)(fwv.y >> 16);
-        S qs[V], gx[V], gy[V], qmn[V], qmx[V], lim[V];
-        PL::get(Q, L.ls, r, qs);
-        S xc, yc, A;
-        if constexpr (sizeof(S) == 4) {
-            const float4 cv = reinterpret_cast<const float4*>(C)[r];
-            xc = cv.x; yc = cv.y; A = cv.z;
-        } else {
-            cent<S>(C, r, xc, yc);
-            A = r < T ? A_own : AR[r - T];
+    // ---- gradients, limiters and face states of the owned cells and ring 1
+    // (calc_gradients + calc_limiters, explicit.cpp:112-258, and the MUSCL
+    // states of calc_time_derivatives, 297-320)
+    if constexpr (PH == 3) {
+        uint4* W = FS;
+        const S gamma = (S)P.gamma;
+        for (int r = l; r < G; r += blockDim.x) {
+            if (r >= nown && r < T) continue;
+            S q[V], w[V];
+            P4::get(Q, L.ls, r, 0, q);
+            fast::speeds(gamma, q, w);
+            P4::put(W, FP.max_grad, r, 0, w);
         }
+        __syncthreads();
+        unsigned long long kmin = ~0ull;
+        if (l < nown) kmin = fused_cell_dt<S, NF>(FP, io, own, W, l, c0 + l, halo_off, flux_off);
+        tile_dt_reduce(P, T, io, t, l, nown, kmin);
+        return true;
+    }
+    const int gslots = PH == 1 ? nown : G;
+    for (int r = r0; r < gslots;) {
+        // unused slots of a last, partial tile and ring-1 ghosts have no faces
+        if (word_nbr(geo.w[0]) != 0xFFFF) {
+            S qs[NV], gx[NV], gy[NV], lim[NV];
+            PL::get(Q, L.ls, r, v0, qs);
+            if constexpr (PH == 2) {
+                const size_t g = r < T ? (size_t)(c0 + r) : (size_t)__ldg(FP.halo + halo_off + r - T);
+                ldv<S, NV>((const S*)io.gx + 4 * g + v0, gx);
+                ldv<S, NV>((const S*)io.gy + 4 * g + v0, gy);
+            } else if constexpr (M::exact) {
+                double qmn[NV], qmx[NV];
 #pragma unroll
-        for (int k = 0; k < V; ++k) { gx[k] = 0; gy[k] = 0; qmn[k] = qs[k]; qmx[k] = qs[k]; lim[k] = 1; }
+                for (int k = 0; k < NV; ++k) { gx[k] = 0; gy[k] = 0; qmn[k] = qs[k]; qmx[k] = qs[k]; lim[k] = 1; }
 #pragma unroll
-        for (int f = 0; f < kMaxFaces; ++f) {
-            if (w[f] == kFaceNone) continue;
-            const int el = w[f] & kFaceEdgeMask, side = w[f] >> 15;
-            const uint32_t ij = sij[el];
-            const int o = side ? (int)(ij & 0xffff) : (int)(ij >> 16);
-            const S nx = snx[el], ny = sny[el], le = sle[el], g = sg[el];
-            S qn[V];
-            PL::get(Q, L.ls, o, qn);
+                for (int f = 0; f < NF; ++f) {
+                    if (!geo.face(f)) continue;
+                    const double nx = geo.a[f][0], ny = geo.a[f][1], le = geo.a[f][2], g = geo.a[f][3];
+                    const bool side = (geo.a[f][2] < 0.);  // a negative length marks the edge's second cell
+                    const double len = fabs(le);
+                    double qn[NV];
+                    PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
 #pragma unroll
-            for (int k = 0; k < V; ++k) {
-                if constexpr (M::exact) {
-                    if (!side) {
-                        const double fl = (qs[k] * (1.0 - g) + qn[k] * g) * le;
-                        gx[k] += fl * nx; gy[k] += fl * ny;
-                    } else {
-                        const double fl = (qn[k] * (1.0 - g) + qs[k] * g) * le;
-                        gx[k] -= fl * nx; gy[k] -= fl * ny;
+                    for (int k = 0; k < NV; ++k) {
+                        if (!side) {
+                            const double fl = (qs[k] * (1.0 - g) + qn[k] * g) * len;
+                            gx[k] += fl * nx; gy[k] += fl * ny;
+                        } else {
+                            const double fl = (qn[k] * (1.0 - g) + qs[k] * g) * len;
+                            gx[k] -= fl * nx; gy[k] -= fl * ny;
+                        }
+                        qmn[k] = exact::dmin(qmn[k], qn[k]); qmx[k] = exact::dmax(qmx[k], qn[k]);
                     }
-                    qmn[k] = exact::dmin(qmn[k], qn[k]); qmx[k] = exact::dmax(qmx[k], qn[k]);
-                } else {
-                    const S qi = side ? qn[k] : qs[k], qj = side ? qs[k] : qn[k];
-                    const S fl = (qi + (qj - qi) * g) * (side ? -le : le);
-                    gx[k] += fl * nx; gy[k] += fl * ny;
-                    qmn[k] = fast::tmin(qmn[k], qn[k]); qmx[k] = fast::tmax(qmx[k], qn[k]);
                 }
-            }
-        }
-        if constexpr (M::exact) {
-            const double invA = 1. / A;
+                const double invA = geo.sl[0], K3a = geo.sl[1];
+                const double tol = 1e-15;
 #pragma unroll
-            for (int k = 0; k < V; ++k) { gx[k] *= invA; gy[k] *= invA; }
-            const double sqrt_area = sqrt(A);
-            const double tol = 1e-15;
-#pragma unroll
-            for (int f = 0; f < kMaxFaces; ++f) {
-                if (w[f] == kFaceNone) continue;
-                const int el = w[f] & kFaceEdgeMask;
-                const double dx = sxf[el] - xc, dy = syf[el] - yc;
-#pragma unroll
-                for (int k = 0; k < V; ++k) {
-                    const double dqg = gx[k] * dx + gy[k] * dy;
+                for (int k = 0; k < NV; ++k) {
+                    gx[k] *= invA; gy[k] *= invA;
                     const double delta_max = qmx[k] - qs[k];
                     const double delta_min = qmn[k] - qs[k];
-                    const double Ka = P.K * sqrt_area;
-                    const double K3a = Ka * Ka * Ka;
                     const double d2 = (delta_max - delta_min) * (delta_max - delta_min);
                     double sig;
                     if (d2 <= K3a) sig = 1.;
@@ -339,266 +505,271 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
                         const double y = (d2 / K3a - 1.0);
                         sig = 2.0 * y * y * y - 3.0 * y * y + 1.0;
                     } else sig = 0.;
-                    double lv = 1.0;
-                    if (sig < 1.0) {
-                        if (dqg > tol) lv = exact::limiter_func(P.limiter, delta_max / dqg);
-                        else if (dqg < -tol) lv = exact::limiter_func(P.limiter, delta_min / dqg);
-                        else lv = 1.0;
-                    }
-                    lv = sig + (1.0 - sig) * lv;
-                    lim[k] = exact::dmin(lim[k], lv);
-                }
-            }
-            PL::put(LM, L.lg, r, lim);
-        } else {
-            const S invA = fast::rcp(A);
 #pragma unroll
-            for (int k = 0; k < V; ++k) { gx[k] *= invA; gy[k] *= invA; }
-            const S Ka = (S)P.K * fast::sqrt_(A);
-            const S K3a = Ka * Ka * Ka, rK3a = fast::rcp(K3a);
-            const S tol = S(1e-15);
-            S sig[V];
-#pragma unroll
-            for (int k = 0; k < V; ++k) {
-                const S d = qmx[k] - qmn[k];
-                const S d2 = d * d;
-                if (d2 <= K3a) sig[k] = 1;
-                else if (d2 <= 2 * K3a) {
-                    const S y = d2 * rK3a - S(1);
-                    sig[k] = (S(2) * y - S(3)) * y * y + S(1);
-                } else sig[k] = 0;
-            }
-#pragma unroll
-            for (int f = 0; f < kMaxFaces; ++f) {
-                if (w[f] == kFaceNone) continue;
-                const int el = w[f] & kFaceEdgeMask;
-                const S dx = sxf[el] - xc, dy = syf[el] - yc;
-#pragma unroll
-                for (int k = 0; k < V; ++k) {
-                    if (sig[k] < S(1)) {
-                        const S dqg = gx[k] * dx + gy[k] * dy;
-                        S phi = 1;
-                        if (dqg > tol) phi = fast::limiter_ratio(P.limiter, qmx[k] - qs[k], dqg);
-                        else if (dqg < -tol) phi = fast::limiter_ratio(P.limiter, qmn[k] - qs[k], dqg);
-                        lim[k] = fast::tmin(lim[k], sig[k] + (S(1) - sig[k]) * phi);
+                    for (int f = 0; f < NF; ++f) {
+                        if (!geo.face(f)) continue;
+                        const double dqg = gx[k] * geo.dx(f) + gy[k] * geo.dy(f);
+                        double lv = 1.0;
+                        if (sig < 1.0) {
+                            if (dqg > tol) lv = exact::limiter_func(P.limiter, delta_max / dqg);
+                            else if (dqg < -tol) lv = exact::limiter_func(P.limiter, delta_min / dqg);
+                            else lv = 1.0;
+                        }
+                        lv = sig + (1.0 - sig) * lv;
+                        lim[k] = exact::dmin(lim[k], lv);
                     }
                 }
-            }
-            // limited gradients
+            } else {
+                S mn[NV], mx[NV], sig[NV];
 #pragma unroll
-            for (int k = 0; k < V; ++k) { gx[k] *= lim[k]; gy[k] *= lim[k]; }
+                for (int k = 0; k < NV; ++k) { gx[k] = 0; gy[k] = 0; mn[k] = 0; mx[k] = 0; lim[k] = 1; }
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    if (!geo.face(f)) continue;
+                    S qn[NV];
+                    PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        const S d = qn[k] - qs[k];
+                        gx[k] = fast::fma_(geo.a[f][0], d, gx[k]);
+                        gy[k] = fast::fma_(geo.a[f][1], d, gy[k]);
+                        mn[k] = fast::vmin(mn[k], d);
+                        mx[k] = fast::vmax(mx[k], d);
+                    }
+                }
+                bool limited = false;
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    sig[k] = fast::smooth_switch(mx[k] - mn[k], geo.sl[0]);
+                    limited |= sig[k] < S(1);
+                }
+                if (limited) {
+                    auto apply = [&](auto kind) {
+#pragma unroll
+                        for (int k = 0; k < NV; ++k) {
+                            // the largest and smallest g . d over the faces
+                            // give the strictest ratio of each sign
+                            S up = 0, lo = 0;
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) {
+                                if (!geo.face(f)) continue;
+                                const S dq = fast::fma_(gy[k], geo.dy(f), gx[k] * geo.dx(f));
+                                up = fast::vmax(up, dq);
+                                lo = fast::vmin(lo, dq);
+                            }
+                            const S lim_k = fast::limiter_min(kind(), sig[k], mx[k], mn[k], up, lo);
+                            gx[k] *= lim_k;
+                            gy[k] *= lim_k;
+                        }
+                    };
+                    if (P.limiter == 2) apply([] { return 2; });
+                    else if (P.limiter == 1) apply([] { return 1; });
+                    else apply([&] { return P.limiter; });
+                }
+            }
+            if constexpr (PH == 1) {
+                stv<S, NV>((S*)io.gx + 4 * (size_t)(c0 + r) + v0, gx);
+                stv<S, NV>((S*)io.gy + 4 * (size_t)(c0 + r) + v0, gy);
+            } else {
+                uint32_t any = 0;
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    if (!geo.face(f)) continue;
+                    S qf[NV];
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        if constexpr (M::exact) qf[k] = qs[k] + (gx[k] * geo.dx(f) + gy[k] * geo.dy(f)) * lim[k];
+                        else qf[k] = fast::fma_(gy[k], geo.dy(f), fast::fma_(gx[k], geo.dx(f), qs[k]));
+                    }
+                    guard_share<S, NV, M::exact>(P, qf, qs);
+                    if (!(geo.w[f] & kWordNoFlux)) PL::put(FS, L.lf, word_unit(geo.w[f]), v0, qf);
+                    any |= geo.w[f];
+                }
+                if (any & kWordGhost) {
+                    // a ghost's face state is its cell value (gradient 0); the
+                    // cell's own gradients are kept for the ghost fill
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        if (!geo.face(f) || !(geo.w[f] & kWordGhost)) continue;
+                        const int u = word_unit(geo.w[f]), el = u < FP.max_flux ? u : u - FP.max_flux;
+                        S qn[NV];
+                        PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
+                        if constexpr (M::exact) {
+                            // the signed zero that the ghost's zero gradient adds
+                            const double z = __ldg((const double*)FP.eg + 4 * (size_t)(flux_off + el) + 3);
+#pragma unroll
+                            for (int k = 0; k < NV; ++k) qn[k] += z;
+                        }
+                        PL::put(FS, L.lf, u < FP.max_flux ? u + FP.max_flux : el, v0, qn);
+                    }
+                    PL::put(GX, L.lt, r, v0, gx);
+                    PL::put(GY, L.lt, r, v0, gy);
+                    if constexpr (M::exact) PL::put(LM, L.lt, r, v0, lim);
+                }
+            }
         }
-        PL::put(GX, L.lg, r, gx);
-        PL::put(GY, L.lg, r, gy);
+        r += rstep;
+        if (r >= gslots) break;
+        geo.load(FP, slot_off, G, r);
     }
+    if constexpr (PH == 1) return true;
     __syncthreads();
 
-    // ---- one flux per flux edge (calc_time_derivatives, explicit.cpp:261-350)
+    // ---- one flux per flux edge (calc_time_derivatives, explicit.cpp:321-350)
     for (int el = l; el < n_flux; el += blockDim.x) {
-        const uint32_t ij = sij[el];
-        const int li = (int)(ij & 0xffff), lj = (int)(ij >> 16);
-        const S n0 = snx[el], n1v = sny[el];
-        FT f[V];
-        S qL[V], qR[V], ci[V], cj[V], gxi[V], gyi[V], gxj[V], gyj[V], pi[2], pj[2];
-        PL::get(Q, L.ls, li, ci);
-        PL::get(Q, L.ls, lj, cj);
-        cent<S>(C, li, pi[0], pi[1]);
-        cent<S>(C, lj, pj[0], pj[1]);
-        PL::get(GX, L.lg, li, gxi); PL::get(GY, L.lg, li, gyi);
-        PL::get(GX, L.lg, lj, gxj); PL::get(GY, L.lg, lj, gyj);
-        const S xf = sxf[el], yf = syf[el];
-        const S di0 = xf - pi[0], di1 = yf - pi[1];
-        const S dj0 = xf - pj[0], dj1 = yf - pj[1];
-        if constexpr (M::exact) {
-            S li_[V], lj_[V];
-            PL::get(LM, L.lg, li, li_); PL::get(LM, L.lg, lj, lj_);
+        S e[4], qL[V], qR[V], f[V];
+        ldg4((const S*)FP.eg + 4 * (size_t)(flux_off + el), e);
+        P4::get(FS, L.lf, el, 0, qL);
+        P4::get(FS, L.lf, el + FP.max_flux, 0, qR);
+        if constexpr (M::exact) exact::flux<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
+        else fast::flux<FLUX, S>((S)P.gamma, f, qL, qR, e[0], e[1]);
 #pragma unroll
-            for (int k = 0; k < V; ++k) {
-                qL[k] = ci[k] + (gxi[k] * di0 + gyi[k] * di1) * li_[k];
-                qR[k] = cj[k] + (gxj[k] * dj0 + gyj[k] * dj1) * lj_[k];
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < V; ++k) {
-                qL[k] = ci[k] + gxi[k] * di0 + gyi[k] * di1;
-                qR[k] = cj[k] + gxj[k] * dj0 + gyj[k] * dj1;
-            }
-        }
-        guard_face<S, V, M::exact>(P, qL, ci);
-        guard_face<S, V, M::exact>(P, qR, cj);
-        if constexpr (M::exact) {
-            exact::flux<FLUX>(P.gamma, f, qL, qR, n0, n1v);
-        } else {
-            fast::flux<FLUX, S>((S)P.gamma, f, qL, qR, n0, n1v);
-            const S le = sle[el];
-#pragma unroll
-            for (int k = 0; k < V; ++k) f[k] *= le;
-        }
-        if (sizeof(FT) == 4) {
-            reinterpret_cast<float4*>(sF)[el] = make_float4((float)f[0], (float)f[1], (float)f[2], (float)f[3]);
-        } else {
-            reinterpret_cast<double2*>(sF)[2 * el] = make_double2((double)f[0], (double)f[1]);
-            reinterpret_cast<double2*>(sF)[2 * el + 1] = make_double2((double)f[2], (double)f[3]);
-        }
+        for (int k = 0; k < V; ++k) { f[k] *= e[2]; qL[k] = -f[k]; }
+        P4::put(FS, L.lf, el, 0, qL);
+        P4::put(FS, L.lf, el + FP.max_flux, 0, f);
     }
+    cpa_wait();  // the base state
     __syncthreads();
 
     // ---- per-cell sums in reference edge order, RK update, ghost fill
     // (update_cells + update_bounds, explicit.cpp:368-417)
-    double res[V];
+    double res[NV];
 #pragma unroll
-    for (int k = 0; k < V; ++k) res[k] = 0.;
-    if (l < nown) {  // fw0 holds the owned cell's faces (slot l < T)
-        uint16_t w[kMaxFaces];
-        w[0] = (uint16_t)(fw0.x & 0xFFFF); w[1] = (uint16_t)(fw0.x >> 16);
-        w[2] = (uint16_t)(fw0.y & 0xFFFF); w[3] = (uint16_t)(fw0.y >> 16);
-        S cr[2];
-        cent<S>(C, l, cr[0], cr[1]);
-        const double A = (double)A_own;
-        double qt[V];
+    for (int k = 0; k < NV; ++k) res[k] = 0.;
+    if (uc < nown) {
+        const int c = c0 + uc;
+        double qt[NV];
 #pragma unroll
-        for (int k = 0; k < V; ++k) qt[k] = 0.;
-        bool has_ghost = false;
+        for (int k = 0; k < NV; ++k) qt[k] = 0.;
+        double A = 1.0;
+        if (M::exact || io.partials != nullptr) A = (double)__ldg((const S*)FP.area + c);
+        uint32_t any = 0;
 #pragma unroll
-        for (int f = 0; f < kMaxFaces; ++f) {
-            if (w[f] == kFaceNone) continue;
-            const int el = w[f] & kFaceEdgeMask, side = w[f] >> 15;
-            has_ghost |= (w[f] & 0x4000) != 0;
-            FT fe[V];
-            lds<FT, V>(sF + (size_t)el * V, fe);
-            if constexpr (M::exact) {
-                const double le = sle[el];
+        for (int f = 0; f < NF; ++f) {
+            if (f == 3 && word_nbr(own[f]) == 0xFFFF) continue;
+            any |= own[f];
+            S fe[NV];
+            PL::get(FS, L.lf, word_unit(own[f]), v0, fe);
 #pragma unroll
-                for (int k = 0; k < V; ++k) {
-                    if (!side) qt[k] -= fe[k] * le / A;
-                    else qt[k] += fe[k] * le / A;
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < V; ++k) qt[k] += side ? (double)fe[k] : -(double)fe[k];
-            }
+            for (int k = 0; k < NV; ++k) qt[k] += M::exact ? (double)fe[k] / A : (double)fe[k];
         }
         if constexpr (!M::exact) {
-            const double rA = 1.0 / A;
+            const double rA = __ldg(FP.ria + c);
 #pragma unroll
-            for (int k = 0; k < V; ++k) qt[k] *= rA;
+            for (int k = 0; k < NV; ++k) qt[k] *= rA;
         }
-        if (global_dt) {
-            // min_dt (explicit.cpp:555-564) of this cell's case; a NaN in its dt[0] wins
-            unsigned long long key = s_dtkey;
-            if (tc < 0) {  // a tile across two cases of a batch: this cell's case
-                const int k = P.cell_case[c];
-                key = ~0ull;
-                for (int i = 0; i < kDtSlots; ++i) key = kmin_(key, io.dtkeys[(size_t)k * kDtSlots + i]);
-                d0 = io.dt[P.case_cell0[k]];
-            }
-            dtc = (d0 != d0) ? d0 : tkey_inv(key);
-        }
-        double qnew[V];
-        if constexpr (M::exact) {
-#pragma unroll
-            for (int k = 0; k < V; ++k) qnew[k] = qb[k] + qt[k] * dtc * io.alpha;
-        } else {
-            const double da = dtc * io.alpha;
-#pragma unroll
-            for (int k = 0; k < V; ++k) qnew[k] = fma(qt[k], da, qb[k]);
-        }
-        if (sizeof(S) == 8) {
-            st<double, V>(io.q_out, c, qnew);
-        } else {
-            S qs[V];
-#pragma unroll
-            for (int k = 0; k < V; ++k) qs[k] = (S)qnew[k];
-            st<S, V>((S*)io.s_out, c, qs);
-            if (io.write_f64) st<double, V>(io.q_out, c, qnew);
-        }
-        if constexpr (REMOTE) {
-            // this cell's new state into every part that reads it
-            const RemoteIO& R = *pio.remote;
-            if (c < R.n_band) {
-                S qs[V];
-#pragma unroll
-                for (int k = 0; k < V; ++k) qs[k] = (S)qnew[k];
-                for (int i = R.cell_off[c]; i < R.cell_off[c + 1]; ++i) {
-                    const int2 d = R.cell_dst[i];
-                    st<S, V>((S*)R.dst[d.x], d.y, qs);
+        {
+            if (global_dt) {
+                dtc = s_dt;
+                if (tc < 0) {  // a tile across two cases of a batch: this cell's case
+                    const int k = P.cell_case[c];
+                    unsigned long long key = ~0ull;
+                    for (int i = 0; i < kDtSlots; ++i) key = kmin_(key, io.dtkeys[(size_t)k * kDtSlots + i]);
+                    const double d0 = io.dt[P.case_cell0[k]];
+                    dtc = (d0 != d0) ? d0 : tkey_inv(key);
                 }
             }
-        }
-        if (has_ghost) {
-            S gxs[V], gys[V];
-            PL::get(GX, L.lg, l, gxs);
-            PL::get(GY, L.lg, l, gys);
+            double qb[NV], qnew[NV];
+            ldv<double, NV>(QB + 4 * uc + v0, qb);
+            if constexpr (M::exact) {
 #pragma unroll
-            for (int f = 0; f < kMaxFaces; ++f) {
-                if (w[f] == kFaceNone || !(w[f] & 0x4000)) continue;
-                const int el = w[f] & kFaceEdgeMask, side = w[f] >> 15;
-                const uint32_t ij = sij[el];
-                const int o = side ? (int)(ij & 0xffff) : (int)(ij >> 16);
-                const int g = FP.halo[halo_off + o - T];
-                const S n0 = snx[el], n1v = sny[el];
-                S qint[V], qc[V], b[V];
+                for (int k = 0; k < NV; ++k) qnew[k] = qb[k] + qt[k] * dtc * io.alpha;
+            } else {
+                const double da = dtc * io.alpha;
 #pragma unroll
-                for (int k = 0; k < V; ++k) { qc[k] = (S)qnew[k]; qint[k] = qc[k]; }
-                const S e0 = sxf[el] - cr[0], e1 = syf[el] - cr[1];
-                if constexpr (M::exact) {
-                    S lms[V];
-                    PL::get(LM, L.lg, l, lms);
+                for (int k = 0; k < NV; ++k) qnew[k] = fma(qt[k], da, qb[k]);
+            }
+            S qs[NV];
 #pragma unroll
-                    for (int k = 0; k < V; ++k) qint[k] = qc[k] + (gxs[k] * e0 + gys[k] * e1) * lms[k];
-                } else {
-#pragma unroll
-                    for (int k = 0; k < V; ++k) qint[k] = qc[k] + gxs[k] * e0 + gys[k] * e1;
-                }
-                guard_face<S, V, M::exact>(P, qint, qc);
-                if constexpr (M::exact) exact::bc<V>(P, P.ghost_group[g - N], g - N, b, qint, n0, n1v);
-                else fast::bc<V, S>(P, P.ghost_group[g - N], g - N, b, qint, n0, n1v);
-                if (sizeof(S) == 8) {
-                    st<double, V>(io.q_out, g, (const double*)b);
-                } else {
-                    st<S, V>((S*)io.s_out, g, b);
-                    if (io.write_f64) {
-                        double bd[V];
-#pragma unroll
-                        for (int k = 0; k < V; ++k) bd[k] = (double)b[k];
-                        st<double, V>(io.q_out, g, bd);
+            for (int k = 0; k < NV; ++k) qs[k] = (S)qnew[k];
+            if (sizeof(S) == 8) {
+                stv<double, NV>(io.q_out + 4 * (size_t)c + v0, qnew);
+            } else {
+                stv<S, NV>((S*)io.s_out + 4 * (size_t)c + v0, qs);
+                if (io.write_f64) stv<double, NV>(io.q_out + 4 * (size_t)c + v0, qnew);
+            }
+            if constexpr (REMOTE) {
+                // this cell's new state into every part that reads it
+                const RemoteIO& R = *pio.remote;
+                if (c < R.n_band) {
+                    for (int i = R.cell_off[c]; i < R.cell_off[c + 1]; ++i) {
+                        const int2 d = R.cell_dst[i];
+                        stv<S, NV>((S*)R.dst[d.x] + 4 * (size_t)d.y + v0, qs);
                     }
                 }
-                if constexpr (REMOTE) {
-                    const RemoteIO& R = *pio.remote;
-                    const int go = g - N;
-                    if (go < R.n_own_ghost)
-                        for (int i = R.ghost_off[go]; i < R.ghost_off[go + 1]; ++i) {
-                            const int2 d = R.ghost_dst[i];
-                            st<S, V>((S*)R.dst[d.x], d.y, b);
+            }
+            if (any & kWordGhost) {
+                S gxs[NV], gys[NV], lms[NV];
+                PL::get(GX, L.lt, uc, v0, gxs);
+                PL::get(GY, L.lt, uc, v0, gys);
+                if constexpr (M::exact) PL::get(LM, L.lt, uc, v0, lms);
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    if ((f == 3 && word_nbr(own[f]) == 0xFFFF) || !(own[f] & kWordGhost)) continue;
+                    const int u = word_unit(own[f]), el = u < FP.max_flux ? u : u - FP.max_flux;
+                    const int g = FP.halo[halo_off + word_nbr(own[f]) - T];
+                    const size_t ri = (size_t)NF * slot_off + (size_t)f * G + uc;
+                    const S* ep = (const S*)FP.eg + 4 * (size_t)(flux_off + el);
+                    const S e0 = M::exact ? ((const S*)FP.rec2)[2 * ri] : ((const S*)FP.rec)[4 * ri + 2];
+                    const S e1 = M::exact ? ((const S*)FP.rec2)[2 * ri + 1] : ((const S*)FP.rec)[4 * ri + 3];
+                    S qint[NV], all[V], b[V], bs[NV];
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        if constexpr (M::exact) qint[k] = qs[k] + (gxs[k] * e0 + gys[k] * e1) * lms[k];
+                        else qint[k] = fast::fma_(gys[k], e1, fast::fma_(gxs[k], e0, qs[k]));
+                    }
+                    guard_share<S, NV, M::exact>(P, qint, qs);
+                    share<S, NV>(qint, all);
+                    if constexpr (M::exact) exact::bc<V>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
+                    else fast::bc<V, S>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
+                    own_share<S, NV>(b, v0, bs);
+                    if (sizeof(S) == 8) {
+                        stv<S, NV>((S*)io.q_out + 4 * (size_t)g + v0, bs);
+                    } else {
+                        stv<S, NV>((S*)io.s_out + 4 * (size_t)g + v0, bs);
+                        if (io.write_f64) {
+                            double bd[NV];
+#pragma unroll
+                            for (int k = 0; k < NV; ++k) bd[k] = (double)bs[k];
+                            stv<double, NV>(io.q_out + 4 * (size_t)g + v0, bd);
                         }
+                    }
+                    if constexpr (REMOTE) {
+                        const RemoteIO& R = *pio.remote;
+                        const int go = g - N;
+                        if (go < R.n_own_ghost)
+                            for (int i = R.ghost_off[go]; i < R.ghost_off[go + 1]; ++i) {
+                                const int2 d = R.ghost_dst[i];
+                                stv<S, NV>((S*)R.dst[d.x] + 4 * (size_t)d.y + v0, bs);
+                            }
+                    }
                 }
             }
-        }
-        if (io.partials != nullptr) {
+            if (io.partials != nullptr) {
 #pragma unroll
-            for (int k = 0; k < V; ++k) res[k] = qt[k] * qt[k] * A;
+                for (int k = 0; k < NV; ++k) res[k] = qt[k] * qt[k] * A;
+            }
         }
     }
     if (io.partials != nullptr) {
+        // butterfly over the cells of a warp (lanes of equal variables), then
+        // the warps in order
 #pragma unroll
-        for (int k = 0; k < V; ++k)
+        for (int k = 0; k < NV; ++k)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) res[k] += __shfl_xor_sync(0xffffffffu, res[k], o);
+            for (int o = 16; o >= LP; o >>= 1) res[k] += __shfl_xor_sync(0xffffffffu, res[k], o);
         // the warp sums share the flux store once every thread has read its fluxes
-        double* red = reinterpret_cast<double*>(sF);
+        double* red = reinterpret_cast<double*>(FS);
         __syncthreads();
-        if ((threadIdx.x & 31) == 0)
+        if ((threadIdx.x & 31) < LP)
 #pragma unroll
-            for (int k = 0; k < V; ++k) red[(threadIdx.x >> 5) * V + k] = res[k];
+            for (int k = 0; k < NV; ++k) red[(threadIdx.x >> 5) * V + v0 + k] = res[k];
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < V) {
             const int nw = blockDim.x >> 5;
-            for (int k = 0; k < V; ++k) {
-                double s = 0.;
-                for (int w = 0; w < nw; ++w) s += red[w * V + k];
-                io.partials[(size_t)t * V + k] = s;
-            }
+            double s = 0.;
+            for (int w = 0; w < nw; ++w) s += red[w * V + threadIdx.x];
+            io.partials[(size_t)t * V + threadIdx.x] = s;
         }
     }
     if constexpr (REMOTE) {
@@ -621,31 +792,59 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
     return true;
 }
 
+// Register budget of the one-lane kernel, as CTAs of 256 threads per SM: FP32
+// 64 registers (32 warps per SM), FP64 128 (16 warps).  Measured in us per
+// RK5 step (64 | 48 | 80 registers): forward step 998k cells 328 | 322 | 358,
+// 99k cells (one wave) 57 | 66 | 54; FP64 with 80 registers spills (998k cells
+// 7 % faster, 65k cells 28 % slower).
+template <class M>
+struct FusedBlocks { static constexpr int v = sizeof(typename M::S) == 4 ? 4 : 2; };
+
 // One CTA per tile, tiles [0, grid).
-template <class M, int FLUX>
-__global__ void __launch_bounds__(kTileMax) k_tile_fused(FusedParams FP, TileIO io) {
+template <class M, int FLUX, int NV, int NF>
+__global__ void __launch_bounds__(NV == 4 ? kTileMax : kFusedThreads, NV == 4 ? FusedBlocks<M>::v : 1)
+    k_tile_fused(FusedParams FP, TileIO io) {
     pdl_trigger();
-    fused_tile<M, FLUX, false, false>(FP, io, (int)blockIdx.x, PartIO{});
+    fused_tile<M, FLUX, NV, NF, 0, false, false>(FP, io, (int)blockIdx.x, PartIO{});
+}
+
+// The split layout of the fast policies, over the same tiles with the same
+// arithmetic: gradients, then the rest of the stage; and the time step (the
+// first kernel of a step).
+template <class M, int NF>
+__global__ void __launch_bounds__(kTileMax) k_tile_fused_grad(FusedParams FP, TileIO io) {
+    pdl_trigger();
+    fused_tile<M, 1, 4, NF, 1, false, false>(FP, io, (int)blockIdx.x, PartIO{});
+}
+template <class M, int NF>
+__global__ void __launch_bounds__(kTileMax) k_tile_fused_flux(FusedParams FP, TileIO io) {
+    pdl_trigger();
+    fused_tile<M, 1, 4, NF, 2, false, false>(FP, io, (int)blockIdx.x, PartIO{});
+}
+
+template <class M, int NF>
+__global__ void __launch_bounds__(kTileMax) k_tile_fused_dt(FusedParams FP, TileIO io) {
+    pdl_trigger();
+    fused_tile<M, 1, 4, NF, 3, false, true>(FP, io, (int)blockIdx.x, PartIO{});
+    // the step's first kernel: the work-list tile counters of its stage
+    // kernels start at zero (every kernel that used them has completed)
+    if (io.work_reset != nullptr && blockIdx.x == 0 && threadIdx.x < kWorkSlots) io.work_reset[threadIdx.x] = 0;
 }
 
 // A decomposition part's launches, one CTA per tile.  MODE 1: tiles
 // [pio.t0, pio.t0 + grid) (the band and interior launches); MODE 2: the halo
-// exchange inside the launch (pio.remote).  Kept apart from k_tile_fused,
-// whose register allocation the tile offset and the owned count from the
-// tile info upset (FP32: 80 registers instead of 64, 5.7 % slower); a
-// register cap on these launches restores 64 registers but runs slower
-// still, so they keep the compiler's choice.
-template <class M, int FLUX, int MODE>
+// exchange inside the launch (pio.remote).
+template <class M, int FLUX, int NF, int MODE>
 __global__ void __launch_bounds__(kTileMax) k_tile_fused_part(FusedParams FP, TileIO io, PartIO pio) {
     pdl_trigger();
-    fused_tile<M, FLUX, MODE == 2, true>(FP, io, (MODE == 1 ? pio.t0 : 0) + (int)blockIdx.x, pio);
+    fused_tile<M, FLUX, 4, NF, 0, MODE == 2, true>(FP, io, (MODE == 1 ? pio.t0 : 0) + (int)blockIdx.x, pio);
 }
 
 // Work-list schedule: as many CTAs as fit on the device at once, each taking
 // the next tile from the launch's counter (reset by the step's dt kernel)
 // until none is left, so no CTA waits at a tail of unevenly sized tiles.
 // The counter is read only after the dependency wait.
-template <class M, int FLUX>
+template <class M, int FLUX, int NF>
 __global__ void __launch_bounds__(kTileMax) k_tile_fused_work(FusedParams FP, TileIO io, int n_tiles) {
     pdl_trigger();
     pdl_wait();
@@ -655,25 +854,24 @@ __global__ void __launch_bounds__(kTileMax) k_tile_fused_work(FusedParams FP, Ti
         __syncthreads();
         const int t = s_t;
         if (t >= n_tiles) return;
-        if (!fused_tile<M, FLUX, false, true>(FP, io, t, PartIO{})) return;
+        if (!fused_tile<M, FLUX, 4, NF, 0, false, true>(FP, io, t, PartIO{})) return;
         __syncthreads();  // every thread is done with this tile's shared memory (and s_t)
     }
 }
 
 template <class M>
 struct FusedLaunch {
-    static size_t smem(const FusedParams& FP) {
-        return fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_edges, FP.max_flux, FP.T).total;
+    // lays out the tiles' shared memory (FP.L); the bytes of the largest launch
+    static size_t smem(FusedParams& FP) {
+        FP.L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_flux, FP.T);
+        return (size_t)(M::exact ? FP.L.total : std::max(FP.L.total, FP.L.total_grad));
     }
-    static cudaError_t prepare(const FusedParams& FP) {
+    static cudaError_t prepare(FusedParams& FP) {
         static std::mutex mu;
         std::lock_guard<std::mutex> lock(mu);
         cudaError_t e = cudaSuccess;
         const size_t bytes = smem(FP);
-        for (const void* fn : {(const void*)k_tile_fused<M, 1>, (const void*)k_tile_fused<M, 2>,
-                               (const void*)k_tile_fused_part<M, 1, 1>, (const void*)k_tile_fused_part<M, 2, 1>,
-                               (const void*)k_tile_fused_part<M, 1, 2>, (const void*)k_tile_fused_part<M, 2, 2>,
-                               (const void*)k_tile_fused_work<M, 1>, (const void*)k_tile_fused_work<M, 2>}) {
+        auto set = [&](const void* fn) {
             // only ever raised: a solver created earlier may launch with more
             cudaFuncAttributes fa{};
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
@@ -682,25 +880,44 @@ struct FusedLaunch {
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
+        };
+        auto all = [&](auto f, auto n) {
+            constexpr int F = decltype(f)::value, NF = decltype(n)::value;
+            for (const void* fn :
+                 {(const void*)k_tile_fused<M, F, 4, NF>, (const void*)k_tile_fused<M, F, 2, NF>,
+                  (const void*)k_tile_fused<M, F, 1, NF>, (const void*)k_tile_fused_part<M, F, NF, 1>,
+                  (const void*)k_tile_fused_part<M, F, NF, 2>, (const void*)k_tile_fused_work<M, F, NF>})
+                set(fn);
+            if constexpr (!M::exact)
+                for (const void* fn : {(const void*)k_tile_fused_grad<M, NF>, (const void*)k_tile_fused_flux<M, NF>, (const void*)k_tile_fused_dt<M, NF>})
+                    set(fn);
+        };
+        using One = std::integral_constant<int, 1>;
+        using Three = std::integral_constant<int, 3>;
+        using Four = std::integral_constant<int, 4>;
+        if (FP.nf == 3) all(One{}, Three{});
+        else all(One{}, Four{});
+        if constexpr (M::exact) {
+            using Two = std::integral_constant<int, 2>;
+            if (FP.nf == 3) all(Two{}, Three{});
+            else all(Two{}, Four{});
         }
         return e;
     }
     // CTAs of the work-list schedule: the device's resident capacity
-    static int work_grid(const FusedParams& FP, int n_tiles) {
+    static int work_grid(FusedParams& FP, int n_tiles) {
         int dev = 0, sms = 0, nb = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tile_fused_work<M, 1>, FP.threads, smem(FP));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &nb, FP.nf == 3 ? k_tile_fused_work<M, 1, 3> : k_tile_fused_work<M, 1, 4>, FP.T, smem(FP));
         return std::max(1, std::min(n_tiles, sms * std::max(nb, 1)));
     }
-    // io.work != nullptr: the work-list schedule on `grid` CTAs
-    // part: a decomposition part's launch (its tile offset, in-launch exchange)
-    static void stage(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int grid,
-                      const PartIO* part = nullptr) {
-        const size_t sm = smem(FP);
+    template <class... A, class... B>
+    static void go(void (*k)(A...), int grid, int threads, size_t sm, cudaStream_t st, bool pdl, const B&... args) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(io.work ? grid : n_tiles));
-        cfg.blockDim = dim3((unsigned)FP.threads);
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)threads);
         cfg.dynamicSmemBytes = sm;
         cfg.stream = st;
         cudaLaunchAttribute at[1];
@@ -708,28 +925,60 @@ struct FusedLaunch {
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
         cfg.numAttrs = pdl ? 1 : 0;
-        if (io.work) {
-            if (FP.P.flux == 1) cudaLaunchKernelEx(&cfg, k_tile_fused_work<M, 1>, FP, io, n_tiles);
-            else cudaLaunchKernelEx(&cfg, k_tile_fused_work<M, 2>, FP, io, n_tiles);
-        } else if (part && part->remote) {
-            if (FP.P.flux == 1) cudaLaunchKernelEx(&cfg, k_tile_fused_part<M, 1, 2>, FP, io, *part);
-            else cudaLaunchKernelEx(&cfg, k_tile_fused_part<M, 2, 2>, FP, io, *part);
-        } else if (part) {
-            if (FP.P.flux == 1) cudaLaunchKernelEx(&cfg, k_tile_fused_part<M, 1, 1>, FP, io, *part);
-            else cudaLaunchKernelEx(&cfg, k_tile_fused_part<M, 2, 1>, FP, io, *part);
-        } else {
-            if (FP.P.flux == 1) cudaLaunchKernelEx(&cfg, k_tile_fused<M, 1>, FP, io);
-            else cudaLaunchKernelEx(&cfg, k_tile_fused<M, 2>, FP, io);
+        cudaLaunchKernelEx(&cfg, k, args...);
+    }
+    template <int F, int NF>
+    static void stage_f(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int grid,
+                        const PartIO* part) {
+        const size_t sm = (size_t)FP.L.total;
+        const int tp = FP.lanes == 1 ? FP.threads : FP.T;  // a part's launch: one lane per cell
+        if (io.work) go(k_tile_fused_work<M, F, NF>, grid, FP.T, sm, st, pdl, FP, io, n_tiles);
+        else if (part && part->remote) go(k_tile_fused_part<M, F, NF, 2>, n_tiles, tp, sm, st, pdl, FP, io, *part);
+        else if (part) go(k_tile_fused_part<M, F, NF, 1>, n_tiles, tp, sm, st, pdl, FP, io, *part);
+        else if (FP.lanes == 4) go(k_tile_fused<M, F, 1, NF>, n_tiles, FP.threads, sm, st, pdl, FP, io);
+        else if (FP.lanes == 2) go(k_tile_fused<M, F, 2, NF>, n_tiles, FP.threads, sm, st, pdl, FP, io);
+        else go(k_tile_fused<M, F, 4, NF>, n_tiles, FP.threads, sm, st, pdl, FP, io);
+    }
+    // io.work != nullptr: the work-list schedule on `grid` CTAs
+    // part: a decomposition part's launch (its tile offset, in-launch exchange)
+    static void stage(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int grid,
+                      const PartIO* part = nullptr) {
+        if constexpr (M::exact) {
+            if (FP.P.flux == 2) {
+                if (FP.nf == 3) stage_f<2, 3>(FP, io, st, pdl, n_tiles, grid, part);
+                else stage_f<2, 4>(FP, io, st, pdl, n_tiles, grid, part);
+                return;
+            }
+        }
+        if (FP.nf == 3) stage_f<1, 3>(FP, io, st, pdl, n_tiles, grid, part);
+        else stage_f<1, 4>(FP, io, st, pdl, n_tiles, grid, part);
+    }
+    // fast policies, one lane per cell: the split layout's two kernels
+    // (phase 1: gradients; phase 2: the rest) and the time step (phase 3)
+    template <int NF>
+    static void split_f(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase) {
+        const FusedSmem& L = FP.L;
+        if (phase == 3) go(k_tile_fused_dt<M, NF>, n_tiles, FP.T, L.total_grad, st, pdl, FP, io);
+        else if (phase == 2) go(k_tile_fused_flux<M, NF>, n_tiles, FP.T, L.total, st, pdl, FP, io);
+        else go(k_tile_fused_grad<M, NF>, n_tiles, FP.T, L.total_grad, st, pdl, FP, io);
+    }
+    static void split(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase) {
+        if constexpr (!M::exact) {
+            if (FP.nf == 3) split_f<3>(FP, io, st, pdl, n_tiles, phase);
+            else split_f<4>(FP, io, st, pdl, n_tiles, phase);
         }
     }
 };
 
 namespace tile {
-cudaError_t prepare_fused(int precision, const FusedParams& FP);
-size_t smem_fused(int precision, const FusedParams& FP);
-int work_grid_fused(int precision, const FusedParams& FP, int n_tiles);
+cudaError_t prepare_fused(int precision, FusedParams& FP);
+size_t smem_fused(int precision, FusedParams& FP);
+int work_grid_fused(int precision, FusedParams& FP, int n_tiles);
 void launch_fused(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
                   int grid, const PartIO* part = nullptr);
+// the fast policies' split kernels over the fused kernel's tiles (FusedLaunch::split)
+void launch_fused_split(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
+                        int phase);
 }  // namespace tile
 
 }  // namespace fvgpu

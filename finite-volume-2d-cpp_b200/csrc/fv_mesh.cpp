@@ -514,6 +514,95 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int T, Tile2Arrays& t
     }
 }
 
+template <class S>
+void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
+                 double K, FusedArrays<S>& out) {
+    const int T = t2.tile_cells, F = HostMesh::MAXF;
+    const int64_t N = m.n_real, NO = m.owned_real();
+    out = FusedArrays<S>();
+    for (int64_t c = 0; c < N && out.nf < F; ++c) out.nf = std::max<int>(out.nf, m.n_faces[c]);
+    const int nf = out.nf;
+    out.info.assign((size_t)t2.n_tiles * 8, 0);
+    int64_t slots = 0, edges = 0;
+    for (int t = 0; t < t2.n_tiles; ++t) {
+        const int32_t* in = &t2.info[(size_t)8 * t];
+        int32_t* inf = &out.info[(size_t)8 * t];
+        inf[0] = (int32_t)slots; inf[1] = in[3]; inf[2] = (int32_t)edges; inf[3] = in[2];
+        inf[4] = in[4]; inf[5] = in[5]; inf[6] = in[7];
+        slots += T + in[4];
+        edges += in[2];
+    }
+    out.hd.assign((size_t)slots * 4, 0x8000FFFFu);
+    const bool packed = nf == 3 && sizeof(S) == 4;  // the fourth word holds sl
+    out.rec.assign((size_t)nf * slots * 4, S(0));
+    if (exact) out.rec2.assign((size_t)nf * slots * 2, S(0));
+    out.sl.assign((size_t)slots * (exact ? 2 : 1), S(0));
+    out.eg.assign((size_t)edges * 4, S(0));
+    out.ria.resize((size_t)NO);
+    for (int64_t c = 0; c < NO; ++c) out.ria[(size_t)c] = 1.0 / (double)(S)fa.area[(size_t)c];
+    auto tiles = [&](int t0, int t1) {
+        for (int t = t0; t < t1; ++t) {
+            const int32_t* in = &t2.info[(size_t)8 * t];
+            const int32_t* inf = &out.info[(size_t)8 * t];
+            const int64_t c0 = (int64_t)t * T;
+            const int eoff = in[0], n_flux = in[2], n1 = in[4], own = in[7], G = T + n1;
+            const int64_t so = inf[0];
+            auto dev = [&](int slot) { return slot < T ? (int32_t)(c0 + slot) : t2.halo[(size_t)in[3] + slot - T]; };
+            for (int r = 0; r < G; ++r) {
+                if (r < T && r >= own) continue;
+                const int32_t c = dev(r);
+                const double A = fa.area[(size_t)c], Ka = K * std::sqrt(A), K3a = Ka * Ka * Ka;
+                if (exact) { out.sl[(size_t)(so + r) * 2] = (S)(1. / A); out.sl[(size_t)(so + r) * 2 + 1] = (S)K3a; }
+                else out.sl[(size_t)(so + r)] = (S)(1. / K3a);
+                if (packed) std::memcpy(&out.hd[(size_t)(so + r) * 4 + 3], &out.sl[(size_t)(so + r)], 4);
+                for (int f = 0; f < F; ++f) {
+                    const uint16_t w = t2.face[((size_t)in[6] + r) * 4 + f];
+                    if (w == 0xFFFF) continue;
+                    const int el = w & 0x3FFF, side = w >> 15;
+                    const size_t e = (size_t)eoff + el;
+                    const uint32_t ij = t2.edge_ij[e];
+                    uint32_t word = side ? (ij & 0xFFFF) : (ij >> 16);
+                    if (el < n_flux) word |= (uint32_t)(el + side * t2.max_flux) << 16 | (uint32_t)(w & 0x4000) << 16;
+                    else word |= 0x80000000u;
+                    out.hd[(size_t)(so + r) * 4 + f] = word;
+                    const size_t b = (size_t)nf * so + (size_t)f * G + r;
+                    const double dx = t2.exf[e] - ta.ccx[(size_t)c], dy = t2.eyf[e] - ta.ccy[(size_t)c];
+                    S* v = &out.rec[b * 4];
+                    if (exact) {
+                        v[0] = (S)t2.enx[e]; v[1] = (S)t2.eny[e];
+                        v[2] = (S)(side ? -t2.ele[e] : t2.ele[e]); v[3] = (S)t2.eg[e];
+                        out.rec2[b * 2] = (S)dx; out.rec2[b * 2 + 1] = (S)dy;
+                    } else {
+                        const double a = (side ? -(1.0 - t2.eg[e]) : t2.eg[e]) * t2.ele[e] / A;
+                        v[0] = (S)(a * t2.enx[e]); v[1] = (S)(a * t2.eny[e]);
+                        v[2] = (S)dx; v[3] = (S)dy;
+                    }
+                }
+            }
+            for (int e = 0; e < n_flux; ++e) {
+                S* v = &out.eg[(size_t)(inf[2] + e) * 4];
+                const size_t g = (size_t)eoff + e;
+                v[0] = (S)t2.enx[g]; v[1] = (S)t2.eny[g]; v[2] = (S)t2.ele[g];
+                // a boundary ghost's zero gradient adds this signed zero to its face state
+                const int32_t j = dev((int)(t2.edge_ij[g] >> 16));
+                if (j >= N)
+                    v[3] = (S)((0.0 * (t2.exf[g] - ta.ccx[(size_t)j]) + 0.0 * (t2.eyf[g] - ta.ccy[(size_t)j])) * 1.0);
+            }
+        }
+    };
+    const int nt = (int)std::min<int64_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency())),
+                                          1 + t2.n_tiles / 256);
+    std::vector<std::thread> pool;
+    for (int k = 1; k < nt; ++k)
+        pool.emplace_back(tiles, (int)((int64_t)t2.n_tiles * k / nt), (int)((int64_t)t2.n_tiles * (k + 1) / nt));
+    tiles(0, t2.n_tiles / nt);
+    for (auto& th : pool) th.join();
+}
+template void build_fused<float>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, double,
+                                 FusedArrays<float>&);
+template void build_fused<double>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, double,
+                                  FusedArrays<double>&);
+
 // ----------------------------------------------------------------------------
 // Domain decomposition.  The reference decomposes with gmsh partitions and
 // exchanges q, gx, gy, limiters and dt of one ring of ghost elements per

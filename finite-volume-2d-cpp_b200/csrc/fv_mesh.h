@@ -105,6 +105,27 @@ struct Tile2Arrays {
 };
 void build_tiles2(const HostMesh& m, const FaceArrays& fa, int tile_cells, Tile2Arrays& ta);
 
+// The fused stage kernel's view of two-ring tiles (fv_fused.cuh): per gradient
+// slot (T + n1 of each tile) face words and one record per
+// face, in the order its threads read them; per flux edge its geometry.  S:
+// the stage precision.  exact: the reference's operands (normal, length with
+// the side in its sign, Green-Gauss weight, face centre - centroid; 1 / A and
+// (K sqrt(A))^3 per slot); otherwise the cell's Green-Gauss coefficients
+// a = w le n / A (outward normal, the neighbour's weight) and face centre -
+// centroid, evaluated in FP64 and rounded once, with 1 / (K sqrt(A))^3 per slot.
+template <class S>
+struct FusedArrays {
+    int nf = 3;                          // faces per slot in rec: 3, or 4 with quadrilaterals
+    std::vector<int32_t> info;           // [n_tiles][8]: slot_off, halo_off, flux_off, n_flux, n1, n2, owned cells, 0
+    std::vector<uint32_t> hd;            // [slots][4] face words (fv_fused.cuh)
+    std::vector<S> rec, rec2, sl;        // [nf * slots][4], exact [nf * slots][2], [slots] (exact [slots][2])
+    std::vector<S> eg;                   // [flux edges][4]
+    std::vector<double> ria;             // [owned cells] 1 / area as the stage precision holds it
+};
+template <class S>
+void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
+                 double K, FusedArrays<S>& out);
+
 // One part of a decomposition of a single mesh into n_parts parts.  Part p
 // owns device real cells [own_off[p], own_off[p+1]) (contiguous ranges of the
 // Hilbert order) and the boundary ghosts of those cells; its local mesh adds

@@ -31,6 +31,38 @@ template <> __device__ __forceinline__ float div_<float>(float a, float b) { ret
 template <class T> __device__ __forceinline__ T tmin(T a, T b) { return (b < a) ? b : a; }
 template <class T> __device__ __forceinline__ T tmax(T a, T b) { return (a < b) ? b : a; }
 
+// Explicit fused multiply-add: one rounding wherever the expression is inlined,
+// so that kernels that share it give the same bits.
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+// minimum and maximum of finite values (one instruction in FP32)
+__device__ __forceinline__ float vmin(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float vmax(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double vmin(double a, double b) { return (b < a) ? b : a; }
+__device__ __forceinline__ double vmax(double a, double b) { return (a < b) ? b : a; }
+
+// Smooth switch of the limiter (explicit.cpp:220-233): 1 up to d^2 = (K h)^3,
+// 0 from twice that on; d = max - min over the stencil, rk3 = 1 / (K h)^3.
+__device__ __forceinline__ float smooth_switch(float d, float rk3) {
+    const float y = __saturatef(__fmaf_rn(d * d, rk3, -1.f));
+    return __fmaf_rn(__fmaf_rn(2.f, y, -3.f), y * y, 1.f);
+}
+__device__ __forceinline__ double smooth_switch(double d, double rk3) {
+    double y = __fma_rn(d * d, rk3, -1.0);
+    y = y > 0.0 ? (y < 1.0 ? y : 1.0) : 0.0;
+    return __fma_rn(__fma_rn(2.0, y, -3.0), y * y, 1.0);
+}
+
+// {u, v, c} of a state
+template <class T>
+__device__ __forceinline__ void speeds(T gamma, const T* q, T* w) {
+    const T ri = rcp(q[0]);
+    w[0] = q[1] * ri;
+    w[1] = q[2] * ri;
+    w[2] = sqrt_(gamma * (gamma - T(1)) * fma_(q[3], ri, T(-0.5) * fma_(w[0], w[0], w[1] * w[1])));
+    w[3] = T(0);
+}
+
 // Roe flux with the "cures" eigenvalues (examples/forwardStep/main.cpp:72-135).
 template <class T>
 __device__ __forceinline__ void roe(T gamma, T* f, const T* qi, const T* qj, T n0, T n1) {
@@ -150,6 +182,22 @@ template <class T>
 __device__ __forceinline__ T limiter_ratio(int kind, T num, T den) {
     if (kind == 2) return num * (num + T(2) * den) * rcp(num * (num + den) + T(2) * den * den);
     return limiter_func(kind, div_(num, den));
+}
+
+// Limiter of one variable of a cell: the minimum over the faces of
+// sig + (1 - sig) phi(delta / dq), delta = mx for dq > 0 and mn for dq < 0
+// (explicit.cpp:234-253).  Every phi here grows up to phi >= 1 and stays
+// there, and the minimum starts at 1, so the strictest face of each sign is
+// the one of largest |dq| (up, lo), and the smaller of the two ratios (by
+// cross-multiplication) decides: one phi per variable instead of one per face.
+template <class T>
+__device__ __forceinline__ T limiter_min(int kind, T sig, T mx, T mn, T up, T lo) {
+    const T tol = T(1e-15);
+    const bool pu = up > tol, pl = lo < -tol;
+    const bool use_up = pu && (!pl || mx * lo > mn * up);
+    const T num = use_up ? mx : mn, den = use_up ? up : lo;
+    if (!pu && !pl) return T(1);
+    return vmin(T(1), fma_(T(1) - sig, limiter_ratio(kind, num, den), sig));
 }
 
 // Boundary conditions (see fv_physics_exact.cuh for the references).

@@ -39,6 +39,8 @@ struct fv_solver {
     TileParams TP{};
     // the fused stage kernel over two-ring tiles (its Params are TP.P at launch)
     bool fused = false;
+    // the two-ring tiles exist (the fast modes' split layout runs over them too)
+    bool two_ring = false;
     // with fused: the first stage of each step runs the split kernels, whose
     // gradient kernel also computes dt (no separate dt kernel)
     bool split_first = false;
@@ -124,7 +126,7 @@ struct EventLog {
 struct StepCursor {
     TileIO io{};
     FusedParams FPl{};
-    bool grads = false, worklist = false, split_first = false;
+    bool grads = false, worklist = false, split_first = false, fast2 = false, dt2 = false;
     int b = 0;
     const void* in = nullptr;
     void* out = nullptr;

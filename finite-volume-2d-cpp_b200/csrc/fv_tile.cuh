@@ -209,18 +209,20 @@ struct Rec {
 // exact mode evaluates p as the oracle does; the fast modes test the same
 // sign without a division: for rho > 0 and gamma > 1,
 // p > 0  <=>  2 rho E - (m_x^2 + m_y^2) > 0.
+template <class S, bool EXACT>
+__device__ __forceinline__ bool face_state_bad(const Params& P, const S* qf) {
+    if constexpr (EXACT) {
+        const S p = ((S)P.gamma - S(1)) * (qf[3] - S(0.5) / qf[0] * (qf[1] * qf[1] + qf[2] * qf[2]));
+        return !(qf[0] > S(0)) || !(p > S(0));
+    } else {
+        const S m2 = fast::fma_(qf[2], qf[2], qf[1] * qf[1]);
+        return !(qf[0] > S(0)) || !(fast::fma_(S(2) * qf[0], qf[3], -m2) > S(0));
+    }
+}
 template <class S, int V, bool EXACT = true>
 __device__ __forceinline__ void guard_face(const Params& P, S* qf, const S* qc) {
     if (V != 4 || !P.positivity_guard) return;
-    bool bad;
-    if constexpr (EXACT) {
-        const S p = ((S)P.gamma - S(1)) * (qf[3] - S(0.5) / qf[0] * (qf[1] * qf[1] + qf[2] * qf[2]));
-        bad = !(qf[0] > S(0)) || !(p > S(0));
-    } else {
-        const S m2 = qf[1] * qf[1] + qf[2] * qf[2];
-        bad = !(qf[0] > S(0)) || !(S(2) * qf[0] * qf[3] - m2 > S(0));
-    }
-    if (bad) {
+    if (face_state_bad<S, EXACT>(P, qf)) {
 #pragma unroll
         for (int k = 0; k < V; ++k) qf[k] = qc[k];
     }
@@ -570,11 +572,9 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
 // min_dt's global minimum (explicit.cpp:555-564): a block minimum, then one
 // atomic per block spread over kDtSlots slots of the tile's case.  Every
 // thread of the block calls it.
-__device__ __forceinline__ void tile_dt_reduce(const TileParams& TP, const TileIO& io, int t, int l, int nown,
+__device__ __forceinline__ void tile_dt_reduce(const Params& P, int T, const TileIO& io, int t, int l, int nown,
                                                unsigned long long kmin) {
     __shared__ unsigned long long wmin[kTileMax / 32];
-    const Params& P = TP.P;
-    const int T = TP.T;
     if (P.global_dt && io.dtkeys != nullptr) {
         const int tc = P.n_cases > 1 ? P.tile_case[t] : 0;
         if (tc >= 0) {
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(kTileMax) k_tile_dt(TileParams TP, TileIO io) 
     __syncthreads();
     unsigned long long kmin = ~0ull;
     if (l < nown) kmin = tile_cell_dt<M, V, R::NR, VISC>(TP, io, inf, l, c0 + l, w, rec, sij, snx, sny, sle);
-    if (P.global_dt && io.dtkeys != nullptr) tile_dt_reduce(TP, io, t, l, nown, kmin);
+    if (P.global_dt && io.dtkeys != nullptr) tile_dt_reduce(P, T, io, t, l, nown, kmin);
 }
 
 // ------------------------------------------------ K1: gradients + limiters --
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(kTileMax) k_tile_gradlim(TileParams TP, TileIO
     if constexpr (DT != 0) {
         unsigned long long kmin = ~0ull;
         if (l < nown) kmin = tile_cell_dt<M, V, R::NR, DT == 2>(TP, io, inf, l, c, w, rec, sij, snx, sny, sle);
-        if (P.global_dt && io.dtkeys != nullptr) tile_dt_reduce(TP, io, t, l, nown, kmin);
+        if (P.global_dt && io.dtkeys != nullptr) tile_dt_reduce(P, T, io, t, l, nown, kmin);
     }
     if (l >= nown) return;
     const S* rs = rec + (size_t)l * R::NR;

@@ -15,9 +15,9 @@ void launch_gradlim_exact(const TileParams& TP, const TileIO& io, cudaStream_t s
 void launch_stage_exact(const TileParams& TP, const TileIO& io, cudaStream_t st, bool pdl, int phase) {
     TileLaunch<MExact>::stage(TP, io, st, pdl, phase);
 }
-cudaError_t prepare_fused_exact(const FusedParams& FP) { return FusedLaunch<MExact>::prepare(FP); }
-size_t smem_fused_exact(const FusedParams& FP) { return FusedLaunch<MExact>::smem(FP); }
-int work_grid_fused_exact(const FusedParams& FP, int n_tiles) { return FusedLaunch<MExact>::work_grid(FP, n_tiles); }
+cudaError_t prepare_fused_exact(FusedParams& FP) { return FusedLaunch<MExact>::prepare(FP); }
+size_t smem_fused_exact(FusedParams& FP) { return FusedLaunch<MExact>::smem(FP); }
+int work_grid_fused_exact(FusedParams& FP, int n_tiles) { return FusedLaunch<MExact>::work_grid(FP, n_tiles); }
 void launch_fused_exact(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int grid,
                         const PartIO* part) {
     FusedLaunch<MExact>::stage(FP, io, st, pdl, n_tiles, grid, part);

@@ -9,9 +9,9 @@ cudaError_t prepare_exact(const TileParams& TP);
 void launch_dt_exact(const TileParams& TP, const TileIO& io, cudaStream_t st, bool pdl);
 void launch_gradlim_exact(const TileParams& TP, const TileIO& io, cudaStream_t st, bool with_dt, bool pdl);
 void launch_stage_exact(const TileParams& TP, const TileIO& io, cudaStream_t st, bool pdl, int phase);
-cudaError_t prepare_fused_exact(const FusedParams& FP);
-size_t smem_fused_exact(const FusedParams& FP);
-int work_grid_fused_exact(const FusedParams& FP, int n_tiles);
+cudaError_t prepare_fused_exact(FusedParams& FP);
+size_t smem_fused_exact(FusedParams& FP);
+int work_grid_fused_exact(FusedParams& FP, int n_tiles);
 void launch_fused_exact(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int grid,
                         const PartIO* part);
 
@@ -35,17 +35,17 @@ void launch_stage(int precision, const TileParams& TP, const TileIO& io, cudaStr
     else if (precision == 1) TileLaunch<MF64>::stage(TP, io, st, pdl, phase);
     else TileLaunch<MF32>::stage(TP, io, st, pdl, phase);
 }
-cudaError_t prepare_fused(int precision, const FusedParams& FP) {
+cudaError_t prepare_fused(int precision, FusedParams& FP) {
     if (precision == 0) return prepare_fused_exact(FP);
     if (precision == 1) return FusedLaunch<MF64>::prepare(FP);
     return FusedLaunch<MF32>::prepare(FP);
 }
-size_t smem_fused(int precision, const FusedParams& FP) {
+size_t smem_fused(int precision, FusedParams& FP) {
     if (precision == 0) return smem_fused_exact(FP);
     if (precision == 1) return FusedLaunch<MF64>::smem(FP);
     return FusedLaunch<MF32>::smem(FP);
 }
-int work_grid_fused(int precision, const FusedParams& FP, int n_tiles) {
+int work_grid_fused(int precision, FusedParams& FP, int n_tiles) {
     if (precision == 0) return work_grid_fused_exact(FP, n_tiles);
     if (precision == 1) return FusedLaunch<MF64>::work_grid(FP, n_tiles);
     return FusedLaunch<MF32>::work_grid(FP, n_tiles);
@@ -55,6 +55,11 @@ void launch_fused(int precision, const FusedParams& FP, const TileIO& io, cudaSt
     if (precision == 0) launch_fused_exact(FP, io, st, pdl, n_tiles, grid, part);
     else if (precision == 1) FusedLaunch<MF64>::stage(FP, io, st, pdl, n_tiles, grid, part);
     else FusedLaunch<MF32>::stage(FP, io, st, pdl, n_tiles, grid, part);
+}
+void launch_fused_split(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
+                        int phase) {
+    if (precision == 1) FusedLaunch<MF64>::split(FP, io, st, pdl, n_tiles, phase);
+    else if (precision == 2) FusedLaunch<MF32>::split(FP, io, st, pdl, n_tiles, phase);
 }
 }  // namespace tile
 }  // namespace fvgpu

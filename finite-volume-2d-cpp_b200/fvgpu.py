@@ -261,8 +261,9 @@ class Solver:
                  tile_cells: int = 0, stage_kernels: str = "auto", schedule: str = "tile"):
         """stage_kernels: "auto" ("hybrid" where the physics allow the fused
         stage kernel, else "split"), "split" (gradient and flux kernels),
-        "fused", or "hybrid" (split first stage with the time step folded into
-        its gradient kernel, fused others); schedule of
+        "fused", or "hybrid" (FP64_EXACT: split first stage with the time step
+        folded into its gradient kernel, fused others; FP64 and FP32: the
+        launches of "fused"); schedule of
         the fused kernel: "tile" (one CTA per tile), "worklist" or "tile2"
         (one CTA of two threads per cell per tile)."""
         self.mesh = mesh
@@ -323,8 +324,8 @@ class Solver:
 
     @property
     def stage_kernels(self):
-        """"fused", "split" or "hybrid" (split first stage, fused others): the
-        stage kernels this solver runs."""
+        """"fused", "split" or "hybrid" (FP64_EXACT: split first stage, fused
+        others): the stage kernels this solver runs."""
         return {3: "hybrid", 2: "fused", 1: "split"}[lib().fv_solver_stage_kernels(self._h)]
 
     @property

@@ -232,10 +232,12 @@ typedef struct {
      * FV_STAGE_FUSED (2): one fused kernel per RK stage (gradients, limiter,
      *   fluxes, update, ghost fill) over two-ring tiles, plus one time-step
      *   kernel per step; FV_ERR_UNSUPPORTED when the physics do not allow it.
-     * FV_STAGE_HYBRID (3): the split kernels for the first stage of each step
-     *   (whose gradient kernel also computes dt, so the step has no separate
-     *   time-step kernel) and the fused kernel for the others; not with the
-     *   work-list schedule.  All four give the same results (bit for bit in
+     * FV_STAGE_HYBRID (3): in FP64_EXACT the split kernels for the first stage
+     *   of each step (whose gradient kernel also computes dt, so the step has
+     *   no separate time-step kernel) and the fused kernel for the others; in
+     *   FP64 and FP32, where the time-step kernel and a fused first stage cost
+     *   less, the launches of FV_STAGE_FUSED.  Not with the work-list
+     *   schedule.  All four give the same results (bit for bit in
      *   FP64_EXACT). */
     int32_t stage_kernels;
     /* Schedule of the fused stage kernel: FV_SCHED_TILE (0) one CTA of one
