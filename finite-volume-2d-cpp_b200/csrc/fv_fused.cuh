@@ -49,7 +49,6 @@ namespace fvgpu {
 //    (exact: the area);
 //  - the limited gradients (and, exact, the limiters) of owned cells with a
 //    boundary ghost, for the ghost fill.
-constexpr int kFusedThreads = 512;  // threads per CTA at most
 struct FusedSmem {
     int q, fs, qb, gx, gy, lm, eg, ria, total, total_grad;
     int ls, lf, lt;  // plane strides (units)
@@ -63,8 +62,8 @@ inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int T) {
     L.lt = T;
     int o = 0;
     L.q = o; o += 16 * NU * max_slots;
-    const int f = 32 * NU * max_flux, red = (kFusedThreads / 32) * 4 * (int)sizeof(double);
-    L.fs = o; o += f > red ? f : red;
+    // the face states, the time step's {u, v, c} or the residual warp sums
+    L.fs = o; o += std::max({32 * NU * max_flux, 16 * NU * max_grad, (kFusedThreads / 32) * 4 * (int)sizeof(double)});
     L.qb = o; o += 32 * T;
     L.gx = o; o += 16 * NU * T;
     L.gy = o; o += 16 * NU * T;
@@ -73,7 +72,7 @@ inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int T) {
     L.ria = o; o += 8 * T;
     L.total = o;
     // the gradient kernel of the split layout and the dt kernel: the states
-    // and, in the flux store's place, {u, v, c} of the gradient slots
+    // and {u, v, c} of the gradient slots
     L.total_grad = L.fs + 16 * NU * max_grad;
     return L;
 }
@@ -100,7 +99,10 @@ struct FusedParams {
     const void* rec;
     const void* rec2;
     const void* sl;            // per gradient slot: fast S 1 / (K sqrt(A))^3; exact double2 {1 / A, (K sqrt(A))^3}
-    const void* eg;            // S[4] per flux edge: n_x, n_y, length, 0
+    // S[4] per flux edge: n_x, n_y, length and, exact, the signed zero that a
+    // boundary ghost's zero gradient adds; first order: its two slots in the
+    // bits of the fourth (edge_slots)
+    const void* eg;
     const double* ria;         // [n_own] 1 / area
     const void* area;          // S [n_total]
     FusedSmem L;               // shared-memory layout (fused_smem)
@@ -110,6 +112,9 @@ constexpr uint32_t kWordGhost = 0x40000000u, kWordNoFlux = 0x80000000u;
 constexpr int kMaxFluxUnits = 0x3FFF;  // 2 * max_flux at most
 __device__ __forceinline__ int word_nbr(uint32_t w) { return (int)(w & 0xFFFFu); }
 __device__ __forceinline__ int word_unit(uint32_t w) { return (int)((w >> 16) & 0x3FFFu); }
+
+__device__ __forceinline__ uint32_t edge_slots(float e3) { return __float_as_uint(e3); }
+__device__ __forceinline__ uint32_t edge_slots(double e3) { return (uint32_t)__double_as_longlong(e3); }
 
 // One 4-vector of S at a 16- or 32-byte aligned global address.
 __device__ __forceinline__ void ldg4(const float* p, float* v) {
@@ -294,13 +299,16 @@ struct SlotGeo {
 
 // CFL or constant time step of owned cell c (slot l) and of its boundary
 // ghosts from {u, v, c} of the tile's slots (calc_dt of
-// examples/forwardStep/main.cpp:140-185 and examples/naca/main.cpp:142-183;
-// fast policies); returns the ordered-key minimum of the values written.
-template <class S, int NF>
+// examples/forwardStep/main.cpp:140-185 and examples/naca/main.cpp:142-183).
+// edge(el, e): normal and length of flux edge el; A: the cell's area, which is
+// its ghosts' too.  Returns the ordered-key minimum of the values written.
+template <class M, int NF, class Edge>
 __device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& FP, const TileIO& io, const uint32_t* fw,
-                                                            const uint4* W, int l, int c, int halo_off, int flux_off) {
+                                                            const uint4* W, int l, int c, int halo_off,
+                                                            typename M::S A, Edge edge, double& di) {
+    using S = typename M::S;
     const Params& P = FP.P;
-    const S cfl = (S)P.cfl, A = __ldg((const S*)FP.area + c);
+    const S cfl = (S)P.cfl;
     const bool sum = P.dt_kind == 1, constant = P.dt_kind == 0;
     unsigned long long kmin = ~0ull;
     S ws[4];
@@ -314,21 +322,40 @@ __device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& F
         const bool ghost = (w & kWordGhost) != 0;
         S e[4], wn[4];
         const int u = word_unit(w);
-        ldg4((const S*)FP.eg + 4 * (size_t)(flux_off + (u < FP.max_flux ? u : u - FP.max_flux)), e);
+        const bool side = u >= FP.max_flux;
+        edge(side ? u - FP.max_flux : u, e);
         Planes<S, 4>::get(W, FP.max_grad, o, 0, wn);
         double dg = P.dt_const;
-        if (sum) {
+        if constexpr (M::exact) {
+            if (sum) {
+                const double es = ws[2] + fabs(ws[0] * e[0] + ws[1] * e[1]);
+                const double en = wn[2] + fabs(wn[0] * e[0] + wn[1] * e[1]);
+                const double center = side ? exact::dmax(en, es) : exact::dmax(es, en);
+                acc += center * e[2];
+                if (ghost) {
+                    double d = 0.;
+                    d += center * e[2];
+                    dg = cfl * A / d;
+                }
+            } else if (!constant) {
+                const double es = (ws[2] + fabs(ws[0])) * e[0] + (ws[2] + fabs(ws[1])) * e[1];
+                acc = exact::dmin(acc, cfl * (A / e[2]) / fabs(es));
+                if (ghost) {
+                    const double en = (wn[2] + fabs(wn[0])) * e[0] + (wn[2] + fabs(wn[1])) * e[1];
+                    dg = exact::dmin(1.0, cfl * (A / e[2]) / fabs(en));
+                }
+            }
+        } else if (sum) {
             const S center = fast::tmax(ws[2] + fabs(fast::fma_(ws[0], e[0], ws[1] * e[1])),
                                         wn[2] + fabs(fast::fma_(wn[0], e[0], wn[1] * e[1])));
             acc = fast::fma_(center, e[2], acc);
-            if (ghost) dg = (double)(cfl * __ldg((const S*)FP.area + FP.halo[halo_off + o - FP.T]) * fast::rcp(center * e[2]));
+            if (ghost) dg = (double)(cfl * A * fast::rcp(center * e[2]));
         } else if (!constant) {
             const S es = fast::fma_(ws[2] + fabs(ws[0]), e[0], (ws[2] + fabs(ws[1])) * e[1]);
             acc = fast::tmin(acc, cfl * A * fast::rcp(e[2] * fabs(es)));
             if (ghost) {
                 const S en = fast::fma_(wn[2] + fabs(wn[0]), e[0], (wn[2] + fabs(wn[1])) * e[1]);
-                const S An = __ldg((const S*)FP.area + FP.halo[halo_off + o - FP.T]);
-                dg = (double)fast::tmin(S(1), cfl * An * fast::rcp(e[2] * fabs(en)));
+                dg = (double)fast::tmin(S(1), cfl * A * fast::rcp(e[2] * fabs(en)));
             }
         }
         if (ghost) {
@@ -336,9 +363,353 @@ __device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& F
             kmin = kmin_(kmin, tkey(dg));
         }
     }
-    const double di = constant ? P.dt_const : (double)(sum ? cfl * A * fast::rcp(acc) : acc);
+    if constexpr (M::exact) di = constant ? P.dt_const : (sum ? cfl * A / acc : acc);
+    else di = constant ? P.dt_const : (double)(sum ? cfl * A * fast::rcp(acc) : acc);
     io.dt[c] = di;
     return kmin_(kmin, tkey(di));
+}
+// {u, v, c} of a state, in the reference's arithmetic (exact) or the fast one
+template <class M>
+__device__ __forceinline__ void fused_speeds(double gamma, const typename M::S* q, typename M::S* w) {
+    if constexpr (M::exact) {
+        const double gm1 = gamma - 1;
+        w[0] = q[1] / q[0];
+        w[1] = q[2] / q[0];
+        w[2] = sqrt((gm1 * (q[3] - 0.5 / q[0] * (q[1] * q[1] + q[2] * q[2]))) * gamma / q[0]);
+        w[3] = 0.;
+    } else {
+        fast::speeds((typename M::S)gamma, q, w);
+    }
+}
+
+// Gradients and limiters of gradient slot r (this lane's variables), and the
+// face states of its flux edges into shared memory.  PH: see fused_tile.
+template <class M, int NV, int NF, int PH>
+__device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& io, unsigned char* smem_raw,
+                                           const SlotGeo<M, NF>& geo, int r, int v0, int c0, int halo_off, int flux_off) {
+    using S = typename M::S;
+    using PL = Planes<S, NV>;
+    const Params& P = FP.P;
+    const FusedSmem& L = FP.L;
+    const int T = FP.T;
+    uint4* Q = reinterpret_cast<uint4*>(smem_raw + L.q);
+    uint4* FS = reinterpret_cast<uint4*>(smem_raw + L.fs);
+    uint4* GX = reinterpret_cast<uint4*>(smem_raw + L.gx);
+    uint4* GY = reinterpret_cast<uint4*>(smem_raw + L.gy);
+    uint4* LM = reinterpret_cast<uint4*>(smem_raw + L.lm);
+    S qs[NV], gx[NV], gy[NV], lim[NV];
+    PL::get(Q, L.ls, r, v0, qs);
+    if constexpr (PH == 2) {
+        const size_t g = r < T ? (size_t)(c0 + r) : (size_t)__ldg(FP.halo + halo_off + r - T);
+        ldv<S, NV>((const S*)io.gx + 4 * g + v0, gx);
+        ldv<S, NV>((const S*)io.gy + 4 * g + v0, gy);
+    } else if constexpr (M::exact) {
+        double qmn[NV], qmx[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) { gx[k] = 0; gy[k] = 0; qmn[k] = qs[k]; qmx[k] = qs[k]; lim[k] = 1; }
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            if (!geo.face(f)) continue;
+            const double nx = geo.a[f][0], ny = geo.a[f][1], le = geo.a[f][2], g = geo.a[f][3];
+            const bool side = (geo.a[f][2] < 0.);  // a negative length marks the edge's second cell
+            const double len = fabs(le);
+            double qn[NV];
+            PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                if (!side) {
+                    const double fl = (qs[k] * (1.0 - g) + qn[k] * g) * len;
+                    gx[k] += fl * nx; gy[k] += fl * ny;
+                } else {
+                    const double fl = (qn[k] * (1.0 - g) + qs[k] * g) * len;
+                    gx[k] -= fl * nx; gy[k] -= fl * ny;
+                }
+                qmn[k] = exact::dmin(qmn[k], qn[k]); qmx[k] = exact::dmax(qmx[k], qn[k]);
+            }
+        }
+        const double invA = geo.sl[0], K3a = geo.sl[1];
+        const double tol = 1e-15;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            gx[k] *= invA; gy[k] *= invA;
+            const double delta_max = qmx[k] - qs[k];
+            const double delta_min = qmn[k] - qs[k];
+            const double d2 = (delta_max - delta_min) * (delta_max - delta_min);
+            double sig;
+            if (d2 <= K3a) sig = 1.;
+            else if (d2 <= 2 * K3a) {
+                const double y = (d2 / K3a - 1.0);
+                sig = 2.0 * y * y * y - 3.0 * y * y + 1.0;
+            } else sig = 0.;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                if (!geo.face(f)) continue;
+                const double dqg = gx[k] * geo.dx(f) + gy[k] * geo.dy(f);
+                double lv = 1.0;
+                if (sig < 1.0) {
+                    if (dqg > tol) lv = exact::limiter_func(P.limiter, delta_max / dqg);
+                    else if (dqg < -tol) lv = exact::limiter_func(P.limiter, delta_min / dqg);
+                    else lv = 1.0;
+                }
+                lv = sig + (1.0 - sig) * lv;
+                lim[k] = exact::dmin(lim[k], lv);
+            }
+        }
+    } else {
+        S mn[NV], mx[NV], sig[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) { gx[k] = 0; gy[k] = 0; mn[k] = 0; mx[k] = 0; lim[k] = 1; }
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            if (!geo.face(f)) continue;
+            S qn[NV];
+            PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                const S d = qn[k] - qs[k];
+                gx[k] = fast::fma_(geo.a[f][0], d, gx[k]);
+                gy[k] = fast::fma_(geo.a[f][1], d, gy[k]);
+                mn[k] = fast::vmin(mn[k], d);
+                mx[k] = fast::vmax(mx[k], d);
+            }
+        }
+        bool limited = false;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            sig[k] = fast::smooth_switch(mx[k] - mn[k], geo.sl[0]);
+            limited |= sig[k] < S(1);
+        }
+        if (limited) {
+            auto apply = [&](auto kind) {
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    // the largest and smallest g . d over the faces
+                    // give the strictest ratio of each sign
+                    S up = 0, lo = 0;
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        if (!geo.face(f)) continue;
+                        const S dq = fast::fma_(gy[k], geo.dy(f), gx[k] * geo.dx(f));
+                        up = fast::vmax(up, dq);
+                        lo = fast::vmin(lo, dq);
+                    }
+                    const S lim_k = fast::limiter_min(kind(), sig[k], mx[k], mn[k], up, lo);
+                    gx[k] *= lim_k;
+                    gy[k] *= lim_k;
+                }
+            };
+            if (P.limiter == 2) apply([] { return 2; });
+            else if (P.limiter == 1) apply([] { return 1; });
+            else apply([&] { return P.limiter; });
+        }
+    }
+    if constexpr (PH == 1) {
+        stv<S, NV>((S*)io.gx + 4 * (size_t)(c0 + r) + v0, gx);
+        stv<S, NV>((S*)io.gy + 4 * (size_t)(c0 + r) + v0, gy);
+    } else {
+        uint32_t any = 0;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            if (!geo.face(f)) continue;
+            S qf[NV];
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                if constexpr (M::exact) qf[k] = qs[k] + (gx[k] * geo.dx(f) + gy[k] * geo.dy(f)) * lim[k];
+                else qf[k] = fast::fma_(gy[k], geo.dy(f), fast::fma_(gx[k], geo.dx(f), qs[k]));
+            }
+            guard_share<S, NV, M::exact>(P, qf, qs);
+            if (!(geo.w[f] & kWordNoFlux)) PL::put(FS, L.lf, word_unit(geo.w[f]), v0, qf);
+            any |= geo.w[f];
+        }
+        if (any & kWordGhost) {
+            // a ghost's face state is its cell value (gradient 0); the
+            // cell's own gradients are kept for the ghost fill
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                if (!geo.face(f) || !(geo.w[f] & kWordGhost)) continue;
+                const int u = word_unit(geo.w[f]), el = u < FP.max_flux ? u : u - FP.max_flux;
+                S qn[NV];
+                PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
+                if constexpr (M::exact) {
+                    // the signed zero that the ghost's zero gradient adds
+                    const double z = __ldg((const double*)FP.eg + 4 * (size_t)(flux_off + el) + 3);
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) qn[k] += z;
+                }
+                PL::put(FS, L.lf, u < FP.max_flux ? u + FP.max_flux : el, v0, qn);
+            }
+            PL::put(GX, L.lt, r, v0, gx);
+            PL::put(GY, L.lt, r, v0, gy);
+            if constexpr (M::exact) PL::put(LM, L.lt, r, v0, lim);
+        }
+    }
+}
+
+// Sum of the fluxes of owned cell uc (this lane's variables) in reference edge
+// order, RK update and ghost fill (update_cells + update_bounds,
+// explicit.cpp:368-417); res: its residual terms when partial sums are due.
+// O2: ghosts from the limited gradients, else from the cell value.
+template <class M, int NV, int NF, bool REMOTE, bool O2>
+__device__ __forceinline__ void fused_update(const FusedParams& FP, const TileIO& io, unsigned char* smem_raw,
+                                             const uint32_t* own, int uc, int v0, int c0, int slot_off, int halo_off,
+                                             int flux_off, int G, int tc, double dtc, const double& s_dt,
+                                             const PartIO& pio, double* res) {
+    using S = typename M::S;
+    using PL = Planes<S, NV>;
+    constexpr int V = 4;
+    const Params& P = FP.P;
+    const FusedSmem& L = FP.L;
+    const int T = FP.T, N = P.n_real;
+    uint4* FS = reinterpret_cast<uint4*>(smem_raw + L.fs);
+    const double* QB = reinterpret_cast<const double*>(smem_raw + L.qb);
+    uint4* GX = reinterpret_cast<uint4*>(smem_raw + L.gx);
+    uint4* GY = reinterpret_cast<uint4*>(smem_raw + L.gy);
+    uint4* LM = reinterpret_cast<uint4*>(smem_raw + L.lm);
+    const double* RA = reinterpret_cast<const double*>(smem_raw + L.ria);
+    const int c = c0 + uc;
+    double qt[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) qt[k] = 0.;
+    const double ra = RA[uc];
+    double A = ra;
+    if (!M::exact && io.partials != nullptr) A = (double)__ldg((const S*)FP.area + c);
+    uint32_t any = 0;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        if (f == 3 && word_nbr(own[f]) == 0xFFFF) continue;
+        any |= own[f];
+        S fe[NV];
+        PL::get(FS, L.lf, word_unit(own[f]), v0, fe);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) qt[k] += M::exact ? (double)fe[k] / A : (double)fe[k];
+    }
+    if constexpr (!M::exact) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) qt[k] *= ra;
+    }
+    {
+        if (io.ctrl != nullptr && P.global_dt) {
+            dtc = s_dt;
+            if (tc < 0) {  // a tile across two cases of a batch: this cell's case
+                const int k = P.cell_case[c];
+                unsigned long long key = ~0ull;
+                for (int i = 0; i < kDtSlots; ++i) key = kmin_(key, io.dtkeys[(size_t)k * kDtSlots + i]);
+                const double d0 = io.dt[P.case_cell0[k]];
+                dtc = (d0 != d0) ? d0 : tkey_inv(key);
+            }
+        }
+        double qb[NV], qnew[NV];
+        ldv<double, NV>(QB + 4 * uc + v0, qb);
+        if constexpr (M::exact) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) qnew[k] = qb[k] + qt[k] * dtc * io.alpha;
+        } else {
+            const double da = dtc * io.alpha;
+#pragma unroll
+            for (int k = 0; k < NV; ++k) qnew[k] = fma(qt[k], da, qb[k]);
+        }
+        S qs[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) qs[k] = (S)qnew[k];
+        if (sizeof(S) == 8) {
+            stv<double, NV>(io.q_out + 4 * (size_t)c + v0, qnew);
+        } else {
+            stv<S, NV>((S*)io.s_out + 4 * (size_t)c + v0, qs);
+            if (io.write_f64) stv<double, NV>(io.q_out + 4 * (size_t)c + v0, qnew);
+        }
+        if constexpr (REMOTE) {
+            // this cell's new state into every part that reads it
+            const RemoteIO& R = *pio.remote;
+            if (c < R.n_band) {
+                for (int i = R.cell_off[c]; i < R.cell_off[c + 1]; ++i) {
+                    const int2 d = R.cell_dst[i];
+                    stv<S, NV>((S*)R.dst[d.x] + 4 * (size_t)d.y + v0, qs);
+                }
+            }
+        }
+        if (any & kWordGhost) {
+            S gxs[NV], gys[NV], lms[NV];
+            if constexpr (O2) {
+                PL::get(GX, L.lt, uc, v0, gxs);
+                PL::get(GY, L.lt, uc, v0, gys);
+                if constexpr (M::exact) PL::get(LM, L.lt, uc, v0, lms);
+            }
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                if ((f == 3 && word_nbr(own[f]) == 0xFFFF) || !(own[f] & kWordGhost)) continue;
+                const int u = word_unit(own[f]), el = u < FP.max_flux ? u : u - FP.max_flux;
+                const int g = FP.halo[halo_off + word_nbr(own[f]) - T];
+                const S* ep = (const S*)FP.eg + 4 * (size_t)(flux_off + el);
+                S qint[NV], all[V], b[V], bs[NV];
+                if constexpr (O2) {
+                    const size_t ri = (size_t)NF * slot_off + (size_t)f * G + uc;
+                    const S e0 = M::exact ? ((const S*)FP.rec2)[2 * ri] : ((const S*)FP.rec)[4 * ri + 2];
+                    const S e1 = M::exact ? ((const S*)FP.rec2)[2 * ri + 1] : ((const S*)FP.rec)[4 * ri + 3];
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        if constexpr (M::exact) qint[k] = qs[k] + (gxs[k] * e0 + gys[k] * e1) * lms[k];
+                        else qint[k] = fast::fma_(gys[k], e1, fast::fma_(gxs[k], e0, qs[k]));
+                    }
+                    guard_share<S, NV, M::exact>(P, qint, qs);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) qint[k] = qs[k];
+                }
+                share<S, NV>(qint, all);
+                if constexpr (M::exact) exact::bc<V>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
+                else fast::bc<V, S>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
+                own_share<S, NV>(b, v0, bs);
+                if (sizeof(S) == 8) {
+                    stv<S, NV>((S*)io.q_out + 4 * (size_t)g + v0, bs);
+                } else {
+                    stv<S, NV>((S*)io.s_out + 4 * (size_t)g + v0, bs);
+                    if (io.write_f64) {
+                        double bd[NV];
+#pragma unroll
+                        for (int k = 0; k < NV; ++k) bd[k] = (double)bs[k];
+                        stv<double, NV>(io.q_out + 4 * (size_t)g + v0, bd);
+                    }
+                }
+                if constexpr (REMOTE) {
+                    const RemoteIO& R = *pio.remote;
+                    const int go = g - N;
+                    if (go < R.n_own_ghost)
+                        for (int i = R.ghost_off[go]; i < R.ghost_off[go + 1]; ++i) {
+                            const int2 d = R.ghost_dst[i];
+                            stv<S, NV>((S*)R.dst[d.x] + 4 * (size_t)d.y + v0, bs);
+                        }
+                }
+            }
+        }
+        if (io.partials != nullptr) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) res[k] = qt[k] * qt[k] * A;
+        }
+    }
+}
+
+// Residual partial sums of tile t: a butterfly over the cells of a warp (lanes
+// of equal variables), then the warps in order.  The warp sums share the flux
+// store once every thread has read its fluxes.
+template <int NV>
+__device__ __forceinline__ void fused_partials(const TileIO& io, unsigned char* store, int t, int v0, double* res) {
+    constexpr int V = 4, LP = V / NV;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int o = 16; o >= LP; o >>= 1) res[k] += __shfl_xor_sync(0xffffffffu, res[k], o);
+    double* red = reinterpret_cast<double*>(store);
+    __syncthreads();
+    if ((threadIdx.x & 31) < LP)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) red[(threadIdx.x >> 5) * V + v0 + k] = res[k];
+    __syncthreads();
+    if (threadIdx.x < V) {
+        const int nw = blockDim.x >> 5;
+        double s = 0.;
+        for (int w = 0; w < nw; ++w) s += red[w * V + threadIdx.x];
+        io.partials[(size_t)t * V + threadIdx.x] = s;
+    }
 }
 
 // One tile t.  Returns false when the step is inactive (nothing written).
@@ -367,9 +738,6 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
     uint4* Q = reinterpret_cast<uint4*>(smem_raw + L.q);
     uint4* FS = reinterpret_cast<uint4*>(smem_raw + L.fs);
     double* QB = reinterpret_cast<double*>(smem_raw + L.qb);
-    uint4* GX = reinterpret_cast<uint4*>(smem_raw + L.gx);
-    uint4* GY = reinterpret_cast<uint4*>(smem_raw + L.gy);
-    uint4* LM = reinterpret_cast<uint4*>(smem_raw + L.lm);
     const S* EG = reinterpret_cast<const S*>(smem_raw + L.eg);
     double* RA = reinterpret_cast<double*>(smem_raw + L.ria);
     const bool global_dt = io.ctrl != nullptr && P.global_dt;
@@ -468,17 +836,19 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
     // states of calc_time_derivatives, 297-320)
     if constexpr (PH == 3) {
         uint4* W = FS;
-        const S gamma = (S)P.gamma;
         for (int r = l; r < G; r += blockDim.x) {
             if (r >= nown && r < T) continue;
             S q[V], w[V];
             P4::get(Q, L.ls, r, 0, q);
-            fast::speeds(gamma, q, w);
+            fused_speeds<M>(P.gamma, q, w);
             P4::put(W, FP.max_grad, r, 0, w);
         }
         __syncthreads();
         unsigned long long kmin = ~0ull;
-        if (l < nown) kmin = fused_cell_dt<S, NF>(FP, io, own, W, l, c0 + l, halo_off, flux_off);
+        double di;
+        auto edge = [&](int el, S* e) { ldg4((const S*)FP.eg + 4 * (size_t)(flux_off + el), e); };
+        if (l < nown)
+            kmin = fused_cell_dt<M, NF>(FP, io, own, W, l, c0 + l, halo_off, __ldg((const S*)FP.area + c0 + l), edge, di);
         tile_dt_reduce(P, T, io, t, l, nown, kmin);
         return true;
     }
@@ -486,152 +856,7 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
     for (int r = r0; r < gslots;) {
         // unused slots of a last, partial tile and ring-1 ghosts have no faces
         if (word_nbr(geo.w[0]) != 0xFFFF) {
-            S qs[NV], gx[NV], gy[NV], lim[NV];
-            PL::get(Q, L.ls, r, v0, qs);
-            if constexpr (PH == 2) {
-                const size_t g = r < T ? (size_t)(c0 + r) : (size_t)__ldg(FP.halo + halo_off + r - T);
-                ldv<S, NV>((const S*)io.gx + 4 * g + v0, gx);
-                ldv<S, NV>((const S*)io.gy + 4 * g + v0, gy);
-            } else if constexpr (M::exact) {
-                double qmn[NV], qmx[NV];
-#pragma unroll
-                for (int k = 0; k < NV; ++k) { gx[k] = 0; gy[k] = 0; qmn[k] = qs[k]; qmx[k] = qs[k]; lim[k] = 1; }
-#pragma unroll
-                for (int f = 0; f < NF; ++f) {
-                    if (!geo.face(f)) continue;
-                    const double nx = geo.a[f][0], ny = geo.a[f][1], le = geo.a[f][2], g = geo.a[f][3];
-                    const bool side = (geo.a[f][2] < 0.);  // a negative length marks the edge's second cell
-                    const double len = fabs(le);
-                    double qn[NV];
-                    PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
-#pragma unroll
-                    for (int k = 0; k < NV; ++k) {
-                        if (!side) {
-                            const double fl = (qs[k] * (1.0 - g) + qn[k] * g) * len;
-                            gx[k] += fl * nx; gy[k] += fl * ny;
-                        } else {
-                            const double fl = (qn[k] * (1.0 - g) + qs[k] * g) * len;
-                            gx[k] -= fl * nx; gy[k] -= fl * ny;
-                        }
-                        qmn[k] = exact::dmin(qmn[k], qn[k]); qmx[k] = exact::dmax(qmx[k], qn[k]);
-                    }
-                }
-                const double invA = geo.sl[0], K3a = geo.sl[1];
-                const double tol = 1e-15;
-#pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    gx[k] *= invA; gy[k] *= invA;
-                    const double delta_max = qmx[k] - qs[k];
-                    const double delta_min = qmn[k] - qs[k];
-                    const double d2 = (delta_max - delta_min) * (delta_max - delta_min);
-                    double sig;
-                    if (d2 <= K3a) sig = 1.;
-                    else if (d2 <= 2 * K3a) {
-                        const double y = (d2 / K3a - 1.0);
-                        sig = 2.0 * y * y * y - 3.0 * y * y + 1.0;
-                    } else sig = 0.;
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) {
-                        if (!geo.face(f)) continue;
-                        const double dqg = gx[k] * geo.dx(f) + gy[k] * geo.dy(f);
-                        double lv = 1.0;
-                        if (sig < 1.0) {
-                            if (dqg > tol) lv = exact::limiter_func(P.limiter, delta_max / dqg);
-                            else if (dqg < -tol) lv = exact::limiter_func(P.limiter, delta_min / dqg);
-                            else lv = 1.0;
-                        }
-                        lv = sig + (1.0 - sig) * lv;
-                        lim[k] = exact::dmin(lim[k], lv);
-                    }
-                }
-            } else {
-                S mn[NV], mx[NV], sig[NV];
-#pragma unroll
-                for (int k = 0; k < NV; ++k) { gx[k] = 0; gy[k] = 0; mn[k] = 0; mx[k] = 0; lim[k] = 1; }
-#pragma unroll
-                for (int f = 0; f < NF; ++f) {
-                    if (!geo.face(f)) continue;
-                    S qn[NV];
-                    PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
-#pragma unroll
-                    for (int k = 0; k < NV; ++k) {
-                        const S d = qn[k] - qs[k];
-                        gx[k] = fast::fma_(geo.a[f][0], d, gx[k]);
-                        gy[k] = fast::fma_(geo.a[f][1], d, gy[k]);
-                        mn[k] = fast::vmin(mn[k], d);
-                        mx[k] = fast::vmax(mx[k], d);
-                    }
-                }
-                bool limited = false;
-#pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    sig[k] = fast::smooth_switch(mx[k] - mn[k], geo.sl[0]);
-                    limited |= sig[k] < S(1);
-                }
-                if (limited) {
-                    auto apply = [&](auto kind) {
-#pragma unroll
-                        for (int k = 0; k < NV; ++k) {
-                            // the largest and smallest g . d over the faces
-                            // give the strictest ratio of each sign
-                            S up = 0, lo = 0;
-#pragma unroll
-                            for (int f = 0; f < NF; ++f) {
-                                if (!geo.face(f)) continue;
-                                const S dq = fast::fma_(gy[k], geo.dy(f), gx[k] * geo.dx(f));
-                                up = fast::vmax(up, dq);
-                                lo = fast::vmin(lo, dq);
-                            }
-                            const S lim_k = fast::limiter_min(kind(), sig[k], mx[k], mn[k], up, lo);
-                            gx[k] *= lim_k;
-                            gy[k] *= lim_k;
-                        }
-                    };
-                    if (P.limiter == 2) apply([] { return 2; });
-                    else if (P.limiter == 1) apply([] { return 1; });
-                    else apply([&] { return P.limiter; });
-                }
-            }
-            if constexpr (PH == 1) {
-                stv<S, NV>((S*)io.gx + 4 * (size_t)(c0 + r) + v0, gx);
-                stv<S, NV>((S*)io.gy + 4 * (size_t)(c0 + r) + v0, gy);
-            } else {
-                uint32_t any = 0;
-#pragma unroll
-                for (int f = 0; f < NF; ++f) {
-                    if (!geo.face(f)) continue;
-                    S qf[NV];
-#pragma unroll
-                    for (int k = 0; k < NV; ++k) {
-                        if constexpr (M::exact) qf[k] = qs[k] + (gx[k] * geo.dx(f) + gy[k] * geo.dy(f)) * lim[k];
-                        else qf[k] = fast::fma_(gy[k], geo.dy(f), fast::fma_(gx[k], geo.dx(f), qs[k]));
-                    }
-                    guard_share<S, NV, M::exact>(P, qf, qs);
-                    if (!(geo.w[f] & kWordNoFlux)) PL::put(FS, L.lf, word_unit(geo.w[f]), v0, qf);
-                    any |= geo.w[f];
-                }
-                if (any & kWordGhost) {
-                    // a ghost's face state is its cell value (gradient 0); the
-                    // cell's own gradients are kept for the ghost fill
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) {
-                        if (!geo.face(f) || !(geo.w[f] & kWordGhost)) continue;
-                        const int u = word_unit(geo.w[f]), el = u < FP.max_flux ? u : u - FP.max_flux;
-                        S qn[NV];
-                        PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
-                        if constexpr (M::exact) {
-                            // the signed zero that the ghost's zero gradient adds
-                            const double z = __ldg((const double*)FP.eg + 4 * (size_t)(flux_off + el) + 3);
-#pragma unroll
-                            for (int k = 0; k < NV; ++k) qn[k] += z;
-                        }
-                        PL::put(FS, L.lf, u < FP.max_flux ? u + FP.max_flux : el, v0, qn);
-                    }
-                    PL::put(GX, L.lt, r, v0, gx);
-                    PL::put(GY, L.lt, r, v0, gy);
-                    if constexpr (M::exact) PL::put(LM, L.lt, r, v0, lim);
-                }
-            }
+            fused_slot<M, NV, NF, PH>(FP, io, smem_raw, geo, r, v0, c0, halo_off, flux_off);
         }
         r += rstep;
         if (r >= gslots) break;
@@ -646,10 +871,15 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
         e[0] = EG[4 * el]; e[1] = EG[4 * el + 1]; e[2] = EG[4 * el + 2];
         P4::get(FS, L.lf, el, 0, qL);
         P4::get(FS, L.lf, el + FP.max_flux, 0, qR);
-        if constexpr (M::exact) exact::flux<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
-        else fast::flux<FLUX, S>((S)P.gamma, f, qL, qR, e[0], e[1]);
+        if constexpr (M::exact) {
+            exact::flux<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
 #pragma unroll
-        for (int k = 0; k < V; ++k) { f[k] *= e[2]; qL[k] = -f[k]; }
+            for (int k = 0; k < V; ++k) f[k] *= e[2];
+        } else {
+            fast::flux_le<FLUX, S>((S)P.gamma, f, qL, qR, e[0], e[1], e[2]);
+        }
+#pragma unroll
+        for (int k = 0; k < V; ++k) qL[k] = -f[k];
         P4::put(FS, L.lf, el, 0, qL);
         P4::put(FS, L.lf, el + FP.max_flux, 0, f);
     }
@@ -662,141 +892,10 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
 #pragma unroll
     for (int k = 0; k < NV; ++k) res[k] = 0.;
     if (uc < nown) {
-        const int c = c0 + uc;
-        double qt[NV];
-#pragma unroll
-        for (int k = 0; k < NV; ++k) qt[k] = 0.;
-        const double ra = RA[uc];
-        double A = ra;
-        if (!M::exact && io.partials != nullptr) A = (double)__ldg((const S*)FP.area + c);
-        uint32_t any = 0;
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            if (f == 3 && word_nbr(own[f]) == 0xFFFF) continue;
-            any |= own[f];
-            S fe[NV];
-            PL::get(FS, L.lf, word_unit(own[f]), v0, fe);
-#pragma unroll
-            for (int k = 0; k < NV; ++k) qt[k] += M::exact ? (double)fe[k] / A : (double)fe[k];
-        }
-        if constexpr (!M::exact) {
-#pragma unroll
-            for (int k = 0; k < NV; ++k) qt[k] *= ra;
-        }
-        {
-            if (global_dt) {
-                dtc = s_dt;
-                if (tc < 0) {  // a tile across two cases of a batch: this cell's case
-                    const int k = P.cell_case[c];
-                    unsigned long long key = ~0ull;
-                    for (int i = 0; i < kDtSlots; ++i) key = kmin_(key, io.dtkeys[(size_t)k * kDtSlots + i]);
-                    const double d0 = io.dt[P.case_cell0[k]];
-                    dtc = (d0 != d0) ? d0 : tkey_inv(key);
-                }
-            }
-            double qb[NV], qnew[NV];
-            ldv<double, NV>(QB + 4 * uc + v0, qb);
-            if constexpr (M::exact) {
-#pragma unroll
-                for (int k = 0; k < NV; ++k) qnew[k] = qb[k] + qt[k] * dtc * io.alpha;
-            } else {
-                const double da = dtc * io.alpha;
-#pragma unroll
-                for (int k = 0; k < NV; ++k) qnew[k] = fma(qt[k], da, qb[k]);
-            }
-            S qs[NV];
-#pragma unroll
-            for (int k = 0; k < NV; ++k) qs[k] = (S)qnew[k];
-            if (sizeof(S) == 8) {
-                stv<double, NV>(io.q_out + 4 * (size_t)c + v0, qnew);
-            } else {
-                stv<S, NV>((S*)io.s_out + 4 * (size_t)c + v0, qs);
-                if (io.write_f64) stv<double, NV>(io.q_out + 4 * (size_t)c + v0, qnew);
-            }
-            if constexpr (REMOTE) {
-                // this cell's new state into every part that reads it
-                const RemoteIO& R = *pio.remote;
-                if (c < R.n_band) {
-                    for (int i = R.cell_off[c]; i < R.cell_off[c + 1]; ++i) {
-                        const int2 d = R.cell_dst[i];
-                        stv<S, NV>((S*)R.dst[d.x] + 4 * (size_t)d.y + v0, qs);
-                    }
-                }
-            }
-            if (any & kWordGhost) {
-                S gxs[NV], gys[NV], lms[NV];
-                PL::get(GX, L.lt, uc, v0, gxs);
-                PL::get(GY, L.lt, uc, v0, gys);
-                if constexpr (M::exact) PL::get(LM, L.lt, uc, v0, lms);
-#pragma unroll
-                for (int f = 0; f < NF; ++f) {
-                    if ((f == 3 && word_nbr(own[f]) == 0xFFFF) || !(own[f] & kWordGhost)) continue;
-                    const int u = word_unit(own[f]), el = u < FP.max_flux ? u : u - FP.max_flux;
-                    const int g = FP.halo[halo_off + word_nbr(own[f]) - T];
-                    const size_t ri = (size_t)NF * slot_off + (size_t)f * G + uc;
-                    const S* ep = (const S*)FP.eg + 4 * (size_t)(flux_off + el);
-                    const S e0 = M::exact ? ((const S*)FP.rec2)[2 * ri] : ((const S*)FP.rec)[4 * ri + 2];
-                    const S e1 = M::exact ? ((const S*)FP.rec2)[2 * ri + 1] : ((const S*)FP.rec)[4 * ri + 3];
-                    S qint[NV], all[V], b[V], bs[NV];
-#pragma unroll
-                    for (int k = 0; k < NV; ++k) {
-                        if constexpr (M::exact) qint[k] = qs[k] + (gxs[k] * e0 + gys[k] * e1) * lms[k];
-                        else qint[k] = fast::fma_(gys[k], e1, fast::fma_(gxs[k], e0, qs[k]));
-                    }
-                    guard_share<S, NV, M::exact>(P, qint, qs);
-                    share<S, NV>(qint, all);
-                    if constexpr (M::exact) exact::bc<V>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
-                    else fast::bc<V, S>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
-                    own_share<S, NV>(b, v0, bs);
-                    if (sizeof(S) == 8) {
-                        stv<S, NV>((S*)io.q_out + 4 * (size_t)g + v0, bs);
-                    } else {
-                        stv<S, NV>((S*)io.s_out + 4 * (size_t)g + v0, bs);
-                        if (io.write_f64) {
-                            double bd[NV];
-#pragma unroll
-                            for (int k = 0; k < NV; ++k) bd[k] = (double)bs[k];
-                            stv<double, NV>(io.q_out + 4 * (size_t)g + v0, bd);
-                        }
-                    }
-                    if constexpr (REMOTE) {
-                        const RemoteIO& R = *pio.remote;
-                        const int go = g - N;
-                        if (go < R.n_own_ghost)
-                            for (int i = R.ghost_off[go]; i < R.ghost_off[go + 1]; ++i) {
-                                const int2 d = R.ghost_dst[i];
-                                stv<S, NV>((S*)R.dst[d.x] + 4 * (size_t)d.y + v0, bs);
-                            }
-                    }
-                }
-            }
-            if (io.partials != nullptr) {
-#pragma unroll
-                for (int k = 0; k < NV; ++k) res[k] = qt[k] * qt[k] * A;
-            }
-        }
+        fused_update<M, NV, NF, REMOTE, true>(FP, io, smem_raw, own, uc, v0, c0, slot_off, halo_off, flux_off, G, tc, dtc,
+                                              s_dt, pio, res);
     }
-    if (io.partials != nullptr) {
-        // butterfly over the cells of a warp (lanes of equal variables), then
-        // the warps in order
-#pragma unroll
-        for (int k = 0; k < NV; ++k)
-#pragma unroll
-            for (int o = 16; o >= LP; o >>= 1) res[k] += __shfl_xor_sync(0xffffffffu, res[k], o);
-        // the warp sums share the flux store once every thread has read its fluxes
-        double* red = reinterpret_cast<double*>(FS);
-        __syncthreads();
-        if ((threadIdx.x & 31) < LP)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) red[(threadIdx.x >> 5) * V + v0 + k] = res[k];
-        __syncthreads();
-        if (threadIdx.x < V) {
-            const int nw = blockDim.x >> 5;
-            double s = 0.;
-            for (int w = 0; w < nw; ++w) s += red[w * V + threadIdx.x];
-            io.partials[(size_t)t * V + threadIdx.x] = s;
-        }
-    }
+    if (io.partials != nullptr) fused_partials<NV>(io, smem_raw + L.fs, t, v0, res);
     if constexpr (REMOTE) {
         // every band tile counts itself once its stores are visible; the
         // last one releases this stage's epoch to the readers
@@ -889,7 +988,7 @@ struct FusedLaunch {
     // lays out the tiles' shared memory (FP.L); the bytes of the largest launch
     static size_t smem(FusedParams& FP) {
         FP.L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_flux, FP.T);
-        return (size_t)(M::exact ? FP.L.total : std::max(FP.L.total, FP.L.total_grad));
+        return (size_t)std::max(FP.L.total, FP.L.total_grad);
     }
     static cudaError_t prepare(FusedParams& FP) {
         static std::mutex mu;

@@ -35,6 +35,9 @@ template <class T> __device__ __forceinline__ T tmax(T a, T b) { return (a < b) 
 // so that kernels that share it give the same bits.
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+// product that is not contracted into a following sum
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
 // minimum and maximum of finite values (one instruction in FP32)
 __device__ __forceinline__ float vmin(float a, float b) { return fminf(a, b); }
 __device__ __forceinline__ float vmax(float a, float b) { return fmaxf(a, b); }
@@ -57,9 +60,9 @@ __device__ __forceinline__ double smooth_switch(double d, double rk3) {
 template <class T>
 __device__ __forceinline__ void speeds(T gamma, const T* q, T* w) {
     const T ri = rcp(q[0]);
-    w[0] = q[1] * ri;
-    w[1] = q[2] * ri;
-    w[2] = sqrt_(gamma * (gamma - T(1)) * fma_(q[3], ri, T(-0.5) * fma_(w[0], w[0], w[1] * w[1])));
+    w[0] = mul_(q[1], ri);
+    w[1] = mul_(q[2], ri);
+    w[2] = sqrt_(gamma * (gamma - T(1)) * fma_(q[3], ri, mul_(T(-0.5), fma_(w[0], w[0], mul_(w[1], w[1])))));
     w[3] = T(0);
 }
 
@@ -102,6 +105,47 @@ __device__ __forceinline__ void roe(T gamma, T* f, const T* qi, const T* qj, T n
                       kF5 * (h + c * V));
 }
 
+// le times the flux of roe(), for the Euler kinds.  The same quantities with
+// every fused multiply-add written out (one rounding wherever it is inlined,
+// so that the kernels that share it give the same bits), the Roe averages as
+// corrections of the left state, and the dissipation collected by the factors
+// that its wave strengths share: with s1 = k1 + k5, s = s1 + k0 and
+// g = c (k5 - k1) - kr dV it is
+//   mass s, momentum (u, v) s + g n + kr (du, dv),
+//   energy h s1 + V g + k0 (u^2 + v^2) / 2 + kr (u du + v dv).
+// About 95 instructions instead of 135.
+template <class T>
+__device__ __forceinline__ void roe_le(T gamma, T* f, const T* qi, const T* qj, T n0, T n1, T le) {
+    const T gm1 = gamma - T(1);
+    const T ri = rcp(qi[0]), rj = rcp(qj[0]);
+    const T uL = mul_(qi[1], ri), vL = mul_(qi[2], ri), uR = mul_(qj[1], rj), vR = mul_(qj[2], rj);
+    const T pL = mul_(gm1, fma_(T(-0.5), fma_(qi[2], vL, mul_(qi[1], uL)), qi[3]));
+    const T pR = mul_(gm1, fma_(T(-0.5), fma_(qj[2], vR, mul_(qj[1], uR)), qj[3]));
+    const T VL = fma_(vL, n1, mul_(uL, n0)), VR = fma_(vR, n1, mul_(uR, n0));
+    const T HL = qi[3] + pL, HR = qj[3] + pR, ps = pL + pR;
+    const T sL = sqrt_(qi[0]), sR = sqrt_(qj[0]);
+    const T b = mul_(sR, rcp(sL + sR));
+    const T hL = mul_(HL, ri), hR = mul_(HR, rj);
+    const T du = uR - uL, dv = vR - vL;
+    const T u = fma_(b, du, uL), v = fma_(b, dv, vL), h = fma_(b, hR - hL, hL);
+    const T q2h = mul_(T(0.5), fma_(v, v, mul_(u, u)));
+    const T c2 = mul_(gm1, h - q2h);
+    const T c = sqrt_(c2), rc2 = rcp(c2);
+    const T V = fma_(v, n1, mul_(u, n0));
+    const T rho = mul_(sL, sR), dp = pR - pL, dV = VR - VL;
+    const T l1 = fabs(tmin(V, VL) - c), l2 = fabs(V), l5 = fabs(tmax(V, VR) + c);
+    const T w = mul_(mul_(rho, c), dV), h2 = mul_(T(0.5), rc2);
+    const T k1 = mul_(mul_(l1, dp - w), h2), k5 = mul_(mul_(l5, dp + w), h2);
+    const T k0 = mul_(l2, fma_(-dp, rc2, qj[0] - qi[0])), kr = mul_(l2, rho);
+    const T s1 = k1 + k5, s = s1 + k0;
+    const T g = fma_(c, k5 - k1, -mul_(kr, dV));
+    const T ku = mul_(kr, du), kv = mul_(kr, dv), a = mul_(T(0.5), le);
+    f[0] = mul_(a, fma_(qi[0], VL, mul_(qj[0], VR)) - s);
+    f[1] = mul_(a, fma_(qi[1], VL, fma_(qj[1], VR, mul_(ps, n0))) - fma_(u, s, fma_(n0, g, ku)));
+    f[2] = mul_(a, fma_(qi[2], VL, fma_(qj[2], VR, mul_(ps, n1))) - fma_(v, s, fma_(n1, g, kv)));
+    f[3] = mul_(a, fma_(HL, VL, mul_(HR, VR)) - fma_(h, s1, fma_(V, g, fma_(k0, q2h, fma_(u, ku, mul_(v, kv))))));
+}
+
 // Upwind advection flux (examples/burgers/main.cpp:68-96).
 template <class T>
 __device__ __forceinline__ void burgers(T* f, const T* qi, const T* qj, T n0, T n1) {
@@ -111,10 +155,16 @@ __device__ __forceinline__ void burgers(T* f, const T* qi, const T* qj, T n0, T 
     f[1] = T(0.5) * (Vi * qi[1] + Vj * qj[1]) - T(0.5) * V * (qj[1] - qi[1]);
 }
 
+// le times the flux (FLUX 3 Burgers, else Roe)
 template <int FLUX, class T>
-__device__ __forceinline__ void flux(T gamma, T* f, const T* qi, const T* qj, T n0, T n1) {
-    if (FLUX == 3) burgers(f, qi, qj, n0, n1);
-    else roe(gamma, f, qi, qj, n0, n1);
+__device__ __forceinline__ void flux_le(T gamma, T* f, const T* qi, const T* qj, T n0, T n1, T le) {
+    if (FLUX == 3) {
+        burgers(f, qi, qj, n0, n1);
+        f[0] *= le;
+        f[1] *= le;
+    } else {
+        roe_le(gamma, f, qi, qj, n0, n1, le);
+    }
 }
 
 // Diffusion flux -grad(u) . n with the corrected face gradient (see
@@ -197,7 +247,15 @@ __device__ __forceinline__ T limiter_min(int kind, T sig, T mx, T mn, T up, T lo
     const bool use_up = pu && (!pl || mx * lo > mn * up);
     const T num = use_up ? mx : mn, den = use_up ? up : lo;
     if (!pu && !pl) return T(1);
-    return vmin(T(1), fma_(T(1) - sig, limiter_ratio(kind, num, den), sig));
+    T phi;
+    if (kind == 2) {
+        phi = mul_(mul_(num, fma_(T(2), den, num)), rcp(fma_(num, num + den, mul_(T(2) * den, den))));
+    } else {
+        const T y = div_(num, den);
+        if (kind == 1) phi = y >= T(2) ? T(1) : fma_(mul_(T(-0.25), y), y, y);
+        else phi = limiter_func(kind, y);
+    }
+    return vmin(T(1), fma_(T(1) - sig, phi, sig));
 }
 
 // Boundary conditions (see fv_physics_exact.cuh for the references).

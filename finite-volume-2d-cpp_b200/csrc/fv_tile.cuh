@@ -36,6 +36,7 @@ struct MF32 { using S = float; static constexpr bool exact = false; };
 
 constexpr int kDtSlots = 64;        // atomic slots of the global dt minimum
 constexpr int kTileMax = 256;       // threads (= cells) per tile at most
+constexpr int kFusedThreads = 512;  // threads per CTA at most (lanes of the fused kernel)
 constexpr uint16_t kFaceNone = 0xFFFF;
 constexpr int kFaceEdgeMask = 0x3FFF;
 
@@ -522,9 +523,9 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
             kmin = kmin_(kmin, tkey(di));
         } else {
             const S gamma = (S)P.gamma, gm1 = gamma - S(1), cfl = (S)P.cfl;
-            const S ri = fast::rcp(qs[0]);
-            const S us = qs[1] * ri, vs = qs[2] * ri;
-            const S cs = fast::sqrt_(gamma * gm1 * (qs[3] * ri - S(0.5) * (us * us + vs * vs)));
+            S ws[4];  // {u, v, c}: the run kernel's arithmetic (fused_cell_dt)
+            fast::speeds(gamma, qs, ws);
+            const S us = ws[0], vs = ws[1], cs = ws[2];
             const S Ai = AR[c];
             S acc = sum ? S(0) : S(1);
 #pragma unroll
@@ -534,15 +535,14 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
                 const uint32_t ij = sij[el];
                 const int o = side ? (int)(ij & 0xffff) : (int)(ij >> 16);
                 const S n0 = snx[el], n1 = sny[el], le = sle[el];
-                S qn[4];
+                S qn[4], wn[4];
                 lds<S, 4>(rec + (size_t)o * NR, qn);
-                const S rn = fast::rcp(qn[0]);
-                const S un = qn[1] * rn, vn = qn[2] * rn;
-                const S cn = fast::sqrt_(gamma * gm1 * (qn[3] * rn - S(0.5) * (un * un + vn * vn)));
+                fast::speeds(gamma, qn, wn);
+                const S un = wn[0], vn = wn[1], cn = wn[2];
                 const bool ghost = (w[f] & 0x4000) != 0;
                 if (sum) {
-                    const S center = fast::tmax(cs + fabs(us * n0 + vs * n1), cn + fabs(un * n0 + vn * n1));
-                    acc += center * le;
+                    const S center = fast::tmax(cs + fabs(fast::fma_(us, n0, vs * n1)), cn + fabs(fast::fma_(un, n0, vn * n1)));
+                    acc = fast::fma_(center, le, acc);
                     if (ghost) {
                         const int g = TP.halo[inf.z + o - T];
                         const double dg = (double)(cfl * AR[g] * fast::rcp(center * le));
@@ -550,11 +550,11 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
                         kmin = kmin_(kmin, tkey(dg));
                     }
                 } else {
-                    const S es = (cs + fabs(us)) * n0 + (cs + fabs(vs)) * n1;
+                    const S es = fast::fma_(cs + fabs(us), n0, (cs + fabs(vs)) * n1);
                     acc = fast::tmin(acc, cfl * Ai * fast::rcp(le * fabs(es)));
                     if (ghost) {
                         const int g = TP.halo[inf.z + o - T];
-                        const S en = (cn + fabs(un)) * n0 + (cn + fabs(vn)) * n1;
+                        const S en = fast::fma_(cn + fabs(un), n0, (cn + fabs(vn)) * n1);
                         const double dg = (double)fast::tmin(S(1), cfl * (S)AR[g] * fast::rcp(le * fabs(en)));
                         io.dt[g] = dg;
                         kmin = kmin_(kmin, tkey(dg));
@@ -574,7 +574,7 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
 // thread of the block calls it.
 __device__ __forceinline__ void tile_dt_reduce(const Params& P, int T, const TileIO& io, int t, int l, int nown,
                                                unsigned long long kmin) {
-    __shared__ unsigned long long wmin[kTileMax / 32];
+    __shared__ unsigned long long wmin[kFusedThreads / 32];
     if (P.global_dt && io.dtkeys != nullptr) {
         const int tc = P.n_cases > 1 ? P.tile_case[t] : 0;
         if (tc >= 0) {
@@ -1000,9 +1000,9 @@ __device__ __forceinline__ void tile_stage(const TileParams& TP, const TileIO& i
             } else if constexpr (M::exact) {
                 exact::flux<FLUX>(P.gamma, f, qL, qR, n0, n1);
             } else {
-                fast::flux<FLUX, S>((S)P.gamma, f, qL, qR, n0, n1);
+                fast::flux_le<FLUX, S>((S)P.gamma, f, qL, qR, n0, n1, sle[el]);
             }
-            if constexpr (!M::exact) {
+            if constexpr (!M::exact && FLUX == 4) {
                 const S le = sle[el];
 #pragma unroll
                 for (int k = 0; k < V; ++k) f[k] *= le;
