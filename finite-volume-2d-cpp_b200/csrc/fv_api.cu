@@ -78,9 +78,9 @@ int upload_v(fv_solver* s, const std::vector<T>& v, const T** out) {
 // the fused kernel's arrays over two-ring tiles (build_fused)
 template <class S>
 int upload_fused(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2,
-                 bool exact, double K) {
+                 bool exact, bool first_order, double K) {
     FusedArrays<S> a;
-    build_fused<S>(m, fa, ta, t2, exact, K, a);
+    build_fused<S>(m, fa, ta, t2, exact, first_order, K, a);
     FusedParams& F = s->FPm;
     F.nf = a.nf;
     const int32_t* info; const uint32_t* hd; const S *rec, *rec2, *sl, *eg;
@@ -97,6 +97,41 @@ int upload_fused(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const Ti
 int fused_lanes(const fv_solver* s) {
     (void)s;
     return 1;
+}
+// The persistent run kernel, where all tiles fit the device at once: the first
+// candidate (fv_persist.cuh) with room for them.
+int choose_run_kernel(fv_solver* s) {
+    int sms = 0, coop = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
+    if (!coop) return FV_OK;
+    FusedParams F = s->FPm;
+    F.P = s->TP.P;
+    RunKernel k[kRunKernels];
+    tile::run_kernels(s->precision, F, k);
+    const size_t smem = tile::smem_fused(s->precision, F);
+    for (int i = 0; i < kRunKernels; ++i) {
+        if (!k[i].fn) continue;
+        {
+            static std::mutex mu;
+            std::lock_guard<std::mutex> lock(mu);
+            // only ever raised: a solver created earlier may launch with more
+            cudaFuncAttributes fa{};
+            CK(cudaFuncGetAttributes(&fa, k[i].fn));
+            if ((size_t)fa.maxDynamicSharedSizeBytes < smem)
+                CK(cudaFuncSetAttribute(k[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaFuncSetAttribute(k[i].fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    (int)cudaSharedmemCarveoutMaxShared));
+        }
+        int nb = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k[i].fn, k[i].threads, smem));
+        if ((int64_t)nb * sms < s->n_tiles) continue;
+        CK(s->alloc(&s->run_keys, (size_t)3 * s->n_cases * kDtSlots));
+        CK(s->alloc(&s->run_bar, 1));
+        s->run_kernel = k[i];
+        return FV_OK;
+    }
+    return FV_OK;
 }
 }  // namespace
 
@@ -396,9 +431,21 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     const bool can_fuse = ph->V == 4 && ph->order2 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST) &&
                           !ph->diffusive && !ph->smooth_residuals;
     const bool two_ring = can_fuse && (sk != FV_STAGE_SPLIT || precision != FV_PREC_FP64_EXACT);
+    // the persistent run kernel (choose_run_kernel): the Roe kinds in their
+    // default layout and schedule with a CFL or constant time step, not on a
+    // part of a decomposition.  Its tiles have to fit the device at once: at
+    // most 8 per SM do.
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const bool roe = ph->V == 4 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST);
+    const bool can_run = roe && ph->dt_kind < FV_DT_VISC_MIN && sk != FV_STAGE_SPLIT &&
+                         !(sk == FV_STAGE_HYBRID && precision == FV_PREC_FP64_EXACT) &&
+                         (!opt || opt->schedule == FV_SCHED_TILE) && m.owned_real() == m.n_real && m.n_real > 0 &&
+                         m.n_real <= (int64_t)8 * sms * tile_cells;
+    const bool run_first_order = can_run && !ph->order2;
     Tile2Arrays t2;
     std::future<void> t2_built;
-    if (two_ring) t2_built = std::async(std::launch::async, [&] { build_tiles2(m, fa, tile_cells, t2); });
+    if (two_ring || run_first_order) t2_built = std::async(std::launch::async, [&] { build_tiles2(m, fa, tile_cells, t2); });
     build_tiles(m, fa, tile_cells, ta);
     if (ta.max_halo + tile_cells > 65535 || ta.max_edges > kFaceEdgeMask)
         return fail(FV_ERR_MESH, "tile halo too large for 16-bit local indices");
@@ -468,8 +515,8 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
             if (!fits && (sk == FV_STAGE_FUSED || sk == FV_STAGE_HYBRID))
                 return fail(FV_ERR_MESH, "two-ring tiles too large for the fused stage kernel at this tile size");
             if (fits) {
-                if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, ph->K);
-                else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, ph->K);
+                if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, false, ph->K);
+                else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, false, ph->K);
                 if (rc) return rc;
                 const int32_t* h2;
                 if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;
@@ -566,6 +613,24 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
         s->nbr = const_cast<uint32_t*>(d);
     }
     launch_fill_ghost_grad(s->gx, s->gy, s->lim, (int)m.n_real, (int)m.n_total, ph->V, s->f32, s->stream);
+    if (run_first_order) {
+        t2_built.get();
+        FusedParams& F = s->FPm;
+        F.T = tile_cells;
+        F.max_slots = t2.max_grad; F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;  // one ring is staged
+        if (t2.max_slots < 65535 && 2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= (size_t)227 * 1024) {
+            if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, true, ph->K);
+            else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, true, ph->K);
+            if (rc) return rc;
+            const int32_t* h2;
+            if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;
+            F.halo = h2;
+            F.area = TP.area;
+            if ((rc = choose_run_kernel(s.get()))) return rc;
+        }
+    } else if (can_run && s->fused) {
+        if ((rc = choose_run_kernel(s.get()))) return rc;
+    }
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s->stream));
     *out = s.release();
@@ -599,7 +664,9 @@ int fv_solver_create_tuned(const fv_mesh* fm, const fv_physics* ph, int32_t prec
         // split; fused with FV_SCHED_TILE, FV_SCHED_WORKLIST, FV_SCHED_TILE2;
         // fused with the split first stage (FV_SCHED_TILE)
         double ms_of[5] = {1e300, 1e300, 1e300, 1e300, 1e300};
+        const RunKernel run = s->run_kernel;  // belongs to the fused tiles' default schedule
         auto set_variant = [&](int v) {
+            s->run_kernel = v == 1 || !can_fuse ? run : RunKernel{};
             s->fused = v >= 1;
             s->sched = (v >= 1 && v <= 3) ? v - 1 : FV_SCHED_TILE;
             s->split_first = v == 4;
@@ -971,6 +1038,27 @@ static int settle_base(fv_solver* s, unsigned long long steps_taken) {
     return FV_OK;
 }
 
+// At most `steps` steps in one launch of the persistent run kernel.
+constexpr int kRunSteps = 2048;  // bounds the duration of a launch
+static int launch_run(fv_solver* s, const std::vector<double>& alpha, int steps) {
+    launch_run_begin(s->ctrl, s->run_keys, 3 * s->n_cases * kDtSlots, s->run_bar, s->stream);
+    PersistIO D{};
+    for (int i = 0; i < 2; ++i) { D.qbase[i] = s->qbase[i]; D.sbase[i] = s->sbase[i]; D.tmp[i] = s->tmp[i]; }
+    D.dt = s->dt; D.partials = s->partials; D.keys = s->run_keys;
+    D.ctrl = s->ctrl; D.limits = s->limits; D.hist = s->hist; D.hist_cap = s->hist_cap;
+    D.bar = s->run_bar;
+    D.n_tiles = s->n_tiles; D.n_cases = s->n_cases; D.f32 = s->f32 ? 1 : 0;
+    D.max_steps = steps;
+    D.ns = (int)alpha.size();
+    for (int k = 0; k < D.ns; ++k) D.alpha[k] = alpha[(size_t)k];
+    FusedParams F = s->FPm;
+    F.P = s->TP.P;
+    void* args[] = {&F, &D};
+    CK(cudaLaunchCooperativeKernel(s->run_kernel.fn, dim3((unsigned)s->n_tiles), dim3((unsigned)s->run_kernel.threads),
+                                   args, (size_t)std::max(F.L.total, F.L.total_grad), s->stream));
+    return FV_OK;
+}
+
 int fv_run(fv_solver* s, const fv_run_options* o, fv_run_info* info) {
     if (!s || !o) return fail(FV_ERR_ARG, "fv_run: null argument");
     if (o->n_alpha < 1 || o->n_alpha > 16 || !o->alpha) return fail(FV_ERR_ARG, "fv_run: need 1..16 RK stages");
@@ -1010,19 +1098,33 @@ int fv_run(fv_solver* s, const fv_run_options* o, fv_run_info* info) {
         const unsigned long long left = o->max_step > cur ? o->max_step - cur : 1ull;
         int len = 1;
         while ((unsigned long long)(len * 2) <= left && len * 2 <= s->chunk) len *= 2;
-        GraphEntry* g = nullptr;
-        int rc = get_graph(s, alpha, len, &g);
-        if (rc) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
-        CK(cudaEventRecord(e0, st));
-        CK(cudaGraphLaunch(g->exec, st));  // its first kernel empties the print records
-        CK(cudaEventRecord(e1, st));
-        launches += g->launches;
+        int rc;
+        if (s->run_kernel.fn) {
+            // a callback hears of its steps every `chunk` steps, as below
+            const unsigned long long most = o->on_print ? std::min(s->chunk, s->hist_cap) : kRunSteps;
+            CK(cudaEventRecord(e0, st));
+            if ((rc = launch_run(s, alpha, (int)std::min(left, most)))) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
+            CK(cudaEventRecord(e1, st));
+            launches += 2;
+        } else {
+            GraphEntry* g = nullptr;
+            rc = get_graph(s, alpha, len, &g);
+            if (rc) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
+            CK(cudaEventRecord(e0, st));
+            CK(cudaGraphLaunch(g->exec, st));  // its first kernel empties the print records
+            CK(cudaEventRecord(e1, st));
+            launches += g->launches;
+        }
         launch_ctrl_copy(s->ctrl, s->hctrl_dev, st);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(st));
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, e0, e1));
         total_ms += ms;
+        if (s->run_kernel.fn && hc.failed) {
+            cudaEventDestroy(e0); cudaEventDestroy(e1);
+            return fail(FV_ERR_CUDA, "fv_run: a grid barrier of the run kernel gave up");
+        }
         if (alpha.size() == 1 && (rc = settle_base(s, hc.step - cur))) return rc;
         cur = hc.step;
         if (o->on_print && hc.n_hist > 0) {

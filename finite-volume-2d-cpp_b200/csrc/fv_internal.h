@@ -19,7 +19,7 @@ struct Ctrl {
     int active;                    // this step runs
     int need_R;                    // residuals are evaluated this step
     int n_hist;                    // print records written this chunk
-    int pad;
+    int failed;                    // a grid barrier of the persistent run kernel gave up
     unsigned long long dtkeys[64]; // global dt minimum, spread over atomic slots
 };
 

@@ -78,6 +78,17 @@ __global__ void k_step_begin(Ctrl* c, const RunLimits* L, int V, unsigned long l
     }
 }
 
+// Before a persistent run kernel, whose phases run while ctrl->active is set.
+__global__ void k_run_begin(Ctrl* c, unsigned long long* keys, int nkeys, unsigned* bar) {
+    for (int i = threadIdx.x; i < nkeys; i += blockDim.x) keys[i] = ~0ull;
+    if (threadIdx.x == 0) {
+        *bar = 0u;
+        c->n_hist = 0;
+        c->active = 1;
+        c->failed = 0;
+    }
+}
+
 // Run control set and read by small kernels, not by copies: a copy would
 // queue behind state transfers that other streams keep the copy engines busy
 // with (the host reads the control through mapped pinned memory).
@@ -203,6 +214,9 @@ __global__ void __launch_bounds__(kEndBlock) k_step_end(Params P, Ctrl* c, const
 
 void launch_step_begin(Ctrl* c, const RunLimits* lim, int V, unsigned long long* keys, int nkeys, cudaStream_t st) {
     k_step_begin<<<1, 128, 0, st>>>(c, lim, V, keys, nkeys);
+}
+void launch_run_begin(Ctrl* c, unsigned long long* keys, int nkeys, unsigned* bar, cudaStream_t st) {
+    k_run_begin<<<1, 256, 0, st>>>(c, keys, nkeys, bar);
 }
 void launch_step_end(const Params& P, Ctrl* c, const RunLimits* lim, const double* partials, int nblocks,
                      const double* dt, unsigned long long* keys, int nkeys, PrintRec* hist, int hist_cap,

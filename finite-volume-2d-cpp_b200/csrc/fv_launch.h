@@ -16,6 +16,9 @@ void launch_ctrl_copy(const Ctrl* src, Ctrl* dst, cudaStream_t st);
 void launch_set_limits(RunLimits* d, const RunLimits& v, cudaStream_t st);
 // keys: the dt minimum's ordered-key slots ([n_cases][64]), reset every step
 void launch_step_begin(Ctrl* c, const RunLimits* lim, int V, unsigned long long* keys, int nkeys, cudaStream_t st);
+// before a persistent run kernel: all its key sets, the barrier counter, the
+// failure flag, an empty print-record list
+void launch_run_begin(Ctrl* c, unsigned long long* keys, int nkeys, unsigned* bar, cudaStream_t st);
 void launch_step_end(const Params& P, Ctrl* c, const RunLimits* lim, const double* partials,
                      int nblocks, const double* dt, unsigned long long* keys, int nkeys, PrintRec* hist, int hist_cap,
                      cudaStream_t st, bool pdl = false);

@@ -516,7 +516,7 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int T, Tile2Arrays& t
 
 template <class S>
 void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
-                 double K, FusedArrays<S>& out) {
+                 bool first_order, double K, FusedArrays<S>& out) {
     const int T = t2.tile_cells, F = HostMesh::MAXF;
     const int64_t N = m.n_real, NO = m.owned_real();
     out = FusedArrays<S>();
@@ -533,10 +533,12 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
         edges += in[2];
     }
     out.hd.assign((size_t)slots * 4, 0x8000FFFFu);
-    const bool packed = nf == 3 && sizeof(S) == 4;  // the fourth word holds sl
-    out.rec.assign((size_t)nf * slots * 4, S(0));
-    if (exact) out.rec2.assign((size_t)nf * slots * 2, S(0));
-    out.sl.assign((size_t)slots * (exact ? 2 : 1), S(0));
+    const bool packed = nf == 3 && sizeof(S) == 4 && !first_order;  // the fourth word holds sl
+    if (!first_order) {
+        out.rec.assign((size_t)nf * slots * 4, S(0));
+        if (exact) out.rec2.assign((size_t)nf * slots * 2, S(0));
+        out.sl.assign((size_t)slots * (exact ? 2 : 1), S(0));
+    }
     out.eg.assign((size_t)edges * 4, S(0));
     out.ria.resize((size_t)NO);
     for (int64_t c = 0; c < NO; ++c) out.ria[(size_t)c] = 1.0 / (double)(S)fa.area[(size_t)c];
@@ -552,7 +554,8 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                 if (r < T && r >= own) continue;
                 const int32_t c = dev(r);
                 const double A = fa.area[(size_t)c], Ka = K * std::sqrt(A), K3a = Ka * Ka * Ka;
-                if (exact) { out.sl[(size_t)(so + r) * 2] = (S)(1. / A); out.sl[(size_t)(so + r) * 2 + 1] = (S)K3a; }
+                if (first_order) { /* no limiter */ }
+                else if (exact) { out.sl[(size_t)(so + r) * 2] = (S)(1. / A); out.sl[(size_t)(so + r) * 2 + 1] = (S)K3a; }
                 else out.sl[(size_t)(so + r)] = (S)(1. / K3a);
                 if (packed) std::memcpy(&out.hd[(size_t)(so + r) * 4 + 3], &out.sl[(size_t)(so + r)], 4);
                 for (int f = 0; f < F; ++f) {
@@ -565,6 +568,7 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                     if (el < n_flux) word |= (uint32_t)(el + side * t2.max_flux) << 16 | (uint32_t)(w & 0x4000) << 16;
                     else word |= 0x80000000u;
                     out.hd[(size_t)(so + r) * 4 + f] = word;
+                    if (first_order) continue;
                     const size_t b = (size_t)nf * so + (size_t)f * G + r;
                     const double dx = t2.exf[e] - ta.ccx[(size_t)c], dy = t2.eyf[e] - ta.ccy[(size_t)c];
                     S* v = &out.rec[b * 4];
@@ -583,6 +587,11 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                 S* v = &out.eg[(size_t)(inf[2] + e) * 4];
                 const size_t g = (size_t)eoff + e;
                 v[0] = (S)t2.enx[g]; v[1] = (S)t2.eny[g]; v[2] = (S)t2.ele[g];
+                if (first_order) {
+                    const uint64_t ij = t2.edge_ij[g];
+                    std::memcpy(&v[3], &ij, sizeof(S));
+                    continue;
+                }
                 // a boundary ghost's zero gradient adds this signed zero to its face state
                 const int32_t j = dev((int)(t2.edge_ij[g] >> 16));
                 if (j >= N)
@@ -598,10 +607,10 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
     tiles(0, t2.n_tiles / nt);
     for (auto& th : pool) th.join();
 }
-template void build_fused<float>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, double,
-                                 FusedArrays<float>&);
-template void build_fused<double>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, double,
-                                  FusedArrays<double>&);
+template void build_fused<float>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, bool,
+                                 double, FusedArrays<float>&);
+template void build_fused<double>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, bool,
+                                  double, FusedArrays<double>&);
 
 // ----------------------------------------------------------------------------
 // Domain decomposition.  The reference decomposes with gmsh partitions and

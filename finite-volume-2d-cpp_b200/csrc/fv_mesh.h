@@ -113,6 +113,8 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int tile_cells, Tile2
 // (K sqrt(A))^3 per slot); otherwise the cell's Green-Gauss coefficients
 // a = w le n / A (outward normal, the neighbour's weight) and face centre -
 // centroid, evaluated in FP64 and rounded once, with 1 / (K sqrt(A))^3 per slot.
+// first_order: no records, and each flux edge's two slots in the bits of its
+// fourth value.
 template <class S>
 struct FusedArrays {
     int nf = 3;                          // faces per slot in rec: 3, or 4 with quadrilaterals
@@ -124,7 +126,7 @@ struct FusedArrays {
 };
 template <class S>
 void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
-                 double K, FusedArrays<S>& out);
+                 bool first_order, double K, FusedArrays<S>& out);
 
 // One part of a decomposition of a single mesh into n_parts parts.  Part p
 // owns device real cells [own_off[p], own_off[p+1]) (contiguous ranges of the

@@ -11,6 +11,7 @@
 #include "fv_fused.cuh"
 #include "fv_launch.h"
 #include "fv_mesh.h"
+#include "fv_persist.cuh"
 #include "fv_tile.cuh"
 
 using namespace fvgpu;
@@ -45,6 +46,11 @@ struct fv_solver {
     // gradient kernel also computes dt (no separate dt kernel)
     bool split_first = false;
     FusedParams FPm{};
+    // the persistent run kernel of a mesh whose tiles are all resident at once
+    // (fn null: none), its dt keys and barrier counter
+    RunKernel run_kernel{};
+    unsigned long long* run_keys = nullptr;
+    unsigned* run_bar = nullptr;
     // its schedule (FV_SCHED_*); the work list's per-stage tile counters and
     // CTAs per launch
     int sched = 0;
