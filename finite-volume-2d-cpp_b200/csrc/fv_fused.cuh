@@ -45,8 +45,7 @@ namespace fvgpu {
 //    replaces them, and after the per-cell sums the store holds the residual
 //    warp sums;
 //  - the base state of the owned cells (FP64, [T][4]);
-//  - the flux edges' geometry [max_flux][4] and 1 / area of the owned cells
-//    (exact: the area);
+//  - the flux edges' geometry [max_flux][4] and 1 / area of the owned cells;
 //  - the limited gradients (and, exact, the limiters) of owned cells with a
 //    boundary ghost, for the ghost fill.
 struct FusedSmem {
@@ -373,9 +372,17 @@ template <class M>
 __device__ __forceinline__ void fused_speeds(double gamma, const typename M::S* q, typename M::S* w) {
     if constexpr (M::exact) {
         const double gm1 = gamma - 1;
-        w[0] = q[1] / q[0];
-        w[1] = q[2] / q[0];
-        w[2] = sqrt((gm1 * (q[3] - 0.5 / q[0] * (q[1] * q[1] + q[2] * q[2]))) * gamma / q[0]);
+        bool ok = true;
+        const exact::Recip r = exact::recip(q[0], ok);
+        w[0] = exact::quot(q[1], r, ok);
+        w[1] = exact::quot(q[2], r, ok);
+        double c2 = exact::quot((gm1 * (q[3] - exact::quot(0.5, r, ok) * (q[1] * q[1] + q[2] * q[2]))) * gamma, r, ok);
+        if (!ok) {
+            w[0] = q[1] / q[0];
+            w[1] = q[2] / q[0];
+            c2 = (gm1 * (q[3] - 0.5 / q[0] * (q[1] * q[1] + q[2] * q[2]))) * gamma / q[0];
+        }
+        w[2] = sqrt(c2);
         w[3] = 0.;
     } else {
         fast::speeds((typename M::S)gamma, q, w);
@@ -429,31 +436,76 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
         }
         const double invA = geo.sl[0], K3a = geo.sl[1];
         const double tol = 1e-15;
+        // the divisions of a group of variables together (exact::quot)
+        constexpr int GK = NV == 4 ? 1 : NV;
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            gx[k] *= invA; gy[k] *= invA;
-            const double delta_max = qmx[k] - qs[k];
-            const double delta_min = qmn[k] - qs[k];
-            const double d2 = (delta_max - delta_min) * (delta_max - delta_min);
-            double sig;
-            if (d2 <= K3a) sig = 1.;
-            else if (d2 <= 2 * K3a) {
-                const double y = (d2 / K3a - 1.0);
-                sig = 2.0 * y * y * y - 3.0 * y * y + 1.0;
-            } else sig = 0.;
+        for (int k0 = 0; k0 < NV; k0 += GK) {
+            double sig[GK], y[GK][NF];
+            bool on[GK][NF], ok = true, limited = false;
 #pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                if (!geo.face(f)) continue;
-                const double dqg = gx[k] * geo.dx(f) + gy[k] * geo.dy(f);
-                double lv = 1.0;
-                if (sig < 1.0) {
-                    if (dqg > tol) lv = exact::limiter_func(P.limiter, delta_max / dqg);
-                    else if (dqg < -tol) lv = exact::limiter_func(P.limiter, delta_min / dqg);
-                    else lv = 1.0;
-                }
-                lv = sig + (1.0 - sig) * lv;
-                lim[k] = exact::dmin(lim[k], lv);
+            for (int i = 0; i < GK; ++i) {
+                const int k = k0 + i;
+                gx[k] *= invA; gy[k] *= invA;
+                const double delta_max = qmx[k] - qs[k];
+                const double delta_min = qmn[k] - qs[k];
+                const double d2 = (delta_max - delta_min) * (delta_max - delta_min);
+                if (d2 <= K3a) sig[i] = 1.;
+                else if (d2 <= 2 * K3a) {
+                    const double z = (d2 / K3a - 1.0);
+                    sig[i] = 2.0 * z * z * z - 3.0 * z * z + 1.0;
+                } else sig[i] = 0.;
+                limited |= sig[i] < 1.0;
             }
+            if (!limited) continue;  // sig = 1: lim = 1
+#pragma unroll
+            for (int i = 0; i < GK; ++i) {
+                const int k = k0 + i;
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    on[i][f] = false;
+                    y[i][f] = 0.;
+                    if (!geo.face(f)) continue;
+                    const double dqg = gx[k] * geo.dx(f) + gy[k] * geo.dy(f);
+                    on[i][f] = sig[i] < 1.0 && (dqg > tol || dqg < -tol);
+                    const double num = on[i][f] ? (dqg > tol ? qmx[k] - qs[k] : qmn[k] - qs[k]) : 0.;
+                    const double den = on[i][f] ? dqg : 1.;
+                    y[i][f] = exact::quot(num, exact::recip(den, ok), ok);
+                }
+            }
+            if (P.limiter == 2) {
+#pragma unroll
+                for (int i = 0; i < GK; ++i)
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        const double z = y[i][f];
+                        y[i][f] = exact::quot(z * z + 2.0 * z, exact::recip(z * z + z + 2.0, ok), ok);
+                    }
+            } else {
+#pragma unroll
+                for (int i = 0; i < GK; ++i)
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) y[i][f] = exact::limiter_func(P.limiter, y[i][f]);
+            }
+            if (!ok) {  // an operand out of exact::quot's range
+#pragma unroll
+                for (int i = 0; i < GK; ++i)
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        if (!on[i][f]) continue;
+                        const int k = k0 + i;
+                        const double dqg = gx[k] * geo.dx(f) + gy[k] * geo.dy(f);
+                        y[i][f] = exact::limiter_func(P.limiter, (dqg > tol ? qmx[k] - qs[k] : qmn[k] - qs[k]) / dqg);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < GK; ++i)
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    if (!geo.face(f)) continue;
+                    double lv = on[i][f] ? y[i][f] : 1.0;
+                    lv = sig[i] + (1.0 - sig[i]) * lv;
+                    lim[k0 + i] = exact::dmin(lim[k0 + i], lv);
+                }
         }
     } else {
         S mn[NV], mx[NV], sig[NV];
@@ -570,9 +622,10 @@ __device__ __forceinline__ void fused_update(const FusedParams& FP, const TileIO
     double qt[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) qt[k] = 0.;
-    const double ra = RA[uc];
-    double A = ra;
-    if (!M::exact && io.partials != nullptr) A = (double)__ldg((const S*)FP.area + c);
+    const double ra = RA[uc];  // 1 / area
+    double A = 1.;
+    if (M::exact || io.partials != nullptr) A = (double)__ldg((const S*)FP.area + c);
+    bool ok = M::exact ? exact::quot_range(A) && exact::quot_range(ra) : true;
     uint32_t any = 0;
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
@@ -581,7 +634,22 @@ __device__ __forceinline__ void fused_update(const FusedParams& FP, const TileIO
         S fe[NV];
         PL::get(FS, L.lf, word_unit(own[f]), v0, fe);
 #pragma unroll
-        for (int k = 0; k < NV; ++k) qt[k] += M::exact ? (double)fe[k] / A : (double)fe[k];
+        for (int k = 0; k < NV; ++k) {
+            if constexpr (M::exact) qt[k] += exact::quot(fe[k], exact::recip_of(A, ra), ok);
+            else qt[k] += (double)fe[k];
+        }
+    }
+    if (M::exact && !ok) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) qt[k] = 0.;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            if (f == 3 && word_nbr(own[f]) == 0xFFFF) continue;
+            S fe[NV];
+            PL::get(FS, L.lf, word_unit(own[f]), v0, fe);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) qt[k] += (double)fe[k] / A;
+        }
     }
     if constexpr (!M::exact) {
 #pragma unroll
@@ -756,7 +824,7 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
         const uint4* src = reinterpret_cast<const uint4*>((const S*)FP.eg + 4 * (size_t)flux_off);
         uint4* dst = reinterpret_cast<uint4*>(smem_raw + L.eg);
         for (int i = l; i < C * n_flux; i += blockDim.x) cpa16(dst + i, src + i);
-        if (l < nown) cpa8(RA + l, (M::exact ? (const double*)FP.area : FP.ria) + c0 + l);
+        if (l < nown) cpa8(RA + l, FP.ria + c0 + l);
     }
     // the owned cell of the update phase (r0 < nown there) and its faces
     const int uc = r0;
@@ -872,7 +940,7 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
         P4::get(FS, L.lf, el, 0, qL);
         P4::get(FS, L.lf, el + FP.max_flux, 0, qR);
         if constexpr (M::exact) {
-            exact::flux<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
+            exact::flux_dev<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
 #pragma unroll
             for (int k = 0; k < V; ++k) f[k] *= e[2];
         } else {

@@ -202,7 +202,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
         const uint4* src = reinterpret_cast<const uint4*>((const S*)FP.eg + 4 * (size_t)flux_off);
         uint4* dst = reinterpret_cast<uint4*>(smem_raw + L.eg);
         for (int i = l; i < NU * n_flux; i += blockDim.x) cpa16(dst + i, src + i);
-        if (l < nown) cpa8(RA + l, (M::exact ? (const double*)FP.area : FP.ria) + c0 + l);
+        if (l < nown) cpa8(RA + l, FP.ria + c0 + l);
         cpa_wait();
     }
     const int tc = (P.global_dt && P.n_cases > 1) ? P.tile_case[t] : 0;
@@ -317,7 +317,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
                     P4::get(Q, L.ls, (int)(ij >> 16), 0, qR);
                 }
                 if constexpr (M::exact) {
-                    exact::flux<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
+                    exact::flux_dev<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
 #pragma unroll
                     for (int i = 0; i < V; ++i) f[i] *= e[2];
                 } else {

@@ -91,6 +91,125 @@ FV_HD void flux(double gamma, double* f, const double* qi, const double* qj,
     else roe<FLUX == 1>(gamma, f, qi, qj, n0, n1);
 }
 
+#ifdef __CUDACC__
+// Correctly rounded quotients without a branch per division: the reciprocal by
+// Newton-Raphson steps and the quotient by Markstein's correction (P. W.
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990).  With y within 1 ulp of 1 / b,
+// y + y (1 - b y) in fused steps is RN(1 / b) unless every mantissa bit of b is
+// set, and q = RN(a y) corrected by (a - b q) y is RN(a / b).  Operands outside
+// 2^+-500 (or that mantissa) clear `ok`: the caller then divides with the
+// operator instead.  One reciprocal serves every quotient by b, and quotients
+// of one b or several overlap, where a division each waits out its own chain.
+struct Recip {
+    double b, y;
+};
+__device__ __forceinline__ bool quot_range(double x) {
+    return (unsigned)((__double2hiint(x) & 0x7fffffff) - ((1023 - 500) << 20)) < (1000u << 20);
+}
+__device__ __forceinline__ Recip recip_of(double b, double y) { return Recip{b, y}; }
+__device__ __forceinline__ Recip recip(double b, bool& ok) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    ok &= quot_range(b) && !(__double2loint(b) == -1 && (__double2hiint(b) & 0xfffff) == 0xfffff);
+    return Recip{b, y};
+}
+__device__ __forceinline__ double quot(double a, const Recip& r, bool& ok) {
+    const double t = __dmul_rn(a, r.y);
+    const double q = __fma_rn(__fma_rn(-r.b, t, a), r.y, t);
+    ok &= quot_range(a) || a == 0.0;
+    return a == 0.0 ? t : q;  // a signed zero keeps its sign
+}
+
+// roe() of doubles with its divisions as above: the same operations in the same
+// order, so the same bits.  16 divisions by 6 different denominators, two of
+// them each other's double.  Returns false when an operand is out of range (f
+// is then not set).
+template <bool FS_ASSOC>
+__device__ __forceinline__ bool roe_quot(double gamma, double* f, const double* qi, const double* qj, double n0,
+                                         double n1) {
+    bool ok = true;
+    const Recip ri = recip(qi[0], ok), rj = recip(qj[0], ok);
+    const double pi = (gamma - 1) * (qi[3] - quot(0.5, ri, ok) * (qi[1] * qi[1] + qi[2] * qi[2]));
+    const double pj = (gamma - 1) * (qj[3] - quot(0.5, rj, ok) * (qj[1] * qj[1] + qj[2] * qj[2]));
+    const double Vi = quot(qi[1] * n0 + qi[2] * n1, ri, ok);
+    const double Vj = quot(qj[1] * n0 + qj[2] * n1, rj, ok);
+    const double uL = quot(qi[1], ri, ok), vL = quot(qi[2], ri, ok);
+    const double uR = quot(qj[1], rj, ok), vR = quot(qj[2], rj, ok);
+    const double pL = pi, pR = pj;
+    const double hL = quot(qi[3] + pL, ri, ok), hR = quot(qj[3] + pR, rj, ok);
+    const double srhoL = sqrt(qi[0]), srhoR = sqrt(qj[0]);
+    const double rho = srhoR * srhoL;
+    const Recip rs = recip(srhoL + srhoR, ok);
+    const double u = quot(uL * srhoL + uR * srhoR, rs, ok);
+    const double v = quot(vL * srhoL + vR * srhoR, rs, ok);
+    const double h = quot(hL * srhoL + hR * srhoR, rs, ok);
+    const double q2 = u * u + v * v;
+    const double c = sqrt((gamma - 1.) * (h - 0.5 * q2));
+    const Recip rc = recip(c * c, ok), r2c = recip_of(2. * rc.b, 0.5 * rc.y);
+    const double V = u * n0 + v * n1;
+    const double VR = uR * n0 + vR * n1;
+    const double VL = uL * n0 + vL * n1;
+    const double lambda_cm = fabs(dmin(V - c, VL - c));
+    const double lambda_c = fabs(V);
+    const double lambda_cp = fabs(dmax(V + c, VR + c));
+    const double kF1 = quot(lambda_cm * ((pR - pL) - rho * c * (VR - VL)), r2c, ok);
+    const double kF234_0 = lambda_c * ((qj[0] - qi[0]) - quot(pR - pL, rc, ok));
+    const double kF234_1 = lambda_c * rho;
+    const double kF5 = quot(lambda_cp * ((pR - pL) + rho * c * (VR - VL)), r2c, ok);
+    if (!ok) return false;
+    if (FS_ASSOC) {
+        f[0] = (qi[0] * Vi + qj[0] * Vj) * 0.5;
+        f[1] = (qi[1] * Vi + pi * n0 + qj[1] * Vj + pj * n0) * 0.5;
+        f[2] = (qi[2] * Vi + pi * n1 + qj[2] * Vj + pj * n1) * 0.5;
+        f[3] = ((qi[3] + pi) * Vi + (qj[3] + pj) * Vj) * 0.5;
+    } else {
+        f[0] = (qi[0] * Vi + qj[0] * Vj) * 0.5;
+        f[1] = ((qi[1] * Vi + pi * n0) + (qj[1] * Vj + pj * n0)) * 0.5;
+        f[2] = ((qi[2] * Vi + pi * n1) + (qj[2] * Vj + pj * n1)) * 0.5;
+        f[3] = ((qi[3] + pi) * Vi + (qj[3] + pj) * Vj) * 0.5;
+    }
+    f[0] -= 0.5 * (kF1 + kF234_0 + kF5);
+    f[1] -= 0.5 * (kF1 * (u - c * n0) + kF234_0 * u + kF234_1 * (uR - uL - (VR - VL) * n0) + kF5 * (u + c * n0));
+    f[2] -= 0.5 * (kF1 * (v - c * n1) + kF234_0 * v + kF234_1 * (vR - vL - (VR - VL) * n1) + kF5 * (v + c * n1));
+    f[3] -= 0.5 * (kF1 * (h - c * V) + kF234_0 * q2 * 0.5 + kF234_1 * (u * (uR - uL) + v * (vR - vL) - V * (VR - VL)) + kF5 * (h + c * V));
+    return true;
+}
+template <bool FS_ASSOC>
+static __device__ __noinline__ void roe_call(double gamma, double* f, const double* qi, const double* qj, double n0,
+                                             double n1) {
+    roe<FS_ASSOC>(gamma, f, qi, qj, n0, n1);
+}
+// flux<FLUX>() in device code
+template <int FLUX>
+__device__ __forceinline__ void flux_dev(double gamma, double* f, const double* qi, const double* qj, double n0,
+                                         double n1) {
+    if constexpr (FLUX == 3) {
+        burgers(f, qi, qj, n0, n1);
+    } else {
+        if (!roe_quot<FLUX == 1>(gamma, f, qi, qj, n0, n1)) {
+            // (through copies, so that the call does not force the arrays of
+            // the fast path into local memory)
+            double a[4], b[4], g[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { a[k] = qi[k]; b[k] = qj[k]; }
+            roe_call<FLUX == 1>(gamma, g, a, b, n0, n1);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f[k] = g[k];
+        }
+    }
+}
+// pressure of a state (the guard's and the time step's expression)
+__device__ __forceinline__ double pres_dev(double gamma, const double* q) {
+    bool ok = true;
+    double h = quot(0.5, recip(q[0], ok), ok);
+    if (!ok) h = 0.5 / q[0];
+    return (gamma - 1) * (q[3] - h * (q[1] * q[1] + q[2] * q[2]));
+}
+#endif
+
 // Face gradient of the diffusive fluxes (gradient_for_diffusion,
 // explicit.cpp:70-109): the mean of the two cell gradients, with its
 // component along the centroid line ci - cj replaced by the difference

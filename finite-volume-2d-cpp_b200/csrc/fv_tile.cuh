@@ -213,7 +213,7 @@ struct Rec {
 template <class S, bool EXACT>
 __device__ __forceinline__ bool face_state_bad(const Params& P, const S* qf) {
     if constexpr (EXACT) {
-        const S p = ((S)P.gamma - S(1)) * (qf[3] - S(0.5) / qf[0] * (qf[1] * qf[1] + qf[2] * qf[2]));
+        const S p = exact::pres_dev(P.gamma, qf);
         return !(qf[0] > S(0)) || !(p > S(0));
     } else {
         const S m2 = fast::fma_(qf[2], qf[2], qf[1] * qf[1]);
@@ -835,7 +835,7 @@ __device__ __forceinline__ void diffusive_edge_flux(const Params& P, const typen
         double gxf[V], gyf[V];
         exact::face_gradient<V>(gxf, gyf, gxi, gyi, gxj, gyj, qci, qcj, cix, ciy, cjx, cjy);
         if constexpr (FLUX == 5) {
-            exact::roe<false>(P.gamma, f, qL, qR, n0, n1);
+            exact::flux_dev<2>(P.gamma, f, qL, qR, n0, n1);
             exact::ns_viscous(P, f, qL, qR, gxf, gyf, n0, n1);
         } else {
             exact::burgers_diffusion(f, qL, qR, gxf, gyf, n0, n1);
@@ -998,7 +998,7 @@ __device__ __forceinline__ void tile_stage(const TileParams& TP, const TileIO& i
                                           ri[R::OC + 1] - rj[R::OC + 1], n0, n1);
                 }
             } else if constexpr (M::exact) {
-                exact::flux<FLUX>(P.gamma, f, qL, qR, n0, n1);
+                exact::flux_dev<FLUX>(P.gamma, f, qL, qR, n0, n1);
             } else {
                 fast::flux_le<FLUX, S>((S)P.gamma, f, qL, qR, n0, n1, sle[el]);
             }
