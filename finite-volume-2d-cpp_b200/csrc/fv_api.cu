@@ -83,14 +83,16 @@ int upload_fused(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const Ti
     build_fused<S>(m, fa, ta, t2, exact, first_order, K, a);
     FusedParams& F = s->FPm;
     F.nf = a.nf;
-    const int32_t* info; const uint32_t* hd; const S *rec, *rec2, *sl, *eg;
+    F.max_ghost = a.max_ghost;
+    const int32_t* info; const uint32_t* hd; const int32_t* gl; const S *rec, *rec2, *sl, *eg, *gd;
     int rc;
     if ((rc = upload_v(s, a.info, &info)) || (rc = upload_v(s, a.hd, &hd)) || (rc = upload_v(s, a.rec, &rec)) || (rc = upload_v(s, a.rec2, &rec2)) || (rc = upload_v(s, a.sl, &sl)) ||
-        (rc = upload_v(s, a.eg, &eg)) || (rc = upload_v(s, a.ria, &F.ria)))
+        (rc = upload_v(s, a.eg, &eg)) || (rc = upload_v(s, a.gl, &gl)) || (rc = upload_v(s, a.gd, &gd)) || (rc = upload_v(s, a.ria, &F.ria)))
         return rc;
     F.info = reinterpret_cast<const int4*>(info);
     F.hd = reinterpret_cast<const uint4*>(hd);
-    F.rec = rec; F.rec2 = rec2; F.sl = sl; F.eg = eg;
+    F.rec = rec; F.rec2 = rec2; F.sl = sl; F.eg = eg; F.gd = gd;
+    F.gl = reinterpret_cast<const int2*>(gl);
     return FV_OK;
 }
 // lanes per cell of the fused kernel's gradient and update phases
@@ -105,11 +107,12 @@ int choose_run_kernel(fv_solver* s) {
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
     if (!coop) return FV_OK;
+    const size_t smem = tile::smem_fused(s->precision, s->FPm);
+    if (smem > (size_t)227 * 1024) return FV_OK;
     FusedParams F = s->FPm;
     F.P = s->TP.P;
     RunKernel k[kRunKernels];
     tile::run_kernels(s->precision, F, k);
-    const size_t smem = tile::smem_fused(s->precision, F);
     for (int i = 0; i < kRunKernels; ++i) {
         if (!k[i].fn) continue;
         {
@@ -1055,7 +1058,7 @@ static int launch_run(fv_solver* s, const std::vector<double>& alpha, int steps)
     F.P = s->TP.P;
     void* args[] = {&F, &D};
     CK(cudaLaunchCooperativeKernel(s->run_kernel.fn, dim3((unsigned)s->n_tiles), dim3((unsigned)s->run_kernel.threads),
-                                   args, (size_t)std::max(F.L.total, F.L.total_grad), s->stream));
+                                   args, (size_t)std::max(F.L.total_run, F.L.total_grad), s->stream));
     return FV_OK;
 }
 

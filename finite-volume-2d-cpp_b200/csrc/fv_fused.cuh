@@ -49,11 +49,11 @@ namespace fvgpu {
 //  - the limited gradients (and, exact, the limiters) of owned cells with a
 //    boundary ghost, for the ghost fill.
 struct FusedSmem {
-    int q, fs, qb, gx, gy, lm, eg, ria, total, total_grad;
+    int q, fs, qb, gx, gy, lm, eg, ria, gl, gd, total, total_grad, total_run;
     int ls, lf, lt;  // plane strides (units)
 };
 template <class M>
-inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int T) {
+inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int max_ghost, int T) {
     constexpr int NU = (int)(4 * sizeof(typename M::S) / 16);
     FusedSmem L{};
     L.ls = max_slots;
@@ -70,6 +70,10 @@ inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int T) {
     L.eg = o; o += 16 * NU * max_flux;
     L.ria = o; o += 8 * T;
     L.total = o;
+    // the run kernel keeps the tile's ghosts behind that
+    L.gd = o; o += 16 * NU * max_ghost;
+    L.gl = o; o += (8 * max_ghost + 15) / 16 * 16;
+    L.total_run = o;
     // the gradient kernel of the split layout and the dt kernel: the states
     // and {u, v, c} of the gradient slots
     L.total_grad = L.fs + 16 * NU * max_grad;
@@ -83,7 +87,9 @@ struct FusedParams {
     int lanes;                 // lanes per cell of the gradient and update phases: 1, 2 or 4
     int nf;                    // faces per gradient slot: 3 (triangles only) or 4
     int max_slots, max_grad, max_flux;
-    const int4* info;          // [n_tiles][2]: {slot_off, halo_off, flux_off, n_flux}, {n1, n2, owned cells, 0}
+    // [n_tiles][2]: {slot_off, halo_off, flux_off, n_flux},
+    // {n1, n2, owned cells | ghosts << 16, ghost_off}
+    const int4* info;
     const int32_t* halo;       // device cell of each ring-1, then ring-2 slot
     // per gradient slot (T owned, then n1 ring-1 slots of every tile) four
     // face words: neighbour slot (0xFFFF = no face) | face-state unit << 16
@@ -105,6 +111,11 @@ struct FusedParams {
     const double* ria;         // [n_own] 1 / area
     const void* area;          // S [n_total]
     FusedSmem L;               // shared-memory layout (fused_smem)
+    // boundary ghosts of the tiles' owned cells, one thread each: {interior
+    // slot | group << 16, device cell}, and S[4] {n_x, n_y, d_x, d_y}
+    const int2* gl;
+    const void* gd;
+    int max_ghost;             // ghosts of a tile at most
 };
 
 constexpr uint32_t kWordGhost = 0x40000000u, kWordNoFlux = 0x80000000u;
@@ -584,7 +595,7 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
                 PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
                 if constexpr (M::exact) {
                     // the signed zero that the ghost's zero gradient adds
-                    const double z = __ldg((const double*)FP.eg + 4 * (size_t)(flux_off + el) + 3);
+                    const double z = reinterpret_cast<const double*>(smem_raw + L.eg)[4 * el + 3];
 #pragma unroll
                     for (int k = 0; k < NV; ++k) qn[k] += z;
                 }
@@ -598,25 +609,18 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
 }
 
 // Sum of the fluxes of owned cell uc (this lane's variables) in reference edge
-// order, RK update and ghost fill (update_cells + update_bounds,
-// explicit.cpp:368-417); res: its residual terms when partial sums are due.
-// O2: ghosts from the limited gradients, else from the cell value.
-template <class M, int NV, int NF, bool REMOTE, bool O2>
+// order and RK update (update_cells, explicit.cpp:368-378); res: its residual
+// terms when partial sums are due.  ghosts: the tile fills boundary ghosts.
+template <class M, int NV, int NF, bool REMOTE>
 __device__ __forceinline__ void fused_update(const FusedParams& FP, const TileIO& io, unsigned char* smem_raw,
-                                             const uint32_t* own, int uc, int v0, int c0, int slot_off, int halo_off,
-                                             int flux_off, int G, int tc, double dtc, const double& s_dt,
-                                             const PartIO& pio, double* res) {
+                                             const uint32_t* own, int uc, int v0, int c0, int tc, double dtc,
+                                             const double& s_dt, bool ghosts, const PartIO& pio, double* res) {
     using S = typename M::S;
     using PL = Planes<S, NV>;
-    constexpr int V = 4;
     const Params& P = FP.P;
     const FusedSmem& L = FP.L;
-    const int T = FP.T, N = P.n_real;
     uint4* FS = reinterpret_cast<uint4*>(smem_raw + L.fs);
     const double* QB = reinterpret_cast<const double*>(smem_raw + L.qb);
-    uint4* GX = reinterpret_cast<uint4*>(smem_raw + L.gx);
-    uint4* GY = reinterpret_cast<uint4*>(smem_raw + L.gy);
-    uint4* LM = reinterpret_cast<uint4*>(smem_raw + L.lm);
     const double* RA = reinterpret_cast<const double*>(smem_raw + L.ria);
     const int c = c0 + uc;
     double qt[NV];
@@ -626,11 +630,9 @@ __device__ __forceinline__ void fused_update(const FusedParams& FP, const TileIO
     double A = 1.;
     if (M::exact || io.partials != nullptr) A = (double)__ldg((const S*)FP.area + c);
     bool ok = M::exact ? exact::quot_range(A) && exact::quot_range(ra) : true;
-    uint32_t any = 0;
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
         if (f == 3 && word_nbr(own[f]) == 0xFFFF) continue;
-        any |= own[f];
         S fe[NV];
         PL::get(FS, L.lf, word_unit(own[f]), v0, fe);
 #pragma unroll
@@ -695,63 +697,68 @@ __device__ __forceinline__ void fused_update(const FusedParams& FP, const TileIO
                 }
             }
         }
-        if (any & kWordGhost) {
-            S gxs[NV], gys[NV], lms[NV];
-            if constexpr (O2) {
-                PL::get(GX, L.lt, uc, v0, gxs);
-                PL::get(GY, L.lt, uc, v0, gys);
-                if constexpr (M::exact) PL::get(LM, L.lt, uc, v0, lms);
-            }
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                if ((f == 3 && word_nbr(own[f]) == 0xFFFF) || !(own[f] & kWordGhost)) continue;
-                const int u = word_unit(own[f]), el = u < FP.max_flux ? u : u - FP.max_flux;
-                const int g = FP.halo[halo_off + word_nbr(own[f]) - T];
-                const S* ep = (const S*)FP.eg + 4 * (size_t)(flux_off + el);
-                S qint[NV], all[V], b[V], bs[NV];
-                if constexpr (O2) {
-                    const size_t ri = (size_t)NF * slot_off + (size_t)f * G + uc;
-                    const S e0 = M::exact ? ((const S*)FP.rec2)[2 * ri] : ((const S*)FP.rec)[4 * ri + 2];
-                    const S e1 = M::exact ? ((const S*)FP.rec2)[2 * ri + 1] : ((const S*)FP.rec)[4 * ri + 3];
-#pragma unroll
-                    for (int k = 0; k < NV; ++k) {
-                        if constexpr (M::exact) qint[k] = qs[k] + (gxs[k] * e0 + gys[k] * e1) * lms[k];
-                        else qint[k] = fast::fma_(gys[k], e1, fast::fma_(gxs[k], e0, qs[k]));
-                    }
-                    guard_share<S, NV, M::exact>(P, qint, qs);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < NV; ++k) qint[k] = qs[k];
-                }
-                share<S, NV>(qint, all);
-                if constexpr (M::exact) exact::bc<V>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
-                else fast::bc<V, S>(P, P.ghost_group[g - N], g - N, b, all, ep[0], ep[1]);
-                own_share<S, NV>(b, v0, bs);
-                if (sizeof(S) == 8) {
-                    stv<S, NV>((S*)io.q_out + 4 * (size_t)g + v0, bs);
-                } else {
-                    stv<S, NV>((S*)io.s_out + 4 * (size_t)g + v0, bs);
-                    if (io.write_f64) {
-                        double bd[NV];
-#pragma unroll
-                        for (int k = 0; k < NV; ++k) bd[k] = (double)bs[k];
-                        stv<double, NV>(io.q_out + 4 * (size_t)g + v0, bd);
-                    }
-                }
-                if constexpr (REMOTE) {
-                    const RemoteIO& R = *pio.remote;
-                    const int go = g - N;
-                    if (go < R.n_own_ghost)
-                        for (int i = R.ghost_off[go]; i < R.ghost_off[go + 1]; ++i) {
-                            const int2 d = R.ghost_dst[i];
-                            stv<S, NV>((S*)R.dst[d.x] + 4 * (size_t)d.y + v0, bs);
-                        }
-                }
-            }
-        }
+        if (ghosts) PL::put(reinterpret_cast<uint4*>(smem_raw + L.q), L.ls, uc, v0, qs);  // for fused_ghosts
         if (io.partials != nullptr) {
 #pragma unroll
             for (int k = 0; k < NV; ++k) res[k] = qt[k] * qt[k] * A;
+        }
+    }
+}
+
+// Ghost fill of the tile's boundary ghosts (update_bounds, explicit.cpp:380-417),
+// one thread each, once every thread has stored its cell's new state.  O2: from
+// the limited gradients, else from the cell value.  gl, gd: the tile's entries.
+template <class M, bool REMOTE, bool O2>
+__device__ __forceinline__ void fused_ghosts(const FusedParams& FP, const TileIO& io, unsigned char* smem_raw,
+                                             const int2* gl, const typename M::S* gd, int n, const PartIO& pio) {
+    using S = typename M::S;
+    using P4 = Planes<S, 4>;
+    const Params& P = FP.P;
+    const FusedSmem& L = FP.L;
+    const int N = P.n_real;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int2 e = gl[i];
+        const int uc = e.x & 0xFFFF, group = e.x >> 16, g = e.y;
+        S qs[4], qint[4], b[4];
+        const S n0 = gd[4 * i], n1 = gd[4 * i + 1];
+        P4::get(reinterpret_cast<const uint4*>(smem_raw + L.q), L.ls, uc, 0, qs);
+        if constexpr (O2) {
+            S gx[4], gy[4], lm[4];
+            const S d0 = gd[4 * i + 2], d1 = gd[4 * i + 3];
+            P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gx), L.lt, uc, 0, gx);
+            P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gy), L.lt, uc, 0, gy);
+            if constexpr (M::exact) P4::get(reinterpret_cast<const uint4*>(smem_raw + L.lm), L.lt, uc, 0, lm);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if constexpr (M::exact) qint[k] = qs[k] + (gx[k] * d0 + gy[k] * d1) * lm[k];
+                else qint[k] = fast::fma_(gy[k], d1, fast::fma_(gx[k], d0, qs[k]));
+            }
+            guard_share<S, 4, M::exact>(P, qint, qs);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) qint[k] = qs[k];
+        }
+        if constexpr (M::exact) exact::bc<4>(P, group, g - N, b, qint, n0, n1);
+        else fast::bc<4, S>(P, group, g - N, b, qint, n0, n1);
+        if (sizeof(S) == 8) {
+            stv<S, 4>((S*)io.q_out + 4 * (size_t)g, b);
+        } else {
+            stv<S, 4>((S*)io.s_out + 4 * (size_t)g, b);
+            if (io.write_f64) {
+                double bd[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) bd[k] = (double)b[k];
+                stv<double, 4>(io.q_out + 4 * (size_t)g, bd);
+            }
+        }
+        if constexpr (REMOTE) {
+            const RemoteIO& R = *pio.remote;
+            const int go = g - N;
+            if (go < R.n_own_ghost)
+                for (int j = R.ghost_off[go]; j < R.ghost_off[go + 1]; ++j) {
+                    const int2 d = R.ghost_dst[j];
+                    stv<S, 4>((S*)R.dst[d.x] + 4 * (size_t)d.y, b);
+                }
         }
     }
 }
@@ -799,8 +806,8 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
     const int N = P.n_real, T = FP.T;
     const int4 ia = FP.info[2 * t], ib = FP.info[2 * t + 1];
     const int slot_off = ia.x, halo_off = ia.y, flux_off = ia.z, n_flux = ia.w;
-    const int n1 = ib.x, nh = ib.x + ib.y;
-    const int c0 = t * T, nown = PART ? ib.z : min(T, N - c0);
+    const int n1 = ib.x, nh = ib.x + ib.y, n_ghost = ib.z >> 16;
+    const int c0 = t * T, nown = PART ? (ib.z & 0xFFFF) : min(T, N - c0);
     const int G = T + n1;
     const FusedSmem& L = FP.L;
     uint4* Q = reinterpret_cast<uint4*>(smem_raw + L.q);
@@ -960,8 +967,11 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
 #pragma unroll
     for (int k = 0; k < NV; ++k) res[k] = 0.;
     if (uc < nown) {
-        fused_update<M, NV, NF, REMOTE, true>(FP, io, smem_raw, own, uc, v0, c0, slot_off, halo_off, flux_off, G, tc, dtc,
-                                              s_dt, pio, res);
+        fused_update<M, NV, NF, REMOTE>(FP, io, smem_raw, own, uc, v0, c0, tc, dtc, s_dt, n_ghost != 0, pio, res);
+    }
+    if (n_ghost != 0) {
+        __syncthreads();
+        fused_ghosts<M, REMOTE, true>(FP, io, smem_raw, FP.gl + ib.w, (const S*)FP.gd + 4 * (size_t)ib.w, n_ghost, pio);
     }
     if (io.partials != nullptr) fused_partials<NV>(io, smem_raw + L.fs, t, v0, res);
     if constexpr (REMOTE) {
@@ -1055,8 +1065,8 @@ template <class M>
 struct FusedLaunch {
     // lays out the tiles' shared memory (FP.L); the bytes of the largest launch
     static size_t smem(FusedParams& FP) {
-        FP.L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_flux, FP.T);
-        return (size_t)std::max(FP.L.total, FP.L.total_grad);
+        FP.L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_flux, FP.max_ghost, FP.T);
+        return (size_t)std::max(FP.L.total_run, FP.L.total_grad);
     }
     static cudaError_t prepare(FusedParams& FP) {
         static std::mutex mu;

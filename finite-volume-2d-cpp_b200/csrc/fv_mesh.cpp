@@ -542,6 +542,28 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
     out.eg.assign((size_t)edges * 4, S(0));
     out.ria.resize((size_t)NO);
     for (int64_t c = 0; c < NO; ++c) out.ria[(size_t)c] = 1.0 / (double)(S)fa.area[(size_t)c];
+    // each tile's boundary ghosts, by interior cell
+    std::vector<int32_t> ghosts;
+    for (int32_t g = 0; g < (int32_t)fa.ghost_cell.size(); ++g)
+        if (fa.ghost_cell[(size_t)g] < NO) ghosts.push_back(g);
+    std::stable_sort(ghosts.begin(), ghosts.end(),
+                     [&](int32_t x, int32_t y) { return fa.ghost_cell[(size_t)x] < fa.ghost_cell[(size_t)y]; });
+    size_t next = 0;
+    for (int t = 0; t < t2.n_tiles; ++t) {
+        const int64_t c0 = (int64_t)t * T, c1 = c0 + t2.info[(size_t)8 * t + 7];
+        int32_t* inf = &out.info[(size_t)8 * t];
+        inf[7] = (int32_t)(out.gl.size() / 2);
+        int n = 0;
+        for (; next < ghosts.size() && fa.ghost_cell[(size_t)ghosts[next]] < c1; ++next, ++n) {
+            const int32_t b = ghosts[next];
+            out.gl.push_back((int32_t)(fa.ghost_cell[(size_t)b] - c0) | fa.ghost_group[(size_t)b] << 16);
+            out.gl.push_back((int32_t)(N + b));
+            for (double v : {fa.g_nx[(size_t)b], fa.g_ny[(size_t)b], fa.g_dx[(size_t)b], fa.g_dy[(size_t)b]})
+                out.gd.push_back((S)v);
+        }
+        inf[6] |= n << 16;
+        out.max_ghost = std::max(out.max_ghost, n);
+    }
     auto tiles = [&](int t0, int t1) {
         for (int t = t0; t < t1; ++t) {
             const int32_t* in = &t2.info[(size_t)8 * t];

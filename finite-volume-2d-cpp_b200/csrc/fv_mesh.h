@@ -118,10 +118,16 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int tile_cells, Tile2
 template <class S>
 struct FusedArrays {
     int nf = 3;                          // faces per slot in rec: 3, or 4 with quadrilaterals
-    std::vector<int32_t> info;           // [n_tiles][8]: slot_off, halo_off, flux_off, n_flux, n1, n2, owned cells, 0
+    // [n_tiles][8]: slot_off, halo_off, flux_off, n_flux, n1, n2, owned cells | ghosts << 16, ghost_off
+    std::vector<int32_t> info;
     std::vector<uint32_t> hd;            // [slots][4] face words (fv_fused.cuh)
     std::vector<S> rec, rec2, sl;        // [nf * slots][4], exact [nf * slots][2], [slots] (exact [slots][2])
     std::vector<S> eg;                   // [flux edges][4]
+    // boundary ghosts of the tiles' owned cells: {interior slot | group << 16,
+    // device cell}, {n_x, n_y, d_x, d_y}
+    std::vector<int32_t> gl;
+    std::vector<S> gd;
+    int max_ghost = 0;
     std::vector<double> ria;             // [owned cells] 1 / area as the stage precision holds it
 };
 template <class S>

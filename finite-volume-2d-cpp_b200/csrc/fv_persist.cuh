@@ -166,8 +166,8 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
     const Params& P = FP.P;
     const int T = FP.T, t = (int)blockIdx.x;
     const int4 ia = FP.info[2 * t], ib = FP.info[2 * t + 1];
-    const int slot_off = ia.x, halo_off = ia.y, flux_off = ia.z, n_flux = ia.w;
-    const int n1 = ib.x, nh = O2 ? ib.x + ib.y : ib.x, nown = ib.z;
+    const int slot_off = ia.x, halo_off = ia.y, flux_off = ia.z, n_flux = ia.w, n_ghost = ib.z >> 16;
+    const int n1 = ib.x, nh = O2 ? ib.x + ib.y : ib.x, nown = ib.z & 0xFFFF;
     const int c0 = t * T, G = T + n1;
     const FusedSmem& L = FP.L;
     uint4* Q = reinterpret_cast<uint4*>(smem_raw + L.q);
@@ -203,6 +203,9 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
         uint4* dst = reinterpret_cast<uint4*>(smem_raw + L.eg);
         for (int i = l; i < NU * n_flux; i += blockDim.x) cpa16(dst + i, src + i);
         if (l < nown) cpa8(RA + l, FP.ria + c0 + l);
+        const uint4* gsrc = reinterpret_cast<const uint4*>((const S*)FP.gd + 4 * (size_t)ib.w);
+        for (int i = l; i < NU * n_ghost; i += blockDim.x) cpa16(reinterpret_cast<uint4*>(smem_raw + L.gd) + i, gsrc + i);
+        for (int i = l; i < n_ghost; i += blockDim.x) cpa8(smem_raw + L.gl + 8 * i, FP.gl + ib.w + i);
         cpa_wait();
     }
     const int tc = (P.global_dt && P.n_cases > 1) ? P.tile_case[t] : 0;
@@ -363,8 +366,12 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
 #pragma unroll
             for (int i = 0; i < NV; ++i) res[i] = 0.;
             if (uc < nown)
-                fused_update<M, NV, NF, false, O2>(FP, io, smem_raw, own, uc, v0, c0, slot_off, halo_off, flux_off, G, tc,
-                                                   dtc, s_dt, PartIO{}, res);
+                fused_update<M, NV, NF, false>(FP, io, smem_raw, own, uc, v0, c0, tc, dtc, s_dt, n_ghost != 0, PartIO{}, res);
+            if (n_ghost != 0) {
+                __syncthreads();
+                fused_ghosts<M, false, O2>(FP, io, smem_raw, reinterpret_cast<const int2*>(smem_raw + L.gl),
+                                           reinterpret_cast<const S*>(smem_raw + L.gd), n_ghost, PartIO{});
+            }
             if (last) fused_partials<NV>(io, smem_raw + L.fs, t, v0, res);
             sync.arrive();
             in = out_s;
