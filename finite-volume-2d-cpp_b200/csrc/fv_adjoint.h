@@ -24,6 +24,9 @@ struct AdjFaces {
     const double *nx, *ny, *le, *g;      // face normal (reference orientation), length, Green-Gauss weight
     const double *dsx, *dsy, *dnx, *dny; // x_f - x_self, x_f - x_neighbour
     const double* area;                  // [n_total]
+    const uint8_t* rev;    // [4][n_real] this cell's face slot in the neighbour (real neighbours)
+    const int32_t* bcells; // [n_bcells] real cells with boundary ghosts
+    int n_bcells;
 };
 
 struct AdjStage {
@@ -39,7 +42,7 @@ struct AdjStage {
     // adjoint
     double* lam_next;      // in: dL/d qs_{k+1}; its real part gains the ghost-fill terms
     double* lam_cur;       // out: dL/d qs_k (written for every cell)
-    double* lam_gx;        // dL/d g_k [n_real][4]
+    double* lam_gx;        // dL/d g_k [n_real][4]: the ghost fill writes the cells with ghosts, the residual the rest
     double* lam_gy;
     double* lam_lim;
     double* lam_qn;        // += dL/d q_n through the update's base state (real cells)
@@ -51,8 +54,8 @@ struct AdjStage {
 void adj_launch_ghosts(const Params& P, const AdjFaces& F, const AdjStage& S, cudaStream_t st);
 // flux residual + RK update: lam_cur = ..., lam_g += ..., lam_qn += lam_next[real], dt partials
 void adj_launch_residual(const Params& P, const AdjFaces& F, const AdjStage& S, cudaStream_t st);
-// gradients + limiters: lam_cur += (d g_k / d qs_k)^T lam_g
-void adj_launch_gradlim(const Params& P, const AdjFaces& F, const AdjStage& S, cudaStream_t st);
+// gradients + limiters: lam_cur += (d g_k / d qs_k)^T lam_g; part: scratch [5][n_real][4]
+void adj_launch_gradlim(const Params& P, const AdjFaces& F, const AdjStage& S, double* part, cudaStream_t st);
 int adj_residual_blocks(const Params& P);
 
 // y[i] += x[i], i < n

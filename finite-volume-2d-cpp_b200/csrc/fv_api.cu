@@ -95,10 +95,13 @@ int upload_fused(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const Ti
     F.gl = reinterpret_cast<const int2*>(gl);
     return FV_OK;
 }
-// lanes per cell of the fused kernel's gradient and update phases
-int fused_lanes(const fv_solver* s) {
-    (void)s;
-    return 1;
+// Lanes per cell of the fused kernel's gradient and update phases: 4 for
+// FP64_EXACT meshes of at most one tile per SM, whose steps outside the run
+// kernel (the adjoint's) wait for one tile's chain.  Measured, us per step of a
+// forward pass with 1 | 4 lanes: 10,206 cells 98 | 82, 18,144 cells 97 | 83,
+// 60,984 cells 144 | 201; in the fast modes 4 lanes gain nothing at any size.
+int fused_lanes(const fv_solver* s, int sms) {
+    return s->precision == FV_PREC_FP64_EXACT && s->n_tiles <= sms && s->FPm.T <= kFusedThreads / 4 ? 4 : 1;
 }
 // The persistent run kernel, where all tiles fit the device at once: the first
 // candidate (fv_persist.cuh) with room for them.
@@ -538,7 +541,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
                 if (sk == FV_STAGE_HYBRID && sched == FV_SCHED_WORKLIST)
                     return fail(FV_ERR_ARG, "the work-list schedule needs the dt kernel of the fused layout");
                 s->sched = sched;
-                F.lanes = fused_lanes(s.get());
+                F.lanes = fused_lanes(s.get(), sms);
                 // automatic choice: in FP32 the split first stage (its gradient
                 // kernel computes dt) saves more than it costs; in FP64 the
                 // fused first stage and the separate dt kernel are faster
@@ -879,8 +882,9 @@ int step_open(fv_solver* s, const std::vector<double>& alpha, int b, bool first,
     c.grads = (TP.P.order2 || TP.P.diffusive) && !s->fused;
     // the fast modes' split kernels over the two-ring tiles
     c.fast2 = s->two_ring && s->precision != FV_PREC_FP64_EXACT;
-    // their time step: the CFL and constant kinds (the viscous ones keep k_tile_dt)
-    c.dt2 = c.fast2 && TP.P.dt_kind < 3;
+    // the time step over those tiles: the CFL and constant kinds (the viscous
+    // ones, and FP64_EXACT's split layouts, keep the one-ring kernels)
+    c.dt2 = s->two_ring && TP.P.dt_kind < 3;
     // FP64_EXACT's hybrid layout: the split first stage's gradient kernel
     // computes dt.  In the fast modes the dt kernel over the fused kernel's
     // tiles and a fused first stage cost less (998k cells, FP32: 80 us against
@@ -939,6 +943,7 @@ int step_stage(fv_solver* s, const std::vector<double>& alpha, int k, StepCursor
     if (r) {
         if (!s->fused || c.worklist || c.split_first) return -1;
         const PartIO pio{r->t0, nullptr, k, ns};
+        so.gx = so.gy = so.lim = nullptr;
         if (r->n > 0) {
             tile::launch_fused(s->precision, c.FPl, so, r->stream ? r->stream : st, r->pdl, r->n, r->n, &pio);
             ++n; mark(KK_FUSED);
@@ -968,6 +973,7 @@ int step_stage(fv_solver* s, const std::vector<double>& alpha, int k, StepCursor
         tile::launch_gradlim(s->precision, TP, so, st, true, pdl); ++n; mark(KK_GRADLIM);
         tile::launch_stage(s->precision, TP, so, st, pdl); ++n; mark(KK_STAGE);
     } else if (s->fused) {
+        so.gx = so.gy = so.lim = nullptr;  // kept by the adjoint only
         so.work = c.worklist ? s->work + k : nullptr;
         const PartIO pio{0, c.worklist ? nullptr : c.remote, k, ns};
         tile::launch_fused(s->precision, c.FPl, so, st, pdl, s->n_tiles, s->work_grid, c.part ? &pio : nullptr);
@@ -1550,10 +1556,10 @@ struct fv_adjoint {
     std::vector<double*> Qs;          // [S] inputs of stages 1..S-1 of the step being reversed (Qs[0] unused)
     std::vector<double*> Gx, Gy, Lim; // [S] gradients and limiters of its stages
     double* dtc = nullptr;            // its per-cell dt
-    double *tmp[2] = {nullptr, nullptr}, *tgx = nullptr, *tgy = nullptr, *tlim = nullptr;
+    double *tmp[2] = {nullptr, nullptr}, *tmp2[2] = {nullptr, nullptr}, *tgx = nullptr, *tgy = nullptr, *tlim = nullptr;
     double *dt_fill = nullptr, *dt_n = nullptr, *loss = nullptr, *lam_dt = nullptr, *partials = nullptr;
     double *lamA = nullptr, *lamB = nullptr, *lam_qn = nullptr, *lgx = nullptr, *lgy = nullptr, *llim = nullptr;
-    double *lam_bv = nullptr;
+    double *lam_bv = nullptr, *glpart = nullptr;
     unsigned long long* keys = nullptr;
     int* argmin = nullptr;
     int32_t* loss_ghosts = nullptr;   // device ghost indices of the loss group
@@ -1589,22 +1595,24 @@ int adj_forward_step(fv_adjoint* a, const double* q, double* q_next, double* dt_
     io.q_stage = q;
     io.dt = dtcells;
     io.dtkeys = a->keys;
-    tile::launch_dt(FV_PREC_FP64_EXACT, TP, io, st);
+    FusedParams FPl = s->FPm;
+    FPl.P = TP.P;
+    fused_schedule(s, FPl, false);
+    if (s->two_ring) tile::launch_fused_split(FV_PREC_FP64_EXACT, FPl, io, st, false, s->n_tiles, 3);
+    else tile::launch_dt(FV_PREC_FP64_EXACT, TP, io, st);
     adj_launch_dt_finalize(a->keys, dtcells, TP.P.cell0, a->dt_fill, (int)nt, dt_slot, st);
     if (with_loss && a->n_loss) adj_launch_loss(TP.P, q, dt_slot, a->loss_ghosts, a->n_loss, a->loss, st);
     const double* in = q;
-    if (!store && s->fused) {
-        // states only: the fused stage kernel (the same bits as the
-        // gradient + stage kernels, without writing the gradients out)
-        FusedParams FPl = s->FPm;
-        FPl.P = TP.P;
-        fused_schedule(s, FPl, false);
+    if (s->fused) {
+        // the fused stage kernel, which writes the gradients and limiters out
+        // where they are kept
         for (int k = 0; k < a->S; ++k) {
-            double* out = (k == a->S - 1) ? q_next : a->tmp[k % 2];
+            double* out = (k == a->S - 1) ? q_next : (store ? a->Qs[(size_t)k + 1] : a->tmp[k % 2]);
             TileIO so{};
             so.q_stage = in;
             so.q_base = q;
             so.q_out = out;
+            if (store) { so.gx = a->Gx[(size_t)k]; so.gy = a->Gy[(size_t)k]; so.lim = a->Lim[(size_t)k]; }
             so.dt = a->dt_fill;
             so.alpha = a->alpha[(size_t)k];
             so.write_f64 = 1;
@@ -1739,7 +1747,25 @@ int fv_adjoint_create(const fv_mesh* fm, const fv_physics* ph, int32_t device, c
         CK(up(&nbr, fa.nbr)); CK(up(&nx, fa.nx)); CK(up(&ny, fa.ny)); CK(up(&le, fa.le)); CK(up(&g, fa.g));
         CK(up(&dsx, fa.dsx)); CK(up(&dsy, fa.dsy)); CK(up(&dnx, fa.dnx)); CK(up(&dny, fa.dny));
         CK(up(&area, fa.area));
-        a->F = AdjFaces{nbr, nx, ny, le, g, dsx, dsy, dnx, dny, area};
+        // each face's slot in the neighbour's list, and the cells with ghosts
+        const size_t N = (size_t)m.n_real;
+        std::vector<uint8_t> rev(4 * N, 0);
+        std::vector<int32_t> bcells;
+        for (size_t c = 0; c < N; ++c) {
+            bool ghost = false;
+            for (int f = 0; f < 4; ++f) {
+                const uint32_t w = fa.nbr[f * N + c];
+                if (w == kNoFace) continue;
+                const size_t j = w & 0x7FFFFFFFu;
+                if (j >= N) { ghost = true; continue; }
+                for (int h = 0; h < m.n_faces[j]; ++h)
+                    if (m.face_edge[j * HostMesh::MAXF + h] == m.face_edge[c * HostMesh::MAXF + f]) rev[f * N + c] = (uint8_t)h;
+            }
+            if (ghost) bcells.push_back((int32_t)c);
+        }
+        uint8_t* d_rev; int32_t* d_bcells;
+        CK(up(&d_rev, rev)); CK(up(&d_bcells, bcells));
+        a->F = AdjFaces{nbr, nx, ny, le, g, dsx, dsy, dnx, dny, area, d_rev, d_bcells, (int)bcells.size()};
     }
     std::vector<int32_t> lg;
     for (int64_t b = 0; b < m.n_bound; ++b)
@@ -1766,6 +1792,7 @@ int fv_adjoint_create(const fv_mesh* fm, const fv_physics* ph, int32_t device, c
     }
     CK(a->alloc(&a->dtc, (size_t)m.n_total));
     CK(a->alloc(&a->tmp[0], nq)); CK(a->alloc(&a->tmp[1], nq));
+    CK(a->alloc(&a->tmp2[0], nq)); CK(a->alloc(&a->tmp2[1], nq));
     CK(a->alloc(&a->tgx, nq)); CK(a->alloc(&a->tgy, nq)); CK(a->alloc(&a->tlim, nq));
     launch_fill_ghost_grad(a->tgx, a->tgy, a->tlim, (int)m.n_real, (int)m.n_total, 4, false, s->stream);
     CK(a->alloc(&a->dt_fill, (size_t)m.n_total));
@@ -1775,6 +1802,7 @@ int fv_adjoint_create(const fv_mesh* fm, const fv_physics* ph, int32_t device, c
     CK(a->alloc(&a->lamA, nq)); CK(a->alloc(&a->lamB, nq)); CK(a->alloc(&a->lam_qn, nq));
     CK(a->alloc(&a->lgx, nq)); CK(a->alloc(&a->lgy, nq)); CK(a->alloc(&a->llim, nq));
     CK(a->alloc(&a->lam_bv, (size_t)m.n_bound * 4));
+    CK(a->alloc(&a->glpart, (size_t)5 * m.n_real * 4));
     CK(a->alloc(&a->keys, (size_t)kDtSlots));
     CK(a->alloc(&a->argmin, 1));
     CK(cudaGetLastError());
@@ -1801,11 +1829,12 @@ int fv_adjoint_run(fv_adjoint* a, const double* theta, double* loss, double* gra
     // ---- forward: checkpoints every `every` steps, loss
     CK(cudaMemsetAsync(a->loss, 0, 8, st));
     double* cur = a->ckpt[0];
-    double* nxt = a->Qn[0];  // scratch for the non-checkpoint states
-    double* alt = a->Qn[1];
+    const int last0 = (a->nseg - 1) * every;  // the last segment's first step
     for (int n = 0; n < N; ++n) {
-        double* dst = ((n + 1) % every == 0 && (n + 1) / every < a->nseg) ? a->ckpt[(size_t)(n + 1) / every]
-                                                                             : (cur == nxt ? alt : nxt);
+        // checkpoints; in between two scratch states, and in the last segment
+        // the states that its reversal starts from
+        double* dst = ((n + 1) % every == 0 && n + 1 <= last0) ? a->ckpt[(size_t)(n + 1) / every]
+                      : n >= last0 ? a->Qn[(size_t)(n - last0) + 1] : a->tmp2[n & 1];
         if ((rc = adj_forward_step(a, cur, dst, a->dt_n + n, false, true))) return rc;
         cur = dst;
     }
@@ -1826,7 +1855,7 @@ int fv_adjoint_run(fv_adjoint* a, const double* theta, double* loss, double* gra
         const int n0 = seg * every, len = std::min(every, N - n0);
         // the segment's step states (the same bits as the forward run's)
         CK(cudaMemcpyAsync(a->Qn[0], a->ckpt[(size_t)seg], nq * 8, cudaMemcpyDeviceToDevice, st));
-        for (int j = 0; j < len; ++j)
+        for (int j = 0; j < len && seg < a->nseg - 1; ++j)  // (the last one's are the forward run's own)
             if ((rc = adj_forward_step(a, a->Qn[(size_t)j], a->Qn[(size_t)j + 1], a->dt_n + n0 + j, false, false)))
                 return rc;
         CK(cudaMemcpyAsync(dts.data(), a->dt_n + n0, (size_t)len * 8, cudaMemcpyDeviceToHost, st));
@@ -1839,7 +1868,7 @@ int fv_adjoint_run(fv_adjoint* a, const double* theta, double* loss, double* gra
                 AdjStage stg = adj_stage(a, a->Qn[(size_t)j], a->Qn[(size_t)j + 1], k, dts[(size_t)j]);
                 adj_launch_ghosts(TP.P, a->F, stg, st);
                 adj_launch_residual(TP.P, a->F, stg, st);
-                if (TP.P.order2) adj_launch_gradlim(TP.P, a->F, stg, st);
+                if (TP.P.order2) adj_launch_gradlim(TP.P, a->F, stg, a->glpart, st);
                 std::swap(a->lamA, a->lamB);
             }
             adj_launch_add(a->lam_qn, a->lamA, nq, st);  // q_n is stage 0's input

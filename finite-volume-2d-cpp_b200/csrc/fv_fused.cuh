@@ -84,7 +84,7 @@ struct FusedParams {
     Params P;
     int T;
     int threads;               // threads per CTA: T, 2T (FV_SCHED_TILE2) or lanes * T
-    int lanes;                 // lanes per cell of the gradient and update phases: 1, 2 or 4
+    int lanes;                 // lanes per cell of the gradient and update phases: 1 or 4 (exact only)
     int nf;                    // faces per gradient slot: 3 (triangles only) or 4
     int max_slots, max_grad, max_flux;
     // [n_tiles][2]: {slot_off, halo_off, flux_off, n_flux},
@@ -564,6 +564,14 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
             if (P.limiter == 2) apply([] { return 2; });
             else if (P.limiter == 1) apply([] { return 1; });
             else apply([&] { return P.limiter; });
+        }
+    }
+    if constexpr (M::exact && PH == 0) {
+        // the adjoint keeps a stage's gradients and limiters
+        if (io.gx != nullptr && r < T) {
+            stv<S, NV>((S*)io.gx + 4 * (size_t)(c0 + r) + v0, gx);
+            stv<S, NV>((S*)io.gy + 4 * (size_t)(c0 + r) + v0, gy);
+            stv<S, NV>((S*)io.lim + 4 * (size_t)(c0 + r) + v0, lim);
         }
     }
     if constexpr (PH == 1) {
@@ -1086,12 +1094,13 @@ struct FusedLaunch {
         auto all = [&](auto f, auto n) {
             constexpr int F = decltype(f)::value, NF = decltype(n)::value;
             for (const void* fn :
-                 {(const void*)k_tile_fused<M, F, 4, NF>, (const void*)k_tile_fused<M, F, 2, NF>,
-                  (const void*)k_tile_fused<M, F, 1, NF>, (const void*)k_tile_fused_part<M, F, NF, 1>,
+                 {(const void*)k_tile_fused<M, F, 4, NF>, (const void*)k_tile_fused_part<M, F, NF, 1>,
                   (const void*)k_tile_fused_part<M, F, NF, 2>, (const void*)k_tile_fused_work<M, F, NF>})
                 set(fn);
+            if constexpr (M::exact) set((const void*)k_tile_fused<M, F, 1, NF>);
+            set((const void*)k_tile_fused_dt<M, NF>);
             if constexpr (!M::exact)
-                for (const void* fn : {(const void*)k_tile_fused_grad<M, NF>, (const void*)k_tile_fused_flux<M, NF>, (const void*)k_tile_fused_dt<M, NF>})
+                for (const void* fn : {(const void*)k_tile_fused_grad<M, NF>, (const void*)k_tile_fused_flux<M, NF>})
                     set(fn);
         };
         using One = std::integral_constant<int, 1>;
@@ -1137,8 +1146,7 @@ struct FusedLaunch {
         if (io.work) go(k_tile_fused_work<M, F, NF>, grid, FP.T, sm, st, pdl, FP, io, n_tiles);
         else if (part && part->remote) go(k_tile_fused_part<M, F, NF, 2>, n_tiles, tp, sm, st, pdl, FP, io, *part);
         else if (part) go(k_tile_fused_part<M, F, NF, 1>, n_tiles, tp, sm, st, pdl, FP, io, *part);
-        else if (FP.lanes == 4) go(k_tile_fused<M, F, 1, NF>, n_tiles, FP.threads, sm, st, pdl, FP, io);
-        else if (FP.lanes == 2) go(k_tile_fused<M, F, 2, NF>, n_tiles, FP.threads, sm, st, pdl, FP, io);
+        else if (M::exact && FP.lanes == 4) go(k_tile_fused<M, F, M::exact ? 1 : 4, NF>, n_tiles, FP.threads, sm, st, pdl, FP, io);
         else go(k_tile_fused<M, F, 4, NF>, n_tiles, FP.threads, sm, st, pdl, FP, io);
     }
     // io.work != nullptr: the work-list schedule on `grid` CTAs
@@ -1155,20 +1163,19 @@ struct FusedLaunch {
         if (FP.nf == 3) stage_f<1, 3>(FP, io, st, pdl, n_tiles, grid, part);
         else stage_f<1, 4>(FP, io, st, pdl, n_tiles, grid, part);
     }
-    // fast policies, one lane per cell: the split layout's two kernels
-    // (phase 1: gradients; phase 2: the rest) and the time step (phase 3)
+    // the time step (phase 3); fast policies: the split layout's two kernels
+    // (phase 1: gradients; phase 2: the rest)
     template <int NF>
     static void split_f(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase) {
         const FusedSmem& L = FP.L;
         if (phase == 3) go(k_tile_fused_dt<M, NF>, n_tiles, FP.T, L.total_grad, st, pdl, FP, io);
+        else if constexpr (M::exact) return;
         else if (phase == 2) go(k_tile_fused_flux<M, NF>, n_tiles, FP.T, L.total, st, pdl, FP, io);
         else go(k_tile_fused_grad<M, NF>, n_tiles, FP.T, L.total_grad, st, pdl, FP, io);
     }
     static void split(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase) {
-        if constexpr (!M::exact) {
-            if (FP.nf == 3) split_f<3>(FP, io, st, pdl, n_tiles, phase);
-            else split_f<4>(FP, io, st, pdl, n_tiles, phase);
-        }
+        if (FP.nf == 3) split_f<3>(FP, io, st, pdl, n_tiles, phase);
+        else split_f<4>(FP, io, st, pdl, n_tiles, phase);
     }
 };
 
@@ -1178,7 +1185,7 @@ size_t smem_fused(int precision, FusedParams& FP);
 int work_grid_fused(int precision, FusedParams& FP, int n_tiles);
 void launch_fused(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
                   int grid, const PartIO* part = nullptr);
-// the fast policies' split kernels over the fused kernel's tiles (FusedLaunch::split)
+// the time step and the fast policies' split kernels over the fused kernel's tiles (FusedLaunch::split)
 void launch_fused_split(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
                         int phase);
 }  // namespace tile

@@ -22,5 +22,8 @@ void launch_fused_exact(const FusedParams& FP, const TileIO& io, cudaStream_t st
                         const PartIO* part) {
     FusedLaunch<MExact>::stage(FP, io, st, pdl, n_tiles, grid, part);
 }
+void launch_fused_split_exact(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase) {
+    FusedLaunch<MExact>::split(FP, io, st, pdl, n_tiles, phase);
+}
 }  // namespace tile
 }  // namespace fvgpu

@@ -15,6 +15,8 @@ int work_grid_fused_exact(FusedParams& FP, int n_tiles);
 void launch_fused_exact(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int grid,
                         const PartIO* part);
 
+void launch_fused_split_exact(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase);
+
 cudaError_t prepare(int precision, const TileParams& TP) {
     if (precision == 0) return prepare_exact(TP);
     if (precision == 1) return TileLaunch<MF64>::prepare(TP);
@@ -58,7 +60,8 @@ void launch_fused(int precision, const FusedParams& FP, const TileIO& io, cudaSt
 }
 void launch_fused_split(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
                         int phase) {
-    if (precision == 1) FusedLaunch<MF64>::split(FP, io, st, pdl, n_tiles, phase);
+    if (precision == 0) launch_fused_split_exact(FP, io, st, pdl, n_tiles, phase);
+    else if (precision == 1) FusedLaunch<MF64>::split(FP, io, st, pdl, n_tiles, phase);
     else if (precision == 2) FusedLaunch<MF32>::split(FP, io, st, pdl, n_tiles, phase);
 }
 }  // namespace tile
