@@ -78,20 +78,21 @@ int upload_v(fv_solver* s, const std::vector<T>& v, const T** out) {
 // the fused kernel's arrays over two-ring tiles (build_fused)
 template <class S>
 int upload_fused(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2,
-                 bool exact, bool first_order, double K) {
+                 bool exact, FusedKind kind, double K) {
     FusedArrays<S> a;
-    build_fused<S>(m, fa, ta, t2, exact, first_order, K, a);
+    build_fused<S>(m, fa, ta, t2, exact, kind, K, a);
     FusedParams& F = s->FPm;
     F.nf = a.nf;
     F.max_ghost = a.max_ghost;
-    const int32_t* info; const uint32_t* hd; const int32_t* gl; const S *rec, *rec2, *sl, *eg, *gd;
+    const int32_t* info; const uint32_t* hd; const int32_t* gl; const S *rec, *rec2, *sl, *eg, *gd, *e2, *ar;
     int rc;
     if ((rc = upload_v(s, a.info, &info)) || (rc = upload_v(s, a.hd, &hd)) || (rc = upload_v(s, a.rec, &rec)) || (rc = upload_v(s, a.rec2, &rec2)) || (rc = upload_v(s, a.sl, &sl)) ||
-        (rc = upload_v(s, a.eg, &eg)) || (rc = upload_v(s, a.gl, &gl)) || (rc = upload_v(s, a.gd, &gd)) || (rc = upload_v(s, a.ria, &F.ria)))
+        (rc = upload_v(s, a.eg, &eg)) || (rc = upload_v(s, a.gl, &gl)) || (rc = upload_v(s, a.gd, &gd)) ||
+        (rc = upload_v(s, a.e2, &e2)) || (rc = upload_v(s, a.ar, &ar)) || (rc = upload_v(s, a.ria, &F.ria)))
         return rc;
     F.info = reinterpret_cast<const int4*>(info);
     F.hd = reinterpret_cast<const uint4*>(hd);
-    F.rec = rec; F.rec2 = rec2; F.sl = sl; F.eg = eg; F.gd = gd;
+    F.rec = rec; F.rec2 = rec2; F.sl = sl; F.eg = eg; F.gd = gd; F.e2 = e2; F.ar = ar;
     F.gl = reinterpret_cast<const int2*>(gl);
     return FV_OK;
 }
@@ -444,14 +445,19 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const bool roe = ph->V == 4 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST);
-    const bool can_run = roe && ph->dt_kind < FV_DT_VISC_MIN && sk != FV_STAGE_SPLIT &&
+    // The Navier-Stokes kind has one in FP64 (flat plate, 13,200 cells: 41
+    // against 104 us per step).  Its FP32 residual norms on low-Mach flows are
+    // mostly rounding noise, which any other order of operations moves by more
+    // than FP32's tolerance, so FP32 keeps its kernels.
+    const bool ns = ph->flux == FV_FLUX_NS && precision == FV_PREC_FP64;
+    const bool can_run = (ns || (roe && ph->dt_kind < FV_DT_VISC_MIN)) && sk != FV_STAGE_SPLIT &&
                          !(sk == FV_STAGE_HYBRID && precision == FV_PREC_FP64_EXACT) &&
                          (!opt || opt->schedule == FV_SCHED_TILE) && m.owned_real() == m.n_real && m.n_real > 0 &&
                          m.n_real <= (int64_t)8 * sms * tile_cells;
-    const bool run_first_order = can_run && !ph->order2;
+    const bool run_own_tiles = can_run && (ns || !ph->order2);  // (the second-order Roe kinds share the fused kernel's)
     Tile2Arrays t2;
     std::future<void> t2_built;
-    if (two_ring || run_first_order) t2_built = std::async(std::launch::async, [&] { build_tiles2(m, fa, tile_cells, t2); });
+    if (two_ring || run_own_tiles) t2_built = std::async(std::launch::async, [&] { build_tiles2(m, fa, tile_cells, t2); });
     build_tiles(m, fa, tile_cells, ta);
     if (ta.max_halo + tile_cells > 65535 || ta.max_edges > kFaceEdgeMask)
         return fail(FV_ERR_MESH, "tile halo too large for 16-bit local indices");
@@ -521,8 +527,8 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
             if (!fits && (sk == FV_STAGE_FUSED || sk == FV_STAGE_HYBRID))
                 return fail(FV_ERR_MESH, "two-ring tiles too large for the fused stage kernel at this tile size");
             if (fits) {
-                if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, false, ph->K);
-                else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, false, ph->K);
+                if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, kFusedEuler, ph->K);
+                else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, kFusedEuler, ph->K);
                 if (rc) return rc;
                 const int32_t* h2;
                 if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;
@@ -619,14 +625,17 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
         s->nbr = const_cast<uint32_t*>(d);
     }
     launch_fill_ghost_grad(s->gx, s->gy, s->lim, (int)m.n_real, (int)m.n_total, ph->V, s->f32, s->stream);
-    if (run_first_order) {
+    if (run_own_tiles) {
         t2_built.get();
         FusedParams& F = s->FPm;
         F.T = tile_cells;
-        F.max_slots = t2.max_grad; F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;  // one ring is staged
+        const FusedKind kind = ns ? kFusedViscous : kFusedFirstOrder;
+        F.P.flux = ph->flux;  // (the shared-memory layout depends on it)
+        F.max_slots = ns ? t2.max_slots : t2.max_grad;  // first order stages one ring
+        F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;
         if (t2.max_slots < 65535 && 2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= (size_t)227 * 1024) {
-            if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, true, ph->K);
-            else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, true, ph->K);
+            if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, kind, ph->K);
+            else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, kind, ph->K);
             if (rc) return rc;
             const int32_t* h2;
             if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;

@@ -47,32 +47,35 @@ namespace fvgpu {
 //  - the base state of the owned cells (FP64, [T][4]);
 //  - the flux edges' geometry [max_flux][4] and 1 / area of the owned cells;
 //  - the limited gradients (and, exact, the limiters) of owned cells with a
-//    boundary ghost, for the ghost fill.
+//    boundary ghost, for the ghost fill; viscous: the unlimited gradients of
+//    every slot, the limiters, and the tile's e2 and ar.
 struct FusedSmem {
-    int q, fs, qb, gx, gy, lm, eg, ria, gl, gd, total, total_grad, total_run;
+    int q, fs, qb, gx, gy, lm, eg, ria, gl, gd, e2, ar, total, total_grad, total_run;
     int ls, lf, lt;  // plane strides (units)
 };
 template <class M>
-inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int max_ghost, int T) {
+inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int max_ghost, int T, bool viscous) {
     constexpr int NU = (int)(4 * sizeof(typename M::S) / 16);
     FusedSmem L{};
     L.ls = max_slots;
     L.lf = 2 * max_flux;
-    L.lt = T;
+    L.lt = viscous ? max_grad : T;
     int o = 0;
     L.q = o; o += 16 * NU * max_slots;
     // the face states, the time step's {u, v, c} or the residual warp sums
     L.fs = o; o += std::max({32 * NU * max_flux, 16 * NU * max_grad, (kFusedThreads / 32) * 4 * (int)sizeof(double)});
     L.qb = o; o += 32 * T;
-    L.gx = o; o += 16 * NU * T;
-    L.gy = o; o += 16 * NU * T;
-    L.lm = o; if (M::exact) o += 16 * NU * T;
+    L.gx = o; o += 16 * NU * L.lt;
+    L.gy = o; o += 16 * NU * L.lt;
+    L.lm = o; if (M::exact || viscous) o += 16 * NU * L.lt;
     L.eg = o; o += 16 * NU * max_flux;
     L.ria = o; o += 8 * T;
     L.total = o;
     // the run kernel keeps the tile's ghosts behind that
     L.gd = o; o += 16 * NU * max_ghost;
     L.gl = o; o += (8 * max_ghost + 15) / 16 * 16;
+    L.e2 = o; if (viscous) o += 16 * NU * max_flux;
+    L.ar = o; if (viscous) o += (4 * NU * max_grad + 15) / 16 * 16;
     L.total_run = o;
     // the gradient kernel of the split layout and the dt kernel: the states
     // and {u, v, c} of the gradient slots
@@ -116,6 +119,8 @@ struct FusedParams {
     const int2* gl;
     const void* gd;
     int max_ghost;             // ghosts of a tile at most
+    const void* e2;            // viscous: S[4] per flux edge {t_x, t_y, 1 / distance, 0} (t: unit vector of c_i - c_j)
+    const void* ar;            // viscous: S per gradient slot: the area
 };
 
 constexpr uint32_t kWordGhost = 0x40000000u, kWordNoFlux = 0x80000000u;
@@ -308,22 +313,28 @@ struct SlotGeo {
 };
 
 // CFL or constant time step of owned cell c (slot l) and of its boundary
-// ghosts from {u, v, c} of the tile's slots (calc_dt of
-// examples/forwardStep/main.cpp:140-185 and examples/naca/main.cpp:142-183).
+// ghosts from {u, v, c, rho} of the tile's slots (calc_dt of
+// examples/forwardStep/main.cpp:140-185 and examples/naca/main.cpp:142-183;
+// VISC, fast policies: and the viscous kinds, AR the slots' areas).
 // edge(el, e): normal and length of flux edge el; A: the cell's area, which is
 // its ghosts' too.  Returns the ordered-key minimum of the values written.
-template <class M, int NF, class Edge>
+template <class M, int NF, bool VISC, class Edge>
 __device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& FP, const TileIO& io, const uint32_t* fw,
                                                             const uint4* W, int l, int c, int halo_off,
-                                                            typename M::S A, Edge edge, double& di) {
+                                                            typename M::S A, Edge edge, double& di,
+                                                            const typename M::S* AR = nullptr) {
     using S = typename M::S;
     const Params& P = FP.P;
     const S cfl = (S)P.cfl;
-    const bool sum = P.dt_kind == 1, constant = P.dt_kind == 0;
+    const bool sum = P.dt_kind == 1 || (VISC && P.dt_kind == 4), constant = P.dt_kind == 0;
+    const bool visc = VISC && P.dt_kind >= 3;
     unsigned long long kmin = ~0ull;
     S ws[4];
     Planes<S, 4>::get(W, FP.max_grad, l, 0, ws);
     S acc = sum ? S(0) : S(1);
+    // viscous kinds (see tile_cell_dt_visc): C mu / pr max(4 / 3, gamma) / rho le^2 / A
+    const S vc = VISC ? S(2) * (S)(P.mu / P.pr) * fast::tmax(S(4.0 / 3.0), (S)P.gamma) : S(0);
+    const S vs = VISC ? vc * fast::rcp(ws[3]) * fast::rcp(A) : S(0);
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
         const uint32_t w = fw[f];
@@ -355,6 +366,21 @@ __device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& F
                     dg = exact::dmin(1.0, cfl * (A / e[2]) / fabs(en));
                 }
             }
+        } else if (visc) {
+            const S le2 = e[2] * e[2], vn = vc * fast::rcp(wn[3]) * le2 * fast::rcp(AR[o]);
+            if (sum) {
+                const S center = fast::tmax(ws[2] + fabs(ws[0] * e[0] + ws[1] * e[1]) + vs * le2,
+                                            wn[2] + fabs(wn[0] * e[0] + wn[1] * e[1]) + vn);
+                acc += center * e[2];
+                if (ghost) dg = (double)(cfl * A * fast::rcp(center * e[2]));
+            } else {
+                const S es = (ws[2] + fabs(e[0] * ws[0]) + fabs(e[1] * ws[1])) * e[2] + vs * le2;
+                acc = fast::tmin(acc, cfl * A * fast::rcp(es));
+                if (ghost) {
+                    const S en = (wn[2] + fabs(e[0] * wn[0]) + fabs(e[1] * wn[1])) * e[2] + vn;
+                    dg = (double)fast::tmin(S(1), cfl * A * fast::rcp(en));
+                }
+            }
         } else if (sum) {
             const S center = fast::tmax(ws[2] + fabs(fast::fma_(ws[0], e[0], ws[1] * e[1])),
                                         wn[2] + fabs(fast::fma_(wn[0], e[0], wn[1] * e[1])));
@@ -378,7 +404,7 @@ __device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& F
     io.dt[c] = di;
     return kmin_(kmin, tkey(di));
 }
-// {u, v, c} of a state, in the reference's arithmetic (exact) or the fast one
+// {u, v, c, rho} of a state, in the reference's arithmetic (exact) or the fast one
 template <class M>
 __device__ __forceinline__ void fused_speeds(double gamma, const typename M::S* q, typename M::S* w) {
     if constexpr (M::exact) {
@@ -394,15 +420,15 @@ __device__ __forceinline__ void fused_speeds(double gamma, const typename M::S* 
             c2 = (gm1 * (q[3] - 0.5 / q[0] * (q[1] * q[1] + q[2] * q[2]))) * gamma / q[0];
         }
         w[2] = sqrt(c2);
-        w[3] = 0.;
     } else {
         fast::speeds((typename M::S)gamma, q, w);
     }
+    w[3] = q[0];
 }
 
 // Gradients and limiters of gradient slot r (this lane's variables), and the
 // face states of its flux edges into shared memory.  PH: see fused_tile.
-template <class M, int NV, int NF, int PH>
+template <class M, int NV, int NF, int PH, bool VISC = false>
 __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& io, unsigned char* smem_raw,
                                            const SlotGeo<M, NF>& geo, int r, int v0, int c0, int halo_off, int flux_off) {
     using S = typename M::S;
@@ -542,7 +568,7 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
             sig[k] = fast::smooth_switch(mx[k] - mn[k], geo.sl[0]);
             limited |= sig[k] < S(1);
         }
-        if (limited) {
+        if (limited && (!VISC || P.order2)) {
             auto apply = [&](auto kind) {
 #pragma unroll
                 for (int k = 0; k < NV; ++k) {
@@ -556,9 +582,11 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
                         up = fast::vmax(up, dq);
                         lo = fast::vmin(lo, dq);
                     }
-                    const S lim_k = fast::limiter_min(kind(), sig[k], mx[k], mn[k], up, lo);
-                    gx[k] *= lim_k;
-                    gy[k] *= lim_k;
+                    lim[k] = fast::limiter_min(kind(), sig[k], mx[k], mn[k], up, lo);
+                    if constexpr (!VISC) {  // the face gradient takes the unlimited ones
+                        gx[k] *= lim[k];
+                        gy[k] *= lim[k];
+                    }
                 }
             };
             if (P.limiter == 2) apply([] { return 2; });
@@ -578,6 +606,10 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
         stv<S, NV>((S*)io.gx + 4 * (size_t)(c0 + r) + v0, gx);
         stv<S, NV>((S*)io.gy + 4 * (size_t)(c0 + r) + v0, gy);
     } else {
+        if constexpr (VISC) {
+            PL::put(GX, L.lt, r, v0, gx);
+            PL::put(GY, L.lt, r, v0, gy);
+        }
         uint32_t any = 0;
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
@@ -586,6 +618,8 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
                 if constexpr (M::exact) qf[k] = qs[k] + (gx[k] * geo.dx(f) + gy[k] * geo.dy(f)) * lim[k];
+                else if constexpr (VISC)
+                    qf[k] = P.order2 ? fast::fma_(fast::fma_(gy[k], geo.dy(f), fast::mul_(gx[k], geo.dx(f))), lim[k], qs[k]) : qs[k];
                 else qf[k] = fast::fma_(gy[k], geo.dy(f), fast::fma_(gx[k], geo.dx(f), qs[k]));
             }
             guard_share<S, NV, M::exact>(P, qf, qs);
@@ -609,9 +643,11 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
                 }
                 PL::put(FS, L.lf, u < FP.max_flux ? u + FP.max_flux : el, v0, qn);
             }
-            PL::put(GX, L.lt, r, v0, gx);
-            PL::put(GY, L.lt, r, v0, gy);
-            if constexpr (M::exact) PL::put(LM, L.lt, r, v0, lim);
+            if constexpr (!VISC) {
+                PL::put(GX, L.lt, r, v0, gx);
+                PL::put(GY, L.lt, r, v0, gy);
+            }
+            if constexpr (M::exact || VISC) PL::put(LM, L.lt, r, v0, lim);
         }
     }
 }
@@ -716,7 +752,7 @@ __device__ __forceinline__ void fused_update(const FusedParams& FP, const TileIO
 // Ghost fill of the tile's boundary ghosts (update_bounds, explicit.cpp:380-417),
 // one thread each, once every thread has stored its cell's new state.  O2: from
 // the limited gradients, else from the cell value.  gl, gd: the tile's entries.
-template <class M, bool REMOTE, bool O2>
+template <class M, bool REMOTE, bool O2, bool VISC = false>
 __device__ __forceinline__ void fused_ghosts(const FusedParams& FP, const TileIO& io, unsigned char* smem_raw,
                                              const int2* gl, const typename M::S* gd, int n, const PartIO& pio) {
     using S = typename M::S;
@@ -730,15 +766,16 @@ __device__ __forceinline__ void fused_ghosts(const FusedParams& FP, const TileIO
         S qs[4], qint[4], b[4];
         const S n0 = gd[4 * i], n1 = gd[4 * i + 1];
         P4::get(reinterpret_cast<const uint4*>(smem_raw + L.q), L.ls, uc, 0, qs);
-        if constexpr (O2) {
+        if (O2 && (!VISC || P.order2)) {
             S gx[4], gy[4], lm[4];
             const S d0 = gd[4 * i + 2], d1 = gd[4 * i + 3];
             P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gx), L.lt, uc, 0, gx);
             P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gy), L.lt, uc, 0, gy);
-            if constexpr (M::exact) P4::get(reinterpret_cast<const uint4*>(smem_raw + L.lm), L.lt, uc, 0, lm);
+            if constexpr (M::exact || VISC) P4::get(reinterpret_cast<const uint4*>(smem_raw + L.lm), L.lt, uc, 0, lm);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if constexpr (M::exact) qint[k] = qs[k] + (gx[k] * d0 + gy[k] * d1) * lm[k];
+                else if constexpr (VISC) qint[k] = fast::fma_(fast::fma_(gy[k], d1, fast::mul_(gx[k], d0)), lm[k], qs[k]);
                 else qint[k] = fast::fma_(gy[k], d1, fast::fma_(gx[k], d0, qs[k]));
             }
             guard_share<S, 4, M::exact>(P, qint, qs);
@@ -931,7 +968,7 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
         double di;
         auto edge = [&](int el, S* e) { ldg4((const S*)FP.eg + 4 * (size_t)(flux_off + el), e); };
         if (l < nown)
-            kmin = fused_cell_dt<M, NF>(FP, io, own, W, l, c0 + l, halo_off, __ldg((const S*)FP.area + c0 + l), edge, di);
+            kmin = fused_cell_dt<M, NF, false>(FP, io, own, W, l, c0 + l, halo_off, __ldg((const S*)FP.area + c0 + l), edge, di);
         tile_dt_reduce(P, T, io, t, l, nown, kmin);
         return true;
     }
@@ -1073,7 +1110,7 @@ template <class M>
 struct FusedLaunch {
     // lays out the tiles' shared memory (FP.L); the bytes of the largest launch
     static size_t smem(FusedParams& FP) {
-        FP.L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_flux, FP.max_ghost, FP.T);
+        FP.L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_flux, FP.max_ghost, FP.T, FP.P.flux == 5);
         return (size_t)std::max(FP.L.total_run, FP.L.total_grad);
     }
     static cudaError_t prepare(FusedParams& FP) {

@@ -516,7 +516,8 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int T, Tile2Arrays& t
 
 template <class S>
 void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
-                 bool first_order, double K, FusedArrays<S>& out) {
+                 FusedKind kind, double K, FusedArrays<S>& out) {
+    const bool first_order = kind == kFusedFirstOrder, viscous = kind == kFusedViscous;
     const int T = t2.tile_cells, F = HostMesh::MAXF;
     const int64_t N = m.n_real, NO = m.owned_real();
     out = FusedArrays<S>();
@@ -540,6 +541,10 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
         out.sl.assign((size_t)slots * (exact ? 2 : 1), S(0));
     }
     out.eg.assign((size_t)edges * 4, S(0));
+    if (viscous) {
+        out.e2.assign((size_t)edges * 4, S(0));
+        out.ar.assign((size_t)slots, S(1));
+    }
     out.ria.resize((size_t)NO);
     for (int64_t c = 0; c < NO; ++c) out.ria[(size_t)c] = 1.0 / (double)(S)fa.area[(size_t)c];
     // each tile's boundary ghosts, by interior cell
@@ -575,6 +580,7 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
             for (int r = 0; r < G; ++r) {
                 if (r < T && r >= own) continue;
                 const int32_t c = dev(r);
+                if (viscous) out.ar[(size_t)(so + r)] = (S)fa.area[(size_t)c];
                 const double A = fa.area[(size_t)c], Ka = K * std::sqrt(A), K3a = Ka * Ka * Ka;
                 if (first_order) { /* no limiter */ }
                 else if (exact) { out.sl[(size_t)(so + r) * 2] = (S)(1. / A); out.sl[(size_t)(so + r) * 2 + 1] = (S)K3a; }
@@ -609,7 +615,14 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                 S* v = &out.eg[(size_t)(inf[2] + e) * 4];
                 const size_t g = (size_t)eoff + e;
                 v[0] = (S)t2.enx[g]; v[1] = (S)t2.eny[g]; v[2] = (S)t2.ele[g];
-                if (first_order) {
+                if (viscous) {
+                    const int32_t ci = dev((int)(t2.edge_ij[g] & 0xFFFF)), cj = dev((int)(t2.edge_ij[g] >> 16));
+                    const double tx = ta.ccx[(size_t)ci] - ta.ccx[(size_t)cj], ty = ta.ccy[(size_t)ci] - ta.ccy[(size_t)cj];
+                    const double len = std::sqrt(tx * tx + ty * ty);
+                    S* u = &out.e2[(size_t)(inf[2] + e) * 4];
+                    u[0] = (S)(tx / len); u[1] = (S)(ty / len); u[2] = (S)(1. / len);
+                }
+                if (first_order || viscous) {
                     const uint64_t ij = t2.edge_ij[g];
                     std::memcpy(&v[3], &ij, sizeof(S));
                     continue;
@@ -629,9 +642,9 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
     tiles(0, t2.n_tiles / nt);
     for (auto& th : pool) th.join();
 }
-template void build_fused<float>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, bool,
+template void build_fused<float>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, FusedKind,
                                  double, FusedArrays<float>&);
-template void build_fused<double>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, bool,
+template void build_fused<double>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, FusedKind,
                                   double, FusedArrays<double>&);
 
 // ----------------------------------------------------------------------------

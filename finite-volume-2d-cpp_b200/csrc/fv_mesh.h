@@ -113,8 +113,11 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int tile_cells, Tile2
 // (K sqrt(A))^3 per slot); otherwise the cell's Green-Gauss coefficients
 // a = w le n / A (outward normal, the neighbour's weight) and face centre -
 // centroid, evaluated in FP64 and rounded once, with 1 / (K sqrt(A))^3 per slot.
-// first_order: no records, and each flux edge's two slots in the bits of its
-// fourth value.
+// kind: kFusedFirstOrder has no records; it and kFusedViscous hold each flux
+// edge's two slots in the bits of its fourth value; kFusedViscous adds the unit
+// vector between the two centroids with the reciprocal of their distance per
+// flux edge, and the slots' areas.
+enum FusedKind { kFusedEuler = 0, kFusedFirstOrder = 1, kFusedViscous = 2 };
 template <class S>
 struct FusedArrays {
     int nf = 3;                          // faces per slot in rec: 3, or 4 with quadrilaterals
@@ -123,6 +126,7 @@ struct FusedArrays {
     std::vector<uint32_t> hd;            // [slots][4] face words (fv_fused.cuh)
     std::vector<S> rec, rec2, sl;        // [nf * slots][4], exact [nf * slots][2], [slots] (exact [slots][2])
     std::vector<S> eg;                   // [flux edges][4]
+    std::vector<S> e2, ar;               // viscous: [flux edges][4], [slots]
     // boundary ghosts of the tiles' owned cells: {interior slot | group << 16,
     // device cell}, {n_x, n_y, d_x, d_y}
     std::vector<int32_t> gl;
@@ -132,7 +136,7 @@ struct FusedArrays {
 };
 template <class S>
 void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
-                 bool first_order, double K, FusedArrays<S>& out);
+                 FusedKind kind, double K, FusedArrays<S>& out);
 
 // One part of a decomposition of a single mesh into n_parts parts.  Part p
 // owns device real cells [own_off[p], own_off[p+1]) (contiguous ranges of the

@@ -1,4 +1,4 @@
-// Persistent run kernel of the Roe kinds: all the time steps of a launch in one
+// Persistent run kernel of the Roe kinds and, in FP64, the Navier-Stokes kind: all the time steps of a launch in one
 // cooperative kernel with one resident CTA per tile, for meshes whose tiles fit
 // the device at once.
 //
@@ -153,13 +153,48 @@ __device__ __forceinline__ double run_min_dt(const unsigned long long* keys, con
     return (d0 != d0) ? d0 : tkey_inv(k);
 }
 
+// le times the Navier-Stokes flux of flux edge el (examples/flatPlate/main.cpp:
+// 126-225): the Roe flux of the face states minus the viscous terms of the
+// corrected face gradient (gradient_for_diffusion, explicit.cpp:70-109).
+template <class S, int NF>
+__device__ __forceinline__ void run_viscous_flux(const FusedParams& FP, const unsigned char* smem_raw, const S* EG,
+                                                 int el, const S* qL, const S* qR, const S* e, S* f) {
+    using P4 = Planes<S, 4>;
+    const FusedSmem& L = FP.L;
+    const uint32_t ij = edge_slots(EG[4 * el + 3]);
+    const int li = (int)(ij & 0xFFFF), lj = (int)(ij >> 16);
+    const S* E2 = reinterpret_cast<const S*>(smem_raw + L.e2) + 4 * el;
+    const S t0 = E2[0], t1 = E2[1], rl = E2[2];
+    S gxi[4], gyi[4], gxj[4], gyj[4], qi[4], qj[4], gx[4], gy[4];
+    P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gx), L.lt, li, 0, gxi);
+    P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gx), L.lt, lj, 0, gxj);
+    P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gy), L.lt, li, 0, gyi);
+    P4::get(reinterpret_cast<const uint4*>(smem_raw + L.gy), L.lt, lj, 0, gyj);
+    P4::get(reinterpret_cast<const uint4*>(smem_raw + L.q), L.ls, li, 0, qi);
+    P4::get(reinterpret_cast<const uint4*>(smem_raw + L.q), L.ls, lj, 0, qj);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const S bx = S(0.5) * (gxi[k] + gxj[k]), by = S(0.5) * (gyi[k] + gyj[k]);
+        const S corr = bx * t0 + by * t1 - (qi[k] - qj[k]) * rl;
+        gx[k] = bx - corr * t0;
+        gy[k] = by - corr * t1;
+    }
+    fast::roe<S>((S)FP.P.gamma, f, qL, qR, e[0], e[1]);
+    fast::ns_viscous<S>(FP.P, f, qL, qR, gx, gy, e[0], e[1]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f[k] *= e[2];
+}
+
 // The time loop of tile blockIdx.x.  NV, NF: as in fused_tile; O2: second order
-// (two-ring tiles), else the face states are the cell values (one ring).
+// (two-ring tiles), else the face states are the cell values (one ring).  FLUX 5
+// (Navier-Stokes, O2; fast policies): the face gradients of its viscous terms
+// come from the same gradients, with or without MUSCL face states (order2).
 template <class M, int FLUX, int NV, int NF, bool O2>
 __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO& D) {
     using S = typename M::S;
     using P4 = Planes<S, 4>;
     constexpr int V = 4, LP = V / NV, NU = (int)sizeof(S) / 4;
+    constexpr bool VISC = FLUX == 5;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ RunState c;
     __shared__ double s_dt, s_time;
@@ -206,6 +241,15 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
         const uint4* gsrc = reinterpret_cast<const uint4*>((const S*)FP.gd + 4 * (size_t)ib.w);
         for (int i = l; i < NU * n_ghost; i += blockDim.x) cpa16(reinterpret_cast<uint4*>(smem_raw + L.gd) + i, gsrc + i);
         for (int i = l; i < n_ghost; i += blockDim.x) cpa8(smem_raw + L.gl + 8 * i, FP.gl + ib.w + i);
+        if constexpr (VISC) {
+            const uint4* esrc = reinterpret_cast<const uint4*>((const S*)FP.e2 + 4 * (size_t)flux_off);
+            for (int i = l; i < NU * n_flux; i += blockDim.x) cpa16(reinterpret_cast<uint4*>(smem_raw + L.e2) + i, esrc + i);
+            for (int i = l; i < G; i += blockDim.x)
+                cpa<(int)sizeof(S)>((S*)(smem_raw + L.ar) + i, (const S*)FP.ar + slot_off + i);
+            // boundary ghosts have no gradient
+            for (int i = l; i < NU * L.lt; i += blockDim.x)
+                reinterpret_cast<uint4*>(smem_raw + L.gx)[i] = reinterpret_cast<uint4*>(smem_raw + L.gy)[i] = make_uint4(0, 0, 0, 0);
+        }
         cpa_wait();
     }
     const int tc = (P.global_dt && P.n_cases > 1) ? P.tile_case[t] : 0;
@@ -280,7 +324,9 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
                 unsigned long long kmin = ~0ull;
                 double di = 0.;
                 auto edge = [&](int el, S* e) { e[0] = EG[4 * el]; e[1] = EG[4 * el + 1]; e[2] = EG[4 * el + 2]; };
-                if (l < nown) kmin = fused_cell_dt<M, NF>(FP, io, dtw, FS, l, c0 + l, halo_off, area, edge, di);
+                if (l < nown)
+                    kmin = fused_cell_dt<M, NF, VISC>(FP, io, dtw, FS, l, c0 + l, halo_off, area, edge, di,
+                                                      reinterpret_cast<const S*>(smem_raw + L.ar));
                 tile_dt_reduce(P, T, io, t, l, nown, kmin);
                 sync.arrive();
                 if (!P.global_dt && uc < nown) dtc = __ldcg(D.dt + c0 + uc);
@@ -292,12 +338,12 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
             // ---- face states
             if constexpr (O2) {
                 if (r0 < G && word_nbr(geo.w[0]) != 0xFFFF)
-                    fused_slot<M, NV, NF, 0>(FP, io, smem_raw, geo, r0, v0, c0, halo_off, flux_off);
+                    fused_slot<M, NV, NF, 0, VISC>(FP, io, smem_raw, geo, r0, v0, c0, halo_off, flux_off);
                 for (int r = r0 + rstep; r < G; r += rstep) {
                     SlotGeo<M, NF> g2;
                     g2.load(FP, slot_off, G, r);
                     if (word_nbr(g2.w[0]) != 0xFFFF)
-                        fused_slot<M, NV, NF, 0>(FP, io, smem_raw, g2, r, v0, c0, halo_off, flux_off);
+                        fused_slot<M, NV, NF, 0, VISC>(FP, io, smem_raw, g2, r, v0, c0, halo_off, flux_off);
                 }
                 __syncthreads();
             } else if (k == 0) {
@@ -323,6 +369,8 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
                     exact::flux_dev<FLUX>(P.gamma, f, qL, qR, e[0], e[1]);
 #pragma unroll
                     for (int i = 0; i < V; ++i) f[i] *= e[2];
+                } else if constexpr (VISC) {
+                    run_viscous_flux<S, NF>(FP, smem_raw, EG, el, qL, qR, e, f);
                 } else {
                     fast::flux_le<FLUX, S>((S)P.gamma, f, qL, qR, e[0], e[1], e[2]);
                 }
@@ -369,7 +417,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
                 fused_update<M, NV, NF, false>(FP, io, smem_raw, own, uc, v0, c0, tc, dtc, s_dt, n_ghost != 0, PartIO{}, res);
             if (n_ghost != 0) {
                 __syncthreads();
-                fused_ghosts<M, false, O2>(FP, io, smem_raw, reinterpret_cast<const int2*>(smem_raw + L.gl),
+                fused_ghosts<M, false, O2, VISC>(FP, io, smem_raw, reinterpret_cast<const int2*>(smem_raw + L.gl),
                                            reinterpret_cast<const S*>(smem_raw + L.gd), n_ghost, PartIO{});
             }
             if (last) fused_partials<NV>(io, smem_raw + L.fs, t, v0, res);
@@ -417,7 +465,9 @@ struct RunLaunch {
     // per cell) 71, 2T 89, T 146, separate kernels 150; FP64 2T 31, T 41,
     // separate 48; FP32 26, 33, 36; 98,784 cells FP32 T 53, separate 55; NACA
     // 65,536 cells FP64 T 53, separate 59; Sod tube (first order) 32,000 cells
-    // FP64 T 9.4, separate 15.8.
+    // FP64 T 9.4, separate 15.8; flat plate (Navier-Stokes) 13,200 cells FP64
+    // 2T 41, separate 104 (two kernels a stage, whose limiter, Green-Gauss and
+    // viscous time-step divisions the run kernel's form does not have).
     template <int F, int NF, bool O2>
     static void list(const FusedParams& FP, RunKernel* k) {
         constexpr int low = sizeof(typename M::S) == 4 ? 4 : 2, high = O2 ? low / 2 : low;
@@ -436,6 +486,13 @@ struct RunLaunch {
         };
         if constexpr (M::exact) {
             if (FP.P.flux == 2) { pick(std::integral_constant<int, 2>{}); return; }
+        }
+        if constexpr (sizeof(typename M::S) == 8 && !M::exact) {
+            if (FP.P.flux == 5) {
+                if (FP.nf == 3) list<5, 3, true>(FP, k);
+                else list<5, 4, true>(FP, k);
+                return;
+            }
         }
         pick(std::integral_constant<int, 1>{});  // the fast policies' two Roe kinds are one function
     }
