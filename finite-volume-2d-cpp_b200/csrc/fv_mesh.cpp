@@ -3,6 +3,7 @@
 #include "fv_mesh.h"
 
 #include <algorithm>
+#include <atomic>
 #include <charconv>
 #include <thread>
 #include <unordered_map>
@@ -513,6 +514,97 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int T, Tile2Arrays& t
         for (int32_t d : touched) local[d] = -1;
     }
 }
+
+template <class S>
+bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, StencilArrays<S>& out) {
+    const int T = ta.tile_cells, nt = ta.n_tiles;
+    const int64_t N = m.n_real;
+    out = StencilArrays<S>();
+    for (int64_t c = 0; c < N && out.nf < HostMesh::MAXF; ++c) out.nf = std::max<int>(out.nf, m.n_faces[c]);
+    const int nf = out.nf;
+    out.coef.assign((size_t)nf * nf * N, S(0));
+    out.slot.resize((size_t)nf * nf * N);
+    out.info.assign((size_t)nt * 4, 0);
+    auto nbr = [&](int64_t c, int f) { return (int64_t)(fa.nbr[(size_t)f * N + c] & 0x7FFFFFFFu); };
+    // outward normal and neighbour's weight of a face; the Green-Gauss
+    // coefficient of q_neighbour - q_c in the cell's gradient
+    struct Face { double nx, ny, le, ax, ay; };
+    auto face = [&](int64_t c, int f) {
+        const size_t i = (size_t)f * N + c;
+        const bool side = fa.nbr[i] >> 31;
+        const double w = side ? 1.0 - fa.g[i] : fa.g[i], s = side ? -1.0 : 1.0, a = w * fa.le[i] / fa.area[(size_t)c];
+        return Face{s * fa.nx[i], s * fa.ny[i], fa.le[i], s * a * fa.nx[i], s * a * fa.ny[i]};
+    };
+    std::vector<std::vector<int32_t>> halos((size_t)nt);
+    std::atomic<bool> ok{true};
+    auto tiles = [&](int t0, int t1) {
+        std::vector<int32_t> slot((size_t)m.n_total, -1);
+        for (int t = t0; t < t1; ++t) {
+            const int64_t c0 = (int64_t)t * T, c1 = std::min<int64_t>(c0 + T, N);
+            std::vector<int32_t>& halo = halos[(size_t)t];
+            auto slot_of = [&](int64_t c) -> int32_t {
+                if (c >= c0 && c < c1) return (int32_t)(c - c0);
+                int32_t& s = slot[(size_t)c];
+                if (s < 0) { s = T + (int32_t)halo.size(); halo.push_back((int32_t)c); }
+                return s;
+            };
+            for (int64_t c = c0; c < c1; ++c) {
+                const double rA = 1.0 / fa.area[(size_t)c];
+                double a[16] = {0.}, Mx = 0., My = 0.;
+                uint16_t sl[16];
+                Face fc[4];
+                for (int k = 0; k < nf * nf; ++k) sl[k] = (uint16_t)(c - c0);
+                for (int f = 0; f < m.n_faces[c]; ++f) {
+                    fc[f] = face(c, f);
+                    const int64_t n = nbr(c, f);
+                    sl[f] = (uint16_t)(slot_of(n) | (n >= N ? 0x8000 : 0));
+                    double tx = ta.ccx[(size_t)c] - ta.ccx[(size_t)n], ty = ta.ccy[(size_t)c] - ta.ccy[(size_t)n];
+                    const double d = std::sqrt(tx * tx + ty * ty);
+                    tx /= d; ty /= d;
+                    const double tn = tx * fc[f].nx + ty * fc[f].ny;
+                    const double mx = 0.5 * rA * fc[f].le * (fc[f].nx - tn * tx), my = 0.5 * rA * fc[f].le * (fc[f].ny - tn * ty);
+                    Mx += mx; My += my;
+                    a[f] -= rA * fc[f].le * tn / d;
+                    if (n >= N) continue;  // a boundary ghost has no gradient
+                    for (int g = 0, k = nf + f * (nf - 1); g < m.n_faces[n]; ++g) {
+                        const Face fn = face(n, g);
+                        const double v = mx * fn.ax + my * fn.ay;
+                        a[f] -= v;
+                        const int64_t o = nbr(n, g);
+                        if (o == c) continue;
+                        a[k] = v;
+                        sl[k] = (uint16_t)slot_of(o);
+                        ++k;
+                    }
+                }
+                for (int f = 0; f < m.n_faces[c]; ++f) a[f] += Mx * fc[f].ax + My * fc[f].ay;
+                for (int k = 0; k < nf * nf; ++k) {
+                    out.coef[(size_t)k * N + c] = (S)a[k];
+                    out.slot[(size_t)k * N + c] = sl[k];
+                }
+            }
+            for (int32_t h : halo) slot[(size_t)h] = -1;
+            if (T + halo.size() > 0x7FFF) ok = false;
+        }
+    };
+    const int th = (int)std::min<int64_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency())), 1 + nt / 256);
+    std::vector<std::thread> pool;
+    for (int k = 1; k < th; ++k) pool.emplace_back(tiles, (int)((int64_t)nt * k / th), (int)((int64_t)nt * (k + 1) / th));
+    tiles(0, nt / th);
+    for (auto& x : pool) x.join();
+    out.max_slots = T;
+    for (int t = 0; t < nt; ++t) {
+        int32_t* inf = &out.info[(size_t)4 * t];
+        inf[0] = (int32_t)out.halo.size();
+        inf[1] = (int32_t)halos[(size_t)t].size();
+        inf[2] = (int32_t)(std::min<int64_t>((int64_t)(t + 1) * T, N) - (int64_t)t * T);
+        out.halo.insert(out.halo.end(), halos[(size_t)t].begin(), halos[(size_t)t].end());
+        out.max_slots = std::max(out.max_slots, T + inf[1]);
+    }
+    return ok;
+}
+template bool build_stencil<float>(const HostMesh&, const FaceArrays&, const TileArrays&, StencilArrays<float>&);
+template bool build_stencil<double>(const HostMesh&, const FaceArrays&, const TileArrays&, StencilArrays<double>&);
 
 template <class S>
 void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,

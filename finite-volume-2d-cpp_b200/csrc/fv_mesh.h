@@ -105,6 +105,20 @@ struct Tile2Arrays {
 };
 void build_tiles2(const HostMesh& m, const FaceArrays& fa, int tile_cells, Tile2Arrays& ta);
 
+// The stencils of the diffusion kind's time derivative (fv_stencil.h) and the
+// two-ring halos of its tiles.  The terms of a cell: its nf faces' neighbours,
+// then the nf - 1 further neighbours of each; unused terms name the cell itself.
+// False if a tile's slots exceed 15 bits.
+template <class S>
+struct StencilArrays {
+    int nf = 3, max_slots = 0;
+    std::vector<int32_t> info, halo;
+    std::vector<S> coef;
+    std::vector<uint16_t> slot;
+};
+template <class S>
+bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, StencilArrays<S>& out);
+
 // The fused stage kernel's view of two-ring tiles (fv_fused.cuh): per gradient
 // slot (T + n1 of each tile) face words and one record per
 // face, in the order its threads read them; per flux edge its geometry.  S:

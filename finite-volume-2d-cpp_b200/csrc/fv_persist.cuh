@@ -87,12 +87,13 @@ __device__ __forceinline__ bool run_divides(unsigned long long step, unsigned lo
     return step % every == 0;
 }
 // Stop criteria of the step about to start (explicit.cpp:717-726).
+template <int V = 4>
 __device__ __forceinline__ void run_step_start(RunState& c, const RunLimits& L) {
     double Rmax = 1.0;
     if (c.step > 0) {
         Rmax = 0.0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) Rmax = exact::dmax(c.R[k], Rmax);
+        for (int k = 0; k < V; ++k) Rmax = exact::dmax(c.R[k], Rmax);
     }
     const bool stop = c.step >= L.max_step || c.time >= L.max_time || Rmax < L.tolerance;
     c.active = !stop;
@@ -100,23 +101,29 @@ __device__ __forceinline__ void run_step_start(RunState& c, const RunLimits& L) 
 }
 // The end of a step (one warp): residual norms from the tiles' partial sums
 // (strided by lane, then a butterfly), time (dt: the step's), print record,
-// the next step's stop criteria.
-__device__ __forceinline__ void run_step_end(const PersistIO& D, RunState& c, const RunLimits& lim, double dt) {
+// the next step's stop criteria.  partials: [n][V], V = 4 or 1.
+template <int V = 4>
+__device__ __forceinline__ void run_step_end(const PersistIO& D, RunState& c, const RunLimits& lim, double dt,
+                                             const double* partials, int n) {
     const int lane = threadIdx.x & 31;
     const bool need_R = c.need_R != 0;
     const unsigned long long step = c.step;
     double s[4] = {0, 0, 0, 0};
     if (need_R) {
-        for (int b = lane; b < D.n_tiles; b += 32) {
-            const double2* p = reinterpret_cast<const double2*>(D.partials + (size_t)b * 4);
-            const double2 x = __ldcg(p), y = __ldcg(p + 1);
-            s[0] += x.x; s[1] += x.y; s[2] += y.x; s[3] += y.y;
+        for (int b = lane; b < n; b += 32) {
+            if constexpr (V == 1) {
+                s[0] += __ldcg(partials + b);
+            } else {
+                const double2* p = reinterpret_cast<const double2*>(partials + (size_t)b * 4);
+                const double2 x = __ldcg(p), y = __ldcg(p + 1);
+                s[0] += x.x; s[1] += x.y; s[2] += y.x; s[3] += y.y;
+            }
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < V; ++k)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-        if (lane < 4) {
+        if (lane < V) {
             const double v = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
             const double r = sqrt(v);
             c.Rraw[lane] = r;
@@ -132,13 +139,13 @@ __device__ __forceinline__ void run_step_end(const PersistIO& D, RunState& c, co
                 r.step = step;
                 r.time = c.time;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) r.R[k] = step == 0 ? 1.0 : c.R[k];
+                for (int k = 0; k < V; ++k) r.R[k] = step == 0 ? 1.0 : c.R[k];
             }
             ++c.n_hist;
         }
         c.time += dt;
         c.step = step + 1;
-        run_step_start(c, lim);
+        run_step_start<V>(c, lim);
     }
     __syncwarp();
 }
@@ -333,7 +340,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
                 // the next step's keys: its set was last read two steps ago
                 if (blockIdx.x == 0)
                     for (int i = l; i < nkeys; i += blockDim.x) D.keys[(size_t)((n + 1) % 3) * nkeys + i] = ~0ull;
-                if (pending && warp == nw - 1) run_step_end(D, c, lim, s_time);
+                if (pending && warp == nw - 1) run_step_end(D, c, lim, s_time, D.partials, D.n_tiles);
             }
             // ---- face states
             if constexpr (O2) {
@@ -428,7 +435,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
     }
     if (pending) {  // the launch's last step
         if (!sync.wait()) return;
-        if (warp == nw - 1) run_step_end(D, c, lim, s_time);
+        if (warp == nw - 1) run_step_end(D, c, lim, s_time, D.partials, D.n_tiles);
         __syncthreads();
     }
     if (blockIdx.x == 0 && l == 0) {

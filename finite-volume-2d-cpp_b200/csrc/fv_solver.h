@@ -12,6 +12,7 @@
 #include "fv_launch.h"
 #include "fv_mesh.h"
 #include "fv_persist.cuh"
+#include "fv_stencil.h"
 #include "fv_tile.cuh"
 
 using namespace fvgpu;
@@ -49,6 +50,9 @@ struct fv_solver {
     // the persistent run kernel of a mesh whose tiles are all resident at once
     // (fn null: none), its dt keys and barrier counter
     RunKernel run_kernel{};
+    bool stencil = false;           // diffusion kind: stages run over stencils
+    StencilParams SP{};
+    double* run_part = nullptr;     // the stencil run kernel's partial sums [2][n_tiles]
     unsigned long long* run_keys = nullptr;
     unsigned* run_bar = nullptr;
     // its schedule (FV_SCHED_*); the work list's per-stage tile counters and
@@ -132,7 +136,7 @@ struct EventLog {
 struct StepCursor {
     TileIO io{};
     FusedParams FPl{};
-    bool grads = false, worklist = false, split_first = false, fast2 = false, dt2 = false;
+    bool grads = false, worklist = false, split_first = false, fast2 = false, dt2 = false, stencil = false;
     int b = 0;
     const void* in = nullptr;
     void* out = nullptr;

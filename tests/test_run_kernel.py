@@ -192,3 +192,61 @@ def test_exact_quotients_out_of_range(scale, order2, oracle):
     got = s.get_state()
     nan = np.isnan(want)
     assert np.array_equal(nan, np.isnan(got)) and bits_equal(got[~nan], want[~nan])
+
+
+@pytest.mark.parametrize("precision", ("fp64", "fp32"))
+@pytest.mark.parametrize("nx, ny, quads", [(1, 1, 0), (8, 8, 0), (13, 5, 0), (24, 6, 1), (130, 90, 0), (420, 260, 0)])
+def test_diffusion_stencil(nx, ny, quads, precision):
+    """One stencil per cell against gradients and fluxes: sums of at most a few
+    dozen products of the differences between neighbouring states, so 64 ulps
+    of the state's range per stage; sizes as in test_sizes, the largest beyond
+    the run kernel (its stages are separate launches)."""
+    em = mixed_strip(nx, ny) if quads else meshgen.rect_tri(nx, ny, 1.0, 0.8, side_names=("wall", "ends"))
+    mesh = fvgpu.Mesh.from_elements(em)
+    g = mesh.geometry()
+    ph = P.heat(dt=0.05 * (0.2 / max(nx, ny)) ** 2)
+    ph.bcs = {"wall": ("copy", None), "ends": ("copy", None)}
+    x, y = np.asarray(g["ccx"]), np.asarray(g["ccy"])
+    q0 = 1.0 + np.sin(9 * x + 1) * np.cos(7 * y) + (np.hypot(x - 0.5, y - 0.4) < 0.2)
+    eps = 1.2e-7 if precision == "fp32" else 2.3e-16
+    for alpha, steps in ((P.RK1_ALPHA, 7), (P.RK5_ALPHA, 4)):
+        a, b = pair(mesh, ph, precision)
+        out = []
+        for s in (a, b):
+            s.set_state(q0)
+            r = s.run(steps, alpha=alpha)
+            recs = []
+            half = s.get_state()
+            s.run(steps + 3, alpha=alpha, restart=False, print_interval=2, on_print=lambda n, t, R: recs.append((n, t)))
+            out.append((half, s.get_state(), r, recs))
+        tol = 64 * eps * (steps + 3) * len(alpha) * np.ptp(q0)
+        for u, v in zip(out[0][:2], out[1][:2]):
+            assert np.abs(u - v).max() <= tol
+        assert out[0][2]["step"] == out[1][2]["step"] == steps and out[0][2]["time"] == out[1][2]["time"]
+        assert out[0][3] == out[1][3]
+        np.testing.assert_allclose(out[0][2]["R"], out[1][2]["R"], rtol=1e4 * eps)
+        if mesh.n_real < 100000:
+            assert a.last_run_stats()[1] <= 4
+
+
+@pytest.mark.parametrize("precision", ("fp64", "fp32"))
+def test_diffusion_stops_and_batch(precision):
+    ph = P.heat(dt=5e-6)
+    ph.bcs = {"wall": ("copy", None), "ends": ("copy", None)}
+    mesh = fvgpu.Mesh.batch([fvgpu.Mesh.from_elements(meshgen.riemann_strip(n, 2)) for n in (40, 7, 64, 1)])
+    q0 = np.sin(7 * np.asarray(mesh.geometry()["ccx"]))
+    eps = 1.2e-7 if precision == "fp32" else 2.3e-16
+    for alpha in (P.RK1_ALPHA, P.RK5_ALPHA):
+        a, b = pair(mesh, ph, precision)
+        recs = []
+        b.set_state(q0)
+        b.run(12, alpha=alpha, on_print=lambda n, t, R: recs.append((t, R[0])))
+        tol = np.sqrt(recs[8][1] * recs[9][1])
+        for kw in (dict(max_time=recs[6][0]), dict(tolerance=tol), dict(max_time=0.0)):
+            got = []
+            for s in (a, b):
+                s.set_state(q0)
+                got.append((s.run(12, alpha=alpha, **kw), s.get_state(), s.case_times()))
+            assert got[0][0]["step"] == got[1][0]["step"] < 12 and got[0][0]["time"] == got[1][0]["time"]
+            assert np.abs(got[0][1] - got[1][1]).max() <= 64 * eps * 12 * len(alpha) * np.ptp(q0)
+            assert bits_equal(got[0][2], got[1][2])
