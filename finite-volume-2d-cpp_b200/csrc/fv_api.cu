@@ -113,13 +113,12 @@ int upload_stencil(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const 
     F.T = ta.tile_cells;
     F.nf = a.nf;
     F.max_slots = a.max_slots;
-    const int32_t* info; const S* coef;
+    const int32_t* info;
     int rc;
-    if ((rc = upload_v(s, a.info, &info)) || (rc = upload_v(s, a.halo, &F.halo)) || (rc = upload_v(s, a.coef, &coef)) ||
+    if ((rc = upload_v(s, a.info, &info)) || (rc = upload_v(s, a.halo, &F.halo)) || (rc = upload_v(s, a.coef, &F.coef)) ||
         (rc = upload_v(s, a.slot, &F.slot)) || (rc = upload_v(s, fa.area, &F.area)))
         return rc;
     F.info = reinterpret_cast<const int4*>(info);
-    F.coef = coef;
     s->stencil = true;
     // the run kernel, where its tiles fit the device at once
     int most = 0;

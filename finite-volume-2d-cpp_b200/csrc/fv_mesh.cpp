@@ -522,18 +522,20 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
     out = StencilArrays<S>();
     for (int64_t c = 0; c < N && out.nf < HostMesh::MAXF; ++c) out.nf = std::max<int>(out.nf, m.n_faces[c]);
     const int nf = out.nf;
-    out.coef.assign((size_t)nf * nf * N, S(0));
+    out.coef.assign((size_t)nf * nf * N, 0.);
     out.slot.resize((size_t)nf * nf * N);
     out.info.assign((size_t)nt * 4, 0);
     auto nbr = [&](int64_t c, int f) { return (int64_t)(fa.nbr[(size_t)f * N + c] & 0x7FFFFFFFu); };
     // outward normal and neighbour's weight of a face; the Green-Gauss
     // coefficient of q_neighbour - q_c in the cell's gradient
+    auto rd = [](double v) { return (double)(S)v; };
     struct Face { double nx, ny, le, ax, ay; };
     auto face = [&](int64_t c, int f) {
         const size_t i = (size_t)f * N + c;
         const bool side = fa.nbr[i] >> 31;
-        const double w = side ? 1.0 - fa.g[i] : fa.g[i], s = side ? -1.0 : 1.0, a = w * fa.le[i] / fa.area[(size_t)c];
-        return Face{s * fa.nx[i], s * fa.ny[i], fa.le[i], s * a * fa.nx[i], s * a * fa.ny[i]};
+        const double gf = rd(fa.g[i]), nx = rd(fa.nx[i]), ny = rd(fa.ny[i]), le = rd(fa.le[i]), w = side ? 1.0 - gf : gf;
+        const double s = side ? -1.0 : 1.0, a = w * le / rd(fa.area[(size_t)c]);
+        return Face{s * nx, s * ny, le, s * a * nx, s * a * ny};
     };
     std::vector<std::vector<int32_t>> halos((size_t)nt);
     std::atomic<bool> ok{true};
@@ -549,7 +551,7 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
                 return s;
             };
             for (int64_t c = c0; c < c1; ++c) {
-                const double rA = 1.0 / fa.area[(size_t)c];
+                const double rA = 1.0 / rd(fa.area[(size_t)c]);
                 double a[16] = {0.}, Mx = 0., My = 0.;
                 uint16_t sl[16];
                 Face fc[4];
@@ -558,7 +560,7 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
                     fc[f] = face(c, f);
                     const int64_t n = nbr(c, f);
                     sl[f] = (uint16_t)(slot_of(n) | (n >= N ? 0x8000 : 0));
-                    double tx = ta.ccx[(size_t)c] - ta.ccx[(size_t)n], ty = ta.ccy[(size_t)c] - ta.ccy[(size_t)n];
+                    double tx = rd(ta.ccx[(size_t)c]) - rd(ta.ccx[(size_t)n]), ty = rd(ta.ccy[(size_t)c]) - rd(ta.ccy[(size_t)n]);
                     const double d = std::sqrt(tx * tx + ty * ty);
                     tx /= d; ty /= d;
                     const double tn = tx * fc[f].nx + ty * fc[f].ny;
@@ -579,7 +581,7 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
                 }
                 for (int f = 0; f < m.n_faces[c]; ++f) a[f] += Mx * fc[f].ax + My * fc[f].ay;
                 for (int k = 0; k < nf * nf; ++k) {
-                    out.coef[(size_t)k * N + c] = (S)a[k];
+                    out.coef[(size_t)k * N + c] = a[k];
                     out.slot[(size_t)k * N + c] = sl[k];
                 }
             }

@@ -113,7 +113,7 @@ template <class S>
 struct StencilArrays {
     int nf = 3, max_slots = 0;
     std::vector<int32_t> info, halo;
-    std::vector<S> coef;
+    std::vector<double> coef;
     std::vector<uint16_t> slot;
 };
 template <class S>

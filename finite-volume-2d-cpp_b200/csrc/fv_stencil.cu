@@ -6,9 +6,9 @@
 // the coefficients (in registers for a whole run, where the tiles fit the
 // device at once) and the latency of a grid barrier or of a launch.  Measured,
 // us per RK5 step, FP64 | FP32, two kernels a stage -> here: 512 cells 28 -> 13 |
-// 26 -> 12, 24,000 cells 33 -> 14 | 30 -> 14, 125,000 cells 58 -> 19 | 54 -> 17,
+// 26 -> 13, 24,000 cells 33 -> 14 | 30 -> 14, 125,000 cells 58 -> 19 | 54 -> 17,
 // 145,800 cells 61 -> 20 | 52 -> 18; a launch per stage: 168,200 cells 75 -> 29 |
-// 66 -> 27, 720,000 cells 267 -> 107 | 162 -> 72.
+// 68 -> 28, 720,000 cells 267 -> 107 | 160 -> 93.
 #include "fv_persist.cuh"
 #include "fv_stencil.h"
 
@@ -19,7 +19,7 @@ namespace {
 template <class S, int NF>
 struct Stencil {
     static constexpr int K = NF * NF;
-    S a[K];
+    double a[K];
     uint32_t w[(K + 1) / 2];
     __device__ __forceinline__ void load(const StencilParams& SP, int c) {
         const size_t N = (size_t)SP.P.n_real;
@@ -27,7 +27,7 @@ struct Stencil {
         for (int k = 0; k < (K + 1) / 2; ++k) w[k] = 0;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            a[k] = __ldg((const S*)SP.coef + k * N + c);
+            a[k] = __ldg(SP.coef + k * N + c);
             w[k / 2] |= (uint32_t)__ldg(SP.slot + k * N + c) << (16 * (k & 1));
         }
     }
@@ -41,10 +41,10 @@ struct Stencil {
     }
     // the time derivative: FP64 sums of the differences from the cell's state
     __device__ __forceinline__ double qt(const S* q, int l) const {
-        const S qc = q[l];
+        const double qc = q[l];
         double s[2] = {0., 0.};
 #pragma unroll
-        for (int k = 0; k < K; ++k) s[k & 1] = fma((double)a[k], (double)(q[slot(k)] - qc), s[k & 1]);
+        for (int k = 0; k < K; ++k) s[k & 1] = fma(a[k], (double)q[slot(k)] - qc, s[k & 1]);
         return s[0] + s[1];
     }
     // the cell's ghosts (copy boundaries) take its new state
@@ -221,9 +221,9 @@ __global__ void __launch_bounds__(THREADS)
 }  // namespace
 
 const void* stencil_run_kernel(bool f32, int nf, int* threads) {
-    // 64 registers; 80 for the quadrilaterals' stencils in FP64
-    *threads = f32 || nf == 3 ? 1024 : 768;
-    if (f32) return nf == 3 ? (const void*)k_run_stencil<float, 3, 1024> : (const void*)k_run_stencil<float, 4, 1024>;
+    // 64 registers; 80 for the quadrilaterals' stencils
+    *threads = nf == 3 ? 1024 : 768;
+    if (f32) return nf == 3 ? (const void*)k_run_stencil<float, 3, 1024> : (const void*)k_run_stencil<float, 4, 768>;
     return nf == 3 ? (const void*)k_run_stencil<double, 3, 1024> : (const void*)k_run_stencil<double, 4, 768>;
 }
 

@@ -6,7 +6,8 @@
 // examples/heatTransfer/main.cpp:33-60) is linear in the states of the cell's
 // two rings: qt_c = sum_k a_k (q_k - q_c), with at most NF^2 terms for cells of
 // NF faces (NF neighbours and NF - 1 further ones of each).  The coefficients
-// are laid out once, evaluated in FP64.
+// are laid out once, evaluated and held in FP64 from the stage precision's
+// geometry: FP32's rounded coordinates are what its results are exact for.
 #pragma once
 #include "fv_launch.h"
 #include "fv_tile.cuh"
@@ -18,7 +19,7 @@ struct StencilParams {
     Params P;
     const int4* info;        // [n_tiles] {halo_off, n_halo, owned cells, 0}
     const int32_t* halo;     // device cell of each halo slot
-    const void* coef;        // S[NF * NF][n_real]
+    const double* coef;      // [NF * NF][n_real]
     const uint16_t* slot;    // [NF * NF][n_real]: slot, 0x8000 set on a ghost neighbour (the first NF)
     const double* area;      // [n_real]
     int T, nf, max_slots;
