@@ -486,7 +486,8 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     // mostly rounding noise, which any other order of operations moves by more
     // than FP32's tolerance, so FP32 keeps its kernels.
     const bool ns = ph->flux == FV_FLUX_NS && precision == FV_PREC_FP64;
-    const bool can_run = (ns || (roe && ph->dt_kind < FV_DT_VISC_MIN)) && sk != FV_STAGE_SPLIT &&
+    // First order in FP32 keeps its kernels for the same reason (flux_le).
+    const bool can_run = (ns || (roe && ph->dt_kind < FV_DT_VISC_MIN && (ph->order2 || precision != FV_PREC_FP32))) && sk != FV_STAGE_SPLIT &&
                          !(sk == FV_STAGE_HYBRID && precision == FV_PREC_FP64_EXACT) &&
                          (!opt || opt->schedule == FV_SCHED_TILE) && m.owned_real() == m.n_real && m.n_real > 0 &&
                          m.n_real <= (int64_t)8 * sms * tile_cells;
@@ -670,8 +671,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
         F.max_slots = ns ? t2.max_slots : t2.max_grad;  // first order stages one ring
         F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;
         if (t2.max_slots < 65535 && 2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= (size_t)227 * 1024) {
-            if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, kind, ph->K);
-            else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, kind, ph->K);
+            rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, kind, ph->K);
             if (rc) return rc;
             const int32_t* h2;
             if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;

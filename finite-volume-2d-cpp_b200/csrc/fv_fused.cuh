@@ -996,7 +996,7 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
 #pragma unroll
             for (int k = 0; k < V; ++k) f[k] *= e[2];
         } else {
-            fast::flux_le<FLUX, S>((S)P.gamma, f, qL, qR, e[0], e[1], e[2]);
+            fast::flux_le<FLUX, true>((S)P.gamma, f, qL, qR, e[0], e[1], e[2]);
         }
 #pragma unroll
         for (int k = 0; k < V; ++k) qL[k] = -f[k];

@@ -379,7 +379,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
                 } else if constexpr (VISC) {
                     run_viscous_flux<S, NF>(FP, smem_raw, EG, el, qL, qR, e, f);
                 } else {
-                    fast::flux_le<FLUX, S>((S)P.gamma, f, qL, qR, e[0], e[1], e[2]);
+                    fast::flux_le<FLUX, O2>((S)P.gamma, f, qL, qR, e[0], e[1], e[2]);
                 }
 #pragma unroll
                 for (int i = 0; i < V; ++i) qL[i] = -f[i];
@@ -488,8 +488,13 @@ struct RunLaunch {
         const bool o2 = FP.P.order2 != 0;
         auto pick = [&](auto f) {
             constexpr int F = decltype(f)::value;
-            if (FP.nf == 3) { if (o2) list<F, 3, true>(FP, k); else list<F, 3, false>(FP, k); }
-            else { if (o2) list<F, 4, true>(FP, k); else list<F, 4, false>(FP, k); }
+            if (o2) {
+                if (FP.nf == 3) list<F, 3, true>(FP, k);
+                else list<F, 4, true>(FP, k);
+            } else if constexpr (sizeof(typename M::S) == 8) {  // (FP32: separate kernels)
+                if (FP.nf == 3) list<F, 3, false>(FP, k);
+                else list<F, 4, false>(FP, k);
+            }
         };
         if constexpr (M::exact) {
             if (FP.P.flux == 2) { pick(std::integral_constant<int, 2>{}); return; }

@@ -155,15 +155,24 @@ __device__ __forceinline__ void burgers(T* f, const T* qi, const T* qj, T n0, T 
     f[1] = T(0.5) * (Vi * qi[1] + Vj * qj[1]) - T(0.5) * V * (qj[1] - qi[1]);
 }
 
-// le times the flux (FLUX 3 Burgers, else Roe)
-template <int FLUX, class T>
+// le times the flux (FLUX 3 Burgers, else Roe).  MUSCL: of second-order face
+// states.  First order in FP32 keeps the unit-normal form: its residual norms
+// hold mostly the rounding noise of the flux sums, which roe_le does not lower
+// (70 Sod tubes of 200 to 200,000 cells: mean error of the norms 1.1e-6 against
+// 0.98e-6, of the state 6.8e-8 against 6.5e-8; the second-order kinds' norms
+// 0.45e-6 against 0.86e-6).
+template <int FLUX, bool MUSCL, class T>
 __device__ __forceinline__ void flux_le(T gamma, T* f, const T* qi, const T* qj, T n0, T n1, T le) {
     if (FLUX == 3) {
         burgers(f, qi, qj, n0, n1);
         f[0] *= le;
         f[1] *= le;
-    } else {
+    } else if (MUSCL || sizeof(T) == 8) {
         roe_le(gamma, f, qi, qj, n0, n1, le);
+    } else {
+        roe(gamma, f, qi, qj, n0, n1);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) f[k] *= le;
     }
 }
 

@@ -523,8 +523,21 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
             kmin = kmin_(kmin, tkey(di));
         } else {
             const S gamma = (S)P.gamma, gm1 = gamma - S(1), cfl = (S)P.cfl;
-            S ws[4];  // {u, v, c}: the run kernel's arithmetic (fused_cell_dt)
-            fast::speeds(gamma, qs, ws);
+            // {u, v, c}; FP64: the run kernel's arithmetic (fused_cell_dt)
+            constexpr bool F64 = sizeof(S) == 8;
+            auto speeds = [&](const S* q, S* w) {
+                if constexpr (F64) {
+                    fast::speeds(gamma, q, w);
+                } else {
+                    const S r = fast::rcp(q[0]);
+                    w[0] = q[1] * r;
+                    w[1] = q[2] * r;
+                    w[2] = fast::sqrt_(gamma * gm1 * (q[3] * r - S(0.5) * (w[0] * w[0] + w[1] * w[1])));
+                }
+            };
+            auto dot = [](S a, S x, S b, S y) { return F64 ? fast::fma_(a, x, b * y) : a * x + b * y; };
+            S ws[4];
+            speeds(qs, ws);
             const S us = ws[0], vs = ws[1], cs = ws[2];
             const S Ai = AR[c];
             S acc = sum ? S(0) : S(1);
@@ -537,12 +550,12 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
                 const S n0 = snx[el], n1 = sny[el], le = sle[el];
                 S qn[4], wn[4];
                 lds<S, 4>(rec + (size_t)o * NR, qn);
-                fast::speeds(gamma, qn, wn);
+                speeds(qn, wn);
                 const S un = wn[0], vn = wn[1], cn = wn[2];
                 const bool ghost = (w[f] & 0x4000) != 0;
                 if (sum) {
-                    const S center = fast::tmax(cs + fabs(fast::fma_(us, n0, vs * n1)), cn + fabs(fast::fma_(un, n0, vn * n1)));
-                    acc = fast::fma_(center, le, acc);
+                    const S center = fast::tmax(cs + fabs(dot(us, n0, vs, n1)), cn + fabs(dot(un, n0, vn, n1)));
+                    acc = F64 ? fast::fma_(center, le, acc) : acc + center * le;
                     if (ghost) {
                         const int g = TP.halo[inf.z + o - T];
                         const double dg = (double)(cfl * AR[g] * fast::rcp(center * le));
@@ -550,11 +563,11 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
                         kmin = kmin_(kmin, tkey(dg));
                     }
                 } else {
-                    const S es = fast::fma_(cs + fabs(us), n0, (cs + fabs(vs)) * n1);
+                    const S es = dot(cs + fabs(us), n0, cs + fabs(vs), n1);
                     acc = fast::tmin(acc, cfl * Ai * fast::rcp(le * fabs(es)));
                     if (ghost) {
                         const int g = TP.halo[inf.z + o - T];
-                        const S en = fast::fma_(cn + fabs(un), n0, (cn + fabs(vn)) * n1);
+                        const S en = dot(cn + fabs(un), n0, cn + fabs(vn), n1);
                         const double dg = (double)fast::tmin(S(1), cfl * (S)AR[g] * fast::rcp(le * fabs(en)));
                         io.dt[g] = dg;
                         kmin = kmin_(kmin, tkey(dg));
@@ -1000,7 +1013,7 @@ __device__ __forceinline__ void tile_stage(const TileParams& TP, const TileIO& i
             } else if constexpr (M::exact) {
                 exact::flux_dev<FLUX>(P.gamma, f, qL, qR, n0, n1);
             } else {
-                fast::flux_le<FLUX, S>((S)P.gamma, f, qL, qR, n0, n1, sle[el]);
+                fast::flux_le<FLUX, MUSCL>((S)P.gamma, f, qL, qR, n0, n1, sle[el]);
             }
             if constexpr (!M::exact && FLUX == 4) {
                 const S le = sle[el];
