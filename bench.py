@@ -68,6 +68,10 @@ ALGO_BYTES = {
 # q_new: FP64 8*3 + 16 + 8 + 1.5*28 + 8 + 8 = 106 (114 exact); FP32 4*3 + 8 +
 # 4 + 1.5*16 + 8 + 4 + 8/5 = 61.6.  Its gradient kernel needs no face centres:
 # FP64 8 + 16 + 8 + 1.5*36 + 24 = 110; FP32 4 + 8 + 4 + 1.5*20 + 12 = 58.
+# In the fast modes' default layout its stage is one stencil kernel: 9
+# FP64 coefficients and 16-bit slots (triangles), q, q_base and q_new: FP64
+# 9*10 + 24 = 114; FP32 9*10 + 4 + 8 + 4 + 8/5 = 107.6.
+ALGO_BYTES_STENCIL = {"fp64": 114.0, "fp32": 107.6}
 ALGO_BYTES_KIND = {
     "ns": {"fp64_exact": {"stage": 290.0, "grad_lim": 230.0}, "fp64": {"stage": 290.0, "grad_lim": 230.0},
            "fp32": {"stage": 174.4, "grad_lim": 118.0}},
@@ -92,10 +96,10 @@ def algo_bytes(ph, precision, kernel):
 TRAFFIC_B_PER_CELL = {
     ("step", "fp32", "split"): (153.2, "ncu --set full -k regex:k_tile_stage -s 30 -c 2, "
                                        "bench.py --precision fp32 --steps 20 --warmup 3 --no-cpu-baseline"),
-    ("step", "fp32", "fused"): (150.6, "ncu --set full -k regex:k_tile_fused -s 10 -c 2, bench.py --precision "
-                                       "fp32 --steps 20 --warmup 3 --no-cpu-baseline --batch-steps 0"),
-    ("step", "fp64", "fused"): (231.3, "ncu --set full -k regex:k_tile_fused -s 10 -c 2, bench.py --precision "
-                                       "fp64 --steps 20 --warmup 3 --no-cpu-baseline --batch-steps 0"),
+    ("step", "fp32", "fused"): (181.5, "ncu -k regex:k_tile_fused, mean of the 5 launches of one RK5 step, "
+                                       "perf/cases.py step_1m_fp32"),
+    ("step", "fp64", "fused"): (304.8, "ncu -k regex:k_tile_fused, mean of the 5 launches of one RK5 step, "
+                                       "perf/cases.py step_1m_fp64"),
 }
 
 
@@ -316,8 +320,9 @@ def measure_mode(args, em, mesh, geo, ph, alpha, ic, precision, local, dist, wor
         s = fvgpu.Solver(mesh, ph, precision, device=local, tile_cells=args.tile_cells,
                          stage_kernels=args.stage_kernels, schedule=args.schedule)
         s.tile_cells = args.tile_cells or 128
-    # hybrid: the split kernels for the first stage, the fused kernel for the
-    # other four (the dominant kernel)
+    # (hybrid launches what fused does in the fast modes; the per-launch times
+    # below are those of the separate kernels, also where the run itself is one
+    # launch of the persistent run kernel)
     fused = s.stage_kernels in ("fused", "hybrid")
     stream = torch.cuda.Stream(device=local)
     s.set_stream(stream.cuda_stream)
@@ -360,11 +365,14 @@ def measure_mode(args, em, mesh, geo, ph, alpha, ic, precision, local, dist, wor
     out["per_launch_ms"] = {kinds[k]: (ms_k[k] / cnt_k[k] if cnt_k[k] else 0.0) for k in range(6)}
     out["share"] = {kinds[k]: float(ms_k[k] / ms_k.sum()) for k in range(6)}
     peak, peak_kind = measured_peak_hbm()
-    kb = (ALGO_BYTES[precision]["fused"] if fused else algo_bytes(ph, precision, "stage")) * N
+    stencil = ph.flux == "diffusion" and out["per_launch_ms"]["grad_lim"] == 0  # the default layout
+    kb = (ALGO_BYTES[precision]["fused"] if fused else ALGO_BYTES_STENCIL[precision] if stencil
+          else algo_bytes(ph, precision, "stage")) * N
     achieved = kb / (out["per_launch_ms"]["fused" if fused else "stage"] / 1e3) / 1e9
     out["stage_kernels"] = s.stage_kernels
     out["schedule"] = s.schedule
     kname = ("gradients + limiter + flux + RK update + ghost fill of a two-ring tile (k_tile_fused)" if fused
+             else "stencil + RK update + ghost fill (k_stencil_stage)" if stencil
              else "flux + RK update + ghost fill (k_tile_stage)")
     out["roofline"] = {"bound": "hbm", "kernel": kname,
                        "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -376,7 +384,7 @@ def measure_mode(args, em, mesh, geo, ph, alpha, ic, precision, local, dist, wor
         out["roofline"]["traffic"] = cap[0] * N
         out["roofline"]["traffic_source"] = ("dram__bytes_read.sum + dram__bytes_write.sum per launch of the "
                                              "stage kernel, from: " + cap[1])
-    if (ph.order2 or ph.diffusive) and not fused:
+    if (ph.order2 or ph.diffusive) and not fused and not stencil:
         kg = algo_bytes(ph, precision, "grad_lim") * N
         out["roofline_grad_lim"] = {"achieved": kg / (out["per_launch_ms"]["grad_lim"] / 1e3) / 1e9,
                                     "frac": kg / (out["per_launch_ms"]["grad_lim"] / 1e3) / 1e9 / peak}
@@ -681,10 +689,11 @@ def measure_decomposed(args, mesh, geo, ph, alpha, ic, prec, parts_per_gpu, loca
             s.run(args.warmup + steps, alpha=alpha, restart=False)
             ms1, _ = s.last_run_stats()
             q1 = s.get_state()
+            s_kernels = s.stage_kernels
             s.close()
             q = grp.get_state()
             out["single_solver"] = {"value": mesh.n_real * len(alpha) * steps / (ms1 / 1e3),
-                                    "ms_per_step": ms1 / steps, "stage_kernels": "hybrid",
+                                    "ms_per_step": ms1 / steps, "stage_kernels": s_kernels,
                                     "decomposition_time_ratio": ms / ms1,
                                     "states_bit_identical": q.tobytes() == q1.tobytes()}
         return out

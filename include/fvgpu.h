@@ -358,7 +358,11 @@ int fv_set_state_device(fv_solver* s, const double* q_device);
 int fv_get_state_device(fv_solver* s, double* q_device);
 /* The run() time loop on the device (explicit.cpp:708-801).  Steps are
  * captured in CUDA graphs of `chunk` steps; stopping criteria are evaluated
- * on the device, so the host only waits once per chunk. */
+ * on the device, so the host only waits once per chunk.  Where the mesh's
+ * tiles fit the device at once (the Roe kinds but FP32 first order,
+ * Navier-Stokes in FP64, the diffusion kind in FP64 and FP32; default layout
+ * and schedule) up to 2,048 steps are one cooperative launch instead; with
+ * on_print, `chunk` steps. */
 int fv_run(fv_solver* s, const fv_run_options* opt, fv_run_info* info);
 /* Continue a run in another solver of the same mesh, typically with another
  * precision (FP32-bulk for the transient, FP64 for the tail of a steady
@@ -384,7 +388,8 @@ int fv_check_state(fv_solver* s);
 /* Pressure force on the faces of boundary group `group` (FP64 sum over the
  * group's faces of p(interior state) * n * length). */
 int fv_boundary_force(fv_solver* s, int32_t group, double* fx, double* fy);
-/* Chunk length of the captured step graphs (default 16). */
+/* Chunk length of the captured step graphs, and of a cooperative launch with
+ * on_print (default 16). */
 int fv_solver_set_chunk(fv_solver* s, int32_t steps);
 /* out[6] = {tiles, cells per tile, max halo cells per tile, max edges per
  * tile, precision, bytes per stored stage value}. */
@@ -406,7 +411,8 @@ int fv_solver_schedule(fv_solver* s);
 int fv_last_run_stats(fv_solver* s, double* device_ms, int64_t* kernel_launches);
 
 /* Per-kernel device timing: runs n_steps more time steps without graph
- * capture, with a CUDA event after every kernel on the solver's stream.
+ * capture (separate kernels also where fv_run takes one cooperative launch),
+ * with a CUDA event after every kernel on the solver's stream.
  * out_ms[6] / out_count[6] per kernel kind: 0 step control, 1 time step,
  * 2 gradients + limiters, 3 flux + update + ghost fill, 4 step end, 5 the
  * fused stage kernel (gradients through ghost fill in one launch). */
