@@ -127,7 +127,7 @@ int upload_stencil(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const 
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
     // the run kernel pays wherever one CTA per SM holds all tiles (145,800
-    // cells FP64: 20 us per step; just above, a launch per stage 29); as few
+    // cells FP64: 20 us per step; just above, a launch per stage 25); as few
     // tiles to a CTA as that allows
     const int per = (s->n_tiles + sms - 1) / sms;
     const size_t smem = (size_t)per * F.max_slots * sizeof(S);
@@ -683,7 +683,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
         if ((rc = choose_run_kernel(s.get()))) return rc;
     }
     // The diffusion kind of the fast modes in its default layout: one linear
-    // stencil per cell and stage (fv_stencil.h), 2.0 to 3.3 times faster than
+    // stencil per cell and stage (fv_stencil.h), 2.0 to 3.7 times faster than
     // gradient and flux kernels at every size from 512 to 720,000 cells.
     // FP64_EXACT keeps the reference's order of operations.
     if (ph->flux == FV_FLUX_DIFFUSION && precision != FV_PREC_FP64_EXACT && sk == FV_STAGE_AUTO &&
@@ -959,7 +959,7 @@ int step_open(fv_solver* s, const std::vector<double>& alpha, int b, bool first,
 int step_dt(fv_solver* s, StepCursor& c, EventLog* log) {
     // every kernel after step_begin is a programmatic dependent of the one
     // before it (its constant tile data is staged during that one's tail)
-    if ((c.grads && !c.fast2) || c.split_first) return 0;
+    if ((c.grads && !c.fast2) || c.split_first || c.stencil) return 0;
     TileIO dio = c.io;
     dio.work_reset = c.worklist ? s->work : nullptr;
     if (c.dt2) tile::launch_fused_split(s->precision, c.FPl, dio, s->stream, true, s->n_tiles, 3);
@@ -1010,6 +1010,7 @@ int step_stage(fv_solver* s, const std::vector<double>& alpha, int k, StepCursor
     if (c.stencil) {
         StencilParams F = s->SP;
         F.P = TP.P;
+        if (k != 0) so.dtkeys = nullptr;
         launch_stencil_stage(s->f32, F, so, s->n_tiles, st, pdl); ++n; mark(KK_STAGE);
         c.in = out_s;
         c.out = out_s;

@@ -7,8 +7,8 @@
 // device at once) and the latency of a grid barrier or of a launch.  Measured,
 // us per RK5 step, FP64 | FP32, two kernels a stage -> here: 512 cells 28 -> 13 |
 // 26 -> 13, 24,000 cells 33 -> 14 | 30 -> 14, 125,000 cells 58 -> 19 | 54 -> 17,
-// 145,800 cells 61 -> 20 | 52 -> 18; a launch per stage: 168,200 cells 75 -> 29 |
-// 68 -> 28, 720,000 cells 267 -> 107 | 160 -> 93.
+// 145,800 cells 61 -> 20 | 52 -> 18; a launch per stage: 168,200 cells 74 -> 25 |
+// 65 -> 23, 720,000 cells 271 -> 72 | 160 -> 64.
 #include "fv_persist.cuh"
 #include "fv_stencil.h"
 
@@ -70,7 +70,10 @@ __device__ __forceinline__ double block_sum(double r) {
     return r;
 }
 
-// One stage of every tile.
+// One stage of every tile.  dtkeys (a step's first stage): the step end's view of
+// the constant time step, one value per case; a time-step kernel over all cells
+// wrote one per cell (21 us of a step; 1,002,528 cells FP64: a step 170 us with
+// it, 139 without).
 template <class S, int NF>
 __global__ void __launch_bounds__(kTileMax) k_stencil_stage(const __grid_constant__ StencilParams SP, TileIO io) {
     pdl_trigger();
@@ -98,6 +101,12 @@ __global__ void __launch_bounds__(kTileMax) k_stencil_stage(const __grid_constan
     for (int h = l; h < inf.y; h += blockDim.x) q[SP.T + h] = in[h == l ? h0 : __ldg(SP.halo + inf.x + h)];
     __syncthreads();
     if (inactive) return;
+    if (io.dtkeys != nullptr && t == 0) {
+        for (int i = l; i < P.n_cases; i += blockDim.x) {
+            io.dtkeys[(size_t)i * kDtSlots] = tkey(P.dt_const);
+            io.dt[P.n_cases > 1 ? P.case_cell0[i] : P.cell0] = P.dt_const;
+        }
+    }
     double res = 0.;
     if (on) {
         const double qt = st.qt(q, l), qnew = fma(qt, P.dt_const * io.alpha, qb);

@@ -239,10 +239,14 @@ def test_diffusion_stencil(nx, ny, quads, precision):
 
 
 @pytest.mark.parametrize("precision", ("fp64", "fp32"))
-def test_diffusion_stops_and_batch(precision):
-    ph = P.heat(dt=5e-6)
+@pytest.mark.parametrize("large", (False, True))  # True: beyond the run kernel
+def test_diffusion_stops_and_batch(large, precision):
+    ph = P.heat(dt=1e-7 if large else 5e-6)
     ph.bcs = {"wall": ("copy", None), "ends": ("copy", None)}
-    mesh = fvgpu.Mesh.batch([fvgpu.Mesh.from_elements(meshgen.riemann_strip(n, 2)) for n in (40, 7, 64, 1)])
+    strips = [meshgen.riemann_strip(n, 2) for n in (40, 7, 64, 1)]
+    if large:
+        strips += [meshgen.rect_tri(300, 280, 1.0, 0.8), meshgen.rect_tri(3, 2, 1.0, 0.8)]
+    mesh = fvgpu.Mesh.batch([fvgpu.Mesh.from_elements(em) for em in strips])
     q0 = np.sin(7 * np.asarray(mesh.geometry()["ccx"]))
     eps = 1.2e-7 if precision == "fp32" else 2.3e-16
     for alpha in (P.RK1_ALPHA, P.RK5_ALPHA):
