@@ -467,13 +467,13 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     const int tile_cells = (opt && opt->tile_cells) ? opt->tile_cells : 128;
     if (tile_cells != 64 && tile_cells != 128 && tile_cells != 256)
         return fail(FV_ERR_ARG, "tile_cells must be 64, 128 or 256");
-    // one fused kernel per stage for the second-order Roe kinds; the fast
-    // modes' split layout runs over the two-ring tiles as well, which are
-    // built beside the one-ring tiles
+    // one fused kernel per stage for the second-order Roe kinds; FP64's
+    // split layout runs over the two-ring tiles as well, which are built beside
+    // the one-ring tiles
     const int sk = opt ? opt->stage_kernels : FV_STAGE_AUTO;
     const bool can_fuse = ph->V == 4 && ph->order2 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST) &&
                           !ph->diffusive && !ph->smooth_residuals;
-    const bool two_ring = can_fuse && (sk != FV_STAGE_SPLIT || precision != FV_PREC_FP64_EXACT);
+    const bool two_ring = can_fuse && (sk != FV_STAGE_SPLIT || precision == FV_PREC_FP64);
     // the persistent run kernel (choose_run_kernel): the Roe kinds in their
     // default layout and schedule with a CFL or constant time step, not on a
     // part of a decomposition.  Its tiles have to fit the device at once: at
@@ -482,11 +482,11 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const bool roe = ph->V == 4 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST);
     // The Navier-Stokes kind has one in FP64 (flat plate, 13,200 cells: 41
-    // against 104 us per step).  Its FP32 residual norms on low-Mach flows are
-    // mostly rounding noise, which any other order of operations moves by more
-    // than FP32's tolerance, so FP32 keeps its kernels.
+    // against 104 us per step).  FP32 results keep their bits (flux_le), which
+    // its other formulas would change, and FP64_EXACT's the oracle's, for which
+    // no such form has been written: both keep the separate kernels.
     const bool ns = ph->flux == FV_FLUX_NS && precision == FV_PREC_FP64;
-    // First order in FP32 keeps its kernels for the same reason (flux_le).
+    // First order in FP32 keeps the bits of its one-ring kernel in the same way.
     const bool can_run = (ns || (roe && ph->dt_kind < FV_DT_VISC_MIN && (ph->order2 || precision != FV_PREC_FP32))) && sk != FV_STAGE_SPLIT &&
                          !(sk == FV_STAGE_HYBRID && precision == FV_PREC_FP64_EXACT) &&
                          (!opt || opt->schedule == FV_SCHED_TILE) && m.owned_real() == m.n_real && m.n_real > 0 &&
@@ -585,9 +585,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
                     return fail(FV_ERR_ARG, "the work-list schedule needs the dt kernel of the fused layout");
                 s->sched = sched;
                 F.lanes = fused_lanes(s.get(), sms);
-                // automatic choice: in FP32 the split first stage (its gradient
-                // kernel computes dt) saves more than it costs; in FP64 the
-                // fused first stage and the separate dt kernel are faster
+                // automatic choice ("hybrid" and "fused" launch the same in FP32)
                 s->split_first = sk == FV_STAGE_HYBRID ||
                                  (sk == FV_STAGE_AUTO && sched != FV_SCHED_WORKLIST && precision == FV_PREC_FP32);
             }
@@ -935,15 +933,14 @@ int step_open(fv_solver* s, const std::vector<double>& alpha, int b, bool first,
     // comes from the dt kernel, as in first order
     c.stencil = s->stencil && !c.part;
     c.grads = (TP.P.order2 || TP.P.diffusive) && !s->fused && !c.stencil;
-    // the fast modes' split kernels over the two-ring tiles
-    c.fast2 = s->two_ring && s->precision != FV_PREC_FP64_EXACT;
+    // FP64's split kernels over the two-ring tiles
+    c.fast2 = s->two_ring && s->precision == FV_PREC_FP64;
     // the time step over those tiles: the CFL and constant kinds (the viscous
     // ones, and FP64_EXACT's split layouts, keep the one-ring kernels)
     c.dt2 = s->two_ring && TP.P.dt_kind < 3;
     // FP64_EXACT's hybrid layout: the split first stage's gradient kernel
     // computes dt.  In the fast modes the dt kernel over the fused kernel's
-    // tiles and a fused first stage cost less (998k cells, FP32: 80 us against
-    // 104 us for the split first stage), so hybrid launches what fused does.
+    // tiles and a fused first stage cost less, so hybrid launches what fused does.
     c.split_first = s->fused && s->split_first && s->precision == FV_PREC_FP64_EXACT;
     // the work-list schedule: one tile counter per stage, zeroed by the dt kernel
     c.worklist = s->fused && s->sched == FV_SCHED_WORKLIST && alpha.size() <= (size_t)kWorkSlots;

@@ -18,9 +18,15 @@
 // and, in the exact policy, bit-identical to the reference's).
 //
 // The geometry of the gradient phase is stored per (gradient cell, face), in
-// the order the threads read it: the fast policies hold the cell's
-// Green-Gauss coefficient (the gradient is the sum of a_f (q_nb - q), since a
-// closed cell's face normals sum to zero) and the vector to the face centre.
+// the order the threads read it: FP64 holds the cell's Green-Gauss
+// coefficient (the gradient is the sum of a_f (q_nb - q), since a closed cell's
+// face normals sum to zero) and the vector to the face centre; FP32 and the exact
+// policy hold what the face value needs.  FP32 takes the face values
+// q_i + (q_j - q_i) g, the limiter per face and the Roe flux on the unit normal
+// with the roundings that its one-ring kernels have: its results are pinned bit
+// for bit, since flows amplify another order of operations to 1e-4 and more of
+// the residual norms.  (The FP64 forms in FP32 take 301 us per step of a 20-step
+// call at 998k cells, these 352; they are nearer to 64 bits, but other results.)
 // It goes from global memory straight into registers, with coalesced 16- or
 // 32-byte loads issued before the dependency wait.
 //
@@ -101,12 +107,12 @@ struct FusedParams {
     // with nf = 3: the fourth word holds `sl`.
     const uint4* hd;
     // per gradient slot and face, at nf * slot_off + f * (T + n1) + slot:
-    // fast S[4] {a_x, a_y, d_x, d_y}; exact S[4] {n_x, n_y, length (negative
+    // FP64 S[4] {a_x, a_y, d_x, d_y}; exact S[4] {n_x, n_y, length (negative
     // on the edge's second side), weight} and S[2] {d_x, d_y} in rec2 (d: face
-    // centre - centroid)
+    // centre - centroid); FP32 as exact, the weight negative with the length
     const void* rec;
     const void* rec2;
-    const void* sl;            // per gradient slot: fast S 1 / (K sqrt(A))^3; exact double2 {1 / A, (K sqrt(A))^3}
+    const void* sl;            // per gradient slot: FP64 1 / (K sqrt(A))^3; FP32 A; exact double2 {1 / A, (K sqrt(A))^3}
     // S[4] per flux edge: n_x, n_y, length and, exact, the signed zero that a
     // boundary ghost's zero gradient adds; first order: its two slots in the
     // bits of the fourth (edge_slots)
@@ -275,13 +281,14 @@ __device__ __forceinline__ void guard_share(const Params& P, S* qf, const S* qc)
 template <class M, int NF>
 struct SlotGeo {
     using S = typename M::S;
+    static constexpr bool faces = M::exact || sizeof(S) == 4;  // face values (rec2), or differences
     uint32_t w[NF];
     S sl[M::exact ? 2 : 1];
     S a[NF][4];
-    S d[M::exact ? NF : 1][2];
+    S d[faces ? NF : 1][2];
     __device__ __forceinline__ bool face(int f) const { return f < 3 || word_nbr(w[f]) != 0xFFFF; }
-    __device__ __forceinline__ S dx(int f) const { if constexpr (M::exact) return d[f][0]; else return a[f][2]; }
-    __device__ __forceinline__ S dy(int f) const { if constexpr (M::exact) return d[f][1]; else return a[f][3]; }
+    __device__ __forceinline__ S dx(int f) const { if constexpr (faces) return d[f][0]; else return a[f][2]; }
+    __device__ __forceinline__ S dy(int f) const { if constexpr (faces) return d[f][1]; else return a[f][3]; }
     __device__ __forceinline__ static void prefetch(const FusedParams& FP, uint32_t slot_off, uint32_t G, uint32_t r) {
         auto pf = [](const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); };
         pf(FP.hd + (slot_off + r));
@@ -306,6 +313,9 @@ struct SlotGeo {
             ldg4((const S*)FP.rec + 4 * (size_t)(b + f * G), a[f]);
             if constexpr (M::exact) {
                 const double2 x = __ldg(reinterpret_cast<const double2*>(FP.rec2) + (b + f * G));
+                d[f][0] = x.x; d[f][1] = x.y;
+            } else if constexpr (faces) {
+                const float2 x = __ldg(reinterpret_cast<const float2*>(FP.rec2) + (b + f * G));
                 d[f][0] = x.x; d[f][1] = x.y;
             }
         }
@@ -382,15 +392,15 @@ __device__ __forceinline__ unsigned long long fused_cell_dt(const FusedParams& F
                 }
             }
         } else if (sum) {
-            const S center = fast::tmax(ws[2] + fabs(fast::fma_(ws[0], e[0], ws[1] * e[1])),
-                                        wn[2] + fabs(fast::fma_(wn[0], e[0], wn[1] * e[1])));
-            acc = fast::fma_(center, e[2], acc);
+            const S center = fast::tmax(ws[2] + fabs(fast::dot2(ws[0], e[0], ws[1], e[1])),
+                                        wn[2] + fabs(fast::dot2(wn[0], e[0], wn[1], e[1])));
+            acc = fast::madd(center, e[2], acc);
             if (ghost) dg = (double)(cfl * A * fast::rcp(center * e[2]));
         } else if (!constant) {
-            const S es = fast::fma_(ws[2] + fabs(ws[0]), e[0], (ws[2] + fabs(ws[1])) * e[1]);
+            const S es = fast::dot2(ws[2] + fabs(ws[0]), e[0], ws[2] + fabs(ws[1]), e[1]);
             acc = fast::tmin(acc, cfl * A * fast::rcp(e[2] * fabs(es)));
             if (ghost) {
-                const S en = fast::fma_(wn[2] + fabs(wn[0]), e[0], (wn[2] + fabs(wn[1])) * e[1]);
+                const S en = fast::dot2(wn[2] + fabs(wn[0]), e[0], wn[2] + fabs(wn[1]), e[1]);
                 dg = (double)fast::tmin(S(1), cfl * A * fast::rcp(e[2] * fabs(en)));
             }
         }
@@ -543,6 +553,66 @@ __device__ __forceinline__ void fused_slot(const FusedParams& FP, const TileIO& 
                     lv = sig[i] + (1.0 - sig[i]) * lv;
                     lim[k0 + i] = exact::dmin(lim[k0 + i], lv);
                 }
+        }
+    } else if constexpr (sizeof(S) == 4) {
+        float qmn[NV], qmx[NV], sig[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) { gx[k] = 0; gy[k] = 0; qmn[k] = qs[k]; qmx[k] = qs[k]; lim[k] = 1; }
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            if (!geo.face(f)) continue;
+            const float nx = geo.a[f][0], ny = geo.a[f][1], le = geo.a[f][2], g = geo.a[f][3];
+            float qn[NV];
+            PL::get(Q, L.ls, word_nbr(geo.w[f]), v0, qn);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                // q_i + (q_j - q_i) g of the edge's first and second cells i and
+                // j; on the second side le and g are negative
+                const float fl = fast::fma_(qn[k] - qs[k], g, le < 0.f ? qn[k] : qs[k]) * le;
+                gx[k] = fast::fma_(fl, nx, gx[k]);
+                gy[k] = fast::fma_(fl, ny, gy[k]);
+                qmn[k] = fast::vmin(qmn[k], qn[k]);
+                qmx[k] = fast::vmax(qmx[k], qn[k]);
+            }
+        }
+        const float A = geo.sl[0], invA = fast::rcp(A), Ka = (float)P.K * fast::sqrt_(A), K3a = Ka * Ka * Ka;
+        const float rK3a = fast::rcp(K3a), tol = 1e-15f;
+        bool limited = false;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            gx[k] *= invA;
+            gy[k] *= invA;
+            const float d = qmx[k] - qmn[k], d2 = d * d;
+            if (d2 <= K3a) sig[k] = 1;
+            else if (d2 <= 2 * K3a) {
+                const float y = d2 * rK3a - 1.f;
+                sig[k] = (2.f * y - 3.f) * y * y + 1.f;
+            } else sig[k] = 0;
+            limited |= sig[k] < 1.f;
+        }
+        if (limited) {
+            auto apply = [&](auto kind) {
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    if (!(sig[k] < 1.f)) continue;
+                    const float mx = qmx[k] - qs[k], mn = qmn[k] - qs[k];
+                    float least = 1.f;  // of phi: the limiter grows with it, rounding included
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        if (!geo.face(f)) continue;
+                        const float dqg = gx[k] * geo.dx(f) + gy[k] * geo.dy(f);
+                        const bool up = dqg > tol;
+                        const float phi = fast::limiter_ratio(kind(), up ? mx : mn, dqg);
+                        if (up || dqg < -tol) least = fast::vmin(least, phi);
+                    }
+                    lim[k] = fast::vmin(1.f, fast::fma_(1.f - sig[k], least, sig[k]));
+                    gx[k] *= lim[k];
+                    gy[k] *= lim[k];
+                }
+            };
+            if (P.limiter == 2) apply([] { return 2; });
+            else if (P.limiter == 1) apply([] { return 1; });
+            else apply([&] { return P.limiter; });
         }
     } else {
         S mn[NV], mx[NV], sig[NV];
@@ -1136,7 +1206,7 @@ struct FusedLaunch {
                 set(fn);
             if constexpr (M::exact) set((const void*)k_tile_fused<M, F, 1, NF>);
             set((const void*)k_tile_fused_dt<M, NF>);
-            if constexpr (!M::exact)
+            if constexpr (!M::exact && sizeof(typename M::S) == 8)
                 for (const void* fn : {(const void*)k_tile_fused_grad<M, NF>, (const void*)k_tile_fused_flux<M, NF>})
                     set(fn);
         };
@@ -1206,7 +1276,7 @@ struct FusedLaunch {
     static void split_f(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase) {
         const FusedSmem& L = FP.L;
         if (phase == 3) go(k_tile_fused_dt<M, NF>, n_tiles, FP.T, L.total_grad, st, pdl, FP, io);
-        else if constexpr (M::exact) return;
+        else if constexpr (M::exact || sizeof(typename M::S) == 4) return;
         else if (phase == 2) go(k_tile_fused_flux<M, NF>, n_tiles, FP.T, L.total, st, pdl, FP, io);
         else go(k_tile_fused_grad<M, NF>, n_tiles, FP.T, L.total_grad, st, pdl, FP, io);
     }

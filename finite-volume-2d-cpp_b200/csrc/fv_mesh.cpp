@@ -629,9 +629,12 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
     }
     out.hd.assign((size_t)slots * 4, 0x8000FFFFu);
     const bool packed = nf == 3 && sizeof(S) == 4 && !first_order;  // the fourth word holds sl
+    const bool faces = exact || sizeof(S) == 4;  // face values, not differences from the cell's state
+    // a difference as the stage precision forms it from its rounded operands
+    auto diff = [](double a, double b) { return (S)((S)a - (S)b); };
     if (!first_order) {
         out.rec.assign((size_t)nf * slots * 4, S(0));
-        if (exact) out.rec2.assign((size_t)nf * slots * 2, S(0));
+        if (faces) out.rec2.assign((size_t)nf * slots * 2, S(0));
         out.sl.assign((size_t)slots * (exact ? 2 : 1), S(0));
     }
     out.eg.assign((size_t)edges * 4, S(0));
@@ -657,8 +660,10 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
             const int32_t b = ghosts[next];
             out.gl.push_back((int32_t)(fa.ghost_cell[(size_t)b] - c0) | fa.ghost_group[(size_t)b] << 16);
             out.gl.push_back((int32_t)(N + b));
-            for (double v : {fa.g_nx[(size_t)b], fa.g_ny[(size_t)b], fa.g_dx[(size_t)b], fa.g_dy[(size_t)b]})
-                out.gd.push_back((S)v);
+            const uint32_t e = m.bound_edges[(size_t)(m.new2ref[(size_t)(N + b)] - N)];
+            const size_t c = (size_t)fa.ghost_cell[(size_t)b];
+            for (S v : {(S)fa.g_nx[(size_t)b], (S)fa.g_ny[(size_t)b], diff(m.ecx[e], ta.ccx[c]), diff(m.ecy[e], ta.ccy[c])})
+                out.gd.push_back(v);
         }
         inf[6] |= n << 16;
         out.max_ghost = std::max(out.max_ghost, n);
@@ -678,7 +683,7 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                 const double A = fa.area[(size_t)c], Ka = K * std::sqrt(A), K3a = Ka * Ka * Ka;
                 if (first_order) { /* no limiter */ }
                 else if (exact) { out.sl[(size_t)(so + r) * 2] = (S)(1. / A); out.sl[(size_t)(so + r) * 2 + 1] = (S)K3a; }
-                else out.sl[(size_t)(so + r)] = (S)(1. / K3a);
+                else out.sl[(size_t)(so + r)] = sizeof(S) == 4 ? (S)A : (S)(1. / K3a);
                 if (packed) std::memcpy(&out.hd[(size_t)(so + r) * 4 + 3], &out.sl[(size_t)(so + r)], 4);
                 for (int f = 0; f < F; ++f) {
                     const uint16_t w = t2.face[((size_t)in[6] + r) * 4 + f];
@@ -692,16 +697,16 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                     out.hd[(size_t)(so + r) * 4 + f] = word;
                     if (first_order) continue;
                     const size_t b = (size_t)nf * so + (size_t)f * G + r;
-                    const double dx = t2.exf[e] - ta.ccx[(size_t)c], dy = t2.eyf[e] - ta.ccy[(size_t)c];
+                    const S dx = diff(t2.exf[e], ta.ccx[(size_t)c]), dy = diff(t2.eyf[e], ta.ccy[(size_t)c]);
                     S* v = &out.rec[b * 4];
-                    if (exact) {
+                    if (faces) {
                         v[0] = (S)t2.enx[e]; v[1] = (S)t2.eny[e];
-                        v[2] = (S)(side ? -t2.ele[e] : t2.ele[e]); v[3] = (S)t2.eg[e];
-                        out.rec2[b * 2] = (S)dx; out.rec2[b * 2 + 1] = (S)dy;
+                        v[2] = (S)(side ? -t2.ele[e] : t2.ele[e]); v[3] = (S)(side && !exact ? -t2.eg[e] : t2.eg[e]);
+                        out.rec2[b * 2] = dx; out.rec2[b * 2 + 1] = dy;
                     } else {
                         const double a = (side ? -(1.0 - t2.eg[e]) : t2.eg[e]) * t2.ele[e] / A;
                         v[0] = (S)(a * t2.enx[e]); v[1] = (S)(a * t2.eny[e]);
-                        v[2] = (S)dx; v[3] = (S)dy;
+                        v[2] = dx; v[3] = dy;
                     }
                 }
             }

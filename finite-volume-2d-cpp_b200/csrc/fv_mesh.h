@@ -124,9 +124,11 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
 // face, in the order its threads read them; per flux edge its geometry.  S:
 // the stage precision.  exact: the reference's operands (normal, length with
 // the side in its sign, Green-Gauss weight, face centre - centroid; 1 / A and
-// (K sqrt(A))^3 per slot); otherwise the cell's Green-Gauss coefficients
+// (K sqrt(A))^3 per slot); FP64 the cell's Green-Gauss coefficients
 // a = w le n / A (outward normal, the neighbour's weight) and face centre -
-// centroid, evaluated in FP64 and rounded once, with 1 / (K sqrt(A))^3 per slot.
+// centroid, with 1 / (K sqrt(A))^3 per slot; FP32 the exact operands rounded (the
+// weight with the length's sign, differences of rounded coordinates), with the
+// area per slot.
 // kind: kFusedFirstOrder has no records; it and kFusedViscous hold each flux
 // edge's two slots in the bits of its fourth value; kFusedViscous adds the unit
 // vector between the two centroids with the reciprocal of their distance per

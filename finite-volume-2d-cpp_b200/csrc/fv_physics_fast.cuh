@@ -60,11 +60,24 @@ __device__ __forceinline__ double smooth_switch(double d, double rk3) {
 template <class T>
 __device__ __forceinline__ void speeds(T gamma, const T* q, T* w) {
     const T ri = rcp(q[0]);
-    w[0] = mul_(q[1], ri);
-    w[1] = mul_(q[2], ri);
-    w[2] = sqrt_(gamma * (gamma - T(1)) * fma_(q[3], ri, mul_(T(-0.5), fma_(w[0], w[0], mul_(w[1], w[1])))));
+    if constexpr (sizeof(T) == 4) {
+        const T gm1 = gamma - T(1);
+        w[0] = q[1] * ri;
+        w[1] = q[2] * ri;
+        w[2] = sqrt_(gamma * gm1 * (q[3] * ri - T(0.5) * (w[0] * w[0] + w[1] * w[1])));
+    } else {
+        w[0] = mul_(q[1], ri);
+        w[1] = mul_(q[2], ri);
+        w[2] = sqrt_(gamma * (gamma - T(1)) * fma_(q[3], ri, mul_(T(-0.5), fma_(w[0], w[0], mul_(w[1], w[1])))));
+    }
     w[3] = T(0);
 }
+// a x + b y: FP64 with its roundings written out
+__device__ __forceinline__ float dot2(float a, float x, float b, float y) { return a * x + b * y; }
+__device__ __forceinline__ double dot2(double a, double x, double b, double y) { return fma_(a, x, mul_(b, y)); }
+// c + a b
+__device__ __forceinline__ float madd(float a, float b, float c) { return c + a * b; }
+__device__ __forceinline__ double madd(double a, double b, double c) { return fma_(a, b, c); }
 
 // Roe flux with the "cures" eigenvalues (examples/forwardStep/main.cpp:72-135).
 template <class T>
@@ -105,7 +118,39 @@ __device__ __forceinline__ void roe(T gamma, T* f, const T* qi, const T* qj, T n
                       kF5 * (h + c * V));
 }
 
-// le times the flux of roe(), for the Euler kinds.  The same quantities with
+// le times the flux of roe() in FP32, each rounding written out.
+__device__ __forceinline__ void roe32_le(float gamma, float* f, const float* qi, const float* qj, float n0, float n1,
+                                         float le) {
+    const float gm1 = gamma - 1.f;
+    const float ri = rcp(qi[0]), rj = rcp(qj[0]);
+    const float uL = mul_(qi[1], ri), vL = mul_(qi[2], ri), uR = mul_(qj[1], rj), vR = mul_(qj[2], rj);
+    const float eL = fma_(-0.5f, fma_(qi[1], uL, mul_(qi[2], vL)), qi[3]);
+    const float eR = fma_(-0.5f, fma_(qj[1], uR, mul_(qj[2], vR)), qj[3]);
+    const float pR = mul_(gm1, eR);
+    const float VL = fma_(uL, n0, mul_(vL, n1)), VR = fma_(uR, n0, mul_(vR, n1));
+    const float HL = fma_(gm1, eL, qi[3]), HR = qj[3] + pR, ps = fma_(gm1, eL, pR), dp = fma_(-gm1, eL, pR);
+    const float sL = sqrt_(qi[0]), sR = sqrt_(qj[0]), rho = mul_(sL, sR), w = rcp(sL + sR);
+    const float u = mul_(fma_(uL, sL, mul_(uR, sR)), w), v = mul_(fma_(vL, sL, mul_(vR, sR)), w);
+    const float h = mul_(fma_(mul_(HL, ri), sL, mul_(mul_(HR, rj), sR)), w);
+    const float q2 = fma_(u, u, mul_(v, v));
+    const float c2 = mul_(gm1, fma_(-0.5f, q2, h)), c = sqrt_(c2), rc2 = rcp(c2);
+    const float V = fma_(u, n0, mul_(v, n1)), dV = VR - VL;
+    const float l1 = fabsf(tmin(V - c, VL - c)), l2 = fabsf(V), l5 = fabsf(tmax(V + c, VR + c));
+    const float rc = mul_(rho, c), h2 = mul_(0.5f, rc2);
+    const float k1 = mul_(mul_(l1, fma_(-rc, dV, dp)), h2), k5 = mul_(mul_(l5, fma_(rc, dV, dp)), h2);
+    const float k0 = mul_(l2, fma_(-dp, rc2, qj[0] - qi[0])), kr = mul_(l2, rho);
+    const float du = uR - uL, dv = vR - vL;
+    const float s1 = fma_(k5, fma_(c, n0, u), fma_(kr, fma_(-dV, n0, du), fma_(k0, u, mul_(k1, fma_(-c, n0, u)))));
+    const float s2 = fma_(k5, fma_(c, n1, v), fma_(kr, fma_(-dV, n1, dv), fma_(k0, v, mul_(k1, fma_(-c, n1, v)))));
+    const float s3 = fma_(k5, fma_(c, V, h), fma_(kr, fma_(-V, dV, fma_(u, du, mul_(v, dv))),
+                                                 fma_(k1, fma_(-c, V, h), mul_(mul_(k0, q2), 0.5f))));
+    f[0] = mul_(mul_(0.5f, fma_(qi[0], VL, mul_(qj[0], VR)) - (k1 + k0 + k5)), le);
+    f[1] = mul_(mul_(0.5f, fma_(ps, n0, fma_(qi[1], VL, mul_(qj[1], VR))) - s1), le);
+    f[2] = mul_(mul_(0.5f, fma_(ps, n1, fma_(qi[2], VL, mul_(qj[2], VR))) - s2), le);
+    f[3] = mul_(mul_(0.5f, fma_(HL, VL, mul_(HR, VR)) - s3), le);
+}
+
+// le times the flux of roe(), for the Euler kinds in FP64.  The same quantities with
 // every fused multiply-add written out (one rounding wherever it is inlined,
 // so that the kernels that share it give the same bits), the Roe averages as
 // corrections of the left state, and the dissipation collected by the factors
@@ -156,19 +201,21 @@ __device__ __forceinline__ void burgers(T* f, const T* qi, const T* qj, T n0, T 
 }
 
 // le times the flux (FLUX 3 Burgers, else Roe).  MUSCL: of second-order face
-// states.  First order in FP32 keeps the unit-normal form: its residual norms
-// hold mostly the rounding noise of the flux sums, which roe_le does not lower
-// (70 Sod tubes of 200 to 200,000 cells: mean error of the norms 1.1e-6 against
-// 0.98e-6, of the state 6.8e-8 against 6.5e-8; the second-order kinds' norms
-// 0.45e-6 against 0.86e-6).
+// states.  FP32 keeps the bits of its results, whose flows can amplify another
+// order of operations to more than 2e-5 (small forward steps and strips after
+// some 100 steps: 2e-5 to 1e-1 of the residual norms under roe_le): second order
+// has the same roundings in every kernel (roe32_le), first order those of its
+// one kernel.
 template <int FLUX, bool MUSCL, class T>
 __device__ __forceinline__ void flux_le(T gamma, T* f, const T* qi, const T* qj, T n0, T n1, T le) {
     if (FLUX == 3) {
         burgers(f, qi, qj, n0, n1);
         f[0] *= le;
         f[1] *= le;
-    } else if (MUSCL || sizeof(T) == 8) {
+    } else if constexpr (sizeof(T) == 8) {
         roe_le(gamma, f, qi, qj, n0, n1, le);
+    } else if constexpr (MUSCL) {
+        roe32_le(gamma, f, qi, qj, n0, n1, le);
     } else {
         roe(gamma, f, qi, qj, n0, n1);
 #pragma unroll

@@ -41,7 +41,7 @@ struct fv_solver {
     TileParams TP{};
     // the fused stage kernel over two-ring tiles (its Params are TP.P at launch)
     bool fused = false;
-    // the two-ring tiles exist (the fast modes' split layout runs over them too)
+    // the two-ring tiles exist (FP64's split layout runs over them too)
     bool two_ring = false;
     // with fused: the first stage of each step runs the split kernels, whose
     // gradient kernel also computes dt (no separate dt kernel)

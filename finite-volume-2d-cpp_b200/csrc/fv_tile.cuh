@@ -216,8 +216,13 @@ __device__ __forceinline__ bool face_state_bad(const Params& P, const S* qf) {
         const S p = exact::pres_dev(P.gamma, qf);
         return !(qf[0] > S(0)) || !(p > S(0));
     } else {
-        const S m2 = fast::fma_(qf[2], qf[2], qf[1] * qf[1]);
-        return !(qf[0] > S(0)) || !(fast::fma_(S(2) * qf[0], qf[3], -m2) > S(0));
+        if constexpr (sizeof(S) == 4) {
+            const S m2 = qf[1] * qf[1] + qf[2] * qf[2];
+            return !(qf[0] > S(0)) || !(S(2) * qf[0] * qf[3] - m2 > S(0));
+        } else {
+            const S m2 = fast::fma_(qf[2], qf[2], qf[1] * qf[1]);
+            return !(qf[0] > S(0)) || !(fast::fma_(S(2) * qf[0], qf[3], -m2) > S(0));
+        }
     }
 }
 template <class S, int V, bool EXACT = true>
@@ -522,22 +527,9 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
             io.dt[c] = di;
             kmin = kmin_(kmin, tkey(di));
         } else {
-            const S gamma = (S)P.gamma, gm1 = gamma - S(1), cfl = (S)P.cfl;
-            // {u, v, c}; FP64: the run kernel's arithmetic (fused_cell_dt)
-            constexpr bool F64 = sizeof(S) == 8;
-            auto speeds = [&](const S* q, S* w) {
-                if constexpr (F64) {
-                    fast::speeds(gamma, q, w);
-                } else {
-                    const S r = fast::rcp(q[0]);
-                    w[0] = q[1] * r;
-                    w[1] = q[2] * r;
-                    w[2] = fast::sqrt_(gamma * gm1 * (q[3] * r - S(0.5) * (w[0] * w[0] + w[1] * w[1])));
-                }
-            };
-            auto dot = [](S a, S x, S b, S y) { return F64 ? fast::fma_(a, x, b * y) : a * x + b * y; };
-            S ws[4];
-            speeds(qs, ws);
+            const S gamma = (S)P.gamma, cfl = (S)P.cfl;
+            S ws[4];  // {u, v, c}
+            fast::speeds(gamma, qs, ws);
             const S us = ws[0], vs = ws[1], cs = ws[2];
             const S Ai = AR[c];
             S acc = sum ? S(0) : S(1);
@@ -550,12 +542,12 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
                 const S n0 = snx[el], n1 = sny[el], le = sle[el];
                 S qn[4], wn[4];
                 lds<S, 4>(rec + (size_t)o * NR, qn);
-                speeds(qn, wn);
+                fast::speeds(gamma, qn, wn);
                 const S un = wn[0], vn = wn[1], cn = wn[2];
                 const bool ghost = (w[f] & 0x4000) != 0;
                 if (sum) {
-                    const S center = fast::tmax(cs + fabs(dot(us, n0, vs, n1)), cn + fabs(dot(un, n0, vn, n1)));
-                    acc = F64 ? fast::fma_(center, le, acc) : acc + center * le;
+                    const S center = fast::tmax(cs + fabs(fast::dot2(us, n0, vs, n1)), cn + fabs(fast::dot2(un, n0, vn, n1)));
+                    acc = fast::madd(center, le, acc);
                     if (ghost) {
                         const int g = TP.halo[inf.z + o - T];
                         const double dg = (double)(cfl * AR[g] * fast::rcp(center * le));
@@ -563,11 +555,11 @@ __device__ __forceinline__ unsigned long long tile_cell_dt(const TileParams& TP,
                         kmin = kmin_(kmin, tkey(dg));
                     }
                 } else {
-                    const S es = dot(cs + fabs(us), n0, cs + fabs(vs), n1);
+                    const S es = fast::dot2(cs + fabs(us), n0, cs + fabs(vs), n1);
                     acc = fast::tmin(acc, cfl * Ai * fast::rcp(le * fabs(es)));
                     if (ghost) {
                         const int g = TP.halo[inf.z + o - T];
-                        const S en = dot(cn + fabs(un), n0, cn + fabs(vn), n1);
+                        const S en = fast::dot2(cn + fabs(un), n0, cn + fabs(vn), n1);
                         const double dg = (double)fast::tmin(S(1), cfl * (S)AR[g] * fast::rcp(le * fabs(en)));
                         io.dt[g] = dg;
                         kmin = kmin_(kmin, tkey(dg));
