@@ -169,6 +169,7 @@ int choose_run_kernel(fv_solver* s) {
         int nb = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k[i].fn, k[i].threads, smem));
         if ((int64_t)nb * sms < s->n_tiles) continue;
+        CK(s->alloc(&s->run_part, (size_t)2 * s->n_tiles * 4));
         CK(s->alloc(&s->run_keys, (size_t)3 * s->n_cases * kDtSlots));
         CK(s->alloc(&s->run_bar, 1));
         s->run_kernel = k[i];
@@ -1114,7 +1115,7 @@ static int launch_run(fv_solver* s, const std::vector<double>& alpha, int steps)
     launch_run_begin(s->ctrl, s->run_keys, 3 * s->n_cases * kDtSlots, s->run_bar, s->stream);
     PersistIO D{};
     for (int i = 0; i < 2; ++i) { D.qbase[i] = s->qbase[i]; D.sbase[i] = s->sbase[i]; D.tmp[i] = s->tmp[i]; }
-    D.dt = s->dt; D.partials = s->partials; D.keys = s->run_keys;
+    D.dt = s->dt; D.partials = s->run_part; D.keys = s->run_keys;
     D.ctrl = s->ctrl; D.limits = s->limits; D.hist = s->hist; D.hist_cap = s->hist_cap;
     D.bar = s->run_bar;
     D.n_tiles = s->n_tiles; D.n_cases = s->n_cases; D.f32 = s->f32 ? 1 : 0;
@@ -1124,7 +1125,6 @@ static int launch_run(fv_solver* s, const std::vector<double>& alpha, int steps)
     if (s->stencil) {
         StencilParams F = s->SP;
         F.P = s->TP.P;
-        D.partials = s->run_part;
         void* sargs[] = {&F, &D};
         const int per = s->run_kernel.threads / F.T;
         CK(cudaLaunchCooperativeKernel(s->run_kernel.fn, dim3((unsigned)((s->n_tiles + per - 1) / per)),

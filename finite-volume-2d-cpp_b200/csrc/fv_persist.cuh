@@ -29,7 +29,10 @@ struct PersistIO {
     void* sbase[2];
     void* tmp[2];
     double* dt;
-    double* partials;              // [n_tiles][4]
+    // residual partial sums, by the step modulo 2: with one stage a CTA may
+    // store its next ones while another still reads these (between the two lies
+    // only the time step's barrier, which a CTA joins before it reads)
+    double* partials;              // [2][n_tiles][4] (stencils: [2][CTAs])
     unsigned long long* keys;      // [3][n_cases][kDtSlots], by the step modulo 3
     Ctrl* ctrl;
     const RunLimits* limits;
@@ -277,10 +280,12 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
     io.dt = D.dt;
     io.ctrl = D.ctrl;
     bool pending = false;  // a step has ended whose norms and time are not evaluated yet
+    const double* part = nullptr;  // its partial sums
     int n = 0;
     for (bool go = c.active != 0; go && n < D.max_steps; ++n) {
         unsigned long long* keys = D.keys + (size_t)(n % 3) * nkeys;
         const int b = D.ns == 1 ? (n & 1) : 0;  // a single stage alternates the base buffers
+        double* part_out = D.partials + (size_t)(n & 1) * D.n_tiles * V;
         io.dtkeys = keys;
         io.q_base = D.qbase[b];
         const void* in = D.sbase[b];
@@ -300,7 +305,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
             }
             io.s_out = D.f32 ? out_s : nullptr;
             io.write_f64 = last ? 1 : 0;
-            io.partials = last ? D.partials : nullptr;
+            io.partials = last ? part_out : nullptr;
             io.q_stage = in;
             io.alpha = D.alpha[k];
             // ---- the stage's input is complete
@@ -340,7 +345,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
                 // the next step's keys: its set was last read two steps ago
                 if (blockIdx.x == 0)
                     for (int i = l; i < nkeys; i += blockDim.x) D.keys[(size_t)((n + 1) % 3) * nkeys + i] = ~0ull;
-                if (pending && warp == nw - 1) run_step_end(D, c, lim, s_time, D.partials, D.n_tiles);
+                if (pending && warp == nw - 1) run_step_end(D, c, lim, s_time, part, D.n_tiles);
             }
             // ---- face states
             if constexpr (O2) {
@@ -431,11 +436,11 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
             sync.arrive();
             in = out_s;
         }
-        if (go) pending = true;
+        if (go) { pending = true; part = part_out; }
     }
     if (pending) {  // the launch's last step
         if (!sync.wait()) return;
-        if (warp == nw - 1) run_step_end(D, c, lim, s_time, D.partials, D.n_tiles);
+        if (warp == nw - 1) run_step_end(D, c, lim, s_time, part, D.n_tiles);
         __syncthreads();
     }
     if (blockIdx.x == 0 && l == 0) {

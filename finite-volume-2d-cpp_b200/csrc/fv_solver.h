@@ -52,7 +52,7 @@ struct fv_solver {
     RunKernel run_kernel{};
     bool stencil = false;           // diffusion kind: stages run over stencils
     StencilParams SP{};
-    double* run_part = nullptr;     // the stencil run kernel's partial sums [2][n_tiles]
+    double* run_part = nullptr;     // the run kernel's partial sums: [2][n_tiles][4], stencils [2][CTAs]
     unsigned long long* run_keys = nullptr;
     unsigned* run_bar = nullptr;
     // its schedule (FV_SCHED_*); the work list's per-stage tile counters and
