@@ -147,8 +147,9 @@ int choose_run_kernel(fv_solver* s) {
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
     if (!coop) return FV_OK;
-    const size_t smem = tile::smem_fused(s->precision, s->FPm);
-    if (smem > (size_t)227 * 1024) return FV_OK;
+    tile::smem_fused(s->precision, s->FPm);  // the layout, with the tiles' ghosts
+    const size_t smem = (size_t)std::max(s->FPm.L.total_run, s->FPm.L.total_grad);
+    if (smem > kSmemMost) return FV_OK;
     FusedParams F = s->FPm;
     F.P = s->TP.P;
     RunKernel k[kRunKernels];
@@ -561,7 +562,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
             F.T = tile_cells;
             F.max_slots = t2.max_slots; F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;
             const bool fits = t2.max_slots < 65535 && t2.max_edges <= kFaceEdgeMask &&
-                              2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= (size_t)227 * 1024;
+                              2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= kSmemMost;
             if (!fits && (sk == FV_STAGE_FUSED || sk == FV_STAGE_HYBRID))
                 return fail(FV_ERR_MESH, "two-ring tiles too large for the fused stage kernel at this tile size");
             if (fits) {
@@ -669,7 +670,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
         F.P.flux = ph->flux;  // (the shared-memory layout depends on it)
         F.max_slots = ns ? t2.max_slots : t2.max_grad;  // first order stages one ring
         F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;
-        if (t2.max_slots < 65535 && 2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= (size_t)227 * 1024) {
+        if (t2.max_slots < 65535 && 2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= kSmemMost) {
             rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, kind, ph->K);
             if (rc) return rc;
             const int32_t* h2;

@@ -89,6 +89,10 @@ inline FusedSmem fused_smem(int max_slots, int max_grad, int max_flux, int max_g
     return L;
 }
 
+// Dynamic shared memory of a CTA at most: 227 KB with the kernels' static
+// variables (under 1 KB).
+constexpr size_t kSmemMost = 226 * 1024;
+
 struct FusedParams {
     Params P;
     int T;
@@ -1179,9 +1183,10 @@ __global__ void __launch_bounds__(kTileMax) k_tile_fused_work(FusedParams FP, Ti
 template <class M>
 struct FusedLaunch {
     // lays out the tiles' shared memory (FP.L); the bytes of the largest launch
+    // but the run kernel's
     static size_t smem(FusedParams& FP) {
         FP.L = fused_smem<M>(FP.max_slots, FP.max_grad, FP.max_flux, FP.max_ghost, FP.T, FP.P.flux == 5);
-        return (size_t)std::max(FP.L.total_run, FP.L.total_grad);
+        return (size_t)std::max(FP.L.total, FP.L.total_grad);
     }
     static cudaError_t prepare(FusedParams& FP) {
         static std::mutex mu;
