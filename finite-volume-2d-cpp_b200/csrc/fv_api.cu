@@ -75,21 +75,56 @@ int upload_v(fv_solver* s, const std::vector<T>& v, const T** out) {
     *out = d;
     return FV_OK;
 }
+// What the fused, run and stencil kernels hold, built on another thread beside
+// the one-ring tiles and their transfer.
+template <class S>
+struct Layouts {
+    Tile2Arrays t2;
+    FusedArrays<S> fused;
+    bool tiles_ok = false;    // within the kernels' index fields
+    StencilArrays<S> stencil;
+    bool stencil_ok = false;
+    void build_two_ring(const HostMesh& m, const FaceArrays& fa, int tile_cells, bool exact, FusedKind kind, double K) {
+        build_tiles2(m, fa, tile_cells, t2);
+        tiles_ok = t2.max_slots < 65535 && t2.max_edges <= kFaceEdgeMask && 2 * t2.max_flux <= kMaxFluxUnits;
+        if (tiles_ok) build_fused<S>(m, fa, t2, exact, kind, K, fused);
+    }
+    // sizes for the kernels' shared-memory layout
+    void sizes(FusedParams& F, FusedKind kind) const {
+        F.T = t2.tile_cells;
+        F.max_slots = kind == kFusedFirstOrder ? t2.max_grad : t2.max_slots;  // first order stages one ring
+        F.max_grad = t2.max_grad;
+        F.max_flux = t2.max_flux;
+        F.nf = fused.nf;
+        F.max_ghost = fused.max_ghost;
+    }
+};
 // the fused kernel's arrays over two-ring tiles (build_fused)
 template <class S>
-int upload_fused(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2,
-                 bool exact, FusedKind kind, double K) {
-    FusedArrays<S> a;
-    build_fused<S>(m, fa, ta, t2, exact, kind, K, a);
+int upload_fused(fv_solver* s, const Layouts<S>& l) {
+    const FusedArrays<S>& a = l.fused;
     FusedParams& F = s->FPm;
-    F.nf = a.nf;
-    F.max_ghost = a.max_ghost;
+    // all in one allocation
+    size_t bytes = 0;
+    unsigned char* base = nullptr;
+    int rc = FV_OK;
+    auto place = [&](const auto& v, const auto** out) {
+        const size_t n = v.size() * sizeof(v[0]);
+        if (base && !rc && n) rc = cudaMemcpy(base + bytes, v.data(), n, cudaMemcpyHostToDevice) == cudaSuccess ? FV_OK : FV_ERR_CUDA;
+        *out = reinterpret_cast<std::remove_reference_t<decltype(*out)>>(base + bytes);
+        bytes += (n + 255) / 256 * 256;
+    };
     const int32_t* info; const uint32_t* hd; const int32_t* gl; const S *rec, *rec2, *sl, *eg, *gd, *e2, *ar;
-    int rc;
-    if ((rc = upload_v(s, a.info, &info)) || (rc = upload_v(s, a.hd, &hd)) || (rc = upload_v(s, a.rec, &rec)) || (rc = upload_v(s, a.rec2, &rec2)) || (rc = upload_v(s, a.sl, &sl)) ||
-        (rc = upload_v(s, a.eg, &eg)) || (rc = upload_v(s, a.gl, &gl)) || (rc = upload_v(s, a.gd, &gd)) ||
-        (rc = upload_v(s, a.e2, &e2)) || (rc = upload_v(s, a.ar, &ar)) || (rc = upload_v(s, a.ria, &F.ria)))
-        return rc;
+    auto all = [&] {
+        place(a.info, &info); place(a.hd, &hd); place(a.rec, &rec); place(a.rec2, &rec2); place(a.sl, &sl); place(a.eg, &eg);
+        place(a.gl, &gl); place(a.gd, &gd); place(a.e2, &e2); place(a.ar, &ar); place(a.ria, &F.ria); place(l.t2.halo, &F.halo);
+    };
+    all();
+    CK(s->alloc(&base, bytes));
+    bytes = 0;
+    all();
+    if (rc) return fail(FV_ERR_CUDA, "copying the fused kernel's arrays");
+    F.area = s->TP.area;
     F.info = reinterpret_cast<const int4*>(info);
     F.hd = reinterpret_cast<const uint4*>(hd);
     F.rec = rec; F.rec2 = rec2; F.sl = sl; F.eg = eg; F.gd = gd; F.e2 = e2; F.ar = ar;
@@ -106,11 +141,11 @@ int fused_lanes(const fv_solver* s, int sms) {
 }
 // The diffusion kind's stencils
 template <class S>
-int upload_stencil(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const TileArrays& ta) {
-    StencilArrays<S> a;
-    if (!build_stencil<S>(m, fa, ta, a) || (size_t)a.max_slots * sizeof(S) > (size_t)40 * 1024) return FV_OK;
+int upload_stencil(fv_solver* s, const FaceArrays& fa, int tile_cells, const Layouts<S>& l) {
+    const StencilArrays<S>& a = l.stencil;
+    if (!l.stencil_ok || (size_t)a.max_slots * sizeof(S) > (size_t)40 * 1024) return FV_OK;
     StencilParams& F = s->SP;
-    F.T = ta.tile_cells;
+    F.T = tile_cells;
     F.nf = a.nf;
     F.max_slots = a.max_slots;
     const int32_t* info;
@@ -139,6 +174,23 @@ int upload_stencil(fv_solver* s, const HostMesh& m, const FaceArrays& fa, const 
     CK(s->alloc(&s->run_bar, 1));
     s->run_kernel = RunKernel{fn, per * F.T};
     return FV_OK;
+}
+// Most tiles of T cells that a run kernel's registers let the device hold.
+int64_t run_room(int precision, const fv_physics* ph, const HostMesh& m, int T, int sms) {
+    FusedParams F{};
+    F.T = T;
+    F.P.flux = ph->flux;
+    F.P.order2 = ph->order2 ? 1 : 0;
+    F.nf = 3;
+    for (int64_t c = 0; c < m.n_real && F.nf < HostMesh::MAXF; ++c) F.nf = std::max<int>(F.nf, m.n_faces[(size_t)c]);
+    RunKernel k[kRunKernels];
+    tile::run_kernels(precision, F, k);
+    int most = 0;
+    for (const RunKernel& r : k) {
+        int nb = 0;
+        if (r.fn && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, r.fn, r.threads, 0) == cudaSuccess) most = std::max(most, nb);
+    }
+    return (int64_t)most * sms;
 }
 // The persistent run kernel, where all tiles fit the device at once: the first
 // candidate (fv_persist.cuh) with room for them.
@@ -478,8 +530,7 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     const bool two_ring = can_fuse && (sk != FV_STAGE_SPLIT || precision == FV_PREC_FP64);
     // the persistent run kernel (choose_run_kernel): the Roe kinds in their
     // default layout and schedule with a CFL or constant time step, not on a
-    // part of a decomposition.  Its tiles have to fit the device at once: at
-    // most 8 per SM do.
+    // part of a decomposition, where its tiles fit the device at once.
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const bool roe = ph->V == 4 && (ph->flux == FV_FLUX_ROE_FS || ph->flux == FV_FLUX_ROE_ST);
@@ -492,11 +543,30 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     const bool can_run = (ns || (roe && ph->dt_kind < FV_DT_VISC_MIN && (ph->order2 || precision != FV_PREC_FP32))) && sk != FV_STAGE_SPLIT &&
                          !(sk == FV_STAGE_HYBRID && precision == FV_PREC_FP64_EXACT) &&
                          (!opt || opt->schedule == FV_SCHED_TILE) && m.owned_real() == m.n_real && m.n_real > 0 &&
-                         m.n_real <= (int64_t)8 * sms * tile_cells;
+                         (m.n_real + tile_cells - 1) / tile_cells <= run_room(precision, ph, m, tile_cells, sms);
     const bool run_own_tiles = can_run && (ns || !ph->order2);  // (the second-order Roe kinds share the fused kernel's)
-    Tile2Arrays t2;
-    std::future<void> t2_built;
-    if (two_ring || run_own_tiles) t2_built = std::async(std::launch::async, [&] { build_tiles2(m, fa, tile_cells, t2); });
+    // The diffusion kind of the fast modes in its default layout: one linear
+    // stencil per cell and stage (fv_stencil.h), 2.0 to 3.7 times faster than
+    // gradient and flux kernels at every size from 512 to 720,000 cells.
+    // FP64_EXACT keeps the reference's order of operations.
+    const bool stencil = ph->flux == FV_FLUX_DIFFUSION && precision != FV_PREC_FP64_EXACT && sk == FV_STAGE_AUTO &&
+                         (!opt || opt->schedule == FV_SCHED_TILE) && m.owned_real() == m.n_real && m.n_real > 0;
+    const FusedKind kind = ns ? kFusedViscous : ph->order2 ? kFusedEuler : kFusedFirstOrder;
+    Layouts<float> l32;
+    Layouts<double> l64;
+    std::future<void> built;
+    auto build = [&](auto& l) {
+        if (stencil) built = run_async([&] { l.stencil_ok = build_stencil(m, fa, tile_cells, l.stencil); });
+        else if (two_ring || run_own_tiles)
+            built = run_async([&] { l.build_two_ring(m, fa, tile_cells, precision == FV_PREC_FP64_EXACT, kind, ph->K); });
+    };
+    if (s->f32) build(l32);
+    else build(l64);
+    const bool& tiles_ok = s->f32 ? l32.tiles_ok : l64.tiles_ok;
+    auto sizes = [&](FusedParams& F) {
+        if (s->f32) l32.sizes(F, kind);
+        else l64.sizes(F, kind);
+    };
     build_tiles(m, fa, tile_cells, ta);
     if (ta.max_halo + tile_cells > 65535 || ta.max_edges > kFaceEdgeMask)
         return fail(FV_ERR_MESH, "tile halo too large for 16-bit local indices");
@@ -542,8 +612,8 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     if ((rc = upload_s(s.get(), ta.eyf, &TP.eyf))) return rc;
     if ((rc = upload_s(s.get(), ta.eg, &TP.eg))) return rc;
     {
-        std::vector<double> cxy(2 * ta.ccx.size());
-        for (size_t i = 0; i < ta.ccx.size(); ++i) { cxy[2 * i] = ta.ccx[i]; cxy[2 * i + 1] = ta.ccy[i]; }
+        std::vector<double> cxy(2 * fa.ccx.size());
+        for (size_t i = 0; i < fa.ccx.size(); ++i) { cxy[2 * i] = fa.ccx[i]; cxy[2 * i + 1] = fa.ccy[i]; }
         if ((rc = upload_s(s.get(), cxy, &TP.ccxy))) return rc;
     }
     if ((rc = upload_s(s.get(), fa.area, &TP.area))) return rc;
@@ -557,22 +627,14 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
             return fail(FV_ERR_UNSUPPORTED, "the fused stage kernel needs a second-order Roe kind without "
                                             "diffusive terms or residual smoothing");
         if (two_ring) {
-            t2_built.get();
+            built.get();
             FusedParams& F = s->FPm;
-            F.T = tile_cells;
-            F.max_slots = t2.max_slots; F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;
-            const bool fits = t2.max_slots < 65535 && t2.max_edges <= kFaceEdgeMask &&
-                              2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= kSmemMost;
+            sizes(F);
+            const bool fits = tiles_ok && tile::smem_fused(precision, F) <= kSmemMost;
             if (!fits && (sk == FV_STAGE_FUSED || sk == FV_STAGE_HYBRID))
                 return fail(FV_ERR_MESH, "two-ring tiles too large for the fused stage kernel at this tile size");
             if (fits) {
-                if (s->f32) rc = upload_fused<float>(s.get(), m, fa, ta, t2, false, kFusedEuler, ph->K);
-                else rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, kFusedEuler, ph->K);
-                if (rc) return rc;
-                const int32_t* h2;
-                if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;
-                F.halo = h2;
-                F.area = TP.area;
+                if ((rc = s->f32 ? upload_fused(s.get(), l32) : upload_fused(s.get(), l64))) return rc;
                 s->two_ring = true;
                 CK(tile::prepare_fused(precision, F));
                 s->fused = sk != FV_STAGE_SPLIT;
@@ -663,32 +725,18 @@ int fv_solver_create_ex(const fv_mesh* fm, const fv_physics* ph, int32_t precisi
     }
     launch_fill_ghost_grad(s->gx, s->gy, s->lim, (int)m.n_real, (int)m.n_total, ph->V, s->f32, s->stream);
     if (run_own_tiles) {
-        t2_built.get();
+        built.get();
         FusedParams& F = s->FPm;
-        F.T = tile_cells;
-        const FusedKind kind = ns ? kFusedViscous : kFusedFirstOrder;
         F.P.flux = ph->flux;  // (the shared-memory layout depends on it)
-        F.max_slots = ns ? t2.max_slots : t2.max_grad;  // first order stages one ring
-        F.max_grad = t2.max_grad; F.max_flux = t2.max_flux;
-        if (t2.max_slots < 65535 && 2 * t2.max_flux <= kMaxFluxUnits && tile::smem_fused(precision, F) <= kSmemMost) {
-            rc = upload_fused<double>(s.get(), m, fa, ta, t2, precision == FV_PREC_FP64_EXACT, kind, ph->K);
-            if (rc) return rc;
-            const int32_t* h2;
-            if ((rc = upload_v(s.get(), t2.halo, &h2))) return rc;
-            F.halo = h2;
-            F.area = TP.area;
-            if ((rc = choose_run_kernel(s.get()))) return rc;
-        }
+        sizes(F);
+        if (tiles_ok && (rc = choose_run_kernel(s.get()))) return rc;
+        if (s->run_kernel.fn && (rc = upload_fused(s.get(), l64))) return rc;
     } else if (can_run && s->fused) {
         if ((rc = choose_run_kernel(s.get()))) return rc;
     }
-    // The diffusion kind of the fast modes in its default layout: one linear
-    // stencil per cell and stage (fv_stencil.h), 2.0 to 3.7 times faster than
-    // gradient and flux kernels at every size from 512 to 720,000 cells.
-    // FP64_EXACT keeps the reference's order of operations.
-    if (ph->flux == FV_FLUX_DIFFUSION && precision != FV_PREC_FP64_EXACT && sk == FV_STAGE_AUTO &&
-        (!opt || opt->schedule == FV_SCHED_TILE) && m.owned_real() == m.n_real && m.n_real > 0) {
-        rc = s->f32 ? upload_stencil<float>(s.get(), m, fa, ta) : upload_stencil<double>(s.get(), m, fa, ta);
+    if (stencil) {
+        built.get();
+        rc = s->f32 ? upload_stencil(s.get(), fa, tile_cells, l32) : upload_stencil(s.get(), fa, tile_cells, l64);
         if (rc) return rc;
     }
     CK(cudaGetLastError());

@@ -378,8 +378,11 @@ void build_face_arrays(const HostMesh& m, FaceArrays& fa) {
         fa.g_dx[b] = m.ecx[e] - m.ccx[ci];
         fa.g_dy[b] = m.ecy[e] - m.ccy[ci];
     }
-    fa.area.assign(NT, 0.);
-    for (int64_t n = 0; n < NT; ++n) fa.area[n] = m.area[m.new2ref[n]];
+    for (auto* v : {&fa.area, &fa.ccx, &fa.ccy}) v->resize(NT);
+    for (int64_t n = 0; n < NT; ++n) {
+        const int32_t r = m.new2ref[n];
+        fa.area[n] = m.area[r]; fa.ccx[n] = m.ccx[r]; fa.ccy[n] = m.ccy[r];
+    }
     fa.cell0 = m.ref2new[0];
 }
 
@@ -437,8 +440,6 @@ void build_tiles(const HostMesh& m, const FaceArrays& fa, int T, TileArrays& ta)
         ta.max_edges = std::max(ta.max_edges, n_edges);
         for (int32_t d : touched) local[d] = -1;
     }
-    ta.ccx.assign(NT, 0.); ta.ccy.assign(NT, 0.);
-    for (int64_t n = 0; n < NT; ++n) { ta.ccx[n] = m.ccx[m.new2ref[n]]; ta.ccy[n] = m.ccy[m.new2ref[n]]; }
 }
 
 void build_tiles2(const HostMesh& m, const FaceArrays& fa, int T, Tile2Arrays& ta) {
@@ -515,10 +516,22 @@ void build_tiles2(const HostMesh& m, const FaceArrays& fa, int T, Tile2Arrays& t
     }
 }
 
+// f(first, last) over the tiles [0, n) on up to 8 threads, of at least 16 tiles
+// each; what a thread throws (or failing to start one) reaches the caller.
+template <class F>
+static void in_parallel(int n, F f) {
+    const int th = (int)std::min<int64_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency())), 1 + n / 16);
+    std::vector<std::future<void>> parts;
+    for (int k = 1; k < th; ++k)
+        parts.push_back(run_async([=] { f((int)((int64_t)n * k / th), (int)((int64_t)n * (k + 1) / th)); }));
+    f(0, n / th);
+    for (auto& p : parts) p.get();
+}
+
 template <class S>
-bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, StencilArrays<S>& out) {
-    const int T = ta.tile_cells, nt = ta.n_tiles;
+bool build_stencil(const HostMesh& m, const FaceArrays& fa, int T, StencilArrays<S>& out) {
     const int64_t N = m.n_real;
+    const int nt = (int)((N + T - 1) / T);
     out = StencilArrays<S>();
     for (int64_t c = 0; c < N && out.nf < HostMesh::MAXF; ++c) out.nf = std::max<int>(out.nf, m.n_faces[c]);
     const int nf = out.nf;
@@ -560,7 +573,7 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
                     fc[f] = face(c, f);
                     const int64_t n = nbr(c, f);
                     sl[f] = (uint16_t)(slot_of(n) | (n >= N ? 0x8000 : 0));
-                    double tx = rd(ta.ccx[(size_t)c]) - rd(ta.ccx[(size_t)n]), ty = rd(ta.ccy[(size_t)c]) - rd(ta.ccy[(size_t)n]);
+                    double tx = rd(fa.ccx[(size_t)c]) - rd(fa.ccx[(size_t)n]), ty = rd(fa.ccy[(size_t)c]) - rd(fa.ccy[(size_t)n]);
                     const double d = std::sqrt(tx * tx + ty * ty);
                     tx /= d; ty /= d;
                     const double tn = tx * fc[f].nx + ty * fc[f].ny;
@@ -589,11 +602,7 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
             if (T + halo.size() > 0x7FFF) ok = false;
         }
     };
-    const int th = (int)std::min<int64_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency())), 1 + nt / 256);
-    std::vector<std::thread> pool;
-    for (int k = 1; k < th; ++k) pool.emplace_back(tiles, (int)((int64_t)nt * k / th), (int)((int64_t)nt * (k + 1) / th));
-    tiles(0, nt / th);
-    for (auto& x : pool) x.join();
+    in_parallel(nt, tiles);
     out.max_slots = T;
     for (int t = 0; t < nt; ++t) {
         int32_t* inf = &out.info[(size_t)4 * t];
@@ -605,11 +614,11 @@ bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta
     }
     return ok;
 }
-template bool build_stencil<float>(const HostMesh&, const FaceArrays&, const TileArrays&, StencilArrays<float>&);
-template bool build_stencil<double>(const HostMesh&, const FaceArrays&, const TileArrays&, StencilArrays<double>&);
+template bool build_stencil<float>(const HostMesh&, const FaceArrays&, int, StencilArrays<float>&);
+template bool build_stencil<double>(const HostMesh&, const FaceArrays&, int, StencilArrays<double>&);
 
 template <class S>
-void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
+void build_fused(const HostMesh& m, const FaceArrays& fa, const Tile2Arrays& t2, bool exact,
                  FusedKind kind, double K, FusedArrays<S>& out) {
     const bool first_order = kind == kFusedFirstOrder, viscous = kind == kFusedViscous;
     const int T = t2.tile_cells, F = HostMesh::MAXF;
@@ -662,7 +671,7 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
             out.gl.push_back((int32_t)(N + b));
             const uint32_t e = m.bound_edges[(size_t)(m.new2ref[(size_t)(N + b)] - N)];
             const size_t c = (size_t)fa.ghost_cell[(size_t)b];
-            for (S v : {(S)fa.g_nx[(size_t)b], (S)fa.g_ny[(size_t)b], diff(m.ecx[e], ta.ccx[c]), diff(m.ecy[e], ta.ccy[c])})
+            for (S v : {(S)fa.g_nx[(size_t)b], (S)fa.g_ny[(size_t)b], diff(m.ecx[e], fa.ccx[c]), diff(m.ecy[e], fa.ccy[c])})
                 out.gd.push_back(v);
         }
         inf[6] |= n << 16;
@@ -697,7 +706,7 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                     out.hd[(size_t)(so + r) * 4 + f] = word;
                     if (first_order) continue;
                     const size_t b = (size_t)nf * so + (size_t)f * G + r;
-                    const S dx = diff(t2.exf[e], ta.ccx[(size_t)c]), dy = diff(t2.eyf[e], ta.ccy[(size_t)c]);
+                    const S dx = diff(t2.exf[e], fa.ccx[(size_t)c]), dy = diff(t2.eyf[e], fa.ccy[(size_t)c]);
                     S* v = &out.rec[b * 4];
                     if (faces) {
                         v[0] = (S)t2.enx[e]; v[1] = (S)t2.eny[e];
@@ -716,7 +725,7 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                 v[0] = (S)t2.enx[g]; v[1] = (S)t2.eny[g]; v[2] = (S)t2.ele[g];
                 if (viscous) {
                     const int32_t ci = dev((int)(t2.edge_ij[g] & 0xFFFF)), cj = dev((int)(t2.edge_ij[g] >> 16));
-                    const double tx = ta.ccx[(size_t)ci] - ta.ccx[(size_t)cj], ty = ta.ccy[(size_t)ci] - ta.ccy[(size_t)cj];
+                    const double tx = fa.ccx[(size_t)ci] - fa.ccx[(size_t)cj], ty = fa.ccy[(size_t)ci] - fa.ccy[(size_t)cj];
                     const double len = std::sqrt(tx * tx + ty * ty);
                     S* u = &out.e2[(size_t)(inf[2] + e) * 4];
                     u[0] = (S)(tx / len); u[1] = (S)(ty / len); u[2] = (S)(1. / len);
@@ -729,21 +738,15 @@ void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, 
                 // a boundary ghost's zero gradient adds this signed zero to its face state
                 const int32_t j = dev((int)(t2.edge_ij[g] >> 16));
                 if (j >= N)
-                    v[3] = (S)((0.0 * (t2.exf[g] - ta.ccx[(size_t)j]) + 0.0 * (t2.eyf[g] - ta.ccy[(size_t)j])) * 1.0);
+                    v[3] = (S)((0.0 * (t2.exf[g] - fa.ccx[(size_t)j]) + 0.0 * (t2.eyf[g] - fa.ccy[(size_t)j])) * 1.0);
             }
         }
     };
-    const int nt = (int)std::min<int64_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency())),
-                                          1 + t2.n_tiles / 256);
-    std::vector<std::thread> pool;
-    for (int k = 1; k < nt; ++k)
-        pool.emplace_back(tiles, (int)((int64_t)t2.n_tiles * k / nt), (int)((int64_t)t2.n_tiles * (k + 1) / nt));
-    tiles(0, t2.n_tiles / nt);
-    for (auto& th : pool) th.join();
+    in_parallel(t2.n_tiles, tiles);
 }
-template void build_fused<float>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, FusedKind,
+template void build_fused<float>(const HostMesh&, const FaceArrays&, const Tile2Arrays&, bool, FusedKind,
                                  double, FusedArrays<float>&);
-template void build_fused<double>(const HostMesh&, const FaceArrays&, const TileArrays&, const Tile2Arrays&, bool, FusedKind,
+template void build_fused<double>(const HostMesh&, const FaceArrays&, const Tile2Arrays&, bool, FusedKind,
                                   double, FusedArrays<double>&);
 
 // ----------------------------------------------------------------------------

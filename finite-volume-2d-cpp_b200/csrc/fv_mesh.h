@@ -4,7 +4,9 @@
 // lists the kernels gather through.
 #pragma once
 #include <cstdint>
+#include <future>
 #include <string>
+#include <system_error>
 #include <vector>
 
 namespace fvgpu {
@@ -48,6 +50,16 @@ struct HostMesh {
     int64_t owned_real() const { return n_own >= 0 ? n_own : n_real; }
 };
 
+// f on another thread, or in the caller's get() where none can be started.
+template <class F>
+std::future<void> run_async(F f) {
+    try {
+        return std::async(std::launch::async, f);
+    } catch (const std::system_error&) {
+        return std::async(std::launch::deferred, f);
+    }
+}
+
 // Per-face arrays of the device kernels, slot-major [MAXF][n_real] in device
 // numbering, plus ghost metadata in device ghost order.
 struct FaceArrays {
@@ -58,7 +70,7 @@ struct FaceArrays {
     std::vector<int32_t> ghost_group, ghost_cell;
     std::vector<uint8_t> ghost_slot;
     std::vector<double> g_nx, g_ny, g_le, g_dx, g_dy;   // per ghost: face normal, length, x_f - x_interior
-    std::vector<double> area;             // [n_total] device numbering
+    std::vector<double> area, ccx, ccy;   // [n_total] device numbering
     int32_t cell0 = 0;                    // device index of reference cell 0
 };
 void build_face_arrays(const HostMesh& m, FaceArrays& fa);
@@ -77,7 +89,6 @@ struct TileArrays {
     std::vector<int32_t> edge_ref;    // reference edge index of each tile edge
     std::vector<double> enx, eny, ele, exf, eyf, eg;  // per tile edge
     std::vector<uint16_t> face;       // [MAXF][n_real]: local edge | side << 15, 0xFFFF = none
-    std::vector<double> ccx, ccy;     // [n_total] device numbering
 };
 void build_tiles(const HostMesh& m, const FaceArrays& fa, int tile_cells, TileArrays& ta);
 
@@ -117,7 +128,7 @@ struct StencilArrays {
     std::vector<uint16_t> slot;
 };
 template <class S>
-bool build_stencil(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, StencilArrays<S>& out);
+bool build_stencil(const HostMesh& m, const FaceArrays& fa, int tile_cells, StencilArrays<S>& out);
 
 // The fused stage kernel's view of two-ring tiles (fv_fused.cuh): per gradient
 // slot (T + n1 of each tile) face words and one record per
@@ -151,7 +162,7 @@ struct FusedArrays {
     std::vector<double> ria;             // [owned cells] 1 / area as the stage precision holds it
 };
 template <class S>
-void build_fused(const HostMesh& m, const FaceArrays& fa, const TileArrays& ta, const Tile2Arrays& t2, bool exact,
+void build_fused(const HostMesh& m, const FaceArrays& fa, const Tile2Arrays& t2, bool exact,
                  FusedKind kind, double K, FusedArrays<S>& out);
 
 // One part of a decomposition of a single mesh into n_parts parts.  Part p

@@ -54,3 +54,34 @@ def test_run_kernel_or_separate_kernels(shapes, run_kernel):
         assert np.all(np.abs(a - b).max(0) <= 1e-12 * np.abs(b).max(0))
     else:
         assert bits_equal(out[0][0], out[1][0])
+
+
+def test_no_arrays_for_a_run_kernel_that_has_no_room():
+    """120,000 Navier-Stokes cells in FP64, beyond the run kernel: the default
+    layout holds what the split layout holds (the run kernel's records would be
+    some 60 MB)."""
+    import torch
+
+    n, m = 400, 300
+    J, I = np.meshgrid(np.arange(m + 1), np.arange(n + 1), indexing="ij")
+    a = (np.arange(m)[:, None] * (n + 1) + np.arange(n)[None]).ravel()
+    e, f = np.arange(n), np.arange(m) * (n + 1)
+    seg = np.concatenate([np.stack(s, 1) for s in ((e, e + 1), (e + m * (n + 1), e + m * (n + 1) + 1), (f, f + n + 1),
+                                                  (f + n, f + 2 * n + 1))]).astype(np.int32)
+    em = meshgen.ElementMesh(I.ravel() / n, J.ravel() / m, np.stack([a, a + 1, a + n + 2, a + n + 1], 1).astype(np.int32),
+                             seg, np.zeros(len(seg), np.int32), ["wall"])
+    mesh = fvgpu.Mesh.from_elements(em)
+    ph = euler(True)
+    ph.flux, ph.diffusive = "ns", True
+    ph.dt_kind, ph.mu, ph.pr, ph.cp, ph.r = "visc_sum", 2e-3, 0.72, 3.5, 1.0
+
+    def held(layout):
+        before = torch.cuda.mem_get_info()[0]
+        s = fvgpu.Solver(mesh, ph, "fp64", stage_kernels=layout)
+        used = before - torch.cuda.mem_get_info()[0]
+        s.close()
+        return used
+
+    held("split")  # (kernels loaded)
+    held("auto")
+    assert abs(held("auto") - held("split")) <= 4 << 20
