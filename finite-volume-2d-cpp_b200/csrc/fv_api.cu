@@ -1158,9 +1158,10 @@ static int settle_base(fv_solver* s, unsigned long long steps_taken) {
     return FV_OK;
 }
 
-// At most `steps` steps in one launch of the persistent run kernel.
+// At most `steps` steps in one launch of the persistent run kernel; an error
+// where the launch is refused (nothing that a captured step relies on has run).
 constexpr int kRunSteps = 2048;  // bounds the duration of a launch
-static int launch_run(fv_solver* s, const std::vector<double>& alpha, int steps) {
+static cudaError_t launch_run(fv_solver* s, const std::vector<double>& alpha, int steps) {
     launch_run_begin(s->ctrl, s->run_keys, 3 * s->n_cases * kDtSlots, s->run_bar, s->stream);
     PersistIO D{};
     for (int i = 0; i < 2; ++i) { D.qbase[i] = s->qbase[i]; D.sbase[i] = s->sbase[i]; D.tmp[i] = s->tmp[i]; }
@@ -1176,17 +1177,15 @@ static int launch_run(fv_solver* s, const std::vector<double>& alpha, int steps)
         F.P = s->TP.P;
         void* sargs[] = {&F, &D};
         const int per = s->run_kernel.threads / F.T;
-        CK(cudaLaunchCooperativeKernel(s->run_kernel.fn, dim3((unsigned)((s->n_tiles + per - 1) / per)),
-                                       dim3((unsigned)s->run_kernel.threads), sargs,
-                                       (size_t)per * F.max_slots * s->ssz, s->stream));
-        return FV_OK;
+        return cudaLaunchCooperativeKernel(s->run_kernel.fn, dim3((unsigned)((s->n_tiles + per - 1) / per)),
+                                           dim3((unsigned)s->run_kernel.threads), sargs,
+                                           (size_t)per * F.max_slots * s->ssz, s->stream);
     }
     FusedParams F = s->FPm;
     F.P = s->TP.P;
     void* args[] = {&F, &D};
-    CK(cudaLaunchCooperativeKernel(s->run_kernel.fn, dim3((unsigned)s->n_tiles), dim3((unsigned)s->run_kernel.threads),
-                                   args, (size_t)std::max(F.L.total_run, F.L.total_grad), s->stream));
-    return FV_OK;
+    return cudaLaunchCooperativeKernel(s->run_kernel.fn, dim3((unsigned)s->n_tiles), dim3((unsigned)s->run_kernel.threads),
+                                       args, (size_t)std::max(F.L.total_run, F.L.total_grad), s->stream);
 }
 
 int fv_run(fv_solver* s, const fv_run_options* o, fv_run_info* info) {
@@ -1222,6 +1221,10 @@ int fv_run(fv_solver* s, const fv_run_options* o, fv_run_info* info) {
     double total_ms = 0.0;
     int64_t launches = 0;
     unsigned long long cur = start_step;
+    // The tiles fit the device as it was at creation; a stream set since may
+    // have fewer SMs (a partitioned context).  A refused launch leaves the run
+    // to the captured steps.
+    bool cooperative = s->run_kernel.fn != nullptr;
     for (;;) {
         // graph length: the largest power of two <= min(chunk, steps left), so
         // runs bounded by max_step launch no idle steps
@@ -1229,14 +1232,19 @@ int fv_run(fv_solver* s, const fv_run_options* o, fv_run_info* info) {
         int len = 1;
         while ((unsigned long long)(len * 2) <= left && len * 2 <= s->chunk) len *= 2;
         int rc;
-        if (s->run_kernel.fn) {
+        if (cooperative) {
             // a callback hears of its steps every `chunk` steps, as below
             const unsigned long long most = o->on_print ? std::min(s->chunk, s->hist_cap) : kRunSteps;
             CK(cudaEventRecord(e0, st));
-            if ((rc = launch_run(s, alpha, (int)std::min(left, most)))) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
-            CK(cudaEventRecord(e1, st));
-            launches += 2;
-        } else {
+            if (launch_run(s, alpha, (int)std::min(left, most)) != cudaSuccess) {
+                (void)cudaGetLastError();
+                cooperative = false;
+            } else {
+                CK(cudaEventRecord(e1, st));
+                launches += 2;
+            }
+        }
+        if (!cooperative) {
             GraphEntry* g = nullptr;
             rc = get_graph(s, alpha, len, &g);
             if (rc) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
@@ -1251,7 +1259,7 @@ int fv_run(fv_solver* s, const fv_run_options* o, fv_run_info* info) {
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, e0, e1));
         total_ms += ms;
-        if (s->run_kernel.fn && hc.failed) {
+        if (cooperative && hc.failed) {
             cudaEventDestroy(e0); cudaEventDestroy(e1);
             return fail(FV_ERR_CUDA, "fv_run: a grid barrier of the run kernel gave up");
         }

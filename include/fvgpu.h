@@ -362,7 +362,8 @@ int fv_get_state_device(fv_solver* s, double* q_device);
  * tiles fit the device at once (the Roe kinds but FP32 first order,
  * Navier-Stokes in FP64, the diffusion kind in FP64 and FP32; default layout
  * and schedule) up to 2,048 steps are one cooperative launch instead; with
- * on_print, `chunk` steps. */
+ * on_print, `chunk` steps.  Where that launch is refused (a stream of fewer SMs
+ * than the device has), the captured steps serve the run. */
 int fv_run(fv_solver* s, const fv_run_options* opt, fv_run_info* info);
 /* Continue a run in another solver of the same mesh, typically with another
  * precision (FP32-bulk for the transient, FP64 for the tail of a steady
