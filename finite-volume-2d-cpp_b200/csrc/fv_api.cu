@@ -816,6 +816,12 @@ int fv_solver_create_tuned(const fv_mesh* fm, const fv_physics* ph, int32_t prec
     return FV_OK;
 }
 
+int fv_solver_set_run_polls(fv_solver* s, int32_t polls) {
+    if (!s || polls < 0 || polls > 1 << 30) return fail(FV_ERR_ARG, "fv_solver_set_run_polls: need 0..2^30 polls");
+    s->run_polls = polls;
+    return FV_OK;
+}
+
 int fv_solver_set_stream(fv_solver* s, void* stream) {
     if (!s) return fail(FV_ERR_ARG, "null solver");
     CK(cudaSetDevice(s->device));
@@ -1170,6 +1176,7 @@ static cudaError_t launch_run(fv_solver* s, const std::vector<double>& alpha, in
     D.bar = s->run_bar;
     D.n_tiles = s->n_tiles; D.n_cases = s->n_cases; D.f32 = s->f32 ? 1 : 0;
     D.max_steps = steps;
+    D.polls = s->run_polls;
     D.ns = (int)alpha.size();
     for (int k = 0; k < D.ns; ++k) D.alpha[k] = alpha[(size_t)k];
     if (s->stencil) {

@@ -41,6 +41,7 @@ struct PersistIO {
     unsigned* bar;                 // arrivals at the grid barrier, zero at launch
     int n_tiles, n_cases, f32;
     int max_steps;                 // steps of this launch at most
+    int polls;                     // polls of a wait at most
     int ns;
     double alpha[kMaxStages];
 };
@@ -50,8 +51,8 @@ struct PersistIO {
 struct GridSync {
     unsigned* bar;
     int* err;
-    unsigned target;
-    static constexpr int kPolls = 1 << 23;  // some seconds
+    int most;  // polls of a wait
+    unsigned target = 0;
     __device__ __forceinline__ void arrive() {
         __syncthreads();
         target += gridDim.x;
@@ -65,7 +66,7 @@ struct GridSync {
                 unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
                 if ((int)(v - target) >= 0) break;
-                if ((++polls & 1023) == 0 && (polls > kPolls || *(volatile int*)err)) {
+                if (++polls > most || ((polls & 1023) == 0 && *(volatile int*)err)) {
                     atomicExch(err, 1);
                     ok = 0;
                     break;
@@ -274,7 +275,7 @@ __device__ __forceinline__ void run_tile(const FusedParams& FP, const PersistIO&
         c.n_hist = 0;
         run_step_start(c, lim);
     }
-    GridSync sync{D.bar, &D.ctrl->failed, 0u};
+    GridSync sync{D.bar, &D.ctrl->failed, D.polls};
     sync.arrive();
     TileIO io{};
     io.dt = D.dt;

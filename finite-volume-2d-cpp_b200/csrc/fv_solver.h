@@ -55,6 +55,7 @@ struct fv_solver {
     double* run_part = nullptr;     // the run kernel's partial sums: [2][n_tiles][4], stencils [2][CTAs]
     unsigned long long* run_keys = nullptr;
     unsigned* run_bar = nullptr;
+    int run_polls = 1 << 23;        // of a wait at most: some seconds
     // its schedule (FV_SCHED_*); the work list's per-stage tile counters and
     // CTAs per launch
     int sched = 0;

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(THREADS)
         c.n_hist = 0;
         run_step_start<1>(c, lim);
     }
-    GridSync sync{D.bar, &D.ctrl->failed, 0u};
+    GridSync sync{D.bar, &D.ctrl->failed, D.polls};
     sync.arrive();
     bool pending = false;
     int n = 0;

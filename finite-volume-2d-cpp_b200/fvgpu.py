@@ -354,6 +354,10 @@ class Solver:
     def sync(self):
         _check(lib().fv_solver_sync(self._h))
 
+    def set_run_polls(self, n):
+        """Polls after which a grid barrier of the run kernel gives up (run raises)."""
+        _check(lib().fv_solver_set_run_polls(self._h, C.c_int32(n)))
+
     def set_chunk(self, n):
         _check(lib().fv_solver_set_chunk(self._h, C.c_int32(n)))
 

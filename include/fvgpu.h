@@ -392,6 +392,11 @@ int fv_boundary_force(fv_solver* s, int32_t group, double* fx, double* fy);
 /* Chunk length of the captured step graphs, and of a cooperative launch with
  * on_print (default 16). */
 int fv_solver_set_chunk(fv_solver* s, int32_t steps);
+/* Polls after which a grid barrier of the cooperative launch gives up (default
+ * 2^23: some seconds).  fv_run then returns FV_ERR_CUDA, with the context as
+ * usable as before; the solver's state and run control are undefined until a
+ * state is set and a run restarted. */
+int fv_solver_set_run_polls(fv_solver* s, int32_t polls);
 /* out[6] = {tiles, cells per tile, max halo cells per tile, max edges per
  * tile, precision, bytes per stored stage value}. */
 int fv_solver_info(fv_solver* s, int64_t* out);

@@ -110,3 +110,31 @@ def test_several_launches_of_many_tiles():
     assert out[0][0]["step"] == out[1][0]["step"] == 2100 and out[0][0]["time"] == out[1][0]["time"]
     assert bits_equal(out[0][1], out[1][1])
     np.testing.assert_allclose(out[0][0]["R"], out[1][0]["R"], rtol=R_RTOL, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ("roe", "stencil"))
+def test_a_barrier_that_gives_up_is_an_error(kind):
+    """No poll allowed beyond the first: the earliest CTA gives up, the others
+    follow at their waits, the kernel ends and the solver serves the next run."""
+    mesh = fvgpu.Mesh.from_elements(meshgen.rect_tri(130, 130, 1.0, 0.8))
+    if kind == "roe":
+        ph, q0 = euler(True), smooth_state(mesh.geometry())
+    else:
+        ph = P.heat(dt=1e-6)
+        ph.bcs = {"wall": ("copy", None), "ends": ("copy", None)}
+        q0 = 1 + np.sin(9 * np.asarray(mesh.geometry()["ccx"]))
+    a, b = (fvgpu.Solver(mesh, ph, "fp64") for _ in range(2))
+    for s in (a, b):
+        s.set_state(q0)
+    a.set_run_polls(0)
+    with pytest.raises(fvgpu.FvError, match="gave up") as e:
+        a.run(200, alpha=P.RK5_ALPHA)
+    assert e.value.code == -2
+    a.set_run_polls(1 << 23)
+    a.set_state(q0)
+    ra, rb = (s.run(20, alpha=P.RK5_ALPHA) for s in (a, b))
+    assert ra["step"] == rb["step"] == 20 and ra["time"] == rb["time"]
+    assert bits_equal(a.get_state(), b.get_state()) and bits_equal(ra["R"], rb["R"])
+    with pytest.raises(fvgpu.FvError):
+        a.set_run_polls(-1)
