@@ -545,6 +545,11 @@ __global__ void k_adj_dt(Params P, AdjFaces F, const double* q, const double* la
     } else if (l <= kFaces) {
         const uint32_t w = F.nbr[(size_t)(l - 1) * N + a];
         if (w != kNone) c = (int)(w & 0x7FFFFFFFu);
+        // a neighbour across several faces is its first one's: its derivative holds all of them
+        for (int f = 0; f < l - 1; ++f) {
+            const uint32_t v = F.nbr[(size_t)f * N + a];
+            if (v != kNone && (int)(v & 0x7FFFFFFFu) == c) c = -1;
+        }
     }
     if (c < 0) return;
     const D4 d = dt_cell_d(P, F, q, a, c);
