@@ -138,3 +138,45 @@ def test_a_barrier_that_gives_up_is_an_error(kind):
     assert bits_equal(a.get_state(), b.get_state()) and bits_equal(ra["R"], rb["R"])
     with pytest.raises(fvgpu.FvError):
         a.set_run_polls(-1)
+
+
+@pytest.mark.gpu
+def test_runs_of_several_solvers_at_once():
+    """Run kernels of several solvers, each on its own stream and host thread:
+    a launch starts where its CTAs have room, so the runs take turns or share the
+    device, with the results that each has alone."""
+    import threading
+
+    heat = P.heat(dt=1e-6)
+    heat.bcs = {"wall": ("copy", None), "ends": ("copy", None)}
+    jobs = []
+    for nx, ny, ph, precision, alpha in ((130, 130, euler(True), "fp64", P.RK5_ALPHA), (180, 180, euler(False), "fp64", P.RK1_ALPHA),
+                                         (31, 23, euler(True, global_dt=False), "fp64_exact", P.RK5_ALPHA),
+                                         (130, 90, heat, "fp64", P.RK5_ALPHA)):
+        mesh = fvgpu.Mesh.from_elements(meshgen.rect_tri(nx, ny, 1.0, 0.8))
+        g = mesh.geometry()
+        q0 = smooth_state(g) if ph is not heat else 1 + np.sin(9 * np.asarray(g["ccx"]))
+        jobs.append((fvgpu.Solver(mesh, ph, precision), q0, alpha))
+
+    def once(job):
+        s, q0, alpha = job
+        s.set_state(q0)
+        r = s.run(40, alpha=alpha)
+        return s.get_state().tobytes(), r["time"], r["R"].tobytes()
+
+    alone = [once(j) for j in jobs]
+    for s, _, _ in jobs:
+        assert s.last_run_stats()[1] <= 2
+    got = [[] for _ in jobs]
+
+    def repeat(k):
+        for _ in range(8):
+            got[k].append(once(jobs[k]))
+
+    threads = [threading.Thread(target=repeat, args=(k,)) for k in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k, want in enumerate(alone):
+        assert len(got[k]) == 8 and all(x == want for x in got[k])
