@@ -96,10 +96,12 @@ def algo_bytes(ph, precision, kernel):
 TRAFFIC_B_PER_CELL = {
     ("step", "fp32", "split"): (153.2, "ncu --set full -k regex:k_tile_stage -s 30 -c 2, "
                                        "bench.py --precision fp32 --steps 20 --warmup 3 --no-cpu-baseline"),
-    ("step", "fp32", "fused"): (181.5, "ncu -k regex:k_tile_fused, mean of the 5 launches of one RK5 step, "
-                                       "perf/cases.py step_1m_fp32"),
-    ("step", "fp64", "fused"): (304.8, "ncu -k regex:k_tile_fused, mean of the 5 launches of one RK5 step, "
-                                       "perf/cases.py step_1m_fp64"),
+    ("step", "fp32", "fused"): (218.1, "mean of the 5 k_tile_fused launches of one RK5 step, ncu --metrics "
+                                       "dram__bytes_read.sum,dram__bytes_write.sum,... --clock-control none "
+                                       "-k regex:k_tile_fused -c 6, profiles/k_tile_fused_forward_step.md"),
+    ("step", "fp64", "fused"): (308.1, "mean of the 5 k_tile_fused launches of one RK5 step, ncu --metrics "
+                                       "dram__bytes_read.sum,dram__bytes_write.sum,... --clock-control none "
+                                       "-k regex:k_tile_fused -c 6, profiles/k_tile_fused_forward_step.md"),
 }
 
 

@@ -37,8 +37,9 @@
 // stage by themselves.  The flux edges' geometry and the cells' 1 / area come
 // through shared memory too, copied before the dependency wait: loaded where
 // they are used, each of the two flux passes and the update waited an L2
-// latency for them (us per RK5 step, before | after: forward step 998k cells
-// FP32 328 | 304, FP64 723 | 676, NACA 1M FP32 307 | 282).
+// latency for them (998k cells FP64: 723 us per RK5 step, 676 with the copies).
+// Now, of a 998k-cell stage: FP32 45 warp instructions per cell at 66 % of the
+// issue rate, 63 us; FP64 58, latency-bound at 16 warps per SM, 125 us.
 #pragma once
 #include "fv_tile.cuh"
 
@@ -1114,10 +1115,12 @@ __device__ __forceinline__ bool fused_tile(const FusedParams& FP, const TileIO& 
 }
 
 // Register budget of the one-lane kernel, as CTAs of 256 threads per SM: FP32
-// 64 registers (32 warps per SM), FP64 128 (16 warps).  Measured in us per
-// RK5 step (64 | 48 | 80 registers): forward step 998k cells 328 | 322 | 358,
-// 99k cells (one wave) 57 | 66 | 54; FP64 with 80 registers spills (998k cells
-// 7 % faster, 65k cells 28 % slower).
+// 64 registers (32 warps per SM), FP64 128 (16 warps).  Measured at sizes beyond
+// the run kernel, us per RK5 step: FP32 with 64 | 48 | 80 registers, forward step
+// 163k cells 79 | 79 | 78, 315k 123 | 133 | 126, 998k 346 | 384 | 389, NACA 1M
+// 316 | 376 | 351, strips of 422k cells 176 | 202 | 191 (48 registers spill);
+// FP64 with 128 | 80 registers (which spill), 163k 133 | 128, 315k 241 | 254,
+// 998k 679 | 693.
 template <class M>
 struct FusedBlocks { static constexpr int v = sizeof(typename M::S) == 4 ? 4 : 2; };
 

@@ -78,7 +78,9 @@ __global__ void k_step_begin(Ctrl* c, const RunLimits* L, int V, unsigned long l
     }
 }
 
-// Before a persistent run kernel, whose phases run while ctrl->active is set.
+// Before a persistent run kernel: key sets, barrier counter, failure flag and
+// print records.  (Its CTAs decide from their own copies of step, time and norms;
+// they set ctrl->active at the end.)
 __global__ void k_run_begin(Ctrl* c, unsigned long long* keys, int nkeys, unsigned* bar) {
     for (int i = threadIdx.x; i < nkeys; i += blockDim.x) keys[i] = ~0ull;
     if (threadIdx.x == 0) {

@@ -474,12 +474,13 @@ struct RunLaunch {
     // The candidates from the most threads and registers per tile down: while
     // the device has room, more threads shorten a tile's chain (one pass over
     // the gradient slots and the flux edges instead of two).  Measured, us per
-    // step of the forward step: 10,206 cells FP64_EXACT 4T threads (two lanes
-    // per cell) 71, 2T 89, T 146, separate kernels 150; FP64 2T 31, T 41,
-    // separate 48; FP32 26, 33, 36; 98,784 cells FP32 T 53, separate 55; NACA
-    // 65,536 cells FP64 T 53, separate 59; Sod tube (first order) 32,000 cells
-    // FP64 T 9.4, separate 15.8; flat plate (Navier-Stokes) 13,200 cells FP64
-    // 2T 41, separate 104 (two kernels a stage, whose limiter, Green-Gauss and
+    // step (k[0] | k[1] | k[2] | k[3] | separate kernels; -: no candidate or no
+    // room): forward step 10,206 cells FP64_EXACT 46.5 | 47.2 | 54.9 | 85.7 |
+    // 57.9, FP64 - | 26.8 | 27.4 | 36.3 | 43.7, FP32 - | 21.5 | 26.4 | 32.9 |
+    // 35.9; 98,784 cells FP32 - | - | - | 54.3 | 61.7; NACA 65,536 cells FP64
+    // - | - | - | 49.7 | 57.9; Sod tube (first order) 32,000 cells FP64 - | 8.8 |
+    // 8.9 | 9.1 | 16.2; flat plate (Navier-Stokes) 13,200 cells FP64 - | 40.0 |
+    // 43.1 | 55.5 | 99.6 (two kernels a stage, whose limiter, Green-Gauss and
     // viscous time-step divisions the run kernel's form does not have).
     template <int F, int NF, bool O2>
     static void list(const FusedParams& FP, RunKernel* k) {
