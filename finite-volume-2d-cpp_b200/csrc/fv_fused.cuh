@@ -911,7 +911,7 @@ __device__ __forceinline__ void fused_partials(const TileIO& io, unsigned char* 
 // NV: variables per lane of the gradient and update phases (4 / NV lanes per cell).
 // PH 0: the whole stage.  PH 1: the limited gradients of the owned cells only,
 // written to io.gx, io.gy; PH 2: the stage with the gradients read from there
-// (the split layout; fast policies).  PH 3: the step's time step only.
+// (FP64's split layout).  PH 3: the step's time step only.
 // PART: a decomposition part's tile, whose owned cells come from the tile
 // info (a part owns fewer real cells than its local mesh holds).
 template <class M, int FLUX, int NV, int NF, int PH, bool REMOTE, bool PART>
@@ -1132,7 +1132,7 @@ __global__ void __launch_bounds__(NV == 4 ? kTileMax : kFusedThreads, NV == 4 ? 
     fused_tile<M, FLUX, NV, NF, 0, false, false>(FP, io, (int)blockIdx.x, PartIO{});
 }
 
-// The split layout of the fast policies, over the same tiles with the same
+// FP64's split layout, over the same tiles with the same
 // arithmetic: gradients, then the rest of the stage; and the time step (the
 // first kernel of a step).
 template <class M, int NF>
@@ -1278,7 +1278,7 @@ struct FusedLaunch {
         if (FP.nf == 3) stage_f<1, 3>(FP, io, st, pdl, n_tiles, grid, part);
         else stage_f<1, 4>(FP, io, st, pdl, n_tiles, grid, part);
     }
-    // the time step (phase 3); fast policies: the split layout's two kernels
+    // the time step (phase 3); FP64: the split layout's two kernels
     // (phase 1: gradients; phase 2: the rest)
     template <int NF>
     static void split_f(const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles, int phase) {
@@ -1300,7 +1300,7 @@ size_t smem_fused(int precision, FusedParams& FP);
 int work_grid_fused(int precision, FusedParams& FP, int n_tiles);
 void launch_fused(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
                   int grid, const PartIO* part = nullptr);
-// the time step and the fast policies' split kernels over the fused kernel's tiles (FusedLaunch::split)
+// the time step and FP64's split kernels over the fused kernel's tiles (FusedLaunch::split)
 void launch_fused_split(int precision, const FusedParams& FP, const TileIO& io, cudaStream_t st, bool pdl, int n_tiles,
                         int phase);
 }  // namespace tile

@@ -46,10 +46,6 @@ __device__ __forceinline__ double vmax(double a, double b) { return (a < b) ? b 
 
 // Smooth switch of the limiter (explicit.cpp:220-233): 1 up to d^2 = (K h)^3,
 // 0 from twice that on; d = max - min over the stencil, rk3 = 1 / (K h)^3.
-__device__ __forceinline__ float smooth_switch(float d, float rk3) {
-    const float y = __saturatef(__fmaf_rn(d * d, rk3, -1.f));
-    return __fmaf_rn(__fmaf_rn(2.f, y, -3.f), y * y, 1.f);
-}
 __device__ __forceinline__ double smooth_switch(double d, double rk3) {
     double y = __fma_rn(d * d, rk3, -1.0);
     y = y > 0.0 ? (y < 1.0 ? y : 1.0) : 0.0;
